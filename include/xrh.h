@@ -283,6 +283,54 @@ int xrh_gemm_fp64_grouped(const xrh_gemm_task* tasks_dev, int n_tasks, int64_t t
 int xrh_gemm_simt_grouped(int precision, const xrh_gemm_task* tasks_dev, int n_tasks, int64_t total_tiles,
                           const xrh_gemm_segment* segs_dev, void* stream);
 
+/* The same contractions with exact products on the tensor cores (no reference counterpart).  Every
+ * row r of an operand is scaled by the power of two above its largest element and written as
+ * XRH_SLICES balanced base-256 digits (integers in [-128, 128], held in BF16): the row in
+ * 62-bit fixed point.  Products of digits are summed in FP32 accumulators that stay below 2^24,
+ * so exactly, for every digit pair (i, j) with i + j < XRH_SLICES; the sums are collected in 64-bit
+ * integers and rounded once per segment to FP64.  Rows with infinities or NaN are recognised and
+ * their results formed by FP64 arithmetic from the operands themselves.
+ *   xrh_slice_grouped: digits of many operands.  The rows of each batch step are padded to blocks of
+ *       `block` rows (128 for an A operand, 64 or 32 for a B operand); digits_dev holds, for every
+ *       block and every 32 K, the shared-memory image of one pipeline stage: [XRH_SLICES][block][32]
+ *       BF16 in 64-byte swizzle (16-byte aligned); Kp is K rounded up to 32.  exps_dev[batch * rows]
+ *       receives the high word of the largest |element| of each row.  Element (b, r, k) of the source
+ *       is src[b * sbatch + r * ld + k], or src[b * sbatch + k * ld + r] with trans = 1 (then exps_dev
+ *       must be zero on entry).  A task owns xrh_slice_ctas(.., 0) CTAs of the launch from cta_begin
+ *       on and, with trans = 1, xrh_slice_ctas(.., 1) CTAs of the row-maximum launch that precedes
+ *       it from max_begin on (tasks without transposed source first).
+ *   xrh_gemm_sliced_grouped: the tasks of xrh_gemm_fp64_grouped (128 x bn output tiles, bn = 32 for
+ *       N <= 32 else 64, times splitk, times batch) over such digits; splitk divides the
+ *       concatenated 32-element K stages.  A device wait that runs out sets *status_dev =
+ *       XRH_ERR_TIMEOUT (XRH_OK on entry). */
+#define XRH_SLICES 8
+typedef struct {
+    const double* src;
+    void* digits;
+    uint32_t* exps;
+    int64_t rows, K, ld, Kp;
+    int64_t batch, sbatch;
+    int64_t trans, block;
+    int64_t cta_begin, max_begin;
+} xrh_slice_task;   /* 104 bytes */
+typedef struct {
+    const void* digA;
+    const void* digB;
+    int64_t stages;            /* Kp / 32 */
+    int64_t rA, rB;            /* rows of the operand per batch step (0: shared by every batch step) */
+    const uint32_t* eA;
+    const uint32_t* eB;
+    const double* A;
+    const double* B;
+    int64_t lda, ldb, K, flags, sA, sB;
+    double alpha;
+} xrh_sliced_segment;   /* 128 bytes */
+int64_t xrh_slice_ctas(int64_t rows, int64_t K, int64_t batch, int trans, int block, int max_pass);
+int xrh_slice_grouped(const xrh_slice_task* tasks_dev, int n_tasks, int64_t total_ctas, int64_t max_ctas,
+                      void* stream);
+int xrh_gemm_sliced_grouped(const xrh_gemm_task* tasks_dev, int n_tasks, int64_t total_tiles,
+                            const xrh_sliced_segment* segs_dev, int32_t* status_dev, void* stream);
+
 /* FP64 Lanczos building blocks for the lowest eigenpairs of H (replaces the dense
  * scipy.linalg.eig of hermitian-XRCC/mains/workflow.py:229 and
  * StateSpaceOptimizer/state_gradients.py:107 for the eigenpairs the optimizer uses):

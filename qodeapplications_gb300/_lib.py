@@ -68,6 +68,9 @@ _SIGS = {
     "xrh_sigma2e": (_i32, [_i32, _i32, _vp, _vp, _i32, _vp, _vp, _i32, _vp, _i64, _vp, _vp, _i32, _vp, _vp]),
     "xrh_gemm_fp64_grouped": (_i32, [_vp, _i32, _i64, _vp, _vp]),
     "xrh_gemm_simt_grouped": (_i32, [_i32, _vp, _i32, _i64, _vp, _vp]),
+    "xrh_slice_ctas": (_i64, [_i64, _i64, _i64, _i32, _i32, _i32]),
+    "xrh_slice_grouped": (_i32, [_vp, _i32, _i64, _i64, _vp]),
+    "xrh_gemm_sliced_grouped": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp]),
     "xrh_gemv_rows": (_i32, [_i64, _i64, _vp, _i64, _vp, _dbl, _dbl, _vp, _vp]),
     "xrh_gemv_cols": (_i32, [_i64, _i64, _vp, _i64, _vp, _dbl, _vp, _vp]),
     "xrh_gemv_split_work": (_i64, [_i64, _i64]),
@@ -135,7 +138,7 @@ class LaunchCounter:
     multi = {"xrh_orbital_terms": 2, "xrh_gemv_rows_split": 2, "xrh_lanczos_normalize_split": 2}
     host_only = {"xrh_abi_version", "xrh_status_string", "xrh_last_cuda_error", "xrh_tc_chunk_elems", "xrh_zero",
                  "xrh_tc_encode_map", "xrh_state_ctas", "xrh_abt_ctas", "xrh_lanczos_coop_work",
-                 "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas"}
+                 "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_slice_ctas"}
     count = 0
 
 
@@ -244,6 +247,16 @@ TASK_DTYPE = np.dtype([("M", np.int64), ("N", np.int64), ("seg_begin", np.int64)
                        ("colB", np.uint64), ("DA", np.uint64), ("DB", np.uint64), ("diagA", np.uint64),
                        ("diagB", np.uint64), ("batch", np.int64), ("sC", np.int64)])
 assert SEGMENT_DTYPE.itemsize == 72 and TASK_DTYPE.itemsize == 152
+SLICES = 8                # XRH_SLICES
+SLICE_TASK_DTYPE = np.dtype([("src", np.uint64), ("digits", np.uint64), ("exps", np.uint64), ("rows", np.int64),
+                             ("K", np.int64), ("ld", np.int64), ("Kp", np.int64), ("batch", np.int64),
+                             ("sbatch", np.int64), ("trans", np.int64), ("block", np.int64),
+                             ("cta_begin", np.int64), ("max_begin", np.int64)])
+SLICED_SEG_DTYPE = np.dtype([("digA", np.uint64), ("digB", np.uint64), ("stages", np.int64), ("rA", np.int64),
+                             ("rB", np.int64), ("eA", np.uint64), ("eB", np.uint64), ("A", np.uint64), ("B", np.uint64),
+                             ("lda", np.int64), ("ldb", np.int64), ("K", np.int64), ("flags", np.int64),
+                             ("sA", np.int64), ("sB", np.int64), ("alpha", np.float64)])
+assert SLICE_TASK_DTYPE.itemsize == 104 and SLICED_SEG_DTYPE.itemsize == 128
 
 
 class Transposes:

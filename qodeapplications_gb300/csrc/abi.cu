@@ -46,3 +46,5 @@ static_assert(sizeof(xrh_tc_task) == 144, "xrh_tc_task layout is part of the ABI
 static_assert(sizeof(xrh_small_mm_task) == 56, "xrh_small_mm_task layout is part of the ABI");
 static_assert(sizeof(xrh_permute_task) == 144, "xrh_permute_task layout is part of the ABI");
 static_assert(sizeof(xrh_gather_terms) == 136, "xrh_gather_terms layout is part of the ABI");
+static_assert(sizeof(xrh_slice_task) == 104, "xrh_slice_task layout is part of the ABI");
+static_assert(sizeof(xrh_sliced_segment) == 128, "xrh_sliced_segment layout is part of the ABI");

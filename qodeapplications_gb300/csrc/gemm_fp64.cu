@@ -9,7 +9,9 @@
 // flat tile index is mapped to (task, tile) by binary search over the tasks' tile_begin.
 //
 // GB300 FP64 throughput is low (about 2 DFMA/clk/SM), so this kernel is DFMA-bound at any
-// reasonable tiling: 64x64 tiles, 256 threads, 4x4 outputs per thread, K staged in 16s.
+// reasonable tiling: 64x64 tiles, 256 threads, 4x4 outputs per thread, K staged in 16s.  FP64
+// launches of any length go to gemm_sliced.cu (the tensor cores); what is left here are short chains
+// (a few K elements) and the FP32 variant.
 #include "xrh_common.cuh"
 
 namespace {

@@ -1,0 +1,780 @@
+// FP64 grouped GEMM with exact digit products on the 5th-generation tensor cores (sm_103a).
+//
+// GB300 runs FP64 at about 2 DFMA/clk/SM (1.1 TFLOP/s), a two-thousandth of its BF16 tensor rate, so
+// the FP64 contractions are rebuilt from integer products (the error-free slicing of Ozaki, Ogita,
+// Oishi and Rump, Numer. Algorithms 59, 95 (2012)): a row x of an operand with |x| < 2^e is the
+// integer V = round(x 2^(62 - e)), written in balanced base-256 digits V = sum_t d_t 256^(7 - t),
+// |d_t| <= 128, |d_0| <= 65, each digit exact in BF16.  With S_w = sum_(i+j=w) sum_k d_i(a_k) d_j(b_k),
+//     sum_k a_k b_k = 2^(ea + eb - 68) sum_(w<8) S_w 256^(7 - w)   (+ terms below 2^-63 of the
+//     largest product),
+// 36 digit pairs.  |d_i d_j| <= 2^14 and a weight has at most 8 pairs, so 128 K elements keep every
+// FP32 accumulator at or below 2^24, where integers are exact: the order and the rounding of the
+// tensor core's additions do not matter.  The eight sums of such a group go into two 64-bit integers
+// per output element and are rounded to FP64 once per segment.
+//
+// What bounds it: 36 pairs of BF16 MMAs are 2 304 cycles of the tensor pipe per 128 x 64 x 32 stage; the
+// integer collection of a group (8 x 8 192 conversions) and the flush of a tile (about 25 000 cycles)
+// overlap with it in part.  Measured at M = N = 3 600, K = 784: 0.77 ms, 26 TFLOP/s of FP64 products
+// (CUDA cores: 1.0); 3 600 x 784 x 784 0.22 + 0.03 ms digits against 4.65 ms; one tile of 128 K 27 us
+// against 160 us.
+//
+// Error: an element within 2^-9 of its row's largest is represented exactly, smaller ones to 2^-63
+// of the largest; there is no rounding per product or per addition, so a result is closer to the
+// exact sum than an FP64 FMA chain of more than a few terms.
+//
+// Per CTA (persistent over 128 x BN tiles, BN = 64, or 32 for N <= 32), 12 warps:
+//   * warp 8: bulk copies of all eight slices of A and B for 32 K (96 KB: two stages); the digits lie
+//     in global memory as the swizzled shared-memory image of a stage, so a stage is two contiguous
+//     copies;
+//   * warp 9: the tcgen05.mma of a stage into eight TMEM accumulators (weight w at column BN w; see
+//     stage_mmas), handed to the epilogue in pairs of weights, the next group starting behind it;
+//   * warps 0-7: tcgen05.ld of two weights (32 columns a warp), integer accumulation, release; at the
+//     end of a segment conversion by integer operations (the FP64 pipe is needed only for alpha
+//     and for additions) and the store, scatter or atomic epilogue through shared memory.
+// Every mbarrier wait is bounded; on timeout *status is set, all roles leave, copies and MMAs in
+// flight are waited for (bounded), TMEM is freed.
+#include "tc_common.cuh"
+#include "xrh_common.cuh"
+
+namespace {
+using namespace xrh_tc;
+
+constexpr int NS = XRH_SLICES;
+constexpr int SL_BM = 128;
+constexpr int SL_KS = 32;                              // K elements per stage (64-byte rows)
+constexpr int SL_GROUP = 4;                            // stages per exact accumulation group
+constexpr int SL_STAGES = 2;
+constexpr int SL_EPI_WARPS = 8;
+constexpr int SL_EPI_THREADS = SL_EPI_WARPS * 32;
+constexpr int SL_THREADS = SL_EPI_THREADS + 128;       // + a warpgroup: loads, MMA, two idle warps
+// registers: 384 threads x 168 at launch = 64512 = 256 x 208 (epilogue) + 128 x 88
+constexpr int SL_EPI_REGS = 208, SL_IO_REGS = 88;
+static_assert(SL_EPI_THREADS * SL_EPI_REGS + 128 * SL_IO_REGS <= SL_THREADS * 168, "register split exceeds the launch");
+constexpr int SL_CW = 32;                              // columns per epilogue warp
+constexpr int NP = NS / 2;                             // weight pairs: the unit handed to the epilogue
+constexpr uint32_t SL_A_SLICE = SL_BM * 64;            // bytes of one slice of a stage
+constexpr uint32_t SL_A_BYTES = NS * SL_A_SLICE;
+constexpr uint32_t SL_B_BYTES = NS * 64 * 64;
+constexpr uint32_t SL_STAGE_BYTES = SL_A_BYTES + SL_B_BYTES;
+constexpr int SL_RUN_GROUPS = 4096;                    // groups collected in 64 bits before a flush (< 2^93)
+static_assert(NS == 8, "digit weights and shifts below are written for eight slices");
+static_assert((long long)SL_GROUP * SL_KS * NS * (1 << 14) <= (1 << 24), "a group must stay exact in FP32");
+
+__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(SL_EPI_THREADS) : "memory"); }
+__device__ __forceinline__ int epi_bar_or(int pred) {
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(pred), "n"(SL_EPI_THREADS)
+        : "memory");
+    return r;
+}
+
+// A persistent CTA's tile: task, batch, output corner, N tile, range of K stages.
+struct Tile {
+    int task, m0, n0, BN;
+    int sb, left;                 // first stage (over the concatenated segments) and their number
+    int64_t batch;
+};
+
+__device__ __forceinline__ Tile tile_of(const xrh_gemm_task* __restrict__ tasks, int n_tasks,
+                                        const xrh_sliced_segment* __restrict__ segs, int64_t tile) {
+    int lo = 0, hi = n_tasks - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tasks[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
+    }
+    const xrh_gemm_task& T = tasks[lo];
+    Tile r;
+    r.task = lo;
+    r.BN = T.N <= 32 ? 32 : 64;
+    const int64_t tiles_m = (T.M + SL_BM - 1) / SL_BM, tiles_n = (T.N + r.BN - 1) / r.BN, mn = tiles_m * tiles_n;
+    int64_t local = tile - T.tile_begin;
+    r.batch = local / (mn * T.splitk);
+    local -= r.batch * mn * T.splitk;
+    const int64_t split = local / mn;
+    local -= split * mn;
+    // concurrent CTAs walk the N tiles of one M tile, or the M tiles of one N tile where those are
+    // the fewer, so that the smaller operand is the one re-read (from L2)
+    if (tiles_m < tiles_n) {
+        r.m0 = (int)((local % tiles_m) * SL_BM);
+        r.n0 = (int)((local / tiles_m) * r.BN);
+    } else {
+        r.m0 = (int)((local / tiles_n) * SL_BM);
+        r.n0 = (int)((local % tiles_n) * r.BN);
+    }
+    int64_t total = 0;
+    for (int64_t s = 0; s < T.seg_count; ++s) total += segs[T.seg_begin + s].stages;
+    const int64_t per = (total + T.splitk - 1) / T.splitk;
+    const int64_t sb = split * per, se = sb + per < total ? sb + per : total;
+    r.sb = (int)sb;
+    r.left = (int)(se > sb ? se - sb : 0);
+    return r;
+}
+
+// What the epilogue needs of its tile, in shared memory: its registers hold 32 x 2 64-bit sums.
+struct EpiTile {
+    double* C;
+    const xrh_sliced_segment* segs;
+    int64_t ldc, batch;
+    int M, N, m0, n0, mode, BN, sb, left, task;
+};
+
+// The stages of a tile as groups: at most SL_GROUP consecutive stages of one segment.  Every role
+// walks the same sequence.
+struct Groups {
+    const xrh_sliced_segment* segs;
+    int si, c, left;              // segment, next stage in it, stages left in the tile
+    int g0;                       // first stage of the current run (stages flushed together)
+    int run;                      // groups in the run so far
+    int take;                     // stages of the current group
+    bool flush;                   // the current group ends its run
+
+    __device__ __forceinline__ Groups(const xrh_sliced_segment* s, int first, int stages)
+        : segs(s), si(0), c(first), left(stages), g0(0), run(0), take(0), flush(true) {}
+    __device__ __forceinline__ bool next() {
+        c += take;
+        left -= take;
+        if (left <= 0) return false;
+        while (c >= segs[si].stages) {
+            c -= (int)segs[si].stages;
+            ++si;
+        }
+        if (flush) {
+            g0 = c;
+            run = 0;
+        }
+        const int in_seg = (int)segs[si].stages - c;
+        int n = in_seg < SL_GROUP ? in_seg : SL_GROUP;
+        if (n > left) n = left;
+        take = n;
+        flush = n == in_seg || n == left || ++run == SL_RUN_GROUPS;
+        return true;
+    }
+};
+
+// (hi 2^32 + lo) 2^(x - 68) rounded to FP64 (nearest, ties to even), |hi 2^32 + lo| < 2^94, by about
+// 45 integer operations without a branch (a branch per element serialises the 32 conversions of
+// a thread: 52 000 cycles a tile; the FP64 pipe would need 16 000).  Results outside the normal
+// range are formed by scalbn.
+__device__ __forceinline__ double sliced_to_double(int64_t hi, uint32_t lo, int x) {
+    const uint32_t sg = (uint32_t)(hi >> 63);           // all ones for a negative value
+    uint32_t w0 = lo ^ sg, w1 = (uint32_t)hi ^ sg, w2 = (uint32_t)(hi >> 32) ^ sg;
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, %2, 0;"
+        : "+r"(w0), "+r"(w1), "+r"(w2)
+        : "r"(sg & 1u));
+    // leading zeros of the 96 bits (w2 < 2^30); the leading one goes to bit 62 of (a : b), c behind
+    const bool z2 = w2 == 0u, z1 = z2 && w1 == 0u;
+    const uint32_t top = z1 ? w0 : (z2 ? w1 : w2);
+    const int z = __clz((int)top);
+    const int lz = z + (z1 ? 64 : (z2 ? 32 : 0));
+    uint32_t a = z1 ? w0 : (z2 ? w1 : w2), b = z1 ? 0u : (z2 ? w0 : w1), c = z2 ? 0u : w0;
+    a = __funnelshift_l(b, a, z);
+    b = __funnelshift_l(c, b, z);
+    c = c << (z & 31);
+    const uint32_t sticky = (c != 0u) | (b & 1u);
+    b = __funnelshift_r(b, a, 1) | sticky;
+    a >>= 1;
+    asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, 0;" : "+r"(b), "+r"(a) : "r"(0x1ffu + ((b >> 10) & 1u)));
+    // 53 bits above bit 10; e - 1 is added above the implicit one
+    const int e = 95 - lz + x - 68 + 1023;
+    const uint32_t mh = a >> 10, ml = __funnelshift_r(b, a, 10);
+    double v = __hiloint2double((int)((mh + ((uint32_t)(e - 1) << 20)) | (sg & 0x80000000u)), (int)ml);
+    if (top == 0u) v = 0.0;
+    else if ((unsigned)(e - 1) >= 2044u) {
+        v = scalbn((double)(((uint64_t)mh << 32) | ml), e - 1075);
+        if (sg) v = -v;
+    }
+    return v;
+}
+
+__device__ __forceinline__ int exp_of(uint32_t hi) {   // |x| < 2^exp_of for the row's largest high word
+    const int E = (int)(hi >> 20);
+    return (E < 1 ? 1 : E) - 1022;
+}
+
+// The MMAs of one stage (two K steps of 16).  The B slices of a stage are consecutive rows and the
+// accumulators consecutive columns (weight w at column BN w), so A_i x [B_j .. B_j+c] adds to the
+// weights i+j .. i+j+c in one MMA of N = BN (c + 1): 12 MMAs a K step for BN = 64 (8 for 32) instead
+// of 36 of N = 64, whose operand reads and dependent additions (about 110 cycles between two
+// MMAs on one accumulator) would bound them: 8 300 cycles a stage against 2 304 of the tensor pipe.
+// The first stage of a group goes weight pair by weight pair instead, each as soon as the epilogue
+// has drained it from the group before; at the last stage a pair is handed over after its own
+// last product.
+template <int BN>
+__device__ __forceinline__ bool stage_mmas(uint32_t tmem, uint64_t dA, uint64_t dB, bool first, bool last,
+                                           uint32_t drained, bool wait_drained, uint32_t drained_parity,
+                                           uint32_t ready, volatile int* abort_flag) {
+    constexpr uint32_t id0 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(SL_BM >> 4) << 24);
+    constexpr uint64_t a_step = SL_A_SLICE >> 4, b_step = (uint64_t)(BN * 64) >> 4;
+    auto mma = [&](int i, int j, int cnt, int ks, uint32_t acc) {       // A_i x [B_j .. B_j+cnt-1]
+        umma<0>(tmem + (uint32_t)(BN * (i + j)), dA + i * a_step + 2 * ks, dB + j * b_step + 2 * ks,
+                id0 | ((uint32_t)(BN * cnt / 8) << 17), acc);
+    };
+    if (first) {
+#pragma unroll
+        for (int p = 0; p < NS / 2; ++p) {
+            if (wait_drained) {
+                if (!mbar_wait(drained + 8u * p, drained_parity, abort_flag)) return false;
+                tc_fence_after();
+            }
+#pragma unroll
+            for (int ks = 0; ks < 2; ++ks) {
+#pragma unroll
+                for (int i = 0; i <= 2 * p; ++i) mma(i, 2 * p - i, 2, ks, (ks || i) ? 1u : 0u);
+                mma(2 * p + 1, 0, 1, ks, 1u);
+            }
+            if (last) umma_commit(ready + 8u * p);
+        }
+        return true;
+    }
+    constexpr int WIDE = 256 / BN;                 // slices of B in the widest MMA
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            mma(i, 0, NS - i < WIDE ? NS - i : WIDE, ks, 1u);
+            if (NS - i > WIDE) mma(i, WIDE, NS - i - WIDE, ks, 1u);
+            if (ks && last && (i & 1)) umma_commit(ready + 8u * (i >> 1));
+        }
+    }
+    return true;
+}
+
+__global__ void __launch_bounds__(SL_THREADS, 1)
+    gemm_sliced_kernel(const xrh_gemm_task* __restrict__ tasks, int n_tasks, int64_t total_tiles,
+                       const xrh_sliced_segment* __restrict__ segs, int32_t* status) {
+    extern __shared__ unsigned char smem_raw[];
+    uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ __align__(8) uint64_t full_bar[SL_STAGES], empty_bar[SL_STAGES];
+    __shared__ __align__(8) uint64_t ready_bar[NP], drained_bar[NP];
+    __shared__ __align__(8) uint64_t done_bar;
+    __shared__ uint32_t tmem_base_sh;
+    __shared__ volatile int abort_sh;
+    __shared__ longlong2 s_raw[SL_BM][9];
+    __shared__ int64_t s_rbase[SL_BM];
+    __shared__ int64_t s_cbase[SL_BM];
+    __shared__ double s_DA[SL_BM], s_DB[64];
+    __shared__ int s_rowB[64], s_colB[64];
+    __shared__ uint32_t s_eA[SL_BM], s_eB[64];
+    __shared__ unsigned char s_diagA[SL_BM], s_diagB[64];
+    __shared__ EpiTile s_t;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    if (tid == 0) {
+        for (int s = 0; s < SL_STAGES; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), 1);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        for (int w = 0; w < NP; ++w) {
+            mbar_init(smem_u32(&ready_bar[w]), 1);
+            mbar_init(smem_u32(&drained_bar[w]), SL_EPI_WARPS);
+        }
+        mbar_init(smem_u32(&done_bar), 1);
+        abort_sh = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_sh;
+
+    if (warp >= SL_EPI_WARPS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SL_IO_REGS));
+        if (warp == SL_EPI_WARPS && lane == 0) {
+            // -------------------------------------------------------------------- TMA loads --
+            uint64_t g = 0;
+            bool ok = true;
+            for (int64_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+                const Tile I = tile_of(tasks, n_tasks, segs, tile);
+                const uint32_t b_bytes = (uint32_t)NS * (uint32_t)I.BN * 64u;
+                Groups G(segs + tasks[I.task].seg_begin, I.sb, I.left);
+                while (ok && G.next()) {
+                    const xrh_sliced_segment& S = G.segs[G.si];
+                    const int64_t blk_a = I.batch * ((S.rA + SL_BM - 1) / SL_BM) + I.m0 / SL_BM;
+                    const int64_t blk_b = I.batch * ((S.rB + I.BN - 1) / I.BN) + I.n0 / I.BN;
+                    const uint8_t* pa = reinterpret_cast<const uint8_t*>(S.digA) + (blk_a * S.stages + G.c) * (int64_t)SL_A_BYTES;
+                    const uint8_t* pb = reinterpret_cast<const uint8_t*>(S.digB) + (blk_b * S.stages + G.c) * b_bytes;
+                    for (int q = 0; q < G.take; ++q, ++g) {
+                        const int s = (int)(g % SL_STAGES);
+                        if (g >= SL_STAGES &&
+                            !mbar_wait(smem_u32(&empty_bar[s]), (uint32_t)(g / SL_STAGES - 1) & 1u, &abort_sh)) {
+                            ok = false;
+                            break;
+                        }
+                        uint8_t* st = stages + (size_t)s * SL_STAGE_BYTES;
+                        const uint32_t bar = smem_u32(&full_bar[s]);
+                        mbar_expect_tx(bar, SL_A_BYTES + b_bytes);
+                        bulk_load(smem_u32(st), pa + (int64_t)q * SL_A_BYTES, SL_A_BYTES, bar);
+                        bulk_load(smem_u32(st + SL_A_BYTES), pb + (int64_t)q * b_bytes, b_bytes, bar);
+                    }
+                }
+            }
+            if (!ok) {
+                abort_sh = 1;
+                atomicExch(status, XRH_ERR_TIMEOUT);
+            }
+            // every copy issued has landed before shared memory goes away
+            for (uint64_t q = g > SL_STAGES ? g - SL_STAGES : 0; q < g; ++q)
+                mbar_wait(smem_u32(&full_bar[q % SL_STAGES]), (uint32_t)(q / SL_STAGES) & 1u, nullptr);
+        } else if (warp == SL_EPI_WARPS + 1 && lane == 0) {
+            // -------------------------------------------------------------------------- MMA --
+            uint64_t g = 0, grp = 0;
+            int bn = 0;                                          // N tile of the previous group
+            bool ok = true;
+            for (int64_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+                const Tile I = tile_of(tasks, n_tasks, segs, tile);
+                Groups G(segs + tasks[I.task].seg_begin, I.sb, I.left);
+                for (; ok && G.next(); ++grp) {
+                    for (int q = 0; q < G.take && ok; ++q, ++g) {
+                        const int s = (int)(g % SL_STAGES);
+                        if (!mbar_wait(smem_u32(&full_bar[s]), (uint32_t)(g / SL_STAGES) & 1u, &abort_sh)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t st = smem_u32(stages + (size_t)s * SL_STAGE_BYTES);
+                        const uint64_t dA = umma_desc_sw64(st), dB = umma_desc_sw64(st + SL_A_BYTES);
+                        const bool wait_d = q == 0 && grp > 0, last = q == G.take - 1;
+                        const uint32_t par = (uint32_t)(grp - 1) & 1u;
+                        if (wait_d && I.BN != bn) {
+                            // the accumulators of the two tile widths overlap: all must be drained
+                            for (int w = 0; w < NP && ok; ++w)
+                                ok = mbar_wait(smem_u32(&drained_bar[w]), par, &abort_sh);
+                            if (!ok) break;
+                        }
+                        bn = I.BN;
+                        ok = I.BN == 64
+                                 ? stage_mmas<64>(tmem, dA, dB, q == 0, last, smem_u32(drained_bar), wait_d, par,
+                                                  smem_u32(ready_bar), &abort_sh)
+                                 : stage_mmas<32>(tmem, dA, dB, q == 0, last, smem_u32(drained_bar), wait_d, par,
+                                                  smem_u32(ready_bar), &abort_sh);
+                        umma_commit(smem_u32(&empty_bar[s]));
+                    }
+                }
+            }
+            if (!ok) {
+                abort_sh = 1;
+                atomicExch(status, XRH_ERR_TIMEOUT);
+            }
+            umma_commit(smem_u32(&done_bar));          // every MMA issued has completed
+            mbar_wait(smem_u32(&done_bar), 0u, nullptr);
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(SL_EPI_REGS));
+        // --------------------------------------------------------------------- epilogue --
+        const int quarter = warp & 3, part = warp >> 2;          // TMEM lanes 32*quarter.., columns 16*part..
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        const int row = quarter * 32 + lane;
+        uint64_t grp = 0;
+        bool failed = false;
+        for (int64_t tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
+            if (tid == 0) {
+                const Tile I = tile_of(tasks, n_tasks, segs, tile);
+                const xrh_gemm_task& T = tasks[I.task];
+                s_t.C = T.C + I.batch * T.sC;
+                s_t.segs = segs + T.seg_begin;
+                s_t.ldc = T.ldc;
+                s_t.batch = I.batch;
+                s_t.M = (int)T.M;
+                s_t.N = (int)T.N;
+                s_t.m0 = I.m0;
+                s_t.n0 = I.n0;
+                s_t.mode = (int)T.mode;
+                s_t.BN = I.BN;
+                s_t.sb = I.sb;
+                s_t.left = I.left;
+                s_t.task = I.task;
+            }
+            epi_bar();
+            if (s_t.left == 0) {                                 // (uniform)
+                epi_bar();                                       // read before the next tile's is written
+                continue;
+            }
+            const int BN = s_t.BN;
+            const bool mine = part * SL_CW < BN;
+            if (s_t.mode == 2) {
+                const xrh_gemm_task& T = tasks[s_t.task];
+                for (int j = tid; j < BN; j += SL_EPI_THREADS) {
+                    const int64_t n = s_t.n0 + j;
+                    const bool ok = n < T.N;
+                    s_rowB[j] = ok ? T.rowB[n] : 0;
+                    s_colB[j] = ok ? T.colB[n] : 0;
+                    s_diagB[j] = ok ? T.diagB[n] : 0;
+                    s_DB[j] = (ok && T.DB) ? T.DB[n] : 0.0;
+                }
+                for (int r = tid; r < SL_BM; r += SL_EPI_THREADS) {
+                    const int64_t m = s_t.m0 + r;
+                    const bool ok = m < T.M;
+                    s_rbase[r] = ok ? T.rowA[m] : 0;
+                    s_cbase[r] = ok ? T.colA[m] : 0;
+                    s_diagA[r] = ok ? T.diagA[m] : 0;
+                    s_DA[r] = (ok && T.DA) ? T.DA[m] : 0.0;
+                }
+            }
+            bool first = true;                                   // first flush of the tile
+            int64_t hi[SL_CW];                                   // sum = hi 2^32 + lo
+            uint32_t lo[SL_CW];
+#pragma unroll
+            for (int j = 0; j < SL_CW; ++j) hi[j] = lo[j] = 0;
+            Groups G(s_t.segs, s_t.sb, s_t.left);
+            while (G.next()) {
+                const uint32_t ph = (uint32_t)grp & 1u;
+                ++grp;
+                // two rolled loops: the code of a group stays small (an unrolled one does not stay in
+                // the instruction cache beside the flush)
+                auto drain = [&](int p, bool low, int mul) {
+                    if (!failed && !mbar_wait(smem_u32(&ready_bar[p]), ph, &abort_sh)) {
+                        failed = true;
+                        abort_sh = 1;
+                    }
+                    if (failed) return;
+                    tc_fence_after();
+#pragma unroll
+                    for (int h = 0; h < SL_CW; h += 16) {
+                        float v[16], u[16];
+                        if (mine)
+                            tmem_ld16_pair(tmem + lane_base + (uint32_t)(2 * p * BN + part * SL_CW + h),
+                                           tmem + lane_base + (uint32_t)((2 * p + 1) * BN + part * SL_CW + h), v, u);
+                        if (h + 16 == SL_CW) {
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(smem_u32(&drained_bar[p]));
+                        }
+                        if (mine) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                // 32 x 32 + 64 bit multiply-adds
+                                const int64_t t = (int64_t)__float2int_rn(u[j]) * mul +
+                                                  ((int64_t)__float2int_rn(v[j]) * (mul * 256) + (low ? 0 : hi[h + j]));
+                                if (!low) {
+                                    hi[h + j] = t;
+                                } else {
+                                    const uint32_t l = lo[h + j] + (uint32_t)t;
+                                    hi[h + j] += (t >> 32) + (l < (uint32_t)t ? 1 : 0);
+                                    lo[h + j] = l;
+                                }
+                            }
+                        }
+                    }
+                };
+#pragma unroll 1
+                for (int p = 0; p < NP / 2; ++p) drain(p, false, p ? 1 : 65536);
+#pragma unroll 1
+                for (int p = NP / 2; p < NP; ++p) drain(p, true, p == 3 ? 1 : 65536);
+                if (!G.flush) continue;
+                // one decision of all epilogue warps per flush (also the barrier before s_eB is reused)
+                if (epi_bar_or(failed)) {
+                    failed = true;
+                    abort_sh = 1;
+                    if (tid == 0) atomicExch(status, XRH_ERR_TIMEOUT);
+                    break;
+                }
+                const xrh_sliced_segment& S = G.segs[G.si];
+                for (int j = tid; j < BN; j += SL_EPI_THREADS)
+                    s_eB[j] = s_t.n0 + j < s_t.N ? S.eB[s_t.batch * S.rB + s_t.n0 + j] : 0u;
+                const uint32_t wa = s_t.m0 + row < s_t.M ? S.eA[s_t.batch * S.rA + s_t.m0 + row] : 0u;
+                const int ea = exp_of(wa);
+                if (part == 0) s_eA[row] = wa;
+                epi_bar();
+                // the integer sums of 4 columns of each warp at a time through shared memory; a thread
+                // converts and writes four elements, lanes on consecutive columns.  The register
+                // arrays need constant indices, everything behind them is one rolled body.
+                const double alpha = S.alpha;
+                const bool scale = alpha != 1.0;
+                const bool any_bad = epi_bar_or((wa >> 20) >= 2047u || (tid < BN && (s_eB[tid] >> 20) >= 2047u)) != 0;
+                const int slot = lane & 7, rr = warp * 16 + (lane >> 3);         // rows rr, rr + 4, ..
+                #pragma unroll 1
+                for (int p = 0; p < SL_CW / 4; ++p) {
+#pragma unroll
+                    for (int u = 0; u < SL_CW / 4; ++u) {
+                        if (u != p) continue;
+#pragma unroll
+                        for (int j = 0; j < 4; ++j)
+                            s_raw[row][part * 4 + j] = make_longlong2(hi[4 * u + j], (long long)lo[4 * u + j]);
+                    }
+                    epi_bar();
+                    longlong2 raw[4];
+#pragma unroll
+                    for (int it = 0; it < 4; ++it) raw[it] = s_raw[rr + 4 * it][slot];
+                    epi_bar();                                   // buffer free
+                    const int jj = (slot >> 2) * SL_CW + 4 * p + (slot & 3);
+                    if (jj < BN && s_t.n0 + jj < s_t.N) {
+                        const uint32_t wb = s_eB[jj];
+                        const int eb = exp_of(wb);
+                        double x[4];
+#pragma unroll
+                        for (int it = 0; it < 4; ++it)
+                            x[it] = sliced_to_double(raw[it].x, (uint32_t)raw[it].y, exp_of(s_eA[rr + 4 * it]) + eb);
+                        if (any_bad) {
+                            // rows or columns with an infinity or a NaN: these K elements in FP64
+#pragma unroll
+                            for (int it = 0; it < 4; ++it) {
+                                const int m = s_t.m0 + rr + 4 * it;
+                                if (m >= s_t.M || !((s_eA[rr + 4 * it] >> 20) >= 2047u || (wb >> 20) >= 2047u)) continue;
+                                const double* a = S.A + s_t.batch * S.sA + (int64_t)m * ((S.flags & 1) ? 1 : S.lda);
+                                const double* b = S.B + s_t.batch * S.sB + (int64_t)(s_t.n0 + jj) * ((S.flags & 2) ? 1 : S.ldb);
+                                const int64_t ka = (S.flags & 1) ? S.lda : 1, kb = (S.flags & 2) ? S.ldb : 1;
+                                const int64_t kt = (int64_t)(G.c + G.take) * SL_KS, ke = kt < S.K ? kt : S.K;
+                                double v = 0.0;
+#pragma unroll 1
+                                for (int64_t k = (int64_t)G.g0 * SL_KS; k < ke; ++k) v = fma(a[k * ka], b[k * kb], v);
+                                x[it] = v;
+                            }
+                        }
+                        if (scale) {
+#pragma unroll
+                            for (int it = 0; it < 4; ++it) x[it] *= alpha;
+                        }
+                        double* d[4];
+#pragma unroll
+                        for (int it = 0; it < 4; ++it) d[it] = s_t.C + (int64_t)(s_t.m0 + rr + 4 * it) * s_t.ldc + s_t.n0 + jj;
+                        if (s_t.mode == 2) {
+#pragma unroll
+                            for (int it = 0; it < 4; ++it) {
+                                const int r = rr + 4 * it;
+                                d[it] = s_t.C + (s_rbase[r] + s_rowB[jj]) * s_t.ldc + s_cbase[r] + s_colB[jj];
+                                if (first) {
+                                    if (s_diagB[jj]) x[it] += s_DA[r];
+                                    if (s_diagA[r]) x[it] += s_DB[jj];
+                                }
+                            }
+                        }
+                        if (s_t.mode == 1) {
+#pragma unroll
+                            for (int it = 0; it < 4; ++it)
+                                if (s_t.m0 + rr + 4 * it < s_t.M) atomicAdd(d[it], x[it]);
+                        } else {
+                            // later segments add to what the same thread stored for the first one
+                            if (!first) {
+#pragma unroll
+                                for (int it = 0; it < 4; ++it)
+                                    if (s_t.m0 + rr + 4 * it < s_t.M) x[it] = *d[it] + x[it];
+                            }
+#pragma unroll
+                            for (int it = 0; it < 4; ++it)
+                                if (s_t.m0 + rr + 4 * it < s_t.M) *d[it] = x[it];
+                        }
+                    }
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int j = 0; j < SL_CW; ++j) hi[j] = lo[j] = 0;
+                first = false;
+            }
+            if (!failed) epi_bar();                              // metadata reads done before the next tile
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// ---- digits -------------------------------------------------------------------------------
+constexpr int DG_THREADS = 256;
+constexpr int DG_WARP_K = 1024;        // rows up to this K: a warp each; longer ones a CTA each
+constexpr int DG_TK = 64;              // transposed operands: 32 rows x 64 K per CTA
+constexpr int DG_MAX_K = 512;          // K per CTA of the row-maximum pass
+
+__device__ __forceinline__ uint32_t abs_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
+
+// V = round(x 2^(62 - e)) for |x| < 2^e, with 128 added to its low seven digits: byte t of the
+// result (t = 0 lowest) is digit 7 - t plus 128, the top byte (signed) is digit 0.
+__device__ __forceinline__ uint64_t fixed62(double x, int E) {
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+    const int ex = (int)(b >> 52) & 0x7ff;
+    uint64_t m = b & 0xfffffffffffffull;
+    if (ex) m |= 1ull << 52;
+    const int s = 9 - (E - (ex ? ex : 1));             // shift of the 53-bit mantissa
+    uint64_t v;
+    if (s >= 0) v = m << s;
+    else if (s > -54) v = ((m >> (-s - 1)) + 1ull) >> 1;   // nearest, ties away
+    else v = 0;
+    const int64_t sv = (b >> 63) ? -(int64_t)v : (int64_t)v;
+    return (uint64_t)sv + 0x0080808080808080ull;
+}
+
+// Digit slices of four consecutive K elements of a row: eight 8-byte stores into the stage image
+// (blocks of `block` rows; per block and 32 K: [slice][row][32 K], 64-byte rows, 64-byte swizzle:
+// 16-byte chunk index xor bits 1..2 of the row).
+__device__ __forceinline__ void put_digits(const uint64_t (&v)[4], const xrh_slice_task& T, int64_t blk, int r, int64_t k) {
+    const int64_t stages = T.Kp / SL_KS;
+    const int kk = (int)(k & (SL_KS - 1));
+    uint8_t* dst = reinterpret_cast<uint8_t*>(T.digits) + (blk * stages + k / SL_KS) * (T.block * 64 * NS) + r * 64 +
+                   (((kk >> 3) ^ ((r >> 1) & 3)) << 4) + (kk & 7) * 2;
+    const int64_t slice_stride = T.block * 64;
+#pragma unroll
+    for (int t = 0; t < NS; ++t) {
+        uint32_t f[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t word = t < 4 ? (uint32_t)(v[e] >> 32) : (uint32_t)v[e];
+            const uint32_t byte = (word >> (8 * (3 - (t & 3)))) & 0xffu;
+            // 2^23 + byte exactly, minus 2^23 and the digit's bias: the digit as a float
+            if (t == 0) f[e] = __float_as_uint((float)(int)(int8_t)byte);
+            else f[e] = __float_as_uint(__uint_as_float(0x4b000000u | byte) - 8388736.0f);
+        }
+        uint2 o;
+        o.x = __byte_perm(f[0], f[1], 0x7632);          // upper halves: BF16
+        o.y = __byte_perm(f[2], f[3], 0x7632);
+        *reinterpret_cast<uint2*>(dst + t * slice_stride) = o;
+    }
+}
+
+__device__ __forceinline__ int find_slice_task(const xrh_slice_task* __restrict__ tasks, int n_tasks, int64_t cta, bool max_pass) {
+    int lo = 0, hi = n_tasks - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if ((max_pass ? tasks[mid].max_begin : tasks[mid].cta_begin) <= cta) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+// Largest |element| of every row of the transposed operands: 32 rows x DG_MAX_K per CTA.
+__global__ void __launch_bounds__(DG_THREADS) slice_max_kernel(const xrh_slice_task* __restrict__ tasks, int n_tasks) {
+    __shared__ uint32_t part[8][32];
+    const xrh_slice_task& T = tasks[find_slice_task(tasks, n_tasks, blockIdx.x, true)];
+    int64_t local = (int64_t)blockIdx.x - T.max_begin;
+    const int64_t nr = (T.rows + 31) / 32, nk = (T.K + DG_MAX_K - 1) / DG_MAX_K;
+    const int64_t b = local / (nr * nk);
+    local -= b * nr * nk;
+    const int64_t r = (local % nr) * 32 + (threadIdx.x & 31), k0 = (local / nr) * DG_MAX_K;
+    const int64_t ke = k0 + DG_MAX_K < T.K ? k0 + DG_MAX_K : T.K;
+    uint32_t m = 0;
+    if (r < T.rows) {
+        const double* p = T.src + b * T.sbatch + r;
+#pragma unroll 4
+        for (int64_t k = k0 + (threadIdx.x >> 5); k < ke; k += 8) m = max(m, abs_hi(__ldg(p + k * T.ld)));
+    }
+    part[threadIdx.x >> 5][threadIdx.x & 31] = m;
+    __syncthreads();
+    if (threadIdx.x < 32 && r < T.rows) {
+        for (int w = 1; w < 8; ++w) m = max(m, part[w][threadIdx.x]);
+        atomicMax(T.exps + b * T.rows + r, m);
+    }
+}
+
+__global__ void __launch_bounds__(DG_THREADS) slice_digits_kernel(const xrh_slice_task* __restrict__ tasks, int n_tasks) {
+    __shared__ uint32_t part[8];
+    __shared__ double tile[DG_TK][33];
+    const xrh_slice_task& T = tasks[find_slice_task(tasks, n_tasks, blockIdx.x, false)];
+    int64_t local = (int64_t)blockIdx.x - T.cta_begin;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // rows are padded with zero digits to whole blocks (block: 32, 64 or 128)
+    const int64_t blocks = (T.rows + T.block - 1) / T.block, rows_p = blocks * T.block;
+    if (T.trans) {
+        const int64_t nr = rows_p / 32, nk = (T.Kp + DG_TK - 1) / DG_TK;
+        const int64_t b = local / (nr * nk);
+        local -= b * nr * nk;
+        const int64_t r0 = (local % nr) * 32, k0 = (local / nr) * DG_TK;
+        const double* p = T.src + b * T.sbatch;
+#pragma unroll
+        for (int i = 0; i < DG_TK / 8; ++i) {
+            const int64_t k = k0 + warp + 8 * i;
+            tile[warp + 8 * i][lane] = (k < T.K && r0 + lane < T.rows) ? __ldg(p + k * T.ld + r0 + lane) : 0.0;
+        }
+        __syncthreads();
+        // 16 threads take the 64 K of a row, four each; 16 rows at a time
+        for (int rr = threadIdx.x >> 4; rr < 32; rr += DG_THREADS / 16) {
+            const int64_t r = r0 + rr, k = k0 + 4 * (threadIdx.x & 15);
+            if (k >= T.Kp) continue;
+            const uint32_t w = r < T.rows ? T.exps[b * T.rows + r] >> 20 : 0u;
+            const int E = w < 1u ? 1 : (int)w;
+            uint64_t v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                v[e] = E >= 2047 ? 0x0080808080808080ull : fixed62(tile[4 * (threadIdx.x & 15) + e][rr], E);
+            put_digits(v, T, b * blocks + r / T.block, (int)(r % T.block), k);
+        }
+        return;
+    }
+    // K-contiguous rows: a warp, or the whole CTA, takes one row: its largest element, then the
+    // digits (the second read of the row hits in cache)
+    const bool wide = T.K > DG_WARP_K;
+    const int64_t row = wide ? local : local * 8 + warp;
+    const int64_t b = row / rows_p, r = row - b * rows_p;
+    const bool ok = b < T.batch && r < T.rows;
+    const double* p = T.src + b * T.sbatch + r * T.ld;
+    const int step = wide ? DG_THREADS : 32, me = wide ? (int)threadIdx.x : lane;
+    uint32_t m = 0;
+    if (ok) {
+#pragma unroll 4
+        for (int64_t k = me; k < T.K; k += step) m = max(m, abs_hi(__ldg(p + k)));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (wide) {
+        if (lane == 0) part[warp] = m;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < 8; ++w) m = max(m, part[w]);
+    }
+    if (b >= T.batch) return;
+    if (ok && me == 0) T.exps[b * T.rows + r] = m;
+    const uint32_t w = m >> 20;
+    const int E = w < 1u ? 1 : (int)w;
+    for (int64_t k = 4 * me; k < T.Kp; k += 4 * step) {
+        uint64_t v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            v[e] = E >= 2047 ? 0x0080808080808080ull : fixed62(ok && k + e < T.K ? __ldg(p + k + e) : 0.0, E);
+        put_digits(v, T, b * blocks + r / T.block, (int)(r % T.block), k);
+    }
+}
+
+}  // namespace
+
+extern "C" int64_t xrh_slice_ctas(int64_t rows, int64_t K, int64_t batch, int trans, int block, int max_pass) {
+    if (rows <= 0 || K <= 0 || batch <= 0 || (block != 32 && block != 64 && block != 128)) return 0;
+    const int64_t rows_p = (rows + block - 1) / block * block;
+    if (trans) {
+        if (max_pass) return batch * ((rows + 31) / 32) * ((K + DG_MAX_K - 1) / DG_MAX_K);
+        return batch * (rows_p / 32) * (((K + SL_KS - 1) / SL_KS * SL_KS + DG_TK - 1) / DG_TK);
+    }
+    if (max_pass) return 0;
+    return K > DG_WARP_K ? rows_p * batch : rows_p * batch / 8;
+}
+
+extern "C" int xrh_slice_grouped(const xrh_slice_task* tasks_dev, int n_tasks, int64_t total_ctas, int64_t max_ctas,
+                                 void* stream) {
+    if (n_tasks < 0 || total_ctas < 0 || max_ctas < 0) return XRH_ERR_ARG;
+    if (n_tasks == 0 || total_ctas == 0) return XRH_OK;
+    if (!tasks_dev) return XRH_ERR_ARG;
+    if (total_ctas > 0x7fffffffLL || max_ctas > 0x7fffffffLL) return XRH_ERR_CAPACITY;
+    if (max_ctas > 0) {
+        slice_max_kernel<<<(unsigned)max_ctas, DG_THREADS, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
+        XRH_CHECK_LAUNCH();
+    }
+    slice_digits_kernel<<<(unsigned)total_ctas, DG_THREADS, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
+    XRH_CHECK_LAUNCH();
+    return XRH_OK;
+}
+
+extern "C" int xrh_gemm_sliced_grouped(const xrh_gemm_task* tasks_dev, int n_tasks, int64_t total_tiles,
+                                       const xrh_sliced_segment* segs_dev, int32_t* status_dev, void* stream) {
+    if (n_tasks < 0 || total_tiles < 0) return XRH_ERR_ARG;
+    if (n_tasks == 0 || total_tiles == 0) return XRH_OK;
+    if (!tasks_dev || !segs_dev || !status_dev) return XRH_ERR_ARG;
+    int dev = 0, n_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    const size_t smem = (size_t)SL_STAGES * SL_STAGE_BYTES + 1024;
+    cudaFuncSetAttribute(gemm_sliced_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int64_t grid = total_tiles < n_sm ? total_tiles : n_sm;
+    gemm_sliced_kernel<<<(unsigned)grid, SL_THREADS, smem, (cudaStream_t)stream>>>(
+        tasks_dev, n_tasks, total_tiles, segs_dev, status_dev);
+    XRH_CHECK_LAUNCH();
+    return XRH_OK;
+}

@@ -11,8 +11,16 @@ import torch
 
 from . import _lib
 from ._lib import SEGMENT_DTYPE, TASK_DTYPE, call, ptr, stream_ptr
+from .sliced import SlicedGemm
 
 FP64_TILE = 64
+# FP64 launches on the tensor cores (sliced.py).  The CUDA-core kernel takes about 1.3 us per K
+# element of a tile's chain and 2 DFMA/clk/SM in all; a sliced launch takes about 32 us (digits and one
+# tile of up to 128 K), then 27 TFLOP/s: measured alone at M = 128, N = 64: K = 32 33 against 47 us,
+# K = 128 38 against 160 us; at 3600 x 784 x 784 249 against 4 650 us.
+SLICED_MIN_CHAIN = 24            # longest K chain of a launch from which it is worth the fixed time
+SLICED_MIN_PRODUCTS = 1 << 24    # or all products of a launch (64 x 64 tiles): 28 us of the FP64 pipe
+SLICED_MIN_K = 8                 # shorter tasks cost the epilogues and stores either way
 
 
 class GroupedGemm:
@@ -61,10 +69,29 @@ class GroupedGemm:
             self._keep += [x for x in (DA, DB) if x is not None]
         self._tasks.append(t)
 
+    def _sliced_tasks(self):
+        """The FP64 tasks that run on the tensor cores (all long enough ones of the launch, or none)."""
+        if self.precision != _lib.FP64:
+            return []
+        K_of = lambda t: [s[4] for s in self._segs[t["seg_begin"]:t["seg_begin"] + t["seg_count"]]]
+        long = [(t, sum(K_of(t))) for t in self._tasks if t["seg_count"] and min(K_of(t)) > 0 and
+                sum(K_of(t)) >= SLICED_MIN_K]
+        chain = max((K // t["splitk"] for t, K in long), default=0)
+        products = sum(-(-t["M"] // 64) * -(-t["N"] // 64) * 4096 * t["batch"] * K for t, K in long)
+        return [t for t, _K in long] if chain >= SLICED_MIN_CHAIN or products >= SLICED_MIN_PRODUCTS else []
+
     def finalize(self, tile=FP64_TILE):
-        tasks = np.zeros(len(self._tasks), dtype=TASK_DTYPE)
+        self.sliced = None
+        chosen = self._sliced_tasks()
+        if chosen:
+            self.sliced = SlicedGemm([dict({k: t[k] for k in t if k not in ("seg_begin", "seg_count", "splitk")},
+                                           segs=self._segs[t["seg_begin"]:t["seg_begin"] + t["seg_count"]])
+                                      for t in chosen], self.device)
+        ids = {id(t) for t in chosen}
+        simt = [t for t in self._tasks if id(t) not in ids]
+        tasks = np.zeros(len(simt), dtype=TASK_DTYPE)
         begin = 0
-        for i, t in enumerate(self._tasks):
+        for i, t in enumerate(simt):
             for k, v in t.items():
                 tasks[i][k] = v
             tasks[i]["tile_begin"] = begin
@@ -76,14 +103,21 @@ class GroupedGemm:
         self.tasks_dev = torch.from_numpy(tasks.view(np.uint8).copy()).to(self.device)
         self.segs_dev = torch.from_numpy(segs.view(np.uint8).copy()).to(self.device) if len(segs) else \
             torch.zeros(SEGMENT_DTYPE.itemsize, dtype=torch.uint8, device=self.device)
-        self.n_tasks = len(self._tasks)
+        self.n_tasks = len(simt)
         return self
 
     def run(self, stream=None):
+        if self.sliced is not None:
+            self.sliced.run(stream)
         if self.n_tasks == 0:
             return
         call("xrh_gemm_simt_grouped", self.precision, _lib.ptr(self.tasks_dev), self.n_tasks, self.total_tiles,
              _lib.ptr(self.segs_dev), stream_ptr(stream))
+
+    def check(self):
+        """Raise if a bounded device wait of a tensor-core launch gave up (synchronises)."""
+        if self.sliced is not None:
+            self.sliced.check()
 
 
 TC_TASK_DTYPE = np.dtype([("M", np.int64), ("N", np.int64), ("seg_begin", np.int64), ("seg_count", np.int64),

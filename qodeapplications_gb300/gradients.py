@@ -523,9 +523,8 @@ class XRDimerAdjoint:
 
     def check_status(self):
         """Raise if a bounded device wait of the tensor-core launch timed out (syncs)."""
-        if self.l3_tc:
-            self.L3.check()
-        self.Lgamma_tc.check()
+        for g in (self.L1, self.L2, self.L3, self.Lgamma, self.Lgamma_tc):
+            g.check()
         st = int(self.tc_status.item())
         if st != 0:
             raise _lib.XRHError(f"tensor-core density adjoint reported status {st}")

@@ -250,7 +250,7 @@ class SigmaBatch:
             self.reg.split("sigW")
 
     def check(self):
-        if self.tc and self.items:
+        if self.items:
             self.gemm.check()
 
 
@@ -803,9 +803,8 @@ class XRDimerPlan:
 
     def check_status(self):
         """Raise if a bounded device wait of the tensor-core kernels timed out (syncs)."""
-        if self.tc:
-            self.pre_tc.check()
-            self.fin_tc.check()
+        for g in (self.pre_tc, self.pre64, self.fin_tc) if self.tc else (self.pre, self.fin):
+            g.check()
         for b in self.builders:
             if hasattr(b, "check"):
                 b.check()

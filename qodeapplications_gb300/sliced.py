@@ -1,0 +1,203 @@
+"""Host-side plan of the FP64 grouped GEMM on the tensor cores (csrc/gemm_sliced.cu).
+
+The tasks of one GroupedGemm launch become waves: the operands of a wave are written as digit
+slices into one workspace (xrh_slice_grouped, every distinct operand once), then one
+xrh_gemm_sliced_grouped launch runs its tasks.  Tasks whose digits exceed the workspace limit are
+divided into panels.  Every table is built once and uploaded in one copy; run() only launches.
+"""
+import numpy as np
+import torch
+
+from . import _lib
+from ._lib import SLICE_TASK_DTYPE, SLICED_SEG_DTYPE, SLICES, TASK_DTYPE, call, ptr, stream_ptr
+
+STAGE_K = 32
+BM = 128
+SMS = 152
+WORKSPACE_LIMIT = 1 << 30        # bytes of digits per wave
+MIN_STAGES_PER_SPLIT = 8         # 256 K: an accumulating tile is not divided below this
+
+
+def _bn(N):
+    return 32 if N <= 32 else 64
+
+
+def _tiles(t):
+    return -(-t["M"] // BM) * -(-t["N"] // _bn(t["N"])) * t["batch"]
+
+
+def _stages(K):
+    return -(-K // STAGE_K)
+
+
+def _operands(t):
+    """(pointer, transposed, rows, K, ld, batch, batch stride, block) of A and B of every segment."""
+    for (A, B, lda, ldb, K, _alpha, flags, sA, sB) in t["segs"]:
+        for p, tr, rows, ld, st, block in ((A, flags & 1, t["M"], lda, sA, BM),
+                                           (B, flags >> 1 & 1, t["N"], ldb, sB, _bn(t["N"]))):
+            batch = t["batch"] if st else 1
+            yield (p, tr, rows, K, ld, batch, st if batch > 1 else 0, block)
+
+
+def _digit_bytes(op):
+    _p, _tr, rows, K, _ld, batch, _st, block = op
+    return 2 * SLICES * -(-rows // block) * block * batch * _stages(K) * STAGE_K
+
+
+def _exp_bytes(op):
+    return -(-4 * op[2] * op[5] // 256) * 256
+
+
+def _part(t, axis, lo, hi):
+    """The part [lo, hi) of a task along its batch, M or N axis."""
+    r = dict(t, segs=list(t["segs"]))
+    n = hi - lo
+    r["batch" if axis == "batch" else axis] = n
+    for i, (A, B, lda, ldb, K, alpha, flags, sA, sB) in enumerate(r["segs"]):
+        if axis == "batch":
+            A, B = A + 8 * lo * sA, B + 8 * lo * sB
+        elif axis == "M":
+            A += 8 * lo * (1 if flags & 1 else lda)
+        else:
+            B += 8 * lo * (1 if flags & 2 else ldb)
+        r["segs"][i] = (A, B, lda, ldb, K, alpha, flags, sA, sB)
+    if axis == "batch":
+        r["C"] += 8 * lo * t["sC"]
+    elif t["mode"] == 2:
+        row, col, diag, D = ("rowA", "colA", "diagA", "DA") if axis == "M" else ("rowB", "colB", "diagB", "DB")
+        r[row] += 4 * lo
+        r[col] += 4 * lo
+        r[diag] += lo
+        if r[D]:
+            r[D] += 8 * lo
+    else:
+        r["C"] += 8 * lo * (t["ldc"] if axis == "M" else 1)
+    return r
+
+
+def _panels(t, limit):
+    """The task as parts whose digits fit the limit."""
+    if sum(_digit_bytes(op) for op in set(_operands(t))) <= limit:
+        return [t]
+    if t["batch"] > 1:
+        axis, n, unit = "batch", t["batch"], 1
+    elif t["M"] >= t["N"]:
+        axis, n, unit = "M", t["M"], BM
+    else:
+        axis, n, unit = "N", t["N"], 64
+    cut = -(-(n // 2) // unit) * unit
+    if not 0 < cut < n:
+        return [t]                   # one tile: its own workspace size
+    return _panels(_part(t, axis, 0, cut), limit) + _panels(_part(t, axis, cut, n), limit)
+
+
+def plan_waves(tasks, limit=None):
+    """[(tasks, {operand: (digit offset, exponent offset)}, bytes, zeroed bytes)]: row exponents of
+    transposed operands first (they are zeroed before each run), then the rest."""
+    limit = WORKSPACE_LIMIT if limit is None else limit
+    waves, cur, ops, size = [], [], {}, 0
+    for t in (p for t in tasks for p in _panels(t, limit)):
+        new = [op for op in dict.fromkeys(_operands(t)) if op not in ops]
+        extra = sum(_digit_bytes(op) + _exp_bytes(op) for op in new)
+        if cur and size + extra > limit:
+            waves.append((cur, ops))
+            cur, ops, size = [], {}, 0
+            new = list(dict.fromkeys(_operands(t)))
+            extra = sum(_digit_bytes(op) + _exp_bytes(op) for op in new)
+        cur.append(t)
+        ops.update(dict.fromkeys(new))
+        size += extra
+    if cur:
+        waves.append((cur, ops))
+    out = []
+    for cur, ops in waves:
+        off, at = 0, {}
+        for op in sorted(ops, key=lambda o: not o[1]):
+            at[op] = off
+            off += _exp_bytes(op)
+        zeroed = sum(_exp_bytes(op) for op in ops if op[1])
+        off = -(-off // 1024) * 1024
+        place = {}
+        for op in ops:
+            place[op] = (off, at[op])
+            off += _digit_bytes(op)
+        out.append((cur, place, off, zeroed))
+    return out
+
+
+def split_factors(tasks):
+    """Split-K factor of every task of a wave: accumulating tasks are divided until the launch has
+    about four tiles per SM, none below MIN_STAGES_PER_SPLIT stages; stored results are not."""
+    stages = [sum(_stages(s[4]) for s in t["segs"]) for t in tasks]
+    work = sum(_tiles(t) * n for t, n in zip(tasks, stages))
+    per = max(MIN_STAGES_PER_SPLIT, -(-work // (4 * SMS)))
+    return [max(1, -(-n // per)) if t["mode"] == 1 else 1 for t, n in zip(tasks, stages)]
+
+
+class SlicedGemm:
+    """tasks: dicts with M, N, mode, C, ldc, batch, sC, mode 2's maps (device addresses) and segs
+    [(A, B, lda, ldb, K, alpha, flags, sA, sB)] (addresses)."""
+
+    def __init__(self, tasks, device):
+        self.device = device
+        waves = plan_waves(tasks)
+        self.work = torch.empty(max(w[2] for w in waves) + 1024, dtype=torch.uint8, device=device)
+        base = -(-self.work.data_ptr() // 1024) * 1024
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        L = _lib.lib()
+        blob, self.waves = bytearray(), []
+
+        def put(raw):
+            at = len(blob)
+            blob.extend(raw)
+            blob.extend(bytes(-len(blob) % 128))
+            return at
+
+        for cur, place, _size, zeroed in waves:
+            st = np.zeros(len(place), dtype=SLICE_TASK_DTYPE)
+            ctas = max_ctas = 0
+            # transposed operands last: their tasks own the CTAs of the row-maximum launch
+            for e, op in zip(st, sorted(place, key=lambda o: o[1])):
+                p, tr, rows, K, ld, batch, sb, block = op
+                e["src"], e["digits"], e["exps"] = p, base + place[op][0], base + place[op][1]
+                e["rows"], e["K"], e["ld"], e["Kp"] = rows, K, ld, _stages(K) * STAGE_K
+                e["batch"], e["sbatch"], e["trans"], e["block"], e["cta_begin"], e["max_begin"] = batch, sb, tr, block, ctas, max_ctas
+                ctas += L.xrh_slice_ctas(rows, K, batch, tr, block, 0)
+                max_ctas += L.xrh_slice_ctas(rows, K, batch, tr, block, 1)
+            gt = np.zeros(len(cur), dtype=TASK_DTYPE)
+            gs = np.zeros(sum(len(t["segs"]) for t in cur), dtype=SLICED_SEG_DTYPE)
+            tiles = k = 0
+            for e, t, sk in zip(gt, cur, split_factors(cur)):
+                for name, v in t.items():
+                    if name != "segs":
+                        e[name] = v
+                e["seg_begin"], e["seg_count"], e["splitk"], e["tile_begin"] = k, len(t["segs"]), sk, tiles
+                tiles += _tiles(t) * sk
+                ops = list(_operands(t))
+                for i, (A, B, lda, ldb, K, alpha, flags, sA, sB) in enumerate(t["segs"]):
+                    a, b, s = ops[2 * i], ops[2 * i + 1], gs[k]
+                    s["digA"], s["digB"], s["stages"] = base + place[a][0], base + place[b][0], _stages(K)
+                    s["rA"], s["rB"] = (a[2] if a[5] > 1 else 0), (b[2] if b[5] > 1 else 0)
+                    s["eA"], s["eB"] = base + place[a][1], base + place[b][1]
+                    s["A"], s["B"], s["lda"], s["ldb"], s["K"], s["alpha"] = A, B, lda, ldb, K, alpha
+                    s["flags"], s["sA"], s["sB"] = flags, sA, sB
+                    k += 1
+            self.waves.append((put(st.tobytes()), len(st), ctas, max_ctas, zeroed, put(gt.tobytes()), len(gt), tiles,
+                               put(gs.tobytes())))
+        self.tables = torch.frombuffer(blob, dtype=torch.uint8).to(device)
+        self.base = base
+
+    def run(self, stream=None):
+        s = stream_ptr(stream)
+        t = self.tables.data_ptr()
+        for st, n_s, ctas, max_ctas, zeroed, gt, n_t, tiles, gs in self.waves:
+            if zeroed:
+                call("xrh_zero", self.base, zeroed, s)
+            call("xrh_slice_grouped", t + st, n_s, ctas, max_ctas, s)
+            call("xrh_gemm_sliced_grouped", t + gt, n_t, tiles, t + gs, ptr(self.status), s)
+
+    def check(self):
+        """Raise if a bounded device wait gave up (synchronises)."""
+        st = int(self.status.item())
+        if st != 0:
+            raise _lib.XRHError(f"sliced FP64 GEMM reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")

@@ -650,6 +650,8 @@ class XRTrimerHamiltonian:
         """Raise if a bounded device wait of a tensor-core launch timed out (syncs)."""
         for pl in self.plans:
             pl.check_status()
+        for g in [self.stage1] + self.simt:
+            g.check()
         for phase in self.tcs:
             for _reg, g in phase:
                 g.check()
