@@ -331,6 +331,49 @@ int xrh_slice_grouped(const xrh_slice_task* tasks_dev, int n_tasks, int64_t tota
 int xrh_gemm_sliced_grouped(const xrh_gemm_task* tasks_dev, int n_tasks, int64_t total_tiles,
                             const xrh_sliced_segment* segs_dev, int32_t* status_dev, void* stream);
 
+/* The FP64 densities of xrh_density_accumulate over digit slices (exact products on the tensor cores;
+ * no reference counterpart).
+ *   xrh_coeff_digits: state coefficients zT[n_conf][n] as digits [ceil(n / npad)][n_conf][XRH_SLICES]
+ *       [npad] BF16 (16-byte aligned; npad = 16, 32 or 64, at least n or 64), each state scaled by the
+ *       power of two above its largest coefficient; exps_dev[n] (zero on entry) receives the high word
+ *       of that coefficient.  A task owns xrh_coeff_digit_ctas(n_conf) CTAs from cta_begin on.
+ *   xrh_density_sliced_grouped: unit u writes rhoT[idx, iblk 64 .., jblk 64 ..] from its `count` couplings
+ *       from c0 on, the first n_pos of sign +1, the rest -1 (count > 0: indices without couplings are
+ *       not written).  npad is that of both digit arrays of every task (state counts above 64 in blocks
+ *       of 64: npad = 64).  A device wait that runs out sets *status_dev = XRH_ERR_TIMEOUT. */
+typedef struct {
+    const double* zT;
+    void* digits;
+    uint32_t* exps;
+    int64_t n_conf;
+    int32_t n, npad;
+    int64_t cta_begin;
+} xrh_coeff_digit_task;   /* 48 bytes */
+typedef struct {
+    const int32_t* P;
+    const int32_t* Q;
+    const void* digb;
+    const void* digk;
+    const uint32_t* eb;
+    const uint32_t* ek;
+    const double* zbT;
+    const double* zkT;
+    double* rhoT;
+    int64_t conf_b, conf_k;    /* determinants of the bra and ket lists */
+    int32_t nb, nk;
+} xrh_dens_sliced_task;   /* 96 bytes */
+typedef struct {
+    int64_t c0;
+    int32_t count, n_pos;
+    int32_t task, idx;
+    int32_t iblk, jblk;
+} xrh_dens_sliced_unit;   /* 32 bytes */
+int64_t xrh_coeff_digit_ctas(int64_t n_conf);
+int xrh_coeff_digits(const xrh_coeff_digit_task* tasks_dev, int n_tasks, int64_t total_ctas, void* stream);
+int xrh_density_sliced_grouped(const xrh_dens_sliced_task* tasks_dev, int n_tasks,
+                               const xrh_dens_sliced_unit* units_dev, int64_t n_units, int npad,
+                               int32_t* status_dev, void* stream);
+
 /* FP64 Lanczos building blocks for the lowest eigenpairs of H (replaces the dense
  * scipy.linalg.eig of hermitian-XRCC/mains/workflow.py:229 and
  * StateSpaceOptimizer/state_gradients.py:107 for the eigenpairs the optimizer uses):

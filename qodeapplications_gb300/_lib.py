@@ -71,6 +71,9 @@ _SIGS = {
     "xrh_slice_ctas": (_i64, [_i64, _i64, _i64, _i32, _i32, _i32]),
     "xrh_slice_grouped": (_i32, [_vp, _i32, _i64, _i64, _vp]),
     "xrh_gemm_sliced_grouped": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp]),
+    "xrh_coeff_digit_ctas": (_i64, [_i64]),
+    "xrh_coeff_digits": (_i32, [_vp, _i32, _i64, _vp]),
+    "xrh_density_sliced_grouped": (_i32, [_vp, _i32, _vp, _i64, _i32, _vp, _vp]),
     "xrh_gemv_rows": (_i32, [_i64, _i64, _vp, _i64, _vp, _dbl, _dbl, _vp, _vp]),
     "xrh_gemv_cols": (_i32, [_i64, _i64, _vp, _i64, _vp, _dbl, _vp, _vp]),
     "xrh_gemv_split_work": (_i64, [_i64, _i64]),
@@ -135,10 +138,11 @@ class LaunchCounter:
     """Counts library calls that launch a kernel (the gpu_launches figure): every entry point
     except the host-only ones below launches one kernel of this library (those in `multi` the
     number given)."""
-    multi = {"xrh_orbital_terms": 2, "xrh_gemv_rows_split": 2, "xrh_lanczos_normalize_split": 2}
+    multi = {"xrh_orbital_terms": 2, "xrh_gemv_rows_split": 2, "xrh_lanczos_normalize_split": 2,
+             "xrh_coeff_digits": 2}
     host_only = {"xrh_abi_version", "xrh_status_string", "xrh_last_cuda_error", "xrh_tc_chunk_elems", "xrh_zero",
                  "xrh_tc_encode_map", "xrh_state_ctas", "xrh_abt_ctas", "xrh_lanczos_coop_work",
-                 "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_slice_ctas"}
+                 "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_slice_ctas", "xrh_coeff_digit_ctas"}
     count = 0
 
 
@@ -256,6 +260,15 @@ SLICED_SEG_DTYPE = np.dtype([("digA", np.uint64), ("digB", np.uint64), ("stages"
                              ("rB", np.int64), ("eA", np.uint64), ("eB", np.uint64), ("A", np.uint64), ("B", np.uint64),
                              ("lda", np.int64), ("ldb", np.int64), ("K", np.int64), ("flags", np.int64),
                              ("sA", np.int64), ("sB", np.int64), ("alpha", np.float64)])
+COEFF_DIGIT_DTYPE = np.dtype([("zT", np.uint64), ("digits", np.uint64), ("exps", np.uint64), ("n_conf", np.int64),
+                              ("n", np.int32), ("npad", np.int32), ("cta_begin", np.int64)])
+DENS_SLICED_TASK_DTYPE = np.dtype([("P", np.uint64), ("Q", np.uint64), ("digb", np.uint64), ("digk", np.uint64),
+                                   ("eb", np.uint64), ("ek", np.uint64), ("zbT", np.uint64), ("zkT", np.uint64),
+                                   ("rhoT", np.uint64), ("conf_b", np.int64), ("conf_k", np.int64), ("nb", np.int32),
+                                   ("nk", np.int32)])
+DENS_SLICED_UNIT_DTYPE = np.dtype([("c0", np.int64), ("count", np.int32), ("n_pos", np.int32), ("task", np.int32),
+                                   ("idx", np.int32), ("iblk", np.int32), ("jblk", np.int32)])
+assert (COEFF_DIGIT_DTYPE.itemsize, DENS_SLICED_TASK_DTYPE.itemsize, DENS_SLICED_UNIT_DTYPE.itemsize) == (48, 96, 32)
 assert SLICE_TASK_DTYPE.itemsize == 104 and SLICED_SEG_DTYPE.itemsize == 128
 
 

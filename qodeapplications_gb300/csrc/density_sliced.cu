@@ -1,0 +1,460 @@
+// FP64 transition densities with exact digit products on the tensor cores (sm_103a).
+//
+//   rho[idx, I, J] = sum_c s_c zb[P_c, I] zk[Q_c, J]   over the couplings c of operator index idx
+//
+// is for every idx a product of two gathered matrices with the couplings as contraction index; on
+// CUDA cores it runs at GB300's FP64 rate (2 DFMA/clk/SM).  Here every state's coefficients are scaled
+// by the power of two above the largest of them and kept as eight BF16 digits per determinant
+// (sliced_common.cuh), rows [8 slices][NPAD states] (NPAD = 16, 32, 64; larger state counts in blocks
+// of 64), so that a coupling is two contiguous rows of 16 NPAD bytes.  They are gathered into
+// shared memory as MN-major operands (128-byte swizzle: 64 elements x 8 couplings per KB) and every
+// digit pair with i + j < 8 comes out of a few wide MMAs: the 128 rows of A tile t are its slices
+// t G .. t G + G - 1 (G = 128 / NPAD), the columns all slices of B, and the accumulator column block
+// t G + j takes A tile t x B slice j, so that lane group g of column block b holds the pairs of weight
+// b + g with i = g mod G.  The sums stay below 2^24, so exact, for GROUP stages; they are collected in
+// 96-bit integers, added over the lane groups and rounded once at the end of the index.
+//
+// A CTA (persistent over a work list ordered by length), 16 warps:
+//   * warps 8-11: cp.async gathers of stages of 32 couplings of one sign (positive ones first: the MMA
+//     negates A for the negative ones), published to the async proxy stage by stage;
+//   * warp 12: MMAs;  * warps 0-7: collection and conversion.
+// Bounds: the gathers, 2 x 16 NPAD bytes of L2 per coupling, against 640 / 192 / 64 cycles of the tensor
+// pipe per 16 couplings at NPAD = 64 / 32 / 16, and the collection (8 NPAD columns a group).  Measured,
+// all blocks of a fragment of 28 spin orbitals: 60 states 115 -> 8.3 ms (97 GFLOP of canonical
+// couplings, 12 TFLOP/s FP64 against the pipe's 1.1), 32 states 2.2, 16 states 1.4; 18 spin orbitals, 10
+// states 3.4 -> 0.13 ms.
+// Every wait is bounded; on timeout *status is set and all roles leave after their copies and MMAs
+// have completed.
+#include "sliced_common.cuh"
+#include "tc_common.cuh"
+#include "xrh_common.cuh"
+
+namespace {
+using namespace xrh_tc;
+using namespace xrh_sliced;
+
+constexpr int DS_KS = 32;                              // couplings per stage
+constexpr int DS_EPI = 256, DS_PROD = 128, DS_THREADS = DS_EPI + DS_PROD + 128;
+constexpr uint32_t DS_ATOM = DS_KS * 128;              // bytes between 64-element atoms of a stage side
+
+template <int NPAD>
+struct Cfg {
+    static constexpr int G = 128 / NPAD;                               // slices per A tile
+    static constexpr int TILES = NS / G;                               // A tiles
+    static constexpr int COLS = NS * NPAD;                             // accumulator columns
+    static constexpr uint32_t SIDE = (uint32_t)DS_KS * NS * NPAD * 2;  // bytes of one side of a stage
+    static constexpr int STAGES = NPAD == 64 ? 3 : (NPAD == 32 ? 2 : 4);
+    static constexpr int LAG = STAGES - 1;
+    static constexpr int CTAS = NPAD == 64 ? 1 : 2;                    // per SM
+    // TILES pairs of |d d| <= 2^14 fall on one accumulator: 2^24 / (TILES 2^14) couplings
+    static constexpr int GROUP = (1 << 10) / TILES / DS_KS;            // stages per exact group
+    static constexpr int CW = NPAD / 2;                                // output columns per epilogue thread
+    // registers: 512 threads x 128 at launch = 65536 >= 256 x 168 + 256 x 72 (NPAD 64, one CTA an SM);
+    // 512 x 64 = 32768 = 256 x 88 + 256 x 40 (two CTAs)
+    static constexpr int EPI_REGS = CTAS == 1 ? 168 : 88, IO_REGS = CTAS == 1 ? 72 : 40;
+    static_assert(DS_EPI * EPI_REGS + (DS_THREADS - DS_EPI) * IO_REGS <= DS_THREADS * (CTAS == 1 ? 128 : 64),
+                  "register split exceeds the launch");
+};
+
+__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(DS_EPI) : "memory"); }
+__device__ __forceinline__ int epi_bar_or(int pred) {
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(pred), "n"(DS_EPI)
+        : "memory");
+    return r;
+}
+
+// MN-major operand: 64-element atoms DS_ATOM apart, 8-coupling groups 1024 B apart.
+__device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(DS_ATOM >> 4) << 16;
+    d |= (uint64_t)(1024 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)2 << 61;
+    return d;
+}
+
+__device__ __forceinline__ int stages_of(int n) { return (n + DS_KS - 1) / DS_KS; }
+
+// 16 bytes to shared memory, zeros where ok is false
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+// columns [c, c + n) of an accumulator, n = 8, 16, 32
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t ta, float (&v)[N]) {
+    uint32_t r[N];
+    if constexpr (N == 8) {
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(ta)
+                     : "memory");
+    } else {
+        static_assert(N == 16, "8 or 16 columns");
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                     "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+                     "tcgen05.wait::ld.sync.aligned;"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                       "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                     : "r"(ta)
+                     : "memory");
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+template <int NPAD>
+__global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
+    density_sliced_kernel(const xrh_dens_sliced_task* __restrict__ tasks, const xrh_dens_sliced_unit* __restrict__ units,
+                          int64_t n_units, int32_t* status) {
+    using C = Cfg<NPAD>;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;       // [STAGES][bra, ket][atoms][couplings]
+    __shared__ __align__(8) uint64_t full_bar[C::STAGES], empty_bar[C::STAGES];
+    __shared__ __align__(8) uint64_t ready_bar, drained_bar, done_bar;
+    __shared__ uint32_t tmem_base_sh;
+    __shared__ volatile int abort_sh;
+    __shared__ longlong2 s_raw[128][9];
+    __shared__ uint32_t s_eb[64], s_ek[64];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < C::STAGES; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), DS_PROD / 32);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        mbar_init(smem_u32(&ready_bar), 1);
+        mbar_init(smem_u32(&drained_bar), DS_EPI / 32);
+        mbar_init(smem_u32(&done_bar), 1);
+        abort_sh = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
+                     "r"(C::COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_sh;
+
+    if (warp >= 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::IO_REGS));
+        if (warp == 12 && lane == 0) {
+            // ------------------------------------------------------------------------ MMA --
+            constexpr uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | (8u << 24);
+            uint32_t st = 0, grp = 0;
+            bool ok = true;
+            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+                const int np = units[u].n_pos, nn = units[u].count - np;
+                const int s_pos = stages_of(np), n_st = s_pos + stages_of(nn);
+                for (int q = 0; q < n_st && ok; ++q, ++st) {
+                    const int in_group = q % C::GROUP;
+                    const uint32_t s = st % C::STAGES;
+                    if (in_group == 0 && grp > 0 && !mbar_wait(smem_u32(&drained_bar), (grp - 1) & 1u, &abort_sh)) ok = false;
+                    if (ok && !mbar_wait(smem_u32(&full_bar[s]), (st / C::STAGES) & 1u, &abort_sh)) ok = false;
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t id = idesc0 | (q >= s_pos ? 1u << 13 : 0u);
+                    const uint64_t da = desc_mn_sw128(ring + s * 2 * C::SIDE), db = desc_mn_sw128(ring + s * 2 * C::SIDE + C::SIDE);
+#pragma unroll
+                    for (int ks = 0; ks < DS_KS / 16; ++ks) {
+#pragma unroll
+                        for (int t = 0; t < C::TILES; ++t) {
+                            const uint32_t acc = (in_group > 0 || ks > 0 || t > 0) ? 1u : 0u;
+                            const uint64_t a = da + (uint64_t)((t * 2 * DS_ATOM + ks * 2048) >> 4);
+                            const int n = C::COLS - 128 * t, n1 = n < 256 ? n : 256;
+                            umma<0>(tmem + 128 * t, a, db + (uint64_t)((ks * 2048) >> 4), id | ((uint32_t)(n1 / 8) << 17), acc);
+                            if (n > 256)
+                                umma<0>(tmem + 128 * t + 256, a, db + (uint64_t)((4 * DS_ATOM + ks * 2048) >> 4),
+                                        id | ((uint32_t)((n - 256) / 8) << 17), acc);
+                        }
+                    }
+                    umma_commit(smem_u32(&empty_bar[s]));
+                    if (in_group == C::GROUP - 1 || q == n_st - 1) {
+                        umma_commit(smem_u32(&ready_bar));
+                        ++grp;
+                    }
+                }
+            }
+            if (!ok) {
+                abort_sh = 1;
+                atomicExch(status, XRH_ERR_TIMEOUT);
+            }
+            umma_commit(smem_u32(&done_bar));
+            mbar_wait(smem_u32(&done_bar), 0u, nullptr);
+        }
+    } else if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::IO_REGS));
+        // -------------------------------------------------------------------- gathers --
+        // warps 8, 9 the bra side, 10, 11 the ket side; a lane per 16-byte chunk of a row
+        const int pw = warp - 8, side = pw >> 1;
+        uint32_t st = 0;
+        bool ok = true;
+        auto publish = [&](uint32_t g) {               // this warp's part of stage g has landed
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&full_bar[g % C::STAGES]));
+        };
+        for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const xrh_dens_sliced_unit U = units[u];
+            const xrh_dens_sliced_task& T = tasks[U.task];
+            const int32_t* list = (side ? T.Q : T.P) + U.c0;
+            const int blk = side ? U.jblk : U.iblk;
+            const uint8_t* rows = reinterpret_cast<const uint8_t*>(side ? T.digk : T.digb) +
+                                  (int64_t)blk * (side ? T.conf_k : T.conf_b) * (NS * NPAD * 2);
+            const int s_pos = stages_of(U.n_pos), n_st = s_pos + stages_of(U.count - U.n_pos);
+            for (int q = 0; q < n_st; ++q, ++st) {
+                const uint32_t s = st % C::STAGES;
+                const int c = (q < s_pos ? q * DS_KS : U.n_pos + (q - s_pos) * DS_KS) + lane;
+                const int mine = c < (q < s_pos ? U.n_pos : U.count) ? __ldg(list + c) : -1;
+                if (st >= C::STAGES) {
+                    const bool free = mbar_wait(smem_u32(&empty_bar[s]), (st / C::STAGES - 1) & 1u, &abort_sh);
+                    if (!__all_sync(0xffffffffu, free)) {
+                        ok = false;
+                        break;
+                    }
+                }
+                const uint32_t base = ring + s * 2 * C::SIDE + side * C::SIDE;
+#pragma unroll 8
+                for (int i = 0; i < NPAD / 2; ++i) {
+                    const int item = i * 64 + (pw & 1) * 32 + lane;
+                    const int cc = item / NPAD, chunk = item % NPAD;           // NPAD 16-byte chunks per row
+                    const int row = __shfl_sync(0xffffffffu, mine, cc);
+                    const uint32_t dst = base + (uint32_t)(chunk >> 3) * DS_ATOM + (uint32_t)(cc >> 3) * 1024u +
+                                         (uint32_t)(cc & 7) * 128u + (uint32_t)(((chunk & 7) ^ (cc & 7)) << 4);
+                    cp_async16_or_zero(dst, rows + (int64_t)(row < 0 ? 0 : row) * (NS * NPAD * 2) + chunk * 16, row >= 0);
+                }
+                cp_async_commit();
+                if (st >= C::LAG) {
+                    cp_async_wait<C::LAG>();
+                    publish(st - C::LAG);
+                }
+            }
+        }
+        cp_async_wait<0>();
+        if (ok) {
+            for (uint32_t g = st > C::LAG ? st - C::LAG : 0; g < st; ++g) publish(g);
+        } else {
+            abort_sh = 1;
+            if (lane == 0) atomicExch(status, XRH_ERR_TIMEOUT);
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::EPI_REGS));
+        // ------------------------------------------------------------------- epilogue --
+        const int quarter = warp & 3, part = warp >> 2;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        const int row = quarter * 32 + lane;
+        const int g = row / NPAD;                      // lane group: weight = column block + g
+        uint32_t grp = 0;
+        bool failed = false;
+        for (int64_t u = blockIdx.x; u < n_units && !failed; u += gridDim.x) {
+            const int np = units[u].n_pos, count = units[u].count;
+            const int n_st = stages_of(np) + stages_of(count - np);
+            int64_t hi[C::CW];                         // sum = hi 2^32 + lo
+            uint32_t lo[C::CW];
+#pragma unroll
+            for (int j = 0; j < C::CW; ++j) hi[j] = lo[j] = 0;
+            for (int q = 0; q < n_st; q += C::GROUP, ++grp) {
+                if (!failed && !mbar_wait(smem_u32(&ready_bar), grp & 1u, &abort_sh)) {
+                    failed = true;
+                    abort_sh = 1;
+                }
+                if (failed) break;
+                tc_fence_after();
+#pragma unroll 1
+                for (int b = 0; b < NS; ++b) {
+                    const int w = b + g;
+                    // weights 0..3 at bits 56 - 8 w of T go to hi, 4..7 to the low words, above 7 nowhere
+                    const int mul = w < 4 ? 1 << (8 * (3 - w)) : (w < NS ? 1 << (8 * (NS - 1 - w)) : 0);
+                    const bool low = w >= 4;
+                    constexpr int CH = C::CW < 16 ? C::CW : 16;
+#pragma unroll
+                    for (int h = 0; h < C::CW; h += CH) {
+                        float v[CH];
+                        tmem_ld<CH>(tmem + lane_base + (uint32_t)(b * NPAD + part * C::CW + h), v);
+#pragma unroll
+                        for (int j = 0; j < CH; ++j) {
+                            const int64_t t = (int64_t)__float2int_rn(v[j]) * mul;
+                            if (!low) {
+                                hi[h + j] += t;
+                            } else {
+                                const uint32_t l = lo[h + j] + (uint32_t)t;
+                                hi[h + j] += (t >> 32) + (l < (uint32_t)t ? 1 : 0);
+                                lo[h + j] = l;
+                            }
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&drained_bar));
+            }
+            if (epi_bar_or(failed)) {                  // (also: s_eb, s_ek of the unit before are read)
+                failed = true;
+                abort_sh = 1;
+                if (tid == 0) atomicExch(status, XRH_ERR_TIMEOUT);
+                break;
+            }
+            const xrh_dens_sliced_unit U = units[u];
+            const xrh_dens_sliced_task& T = tasks[U.task];
+            const int i0 = U.iblk * 64, j0 = U.jblk * 64;
+            if (tid < 64) s_eb[tid] = i0 + tid < T.nb ? T.eb[i0 + tid] : 0u;
+            else if (tid < 128) s_ek[tid - 64] = j0 + tid - 64 < T.nk ? T.ek[j0 + tid - 64] : 0u;
+            epi_bar();
+            // 4 columns of each part at a time: the lane groups of an element are added, converted, stored
+#pragma unroll 1
+            for (int p = 0; p < C::CW / 4; ++p) {
+#pragma unroll
+                for (int v = 0; v < C::CW / 4; ++v) {
+                    if (v != p) continue;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        s_raw[row][part * 4 + j] = make_longlong2(hi[4 * v + j], (long long)lo[4 * v + j]);
+                }
+                epi_bar();
+#pragma unroll
+                for (int e = 0; e < (NPAD * 8 + DS_EPI - 1) / DS_EPI; ++e) {
+                    const int item = e * DS_EPI + tid, slot = item & 7, I = item >> 3;
+                    const int J = (slot >> 2) * C::CW + 4 * p + (slot & 3);
+                    if (I >= NPAD || i0 + I >= T.nb || j0 + J >= T.nk) continue;
+                    long long h = 0, l = 0;
+#pragma unroll
+                    for (int k = 0; k < C::G; ++k) {
+                        const longlong2 r = s_raw[k * NPAD + I][slot];
+                        h += r.x;
+                        l += r.y;
+                    }
+                    h += l >> 32;
+                    double x = sliced_to_double(h, (uint32_t)l, exp_of(s_eb[I]) + exp_of(s_ek[J]));
+                    if ((s_eb[I] >> 20) >= 2047u || (s_ek[J] >> 20) >= 2047u) {
+                        // a state with an infinity or a NaN: the couplings in FP64
+                        x = 0.0;
+#pragma unroll 1
+                        for (int c = 0; c < count; ++c) {
+                            const double a = T.zbT[(int64_t)T.P[U.c0 + c] * T.nb + i0 + I];
+                            x = fma(c < np ? a : -a, T.zkT[(int64_t)T.Q[U.c0 + c] * T.nk + j0 + J], x);
+                        }
+                    }
+                    T.rhoT[((int64_t)U.idx * T.nb + i0 + I) * T.nk + j0 + J] = x;
+                }
+                epi_bar();
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::COLS) : "memory");
+}
+
+// ---- digits of the state coefficients ------------------------------------------------------
+constexpr int CD_ROWS = 64;                            // determinants per CTA
+
+__device__ __forceinline__ const xrh_coeff_digit_task& find_coeff(const xrh_coeff_digit_task* __restrict__ tasks, int n_tasks) {
+    int lo = 0, hi = n_tasks - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tasks[mid].cta_begin <= (int64_t)blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    return tasks[lo];
+}
+
+// exps[state] = high word of the largest |coefficient| (zero on entry)
+__global__ void __launch_bounds__(256) coeff_max_kernel(const xrh_coeff_digit_task* __restrict__ tasks, int n_tasks) {
+    const xrh_coeff_digit_task& T = find_coeff(tasks, n_tasks);
+    const int64_t r0 = ((int64_t)blockIdx.x - T.cta_begin) * CD_ROWS;
+    const int rows = T.n_conf - r0 < CD_ROWS ? (int)(T.n_conf - r0) : CD_ROWS;
+    const int lanes = T.n <= 8 ? 8 : (T.n <= 16 ? 16 : (T.n <= 32 ? 32 : 64));   // threads along the states
+    for (int s0 = 0; s0 < T.n; s0 += lanes) {
+        const int s = s0 + threadIdx.x % lanes;
+        uint32_t m = 0;
+        if (s < T.n)
+            for (int r = threadIdx.x / lanes; r < rows; r += 256 / lanes) m = max(m, abs_hi(__ldg(T.zT + (r0 + r) * T.n + s)));
+        if (m) atomicMax(T.exps + s, m);
+    }
+}
+
+// rows [block of 64 states][determinant][slice][NPAD]: a thread per (determinant, 8 states)
+__global__ void __launch_bounds__(256) coeff_digits_kernel(const xrh_coeff_digit_task* __restrict__ tasks, int n_tasks) {
+    const xrh_coeff_digit_task& T = find_coeff(tasks, n_tasks);
+    const int64_t r0 = ((int64_t)blockIdx.x - T.cta_begin) * CD_ROWS;
+    const int rows = T.n_conf - r0 < CD_ROWS ? (int)(T.n_conf - r0) : CD_ROWS;
+    const int blocks = (T.n + T.npad - 1) / T.npad, oct = T.npad / 8, per = blocks * oct;
+    for (int x = threadIdx.x; x < rows * per; x += 256) {
+        const int r = x / per, o = x - r * per, blk = o / oct, s0 = blk * T.npad + (o - blk * oct) * 8;
+        const double* z = T.zT + (r0 + r) * T.n;
+        uint64_t v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int s = s0 + k;
+            v[k] = 0x0080808080808080ull;
+            if (s < T.n) {
+                const uint32_t w = T.exps[s] >> 20;
+                if (w < 2047u) v[k] = fixed62(__ldg(z + s), w < 1u ? 1 : (int)w);
+            }
+        }
+        uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(T.digits) +
+                                              ((int64_t)blk * T.n_conf + r0 + r) * (NS * T.npad)) + (o - blk * oct);
+#pragma unroll
+        for (int t = 0; t < NS; ++t) {
+            uint32_t q[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q[k] = __byte_perm(digit_float(v[2 * k], t), digit_float(v[2 * k + 1], t), 0x7632);
+            dst[t * oct] = make_uint4(q[0], q[1], q[2], q[3]);
+        }
+    }
+}
+
+template <int NPAD>
+int launch(const xrh_dens_sliced_task* tasks, const xrh_dens_sliced_unit* units, int64_t n_units, int32_t* status,
+           cudaStream_t s) {
+    using C = Cfg<NPAD>;
+    int dev = 0, n_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    const size_t smem = (size_t)C::STAGES * 2 * C::SIDE + 1024;
+    cudaFuncSetAttribute(density_sliced_kernel<NPAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int64_t grid = n_units < (int64_t)n_sm * C::CTAS ? n_units : (int64_t)n_sm * C::CTAS;
+    density_sliced_kernel<NPAD><<<(unsigned)grid, DS_THREADS, smem, s>>>(tasks, units, n_units, status);
+    XRH_CHECK_LAUNCH();
+    return XRH_OK;
+}
+
+}  // namespace
+
+extern "C" int64_t xrh_coeff_digit_ctas(int64_t n_conf) { return n_conf > 0 ? (n_conf + CD_ROWS - 1) / CD_ROWS : 0; }
+
+extern "C" int xrh_coeff_digits(const xrh_coeff_digit_task* tasks_dev, int n_tasks, int64_t total_ctas, void* stream) {
+    if (n_tasks < 0 || total_ctas < 0) return XRH_ERR_ARG;
+    if (n_tasks == 0 || total_ctas == 0) return XRH_OK;
+    if (!tasks_dev) return XRH_ERR_ARG;
+    if (total_ctas > 0x7fffffffLL) return XRH_ERR_CAPACITY;
+    coeff_max_kernel<<<(unsigned)total_ctas, 256, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
+    XRH_CHECK_LAUNCH();
+    coeff_digits_kernel<<<(unsigned)total_ctas, 256, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
+    XRH_CHECK_LAUNCH();
+    return XRH_OK;
+}
+
+extern "C" int xrh_density_sliced_grouped(const xrh_dens_sliced_task* tasks_dev, int n_tasks,
+                                          const xrh_dens_sliced_unit* units_dev, int64_t n_units, int npad,
+                                          int32_t* status_dev, void* stream) {
+    if (n_tasks < 0 || n_units < 0 || (npad != 16 && npad != 32 && npad != 64)) return XRH_ERR_ARG;
+    if (n_tasks == 0 || n_units == 0) return XRH_OK;
+    if (!tasks_dev || !units_dev || !status_dev) return XRH_ERR_ARG;
+    if (npad == 16) return launch<16>(tasks_dev, units_dev, n_units, status_dev, (cudaStream_t)stream);
+    if (npad == 32) return launch<32>(tasks_dev, units_dev, n_units, status_dev, (cudaStream_t)stream);
+    return launch<64>(tasks_dev, units_dev, n_units, status_dev, (cudaStream_t)stream);
+}

@@ -33,13 +33,13 @@
 //     and for additions) and the store, scatter or atomic epilogue through shared memory.
 // Every mbarrier wait is bounded; on timeout *status is set, all roles leave, copies and MMAs in
 // flight are waited for (bounded), TMEM is freed.
+#include "sliced_common.cuh"
 #include "tc_common.cuh"
-#include "xrh_common.cuh"
 
 namespace {
 using namespace xrh_tc;
+using namespace xrh_sliced;
 
-constexpr int NS = XRH_SLICES;
 constexpr int SL_BM = 128;
 constexpr int SL_KS = 32;                              // K elements per stage (64-byte rows)
 constexpr int SL_GROUP = 4;                            // stages per exact accumulation group
@@ -154,46 +154,6 @@ struct Groups {
         return true;
     }
 };
-
-// (hi 2^32 + lo) 2^(x - 68) rounded to FP64 (nearest, ties to even), |hi 2^32 + lo| < 2^94, by about
-// 45 integer operations without a branch (a branch per element serialises the 32 conversions of
-// a thread: 52 000 cycles a tile; the FP64 pipe would need 16 000).  Results outside the normal
-// range are formed by scalbn.
-__device__ __forceinline__ double sliced_to_double(int64_t hi, uint32_t lo, int x) {
-    const uint32_t sg = (uint32_t)(hi >> 63);           // all ones for a negative value
-    uint32_t w0 = lo ^ sg, w1 = (uint32_t)hi ^ sg, w2 = (uint32_t)(hi >> 32) ^ sg;
-    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, %2, 0;"
-        : "+r"(w0), "+r"(w1), "+r"(w2)
-        : "r"(sg & 1u));
-    // leading zeros of the 96 bits (w2 < 2^30); the leading one goes to bit 62 of (a : b), c behind
-    const bool z2 = w2 == 0u, z1 = z2 && w1 == 0u;
-    const uint32_t top = z1 ? w0 : (z2 ? w1 : w2);
-    const int z = __clz((int)top);
-    const int lz = z + (z1 ? 64 : (z2 ? 32 : 0));
-    uint32_t a = z1 ? w0 : (z2 ? w1 : w2), b = z1 ? 0u : (z2 ? w0 : w1), c = z2 ? 0u : w0;
-    a = __funnelshift_l(b, a, z);
-    b = __funnelshift_l(c, b, z);
-    c = c << (z & 31);
-    const uint32_t sticky = (c != 0u) | (b & 1u);
-    b = __funnelshift_r(b, a, 1) | sticky;
-    a >>= 1;
-    asm("add.cc.u32 %0, %0, %2;\n\taddc.u32 %1, %1, 0;" : "+r"(b), "+r"(a) : "r"(0x1ffu + ((b >> 10) & 1u)));
-    // 53 bits above bit 10; e - 1 is added above the implicit one
-    const int e = 95 - lz + x - 68 + 1023;
-    const uint32_t mh = a >> 10, ml = __funnelshift_r(b, a, 10);
-    double v = __hiloint2double((int)((mh + ((uint32_t)(e - 1) << 20)) | (sg & 0x80000000u)), (int)ml);
-    if (top == 0u) v = 0.0;
-    else if ((unsigned)(e - 1) >= 2044u) {
-        v = scalbn((double)(((uint64_t)mh << 32) | ml), e - 1075);
-        if (sg) v = -v;
-    }
-    return v;
-}
-
-__device__ __forceinline__ int exp_of(uint32_t hi) {   // |x| < 2^exp_of for the row's largest high word
-    const int E = (int)(hi >> 20);
-    return (E < 1 ? 1 : E) - 1022;
-}
 
 // The MMAs of one stage (two K steps of 16).  The B slices of a stage are consecutive rows and the
 // accumulators consecutive columns (weight w at column BN w), so A_i x [B_j .. B_j+c] adds to the
@@ -588,24 +548,6 @@ constexpr int DG_WARP_K = 1024;        // rows up to this K: a warp each; longer
 constexpr int DG_TK = 64;              // transposed operands: 32 rows x 64 K per CTA
 constexpr int DG_MAX_K = 512;          // K per CTA of the row-maximum pass
 
-__device__ __forceinline__ uint32_t abs_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
-
-// V = round(x 2^(62 - e)) for |x| < 2^e, with 128 added to its low seven digits: byte t of the
-// result (t = 0 lowest) is digit 7 - t plus 128, the top byte (signed) is digit 0.
-__device__ __forceinline__ uint64_t fixed62(double x, int E) {
-    const uint64_t b = (uint64_t)__double_as_longlong(x);
-    const int ex = (int)(b >> 52) & 0x7ff;
-    uint64_t m = b & 0xfffffffffffffull;
-    if (ex) m |= 1ull << 52;
-    const int s = 9 - (E - (ex ? ex : 1));             // shift of the 53-bit mantissa
-    uint64_t v;
-    if (s >= 0) v = m << s;
-    else if (s > -54) v = ((m >> (-s - 1)) + 1ull) >> 1;   // nearest, ties away
-    else v = 0;
-    const int64_t sv = (b >> 63) ? -(int64_t)v : (int64_t)v;
-    return (uint64_t)sv + 0x0080808080808080ull;
-}
-
 // Digit slices of four consecutive K elements of a row: eight 8-byte stores into the stage image
 // (blocks of `block` rows; per block and 32 K: [slice][row][32 K], 64-byte rows, 64-byte swizzle:
 // 16-byte chunk index xor bits 1..2 of the row).
@@ -620,11 +562,7 @@ __device__ __forceinline__ void put_digits(const uint64_t (&v)[4], const xrh_sli
         uint32_t f[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const uint32_t word = t < 4 ? (uint32_t)(v[e] >> 32) : (uint32_t)v[e];
-            const uint32_t byte = (word >> (8 * (3 - (t & 3)))) & 0xffu;
-            // 2^23 + byte exactly, minus 2^23 and the digit's bias: the digit as a float
-            if (t == 0) f[e] = __float_as_uint((float)(int)(int8_t)byte);
-            else f[e] = __float_as_uint(__uint_as_float(0x4b000000u | byte) - 8388736.0f);
+            f[e] = digit_float(v[e], t);
         }
         uint2 o;
         o.x = __byte_perm(f[0], f[1], 0x7632);          // upper halves: BF16

@@ -31,10 +31,24 @@ class Couplings:
     def __init__(self, op, K, idx_ptr, P, Q, sign):
         self.op, self.K = op, K
         self.idx_ptr, self.P, self.Q, self.sign = idx_ptr, P, Q, sign
+        self._ranges = None
 
     @property
     def count(self):
         return int(self.P.numel())
+
+    def ranges(self):
+        """(operator indices with couplings, first coupling, number, number of sign +1) on the host;
+        kept with the list."""
+        if self._ranges is None:
+            dev = self.idx_ptr.device
+            pos = torch.zeros(self.count + 1, dtype=torch.int64, device=dev)
+            pos[1:] = torch.cumsum((self.sign > 0).to(torch.int64), 0)
+            p = torch.stack([self.idx_ptr, pos[self.idx_ptr]]).cpu().numpy()
+            n = np.diff(p, axis=1)
+            idx = np.nonzero(n[0])[0]
+            self._ranges = (idx, p[0, idx], n[0, idx], n[1, idx])
+        return self._ranges
 
 
 # op strings with two adjacent operators of one kind: position u of the anticommuting pair
@@ -301,6 +315,68 @@ def _coupling_units(cp):
     return units, bool((nu > 1).any())
 
 
+class SlicedDensities:
+    """The FP64 coupling-list densities of one builder on the tensor cores
+    (xrh_density_sliced_grouped): digit copies of the state coefficients per charge and side, one unit
+    per operator index with couplings and block of 64 x 64 states, longest first (the CTAs take them
+    in turn, so the long ones do not end up last).
+    blocks: [(couplings, bra side, bra charge, ket side, ket charge, rhoT)]; sides: {side: {charge: zT}}.
+    Operator indices without couplings are never written: rhoT must hold zeros there."""
+
+    def __init__(self, blocks, sides, device):
+        n_max = max(z.shape[1] for zs in sides.values() for z in zs.values())
+        self.npad = 16 if n_max <= 16 else 32 if n_max <= 32 else 64
+        tabs = [(s, c, z) for s, zs in sides.items() for c, z in zs.items()]
+        ct = np.zeros(len(tabs), dtype=_lib.COEFF_DIGIT_DTYPE)
+        self.exps = torch.zeros(sum(z.shape[1] for _, _, z in tabs), dtype=torch.int32, device=device)
+        self.digits, at, e0, cta = {}, {}, 0, 0
+        for e, (s, c, z) in zip(ct, tabs):
+            n_conf, n = z.shape
+            nblk = -(-n // self.npad)
+            d = self.digits[(s, c)] = torch.empty((nblk, max(n_conf, 1), _lib.SLICES, self.npad), dtype=torch.bfloat16,
+                                                  device=device)
+            at[(s, c)] = self.exps.data_ptr() + 4 * e0
+            e["zT"], e["digits"], e["exps"], e["n_conf"] = z.data_ptr(), d.data_ptr(), at[(s, c)], n_conf
+            e["n"], e["npad"], e["cta_begin"] = n, self.npad, cta
+            e0 += n
+            cta += _lib.lib().xrh_coeff_digit_ctas(n_conf)
+        self.n_coeff, self.coeff_ctas = len(ct), cta
+        tasks = np.zeros(len(blocks), dtype=_lib.DENS_SLICED_TASK_DTYPE)
+        units = []
+        for i, (cp, bs, bc, ks, kc, rhoT) in enumerate(blocks):
+            t, zb, zk = tasks[i], sides[bs][bc], sides[ks][kc]
+            t["P"], t["Q"], t["rhoT"] = cp.P.data_ptr(), cp.Q.data_ptr(), rhoT.data_ptr()
+            t["digb"], t["digk"] = self.digits[(bs, bc)].data_ptr(), self.digits[(ks, kc)].data_ptr()
+            t["eb"], t["ek"], t["zbT"], t["zkT"] = at[(bs, bc)], at[(ks, kc)], zb.data_ptr(), zk.data_ptr()
+            t["conf_b"], t["conf_k"], t["nb"], t["nk"] = zb.shape[0], zk.shape[0], zb.shape[1], zk.shape[1]
+            idx, c0, count, n_pos = cp.ranges()
+            for ib in range(-(-int(t["nb"]) // 64)):
+                for jb in range(-(-int(t["nk"]) // 64)):
+                    un = np.zeros(len(idx), dtype=_lib.DENS_SLICED_UNIT_DTYPE)
+                    un["c0"], un["count"], un["n_pos"] = c0, count, n_pos
+                    un["task"], un["idx"], un["iblk"], un["jblk"] = i, idx, ib, jb
+                    units.append(un)
+        units = np.concatenate(units) if units else np.zeros(0, dtype=_lib.DENS_SLICED_UNIT_DTYPE)
+        units = units[np.argsort(-units["count"], kind="stable")]
+        self.n_tasks, self.n_units = len(tasks), len(units)
+        up = lambda a: torch.from_numpy(np.frombuffer(a.tobytes() or bytes(1), dtype=np.uint8).copy()).to(device)
+        self.coeff_dev, self.tasks_dev, self.units_dev = up(ct), up(tasks), up(units)
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.keep = (blocks, sides)
+
+    def run(self, s):
+        _lib.zero_(self.exps)
+        call("xrh_coeff_digits", ptr(self.coeff_dev), self.n_coeff, self.coeff_ctas, s)
+        call("xrh_density_sliced_grouped", ptr(self.tasks_dev), self.n_tasks, ptr(self.units_dev), self.n_units,
+             self.npad, ptr(self.status), s)
+
+    def check(self):
+        """Raise if a bounded device wait gave up (synchronises)."""
+        st = int(self.status.item())
+        if st != 0:
+            raise _lib.XRHError(f"sliced FP64 densities reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")
+
+
 class DensityBuilder:
     """Preallocated, reusable density build for one fragment and fixed state counts.
 
@@ -347,7 +423,8 @@ class DensityBuilder:
                 self._tmp[(op, bc, kc)] = self._unit_zero[arena_off:arena_off + cp.K * nb * nk]
                 arena_off += cp.K * nb * nk
             else:
-                self._tmp[(op, bc, kc)] = torch.empty(cp.K * nb * nk, dtype=torch.float64, device=dev)
+                # (the FP64 path writes the operator indices that have couplings only)
+                self._tmp[(op, bc, kc)] = torch.zeros(cp.K * nb * nk, dtype=torch.float64, device=dev)
         # canonical lists for the accumulated blocks of op strings with an anticommuting pair (not
         # the warp-per-unit blocks, whose unit tables index the full lists)
         self._canon = {}
@@ -369,6 +446,17 @@ class DensityBuilder:
             c: torch.empty((space.n_conf[c], self.n_states_bra[c]), dtype=torch.float64, device=dev)
             for c in space.charges}
         self._stage = None
+        # FP64 path: the accumulated blocks in one launch on the tensor cores.  State counts the
+        # CUDA-core kernel refuses (empty ones, or rows beyond its shared memory) keep its answer.
+        self.sliced = None
+        direct = [(key, self._canon.get(key, cp)) for key, cp in space.couplings.items() if key not in self.mirror]
+        sizes = [(self.n_states_bra[key[1]], self.n_states[key[2]]) for key, _ in direct]
+        if not self.f32 and direct and all(min(s) > 0 and sum((x + 3) // 4 * 4 for x in s) <= 400 for s in sizes) and \
+                min(self.n_states.values()) > 0 and min(self.n_states_bra.values()) > 0:
+            kside = "ket" if self.same_bra else "bra"
+            self.sliced = SlicedDensities(
+                [(cp, kside, key[1], "ket", key[2], self._tmp[key]) for key, cp in direct],
+                {"ket": self.zT} if self.same_bra else {"ket": self.zT, "bra": self.zbT}, dev)
         self._tr_direct = self._tr_derived = None
         self._mirrors = None
         # FP32 path: coefficients converted once per build, rows padded to 16 bytes
@@ -478,7 +566,9 @@ class DensityBuilder:
                     _lib.zero_(self._unit_zero)
                 call("xrh_density_accumulate_f32_units", ptr(self._unit_tasks), self._n_unit_tasks, ptr(self._units),
                      self._n_units, self._max_n, s)
-        if not self.f32:
+        if self.sliced is not None:
+            self.sliced.run(s)
+        elif not self.f32:
             for (op, bc, kc), cp in self.space.couplings.items():
                 if (op, bc, kc) in self.mirror:
                     continue
@@ -514,6 +604,11 @@ class DensityBuilder:
         self._mirrors.run()
         self._tr_derived.run()
         return self.rho
+
+    def check(self):
+        """Raise if a bounded device wait of the last builds gave up (synchronises)."""
+        if self.sliced is not None:
+            self.sliced.check()
 
 
 def as_device_sectors(states, device="cuda"):
