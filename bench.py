@@ -385,9 +385,9 @@ def density_adjoint_work(adj, m):
 
 def dominant_kernel_roofline(it, config, reps=20):
     """Live CUDA-event timing, on the launching stream, of the dominant kernel of the step in
-    the ncu launch list: the FP32 density adjoint (dE/dz from dE/drho), one launch per
-    fragment (lane per coupling on unit tables for blocks of at most 16 states, one CTA per
-    operator index above).  Timed with the buffers the last iteration left (the launches add
+    the ncu launch list: the FP32 density adjoint (dE/dz from dE/drho): lane per coupling on unit
+    tables for blocks of at most 16 states, one launch per fragment; above, digit slices on the
+    tensor cores, both fragments in one launch.  Timed with the buffers the last iteration left (the launches add
     into the gradient buffers, which the next iteration zeroes)."""
     import torch
     from qodeapplications_gb300 import _lib
@@ -395,13 +395,17 @@ def dominant_kernel_roofline(it, config, reps=20):
     launches = []
     for m, (tasks, n_t, units, n_u, mx) in enumerate(getattr(adj, "dens_adj_units", ())):
         launches.append(("xrh_density_adjoint_f32_units", (_lib.ptr(tasks), n_t, _lib.ptr(units), n_u, mx, 1)))
-    for (tasks, n_t, ctas, mnb, mnk) in adj.dens_adj_groups:
-        launches.append(("xrh_density_adjoint_f32_grouped", (_lib.ptr(tasks), n_t, ctas, mnb, mnk)))
+    for sl in adj.dens_adj_sliced:
+        launches.append(("xrh_density_adjoint_sliced_grouped",
+                         (sl.precision, _lib.ptr(sl.tasks_dev), sl.n_tasks, _lib.ptr(sl.units_dev), sl.n_units, sl.npad,
+                          _lib.ptr(sl.status))))
     if not launches:
         return None
     name = launches[0][0]
     launches = [l for l in launches if l[0] == name]
     work = [density_adjoint_work(adj, m) for m in (0, 1)]
+    if name.endswith("sliced_grouped"):          # both fragments in one launch
+        work = [tuple(a + b for a, b in zip(*work))]
     stream = torch.cuda.current_stream()
     s = _lib.stream_ptr(stream)
     for _ in range(3):
@@ -418,8 +422,8 @@ def dominant_kernel_roofline(it, config, reps=20):
     ms = e0.elapsed_time(e1) / (reps * len(launches))
     by = sum(w[0] for w in work) / len(work)
     fl = sum(w[1] for w in work) / len(work)
-    kname = ("density_adjoint_units_kernel" if name.endswith("units") else "density_adjoint_f32_grouped_kernel")
-    return dict(name=f"{kname} (FP32 density adjoint, one launch per fragment)", ms=ms, bytes=by, flops=fl,
+    kname = "density_adjoint_units_kernel" if name.endswith("units") else "adjoint_sliced_kernel"
+    return dict(name=f"{kname} (FP32 density adjoint)", ms=ms, bytes=by, flops=fl,
                 kernel=kname, traffic=DENSITY_ADJ_TRAFFIC.get((config, kname)))
 
 
@@ -521,9 +525,10 @@ def run_ours(args):
                     "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel in a "
                                        "capture of the bench command (profiles/)") if dk["traffic"] else
                                       "null: no ncu capture of the current kernel build at this workload",
-                    "note": "sparse outer products over coupling lists (4 n_b n_k FLOPs and 9 bytes per coupling; "
-                            "coefficient rows gathered from L2): bound by the FP32 pipe, not by HBM or the tensor "
-                            "cores; the HBM fraction is given beside it"}
+                    "note": "products over coupling lists (4 n_b n_k FLOPs and 9 bytes per coupling; coefficient rows "
+                            "gathered from L2), FLOPs as on the CUDA cores; above 16 states the kernel forms them from "
+                            "21 BF16 digit-slice products on the tensor cores, so the FP32 rate is a yardstick there, "
+                            "not its bound; the HBM fraction is given beside it"}
     else:
         roofline = None
 

@@ -333,7 +333,7 @@ int xrh_gemm_sliced_grouped(const xrh_gemm_task* tasks_dev, int n_tasks, int64_t
 
 /* The FP64 densities of xrh_density_accumulate over digit slices (exact products on the tensor cores;
  * no reference counterpart).
- *   xrh_coeff_digits: state coefficients zT[n_conf][n] as digits [ceil(n / npad)][n_conf][XRH_SLICES]
+ *   xrh_coeff_digits: state coefficients zT[n_conf][n] as digits [ceil(n / npad)][n_conf][slices]
  *       [npad] BF16 (16-byte aligned; npad = 16, 32 or 64, at least n or 64), each state scaled by the
  *       power of two above its largest coefficient; exps_dev[n] (zero on entry) receives the high word
  *       of that coefficient.  A task owns xrh_coeff_digit_ctas(n_conf) CTAs from cta_begin on.
@@ -347,8 +347,9 @@ typedef struct {
     uint32_t* exps;
     int64_t n_conf;
     int32_t n, npad;
+    int64_t slices;            /* digit slices written: 8, or 6 (the leading ones) */
     int64_t cta_begin;
-} xrh_coeff_digit_task;   /* 48 bytes */
+} xrh_coeff_digit_task;   /* 56 bytes */
 typedef struct {
     const int32_t* P;
     const int32_t* Q;
@@ -368,6 +369,29 @@ typedef struct {
     int32_t task, idx;
     int32_t iblk, jblk;
 } xrh_dens_sliced_unit;   /* 32 bytes */
+/* The adjoint of those densities (xrh_density_adjoint) over the same digit rows: gzk[Q, J] += s sum_I
+ * zb[P, I] gT[idx, I, J] (units with n_pos >= 0) and gzb[P, I] += s sum_J zk[Q, J] gT[idx, I, J] (units
+ * with the sign bit of n_pos set), one unit per direction, operator index and blocks of 64 states.
+ * precision XRH_FP64: digit rows of 8 slices, gz* double; XRH_FP32: rows of 6 slices (8 for npad = 16),
+ * gz* float. */
+typedef struct {
+    const int32_t* P;
+    const int32_t* Q;
+    const void* digb;
+    const void* digk;
+    const uint32_t* eb;
+    const uint32_t* ek;
+    const double* zbT;
+    const double* zkT;
+    const double* gT;
+    void* gzb;
+    void* gzk;
+    int64_t conf_b, conf_k;
+    int32_t nb, nk;
+} xrh_adj_sliced_task;   /* 112 bytes */
+int xrh_density_adjoint_sliced_grouped(int precision, const xrh_adj_sliced_task* tasks_dev, int n_tasks,
+                                       const xrh_dens_sliced_unit* units_dev, int64_t n_units, int npad,
+                                       int32_t* status_dev, void* stream);
 int64_t xrh_coeff_digit_ctas(int64_t n_conf);
 int xrh_coeff_digits(const xrh_coeff_digit_task* tasks_dev, int n_tasks, int64_t total_ctas, void* stream);
 int xrh_density_sliced_grouped(const xrh_dens_sliced_task* tasks_dev, int n_tasks,

@@ -73,6 +73,7 @@ _SIGS = {
     "xrh_gemm_sliced_grouped": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp]),
     "xrh_coeff_digit_ctas": (_i64, [_i64]),
     "xrh_coeff_digits": (_i32, [_vp, _i32, _i64, _vp]),
+    "xrh_density_adjoint_sliced_grouped": (_i32, [_i32, _vp, _i32, _vp, _i64, _i32, _vp, _vp]),
     "xrh_density_sliced_grouped": (_i32, [_vp, _i32, _vp, _i64, _i32, _vp, _vp]),
     "xrh_gemv_rows": (_i32, [_i64, _i64, _vp, _i64, _vp, _dbl, _dbl, _vp, _vp]),
     "xrh_gemv_cols": (_i32, [_i64, _i64, _vp, _i64, _vp, _dbl, _vp, _vp]),
@@ -261,14 +262,19 @@ SLICED_SEG_DTYPE = np.dtype([("digA", np.uint64), ("digB", np.uint64), ("stages"
                              ("lda", np.int64), ("ldb", np.int64), ("K", np.int64), ("flags", np.int64),
                              ("sA", np.int64), ("sB", np.int64), ("alpha", np.float64)])
 COEFF_DIGIT_DTYPE = np.dtype([("zT", np.uint64), ("digits", np.uint64), ("exps", np.uint64), ("n_conf", np.int64),
-                              ("n", np.int32), ("npad", np.int32), ("cta_begin", np.int64)])
+                              ("n", np.int32), ("npad", np.int32), ("slices", np.int64), ("cta_begin", np.int64)])
+ADJ_SLICED_TASK_DTYPE = np.dtype([("P", np.uint64), ("Q", np.uint64), ("digb", np.uint64), ("digk", np.uint64),
+                                  ("eb", np.uint64), ("ek", np.uint64), ("zbT", np.uint64), ("zkT", np.uint64),
+                                  ("gT", np.uint64), ("gzb", np.uint64), ("gzk", np.uint64), ("conf_b", np.int64),
+                                  ("conf_k", np.int64), ("nb", np.int32), ("nk", np.int32)])
 DENS_SLICED_TASK_DTYPE = np.dtype([("P", np.uint64), ("Q", np.uint64), ("digb", np.uint64), ("digk", np.uint64),
                                    ("eb", np.uint64), ("ek", np.uint64), ("zbT", np.uint64), ("zkT", np.uint64),
                                    ("rhoT", np.uint64), ("conf_b", np.int64), ("conf_k", np.int64), ("nb", np.int32),
                                    ("nk", np.int32)])
 DENS_SLICED_UNIT_DTYPE = np.dtype([("c0", np.int64), ("count", np.int32), ("n_pos", np.int32), ("task", np.int32),
                                    ("idx", np.int32), ("iblk", np.int32), ("jblk", np.int32)])
-assert (COEFF_DIGIT_DTYPE.itemsize, DENS_SLICED_TASK_DTYPE.itemsize, DENS_SLICED_UNIT_DTYPE.itemsize) == (48, 96, 32)
+assert (COEFF_DIGIT_DTYPE.itemsize, DENS_SLICED_TASK_DTYPE.itemsize, DENS_SLICED_UNIT_DTYPE.itemsize,
+        ADJ_SLICED_TASK_DTYPE.itemsize) == (56, 96, 32, 112)
 assert SLICE_TASK_DTYPE.itemsize == 104 and SLICED_SEG_DTYPE.itemsize == 128
 
 

@@ -48,6 +48,7 @@ static_assert(sizeof(xrh_permute_task) == 144, "xrh_permute_task layout is part 
 static_assert(sizeof(xrh_gather_terms) == 136, "xrh_gather_terms layout is part of the ABI");
 static_assert(sizeof(xrh_slice_task) == 104, "xrh_slice_task layout is part of the ABI");
 static_assert(sizeof(xrh_sliced_segment) == 128, "xrh_sliced_segment layout is part of the ABI");
-static_assert(sizeof(xrh_coeff_digit_task) == 48, "xrh_coeff_digit_task layout is part of the ABI");
+static_assert(sizeof(xrh_coeff_digit_task) == 56, "xrh_coeff_digit_task layout is part of the ABI");
 static_assert(sizeof(xrh_dens_sliced_task) == 96, "xrh_dens_sliced_task layout is part of the ABI");
 static_assert(sizeof(xrh_dens_sliced_unit) == 32, "xrh_dens_sliced_unit layout is part of the ABI");
+static_assert(sizeof(xrh_adj_sliced_task) == 112, "xrh_adj_sliced_task layout is part of the ABI");

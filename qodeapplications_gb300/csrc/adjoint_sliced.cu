@@ -1,0 +1,617 @@
+// Adjoint of the transition densities with exact digit products on the tensor cores (sm_103a).
+//
+// For an operator index with gradient G = dE/drho[idx] (n_b x n_k) and couplings (P_c, Q_c, s_c)
+//     dE/dzk[Q_c, J] += s_c sum_I zb[P_c, I] G[I, J]        (ket direction)
+//     dE/dzb[P_c, I] += s_c sum_J zk[Q_c, J] G[I, J]        (bra direction)
+// Each direction of an index is one unit: A = gathered digit rows of 128 couplings (K = states, the
+// rows the density kernel uses, density_sliced.cu), B = the digits of G for this direction, made in
+// shared memory once per unit.  A's digits are scaled per state, by 2^e_I; that factor goes into G
+// before its columns are scaled by their own largest element.  Slice i of A times all slices j of B
+// with i + j < NS is one MMA of N = (NS - i) NPAD columns that lands on the accumulators of the weights
+// i + j; a tile sums at most 8 pairs of 64 states, 2^23, exactly.
+//   FP64 (NS = 8): the eight weights of a sum become one 96-bit integer, rounded once;
+//   FP32 (NS = 6, 46 bits: states and gradients down to 2^-22 of their column's largest keep the 24 bits
+//   of FP32): the weights are combined by FP32 fused multiply-adds.
+// The results of a tile are staged in shared memory and added to the gradient rows with the lanes along
+// the outputs of a row: additions by a lane per row (one 32-byte sector each) held up the gathers on
+// the way to L2, 13.5 against 11.9 ms at the FP32 size below; one bulk reduction per row was slower
+// than either (12.9 ms, and 9.9 against 7.6 at the FP64 size, whose rows are not 16-byte units).
+//
+// A CTA (persistent), 16 or 20 warps: 8-11 gather (ring of 16 KB slots: 128 couplings x 64 elements,
+// K-major, 128-byte swizzle), 12 issues the MMAs, 13 and up make the digits of the next unit's G, 0-7
+// collect and add.
+//
+// What bounds it: FP64, the collection, about 75 integer operations a result, and the FP64 additions in
+// L2; FP32, the gathers, 96 KB a tile for 60 states, and the MMAs (3 500 cycles a tile, of about 5 500).
+// Measured, all indices of a fragment: FP64 24 spin orbitals, 21 states 48.6 (FP64 FMAs) -> 4.4 ms; FP64
+// 18 spin orbitals, 10 states 3.5 -> 0.53 ms; FP32 28 spin orbitals, 60 states 16.4 (TF32 x 3) -> 11.7 ms.
+// Every wait is bounded; on timeout *status is set and all roles leave after their copies and MMAs
+// have completed.
+#include "sliced_common.cuh"
+#include "tc_common.cuh"
+#include <type_traits>
+
+namespace {
+using namespace xrh_tc;
+using namespace xrh_sliced;
+
+constexpr int AS_EPI = 256, AS_PROD = 128;
+constexpr int AS_M = 128;                              // couplings per tile
+constexpr uint32_t AS_SLOT = AS_M * 128;
+
+template <int NPAD, int NSL>
+struct Cfg {
+    static constexpr int PER = 64 / NPAD;                              // slices per 128-byte row chunk
+    static constexpr int CHUNKS = (NSL + PER - 1) / PER;               // chunks of a tile
+    static constexpr int ROW = CHUNKS * 128;                           // bytes of a determinant's digit row
+    static constexpr int GROW = NPAD == 32 ? 64 : 128;                 // bytes of a row of B: (slice, output)
+    static constexpr uint32_t GBYTES = (uint32_t)NSL * NPAD * GROW;    // one buffer of it
+    static constexpr int NBUF = NPAD == 64 && NSL == 8 ? 1 : 2;        // buffers of B
+    static constexpr int ESIZE = NSL == 8 ? 8 : 4;                     // bytes of a result
+    static constexpr int SROW = NPAD * ESIZE + (NSL == 8 ? 8 : 16);                   // bytes of a staged row of results
+    static constexpr int SLOTS = NPAD == 64 ? 5 : (NPAD == 32 && NSL == 8 ? 2 : 3);
+    static constexpr uint32_t SMEM = NBUF * GBYTES + SLOTS * AS_SLOT + AS_M * SROW + 1024;
+    static constexpr int CTAS = NPAD == 64 ? 1 : 2;
+    static constexpr int DIG = NPAD == 64 ? 7 : 3;                     // warps that make digits of G
+    static constexpr int THREADS = AS_EPI + AS_PROD + 32 + DIG * 32;
+    static constexpr uint32_t COLS = NPAD == 64 ? 512 : 8 * NPAD;      // TMEM columns (a power of two)
+    static constexpr int CW = NPAD / 2;
+    // registers: 640 threads x 96 (one CTA an SM) or 512 x 64 (two) at launch
+    static constexpr int EPI_REGS = CTAS == 2 ? 80 : (NSL == 8 ? 168 : 152);
+    static constexpr int IO_REGS = CTAS == 1 && NSL == 6 ? 56 : 48;
+    static_assert(AS_EPI * EPI_REGS + (THREADS - AS_EPI) * IO_REGS <= THREADS * (CTAS == 1 ? 96 : 64),
+                  "register split exceeds the launch");
+};
+
+template <int N>
+__device__ __forceinline__ bool all_digit(bool x) {        // barrier of the warps that make digits of G
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 3, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((int)x), "n"(N)
+        : "memory");
+    return r != 0;
+}
+__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(AS_EPI) : "memory"); }
+__device__ __forceinline__ int epi_bar_or(int pred) {
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(pred), "n"(AS_EPI)
+        : "memory");
+    return r;
+}
+
+// The barrier counts this thread's copies as one arrival once they have landed; their reader, not the
+// thread that issued them, orders them before the MMAs (a proxy fence here would wait for the copies
+// in flight: one gather at a time).
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void fence_copies() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t ta, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(ta)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t ta, float (&v)[32]) {       // v is there after tmem_wait
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]), "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]), "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
+        : "r"(ta)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait(float (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]), "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15]), "+f"(v[16]), "+f"(v[17]), "+f"(v[18]), "+f"(v[19]), "+f"(v[20]), "+f"(v[21]), "+f"(v[22]), "+f"(v[23]), "+f"(v[24]), "+f"(v[25]), "+f"(v[26]), "+f"(v[27]), "+f"(v[28]), "+f"(v[29]), "+f"(v[30]), "+f"(v[31])
+                 :
+                 : "memory");
+}
+
+__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }      // -126 <= e <= 127
+
+__device__ __forceinline__ void tmem_ld4(uint32_t ta, float* v) {         // v is there after a wait
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                 : "r"(ta)
+                 : "memory");
+}
+
+template <typename T>
+__device__ __forceinline__ T ld_shared(uint32_t at) {
+    T x;
+    if constexpr (sizeof(T) == 8) asm volatile("ld.shared.f64 %0, [%1];" : "=d"(x) : "r"(at) : "memory");
+    else asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(at) : "memory");
+    return x;
+}
+
+template <int NPAD, int NSL>
+__global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
+    adjoint_sliced_kernel(const xrh_adj_sliced_task* __restrict__ tasks, const xrh_dens_sliced_unit* __restrict__ units,
+                          int64_t n_units, int32_t* status) {
+    using C = Cfg<NPAD, NSL>;
+    constexpr bool F64 = NSL == 8;
+    using Out = std::conditional_t<F64, double, float>;
+    extern __shared__ unsigned char smem_raw[];
+    const uint32_t gsm = (smem_u32(smem_raw) + 1023u) & ~1023u, ring = gsm + C::NBUF * C::GBYTES;
+    const uint32_t stage = ring + C::SLOTS * AS_SLOT;  // [row][output] results of a tile, on their way to memory
+    __shared__ __align__(8) uint64_t full_bar[C::SLOTS], empty_bar[C::SLOTS];
+    __shared__ __align__(8) uint64_t ready_bar, drained_bar, gfull_bar[2], gfree_bar[2], done_bar;
+    __shared__ uint32_t tmem_base_sh;
+    __shared__ volatile int abort_sh;
+    __shared__ int s_src[2][AS_M];                     // gathered rows of a tile (producers)
+    __shared__ int s_dst[AS_M];                        // output rows of a tile (epilogue)
+    __shared__ int s_max[2][64];                       // exponents of the columns of G
+    __shared__ float2 s_scale[2][F64 ? 1 : 64];        // factor of a column's sums, as a product of two floats
+    __shared__ int s_bad[2];                           // an infinity or a NaN in G or its states
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) {
+        for (int s = 0; s < C::SLOTS; ++s) {
+            mbar_init(smem_u32(&full_bar[s]), AS_PROD);
+            mbar_init(smem_u32(&empty_bar[s]), 1);
+        }
+        mbar_init(smem_u32(&ready_bar), 1);
+        mbar_init(smem_u32(&drained_bar), AS_EPI / 32);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(smem_u32(&gfull_bar[b]), C::DIG);
+            mbar_init(smem_u32(&gfree_bar[b]), 2);     // the MMAs and the epilogue of the unit
+        }
+        mbar_init(smem_u32(&done_bar), 1);
+        abort_sh = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncwarp();
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_sh)),
+                     "r"(C::COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_sh;
+
+    if (warp >= 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::IO_REGS));
+        if (warp == 12 && lane == 0) {
+            // ------------------------------------------------------------------------ MMA --
+            constexpr uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
+            uint32_t ch = 0, tile = 0, un = 0;
+            bool ok = true;
+            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++un) {
+                const int n_tiles = (units[u].count + AS_M - 1) / AS_M;
+                if (!mbar_wait(smem_u32(&gfull_bar[un % C::NBUF]), (un / C::NBUF) & 1u, &abort_sh)) ok = false;
+                const uint32_t gb = gsm + (un % C::NBUF) * C::GBYTES;
+                const uint64_t db = NPAD == 32 ? umma_desc_sw64(gb) : umma_desc_sw128(gb);
+                for (int q = 0; q < n_tiles && ok; ++q, ++tile) {
+                    if (tile > 0 && !mbar_wait(smem_u32(&drained_bar), (tile - 1) & 1u, &abort_sh)) {
+                        ok = false;
+                        break;
+                    }
+                    for (int k = 0; k < C::CHUNKS; ++k, ++ch) {
+                        const uint32_t s = ch % C::SLOTS;
+                        if (!mbar_wait(smem_u32(&full_bar[s]), (ch / C::SLOTS) & 1u, &abort_sh)) {
+                            ok = false;
+                            break;
+                        }
+                        fence_copies();
+                        tc_fence_after();
+                        const uint64_t da = umma_desc_sw128(ring + s * AS_SLOT);
+#pragma unroll
+                        for (int p = 0; p < C::PER; ++p) {
+                            const int i = k * C::PER + p;
+                            if (i >= NSL) break;
+                            const int n = (NSL - i) * NPAD, n1 = n < 256 ? n : 256;
+#pragma unroll
+                            for (int ks = 0; ks < NPAD / 16; ++ks) {
+                                const uint64_t a = da + (uint64_t)((p * NPAD * 2 + ks * 32) >> 4), b = db + 2 * ks;
+                                const uint32_t acc = (i > 0 || ks > 0) ? 1u : 0u;
+                                umma<0>(tmem + i * NPAD, a, b, idesc0 | ((uint32_t)(n1 / 8) << 17), acc);
+                                if (n > 256)
+                                    umma<0>(tmem + i * NPAD + 256, a, b + (uint64_t)((256 * C::GROW) >> 4),
+                                            idesc0 | ((uint32_t)((n - 256) / 8) << 17), acc);
+                            }
+                        }
+                        umma_commit(smem_u32(&empty_bar[s]));
+                    }
+                    if (ok) umma_commit(smem_u32(&ready_bar));
+                }
+                if (ok) umma_commit(smem_u32(&gfree_bar[un % C::NBUF]));
+            }
+            if (!ok) {
+                abort_sh = 1;
+                atomicExch(status, XRH_ERR_TIMEOUT);
+            }
+            umma_commit(smem_u32(&done_bar));
+            mbar_wait(smem_u32(&done_bar), 0u, nullptr);
+        } else if (warp > 12) {
+            // ------------------------------------------------------------ digits of G --
+            // an item: OL outputs along the lanes, KC consecutive contracted states per lane
+            constexpr int OL = NPAD < 32 ? NPAD : 32, KC = 4, KL = 32 / OL;
+            constexpr int ITEMS = (NPAD / OL) * (NPAD / (KC * KL));
+            const int dw = warp - 13;
+            uint32_t un = 0;
+            bool ok = true;
+            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++un) {
+                const uint32_t b = un % C::NBUF;
+                if (un >= C::NBUF) {
+                    const bool free = mbar_wait(smem_u32(&gfree_bar[b]), (un / C::NBUF - 1) & 1u, &abort_sh);
+                    if (!__all_sync(0xffffffffu, free)) ok = false;
+                }
+                if (dw == 0) {
+                    for (int o = lane; o < 64; o += 32) s_max[b][o] = -100000;
+                    if (lane == 0) s_bad[b] = 0;
+                }
+                ok = all_digit<C::DIG * 32>(ok);                        // (the three warps go on or stop together)
+                if (!ok) break;
+                const xrh_dens_sliced_unit U = units[u];
+                const xrh_adj_sliced_task& T = tasks[U.task];
+                const bool bra = U.n_pos < 0;
+                const int i0 = U.iblk * 64, j0 = U.jblk * 64;
+                const int nk_ = bra ? T.nk - j0 : T.nb - i0, no_ = bra ? T.nb - i0 : T.nk - j0;
+                const int n_con = nk_ < NPAD ? nk_ : NPAD, n_out = no_ < NPAD ? no_ : NPAD;
+                const uint32_t* ecoef = bra ? T.ek + j0 : T.eb + i0;
+                const double* g = T.gT + ((int64_t)U.idx * T.nb + i0) * T.nk + j0;
+                const int64_t so = bra ? T.nk : 1, sk = bra ? 1 : T.nk;
+                // x and the exponent (biased as FP64's) of x 2^e_k
+                auto load = [&](int item, double (&x)[KC], int (&ex)[KC], int& o, int& k0) {
+                    o = (item % (NPAD / OL)) * OL + lane % OL;
+                    k0 = (item / (NPAD / OL) * KL + lane / OL) * KC;
+                    bool odd = false;
+#pragma unroll
+                    for (int k = 0; k < KC; ++k) {
+                        const bool in = o < n_out && k0 + k < n_con;
+                        x[k] = in ? g[o * so + (k0 + k) * sk] : 0.0;
+                        const uint32_t we = in ? ecoef[k0 + k] >> 20 : 0u, wx = abs_hi(x[k]) >> 20;
+                        odd = odd || we >= 2047u || wx >= 2047u;
+                        ex[k] = (int)(wx < 1u ? 1u : wx) + (int)(we < 1u ? 1u : we) - 1022;
+                    }
+                    return odd;
+                };
+#pragma unroll 1
+                for (int item = dw; item < ITEMS; item += C::DIG) {
+                    double x[KC];
+                    int ex[KC], o, k0, top = -100000;
+                    if (load(item, x, ex, o, k0)) s_bad[b] = 1;
+#pragma unroll
+                    for (int k = 0; k < KC; ++k)
+                        if (x[k] != 0.0 && ex[k] > top) top = ex[k];
+                    if (top > -100000) atomicMax(&s_max[b][o], top);
+                }
+                asm volatile("bar.sync 3, %0;" ::"n"(C::DIG * 32) : "memory");
+                const bool bad = s_bad[b] != 0;
+                if (!F64 && dw == 0) {
+                    for (int o = lane; o < NPAD; o += 32) {
+                        int e = s_max[b][o] - 1022 - 12;
+                        e = e < -250 ? -250 : (e > 250 ? 250 : e);
+                        s_scale[b][o] = make_float2(pow2f(e / 2), pow2f(e - e / 2));
+                    }
+                }
+#pragma unroll 1
+                for (int item = dw; item < ITEMS; item += C::DIG) {
+                    double x[KC];
+                    int ex[KC], o, k0;
+                    load(item, x, ex, o, k0);
+                    const int E = s_max[b][o];
+                    uint64_t v[KC];
+#pragma unroll
+                    for (int k = 0; k < KC; ++k)
+                        v[k] = bad || x[k] == 0.0 ? 0x0080808080808080ull
+                                                  : fixed62(x[k], E - (ex[k] - (int)max(1u, abs_hi(x[k]) >> 20)));
+#pragma unroll
+                    for (int t = 0; t < NSL; ++t) {
+                        const uint32_t r = (uint32_t)(t * NPAD + o), kk = (uint32_t)k0;
+                        const uint32_t sw = NPAD == 32 ? (r >> 1) & 3u : r & 7u;
+                        const uint32_t dst = gsm + b * C::GBYTES + r * C::GROW + (((kk >> 3) ^ sw) << 4) + (kk & 7u) * 2u;
+                        uint32_t q[KC / 2];
+#pragma unroll
+                        for (int k = 0; k < KC / 2; ++k)
+                            q[k] = __byte_perm(digit_float(v[2 * k], t), digit_float(v[2 * k + 1], t), 0x7632);
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"(q[0]), "r"(q[1]) : "memory");
+                    }
+                }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&gfull_bar[b]));
+            }
+            if (!ok && lane == 0) {
+                abort_sh = 1;
+                atomicExch(status, XRH_ERR_TIMEOUT);
+            }
+        }
+    } else if (warp >= 8) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::IO_REGS));
+        // -------------------------------------------------------------------- gathers --
+        const int pt = tid - AS_EPI, pw = pt >> 5;
+        uint32_t ch = 0, tile = 0;
+        bool ok = true;
+        for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const xrh_dens_sliced_unit U = units[u];
+            const xrh_adj_sliced_task& T = tasks[U.task];
+            const int bra = U.n_pos < 0;               // direction: the sign bit of n_pos
+            const int32_t* list = (bra ? T.Q : T.P) + U.c0;
+            const uint8_t* rows = reinterpret_cast<const uint8_t*>(bra ? T.digk : T.digb) +
+                                  (int64_t)(bra ? U.jblk : U.iblk) * (bra ? T.conf_k : T.conf_b) * C::ROW;
+            const int n_tiles = (U.count + AS_M - 1) / AS_M;
+            int next = pt < U.count ? __ldg(list + pt) : -1;         // a tile ahead: its latency stays hidden
+            for (int q = 0; q < n_tiles && ok; ++q, ++tile) {
+                int* src = s_src[tile & 1];
+                src[pt] = next;
+                next = (q + 1) * AS_M + pt < U.count ? __ldg(list + (q + 1) * AS_M + pt) : -1;
+                asm volatile("bar.sync 2, %0;" ::"n"(AS_PROD) : "memory");
+                for (int k = 0; k < C::CHUNKS; ++k, ++ch) {
+                    const uint32_t s = ch % C::SLOTS;
+                    if (ch >= C::SLOTS) {
+                        const bool free = mbar_wait(smem_u32(&empty_bar[s]), (ch / C::SLOTS - 1) & 1u, &abort_sh);
+                        if (!__all_sync(0xffffffffu, free)) ok = false;
+                    }
+                    if (ok) {
+                        // 8 lanes per 128-byte row piece, 16 rows at a time
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int r = i * 16 + pw * 4 + (lane >> 3), c16 = lane & 7;
+                            const int row = src[r];
+                            cp_async16_or_zero(ring + s * AS_SLOT + (uint32_t)r * 128u + (uint32_t)((c16 ^ (r & 7)) << 4),
+                                               rows + (int64_t)(row < 0 ? 0 : row) * C::ROW + k * 128 + c16 * 16, row >= 0);
+                        }
+                    }
+                    cp_async_arrive(smem_u32(&full_bar[s]));
+                }
+            }
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        if (!ok) {
+            abort_sh = 1;
+            if (lane == 0) atomicExch(status, XRH_ERR_TIMEOUT);
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::EPI_REGS));
+        // ------------------------------------------------------------------- epilogue --
+        const int quarter = warp & 3, part = warp >> 2;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        const int row = quarter * 32 + lane;
+        uint32_t tile = 0, un = 0;
+        bool failed = false;
+        for (int64_t u = blockIdx.x; u < n_units && !failed; u += gridDim.x, ++un) {
+            const xrh_dens_sliced_unit U = units[u];
+            const xrh_adj_sliced_task& T = tasks[U.task];
+            const bool bra = U.n_pos < 0;
+            const int n_pos = U.n_pos & 0x7fffffff;
+            const int i0 = U.iblk * 64, j0 = U.jblk * 64;
+            const int nk_ = bra ? T.nk - j0 : T.nb - i0, no_ = bra ? T.nb - i0 : T.nk - j0;
+            const int n_con = nk_ < NPAD ? nk_ : NPAD, n_out = no_ < NPAD ? no_ : NPAD;   // contracted, output states
+            const uint32_t b = un % C::NBUF;
+            if (!mbar_wait(smem_u32(&gfull_bar[b]), (un / C::NBUF) & 1u, &abort_sh)) failed = true;
+            const bool bad = s_bad[b] != 0;
+            const double* g = T.gT + ((int64_t)U.idx * T.nb + i0) * T.nk + j0;             // G[i][j], row stride nk
+            const int64_t so = bra ? T.nk : 1, sk = bra ? 1 : T.nk;
+            // ---- tiles ----
+            const int32_t* out_list = (bra ? T.P : T.Q) + U.c0;
+            const int64_t n_row = bra ? T.nb : T.nk;
+            const int o0 = bra ? i0 : j0;
+            const int n_tiles = (U.count + AS_M - 1) / AS_M;
+            const bool vec = ((n_out | (int)n_row) & 3) == 0;      // rows of whole 16-byte units (FP32)
+            int next_dst = tid < AS_M && tid < U.count ? __ldg(out_list + tid) : -1;
+            for (int q = 0; q < n_tiles; ++q, ++tile) {
+                // this tile's output rows (loaded during the tile before)
+                if (tid < AS_M) s_dst[tid] = next_dst;
+                if (tid < AS_M) next_dst = (q + 1) * AS_M + tid < U.count ? __ldg(out_list + (q + 1) * AS_M + tid) : -1;
+                if (!failed && !mbar_wait(smem_u32(&ready_bar), tile & 1u, &abort_sh)) {
+                    failed = true;
+                    abort_sh = 1;
+                }
+                if (epi_bar_or(failed)) {              // also: s_dst is written
+                    failed = true;
+                    abort_sh = 1;
+                    if (tid == 0) atomicExch(status, XRH_ERR_TIMEOUT);
+                    break;
+                }
+                tc_fence_after();
+                const int d = s_dst[row];
+                const bool neg = q * AS_M + row >= n_pos;
+                const uint32_t srow = stage + (uint32_t)row * C::SROW;
+                if constexpr (F64) {
+                    // columns in groups of 4, alternately of the two parts
+                    const int n_grp = (n_out - 4 * part + 7) >> 3;
+#pragma unroll 1
+                    for (int p = 0; p < n_grp; ++p) {
+                        Sum96 t[4];
+                        int te[4];
+                        double y[4];
+                        float v[NSL][4];
+                        const int J = 8 * p + 4 * part;
+#pragma unroll
+                        for (int w = 0; w < NSL; ++w) tmem_ld4(tmem + lane_base + (uint32_t)(w * NPAD + J), v[w]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            float x[NSL];
+#pragma unroll
+                            for (int w = 0; w < NSL; ++w) {
+                                asm volatile("" : "+f"(v[w][j]));      // (not before the wait)
+                                x[w] = v[w][j];
+                            }
+                            if constexpr (NSL == 8) t[j] = collect_weights<NPAD>(x);
+                            te[j] = s_max[b][J + j] - 1022;
+                        }
+                        sliced_to_doubles<4>(t, te, y);
+                        if (bad && d >= 0) {
+                            // an infinity or a NaN in G or the states: the products in FP64
+                            const double* z = bra ? T.zkT + (int64_t)T.Q[U.c0 + q * AS_M + row] * T.nk + j0
+                                                  : T.zbT + (int64_t)T.P[U.c0 + q * AS_M + row] * T.nb + i0;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                y[j] = 0.0;
+#pragma unroll 1
+                                for (int k = 0; k < n_con && J + j < n_out; ++k) y[j] = fma(z[k], g[(J + j) * so + k * sk], y[j]);
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            if (neg) y[j] = -y[j];
+                            if (J + j < n_out) asm volatile("st.shared.f64 [%0], %1;" ::"r"(srow + (uint32_t)(J + j) * 8u), "d"(y[j]) : "memory");
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&drained_bar));
+                } else {
+                    // the sums of this thread's columns into registers, the accumulators back to the MMA
+                    // warp, then scaling and additions while the next tile is multiplied
+                    float acc[C::CW];
+#pragma unroll
+                    for (int j = 0; j < C::CW; ++j) acc[j] = 0.f;
+                    if constexpr (NPAD == 64) {        // two weights in flight
+                        float va[32], vb[32];
+                        const uint32_t t0 = tmem + lane_base + (uint32_t)(part * 32);
+                        tmem_ld32(t0 + (NSL - 1) * 64, va);
+                        tmem_wait(va);
+#pragma unroll
+                        for (int w = NSL - 1; w > 0; w -= 2) {
+                            tmem_ld32(t0 + (w - 1) * 64, vb);
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) acc[j] = fmaf(acc[j], 0.00390625f, va[j]);
+                            tmem_wait(vb);
+                            if (w > 1) tmem_ld32(t0 + (w - 2) * 64, va);
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) acc[j] = fmaf(acc[j], 0.00390625f, vb[j]);
+                            if (w > 1) tmem_wait(va);
+                        }
+                    } else {
+#pragma unroll 1
+                        for (int w = NSL - 1; w >= 0; --w) {
+#pragma unroll
+                            for (int h = 0; h < C::CW; h += 8) {
+                                float v[8];
+                                tmem_ld8(tmem + lane_base + (uint32_t)(w * NPAD + part * C::CW + h), v);
+#pragma unroll
+                                for (int j = 0; j < 8; ++j) acc[h + j] = fmaf(acc[h + j], 0.00390625f, v[j]);
+                            }
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&drained_bar));
+                    const float sg = neg ? -1.f : 1.f;
+#pragma unroll
+                    for (int h = 0; h < C::CW; h += 4) {
+                        const int J = part * C::CW + h;
+                        if (J < n_out) {
+                            float v[4];
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) v[j] = (acc[h + j] * s_scale[b][J + j].x) * (sg * s_scale[b][J + j].y);
+                            if (bad && d >= 0) {
+                                // an infinity or a NaN in G or the states: FP32 products of the operands
+                                const double* z = bra ? T.zkT + (int64_t)T.Q[U.c0 + q * AS_M + row] * T.nk + j0
+                                                      : T.zbT + (int64_t)T.P[U.c0 + q * AS_M + row] * T.nb + i0;
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    float y = 0.f;
+#pragma unroll 1
+                                    for (int k = 0; k < n_con && J + j < n_out; ++k)
+                                        y = fmaf((float)z[k], (float)g[(J + j) * so + k * sk], y);
+                                    v[j] = sg * y;
+                                }
+                            }
+                            const uint32_t at = srow + (uint32_t)J * 4u;
+                            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+                        }
+                    }
+                }
+                epi_bar();                             // the tile is staged
+                // a warp adds 16 rows, lanes along the outputs of a row: whole sectors in every addition
+                const int to_lane = s_dst[warp * 16 + (lane & 15)];
+                const uint32_t rows = stage + (uint32_t)(warp * 16) * C::SROW;
+                unsigned char* out = reinterpret_cast<unsigned char*>(bra ? T.gzb : T.gzk) + o0 * C::ESIZE;
+                if (!F64 && vec) {
+#pragma unroll
+                    for (int i = 0; i < NPAD / 8; ++i) {
+                        const int x = i * 32 + lane, r = x / (NPAD / 4), c = x % (NPAD / 4) * 4;
+                        const int to = __shfl_sync(0xffffffffu, to_lane, r);
+                        if (to < 0 || c >= n_out) continue;
+                        float v[4];
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                                     : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                                     : "r"(rows + (uint32_t)(r * C::SROW + c * 4))
+                                     : "memory");
+                        xrh_red_add_v4(reinterpret_cast<float*>(out) + (int64_t)to * n_row + c, v[0], v[1], v[2], v[3]);
+                    }
+                } else {
+#pragma unroll 1
+                    for (int i0_ = 0; i0_ < NPAD / 2; i0_ += 8) {
+                        Out v[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int x = (i0_ + i) * 32 + lane, r = x / NPAD, c = x % NPAD;
+                            v[i] = ld_shared<Out>(rows + (uint32_t)(r * C::SROW + c * C::ESIZE));
+                        }
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int x = (i0_ + i) * 32 + lane, r = x / NPAD, c = x % NPAD;
+                            const int to = __shfl_sync(0xffffffffu, to_lane, r);
+                            if (to >= 0 && c < n_out) atomicAdd(reinterpret_cast<Out*>(out) + (int64_t)to * n_row + c, v[i]);
+                        }
+                    }
+                }
+                epi_bar();                             // s_dst is read
+            }
+            if (!failed && tid == 0) mbar_arrive(smem_u32(&gfree_bar[b]));     // (behind a barrier of the tile)
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::COLS) : "memory");
+}
+
+template <int NPAD, int NSL>
+int launch(const xrh_adj_sliced_task* tasks, const xrh_dens_sliced_unit* units, int64_t n_units, int32_t* status,
+           cudaStream_t s) {
+    using C = Cfg<NPAD, NSL>;
+    int dev = 0, n_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
+    cudaFuncSetAttribute(adjoint_sliced_kernel<NPAD, NSL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    const int64_t grid = n_units < (int64_t)n_sm * C::CTAS ? n_units : (int64_t)n_sm * C::CTAS;
+    adjoint_sliced_kernel<NPAD, NSL><<<(unsigned)grid, C::THREADS, C::SMEM, s>>>(tasks, units, n_units, status);
+    XRH_CHECK_LAUNCH();
+    return XRH_OK;
+}
+
+}  // namespace
+
+extern "C" int xrh_density_adjoint_sliced_grouped(int precision, const xrh_adj_sliced_task* tasks_dev, int n_tasks,
+                                                  const xrh_dens_sliced_unit* units_dev, int64_t n_units, int npad,
+                                                  int32_t* status_dev, void* stream) {
+    if (n_tasks < 0 || n_units < 0 || (npad != 16 && npad != 32 && npad != 64)) return XRH_ERR_ARG;
+    if (precision != XRH_FP64 && precision != XRH_FP32) return XRH_ERR_UNSUPPORTED;
+    if (n_tasks == 0 || n_units == 0) return XRH_OK;
+    if (!tasks_dev || !units_dev || !status_dev) return XRH_ERR_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (precision == XRH_FP64) {
+        if (npad == 16) return launch<16, 8>(tasks_dev, units_dev, n_units, status_dev, s);
+        if (npad == 32) return launch<32, 8>(tasks_dev, units_dev, n_units, status_dev, s);
+        return launch<64, 8>(tasks_dev, units_dev, n_units, status_dev, s);
+    }
+    if (npad == 16) return launch<16, 6>(tasks_dev, units_dev, n_units, status_dev, s);
+    if (npad == 32) return launch<32, 6>(tasks_dev, units_dev, n_units, status_dev, s);
+    return launch<64, 6>(tasks_dev, units_dev, n_units, status_dev, s);
+}

@@ -16,7 +16,7 @@
 //
 // A CTA (persistent over a work list ordered by length), 16 warps:
 //   * warps 8-11: cp.async gathers of stages of 32 couplings of one sign (positive ones first: the MMA
-//     negates A for the negative ones), published to the async proxy stage by stage;
+//     negates A for the negative ones);
 //   * warp 12: MMAs;  * warps 0-7: collection and conversion.
 // Bounds: the gathers, 2 x 16 NPAD bytes of L2 per coupling, against 640 / 192 / 64 cycles of the tensor
 // pipe per 16 couplings at NPAD = 64 / 32 / 16, and the collection (8 NPAD columns a group).  Measured,
@@ -44,7 +44,6 @@ struct Cfg {
     static constexpr int COLS = NS * NPAD;                             // accumulator columns
     static constexpr uint32_t SIDE = (uint32_t)DS_KS * NS * NPAD * 2;  // bytes of one side of a stage
     static constexpr int STAGES = NPAD == 64 ? 3 : (NPAD == 32 ? 2 : 4);
-    static constexpr int LAG = STAGES - 1;
     static constexpr int CTAS = NPAD == 64 ? 1 : 2;                    // per SM
     // TILES pairs of |d d| <= 2^14 fall on one accumulator: 2^24 / (TILES 2^14) couplings
     static constexpr int GROUP = (1 << 10) / TILES / DS_KS;            // stages per exact group
@@ -82,6 +81,14 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t saddr) {
 __device__ __forceinline__ int stages_of(int n) { return (n + DS_KS - 1) / DS_KS; }
 
 // 16 bytes to shared memory, zeros where ok is false
+// The barrier counts this thread's copies as one arrival once they have landed; their reader, not the
+// thread that issued them, orders them before the MMAs (a proxy fence here would wait for the copies
+// in flight: one gather at a time).
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void fence_copies() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
 __device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
@@ -121,12 +128,12 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
     __shared__ __align__(8) uint64_t ready_bar, drained_bar, done_bar;
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_sh;
-    __shared__ longlong2 s_raw[128][9];
+    __shared__ uint4 s_raw[128][9];
     __shared__ uint32_t s_eb[64], s_ek[64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < C::STAGES; ++s) {
-            mbar_init(smem_u32(&full_bar[s]), DS_PROD / 32);
+            mbar_init(smem_u32(&full_bar[s]), DS_PROD);
             mbar_init(smem_u32(&empty_bar[s]), 1);
         }
         mbar_init(smem_u32(&ready_bar), 1);
@@ -164,6 +171,7 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                     if (in_group == 0 && grp > 0 && !mbar_wait(smem_u32(&drained_bar), (grp - 1) & 1u, &abort_sh)) ok = false;
                     if (ok && !mbar_wait(smem_u32(&full_bar[s]), (st / C::STAGES) & 1u, &abort_sh)) ok = false;
                     if (!ok) break;
+                    fence_copies();
                     tc_fence_after();
                     const uint32_t id = idesc0 | (q >= s_pos ? 1u << 13 : 0u);
                     const uint64_t da = desc_mn_sw128(ring + s * 2 * C::SIDE), db = desc_mn_sw128(ring + s * 2 * C::SIDE + C::SIDE);
@@ -201,11 +209,6 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
         const int pw = warp - 8, side = pw >> 1;
         uint32_t st = 0;
         bool ok = true;
-        auto publish = [&](uint32_t g) {               // this warp's part of stage g has landed
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&full_bar[g % C::STAGES]));
-        };
         for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const xrh_dens_sliced_unit U = units[u];
             const xrh_dens_sliced_task& T = tasks[U.task];
@@ -235,17 +238,12 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                                          (uint32_t)(cc & 7) * 128u + (uint32_t)(((chunk & 7) ^ (cc & 7)) << 4);
                     cp_async16_or_zero(dst, rows + (int64_t)(row < 0 ? 0 : row) * (NS * NPAD * 2) + chunk * 16, row >= 0);
                 }
-                cp_async_commit();
-                if (st >= C::LAG) {
-                    cp_async_wait<C::LAG>();
-                    publish(st - C::LAG);
-                }
+                cp_async_arrive(smem_u32(&full_bar[s]));
             }
         }
+        cp_async_commit();
         cp_async_wait<0>();
-        if (ok) {
-            for (uint32_t g = st > C::LAG ? st - C::LAG : 0; g < st; ++g) publish(g);
-        } else {
+        if (!ok) {
             abort_sh = 1;
             if (lane == 0) atomicExch(status, XRH_ERR_TIMEOUT);
         }
@@ -261,10 +259,9 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
         for (int64_t u = blockIdx.x; u < n_units && !failed; u += gridDim.x) {
             const int np = units[u].n_pos, count = units[u].count;
             const int n_st = stages_of(np) + stages_of(count - np);
-            int64_t hi[C::CW];                         // sum = hi 2^32 + lo
-            uint32_t lo[C::CW];
+            Sum96 sum[C::CW];
 #pragma unroll
-            for (int j = 0; j < C::CW; ++j) hi[j] = lo[j] = 0;
+            for (int j = 0; j < C::CW; ++j) sum[j] = Sum96{0u, 0u, 0u};
             for (int q = 0; q < n_st; q += C::GROUP, ++grp) {
                 if (!failed && !mbar_wait(smem_u32(&ready_bar), grp & 1u, &abort_sh)) {
                     failed = true;
@@ -274,26 +271,14 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                 tc_fence_after();
 #pragma unroll 1
                 for (int b = 0; b < NS; ++b) {
-                    const int w = b + g;
-                    // weights 0..3 at bits 56 - 8 w of T go to hi, 4..7 to the low words, above 7 nowhere
-                    const int mul = w < 4 ? 1 << (8 * (3 - w)) : (w < NS ? 1 << (8 * (NS - 1 - w)) : 0);
-                    const bool low = w >= 4;
                     constexpr int CH = C::CW < 16 ? C::CW : 16;
+                    const int w = b + g;               // above 7: not needed
 #pragma unroll
                     for (int h = 0; h < C::CW; h += CH) {
                         float v[CH];
                         tmem_ld<CH>(tmem + lane_base + (uint32_t)(b * NPAD + part * C::CW + h), v);
-#pragma unroll
-                        for (int j = 0; j < CH; ++j) {
-                            const int64_t t = (int64_t)__float2int_rn(v[j]) * mul;
-                            if (!low) {
-                                hi[h + j] += t;
-                            } else {
-                                const uint32_t l = lo[h + j] + (uint32_t)t;
-                                hi[h + j] += (t >> 32) + (l < (uint32_t)t ? 1 : 0);
-                                lo[h + j] = l;
-                            }
-                        }
+                        if (w < NS) add_weight<CH>(sum + h, v, w);
+                        __syncwarp();                  // (w differs within a warp for NPAD = 16)
                     }
                 }
                 tc_fence_before();
@@ -320,7 +305,7 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                     if (v != p) continue;
 #pragma unroll
                     for (int j = 0; j < 4; ++j)
-                        s_raw[row][part * 4 + j] = make_longlong2(hi[4 * v + j], (long long)lo[4 * v + j]);
+                        s_raw[row][part * 4 + j] = make_uint4(sum[4 * v + j].w0, sum[4 * v + j].w1, sum[4 * v + j].w2, 0u);
                 }
                 epi_bar();
 #pragma unroll
@@ -328,15 +313,16 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                     const int item = e * DS_EPI + tid, slot = item & 7, I = item >> 3;
                     const int J = (slot >> 2) * C::CW + 4 * p + (slot & 3);
                     if (I >= NPAD || i0 + I >= T.nb || j0 + J >= T.nk) continue;
-                    long long h = 0, l = 0;
+                    Sum96 t[1] = {Sum96{0u, 0u, 0u}};
 #pragma unroll
                     for (int k = 0; k < C::G; ++k) {
-                        const longlong2 r = s_raw[k * NPAD + I][slot];
-                        h += r.x;
-                        l += r.y;
+                        const uint4 r = s_raw[k * NPAD + I][slot];
+                        add96(t[0], r.x, r.y, r.z);
                     }
-                    h += l >> 32;
-                    double x = sliced_to_double(h, (uint32_t)l, exp_of(s_eb[I]) + exp_of(s_ek[J]));
+                    const int te[1] = {exp_of(s_eb[I]) + exp_of(s_ek[J])};
+                    double tv[1];
+                    sliced_to_doubles<1>(t, te, tv);
+                    double x = tv[0];
                     if ((s_eb[I] >> 20) >= 2047u || (s_ek[J] >> 20) >= 2047u) {
                         // a state with an infinity or a NaN: the couplings in FP64
                         x = 0.0;
@@ -348,6 +334,7 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                     }
                     T.rhoT[((int64_t)U.idx * T.nb + i0 + I) * T.nk + j0 + J] = x;
                 }
+                __syncwarp();
                 epi_bar();
             }
         }
@@ -406,9 +393,10 @@ __global__ void __launch_bounds__(256) coeff_digits_kernel(const xrh_coeff_digit
             }
         }
         uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(T.digits) +
-                                              ((int64_t)blk * T.n_conf + r0 + r) * (NS * T.npad)) + (o - blk * oct);
+                                              ((int64_t)blk * T.n_conf + r0 + r) * (T.slices * T.npad)) + (o - blk * oct);
 #pragma unroll
         for (int t = 0; t < NS; ++t) {
+            if (t >= T.slices) break;
             uint32_t q[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) q[k] = __byte_perm(digit_float(v[2 * k], t), digit_float(v[2 * k + 1], t), 0x7632);

@@ -47,10 +47,13 @@ constexpr int SL_STAGES = 2;
 constexpr int SL_EPI_WARPS = 8;
 constexpr int SL_EPI_THREADS = SL_EPI_WARPS * 32;
 constexpr int SL_THREADS = SL_EPI_THREADS + 128;       // + a warpgroup: loads, MMA, two idle warps
-// registers: 384 threads x 168 at launch = 64512 = 256 x 208 (epilogue) + 128 x 88
+// registers: 384 threads x 168 at launch = 64512 = 256 x 208 (epilogue) + 128 x 88; 16 epilogue
+// warps of 104 registers spill and are 20 % slower
 constexpr int SL_EPI_REGS = 208, SL_IO_REGS = 88;
 static_assert(SL_EPI_THREADS * SL_EPI_REGS + 128 * SL_IO_REGS <= SL_THREADS * 168, "register split exceeds the launch");
-constexpr int SL_CW = 32;                              // columns per epilogue warp
+constexpr int SL_CW = 64 / (SL_EPI_WARPS / 4);         // columns per epilogue warp
+constexpr int SL_SUB = SL_CW / 8;                      // of them per pass of a flush (8 passes, 8 slots a row)
+constexpr int SL_NEL = 1024 / SL_EPI_THREADS;          // elements a thread converts per pass
 constexpr int NP = NS / 2;                             // weight pairs: the unit handed to the epilogue
 constexpr uint32_t SL_A_SLICE = SL_BM * 64;            // bytes of one slice of a stage
 constexpr uint32_t SL_A_BYTES = NS * SL_A_SLICE;
@@ -213,11 +216,9 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
     __shared__ __align__(8) uint64_t done_bar;
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_sh;
-    __shared__ longlong2 s_raw[SL_BM][9];
-    __shared__ int64_t s_rbase[SL_BM];
-    __shared__ int64_t s_cbase[SL_BM];
+    __shared__ uint4 s_raw[SL_BM][9];
+    __shared__ int64_t s_roff[SL_BM], s_coff[64];      // element (m, n) lies at C[s_roff[m] + s_coff[n]]
     __shared__ double s_DA[SL_BM], s_DB[64];
-    __shared__ int s_rowB[64], s_colB[64];
     __shared__ uint32_t s_eA[SL_BM], s_eB[64];
     __shared__ unsigned char s_diagA[SL_BM], s_diagB[64];
     __shared__ EpiTile s_t;
@@ -363,42 +364,41 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
             }
             const int BN = s_t.BN;
             const bool mine = part * SL_CW < BN;
-            if (s_t.mode == 2) {
+            {
                 const xrh_gemm_task& T = tasks[s_t.task];
+                const bool scatter = s_t.mode == 2;
                 for (int j = tid; j < BN; j += SL_EPI_THREADS) {
                     const int64_t n = s_t.n0 + j;
-                    const bool ok = n < T.N;
-                    s_rowB[j] = ok ? T.rowB[n] : 0;
-                    s_colB[j] = ok ? T.colB[n] : 0;
+                    const bool ok = scatter && n < s_t.N;
+                    s_coff[j] = ok ? (int64_t)T.rowB[n] * s_t.ldc + T.colB[n] : n;
                     s_diagB[j] = ok ? T.diagB[n] : 0;
                     s_DB[j] = (ok && T.DB) ? T.DB[n] : 0.0;
                 }
                 for (int r = tid; r < SL_BM; r += SL_EPI_THREADS) {
                     const int64_t m = s_t.m0 + r;
-                    const bool ok = m < T.M;
-                    s_rbase[r] = ok ? T.rowA[m] : 0;
-                    s_cbase[r] = ok ? T.colA[m] : 0;
+                    const bool ok = scatter && m < s_t.M;
+                    s_roff[r] = ok ? (int64_t)T.rowA[m] * s_t.ldc + T.colA[m] : m * s_t.ldc;
                     s_diagA[r] = ok ? T.diagA[m] : 0;
                     s_DA[r] = (ok && T.DA) ? T.DA[m] : 0.0;
                 }
             }
             bool first = true;                                   // first flush of the tile
-            int64_t hi[SL_CW];                                   // sum = hi 2^32 + lo
-            uint32_t lo[SL_CW];
+            Sum96 sum[SL_CW];
 #pragma unroll
-            for (int j = 0; j < SL_CW; ++j) hi[j] = lo[j] = 0;
+            for (int j = 0; j < SL_CW; ++j) sum[j] = Sum96{0u, 0u, 0u};
             Groups G(s_t.segs, s_t.sb, s_t.left);
             while (G.next()) {
                 const uint32_t ph = (uint32_t)grp & 1u;
                 ++grp;
-                // two rolled loops: the code of a group stays small (an unrolled one does not stay in
-                // the instruction cache beside the flush)
-                auto drain = [&](int p, bool low, int mul) {
+                // a rolled loop over the weight pairs: the code of a group stays small (an unrolled one does
+                // not stay in the instruction cache beside the flush)
+#pragma unroll 1
+                for (int p = 0; p < NP; ++p) {
                     if (!failed && !mbar_wait(smem_u32(&ready_bar[p]), ph, &abort_sh)) {
                         failed = true;
                         abort_sh = 1;
                     }
-                    if (failed) return;
+                    if (failed) break;
                     tc_fence_after();
 #pragma unroll
                     for (int h = 0; h < SL_CW; h += 16) {
@@ -412,26 +412,11 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                             if (lane == 0) mbar_arrive(smem_u32(&drained_bar[p]));
                         }
                         if (mine) {
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                // 32 x 32 + 64 bit multiply-adds
-                                const int64_t t = (int64_t)__float2int_rn(u[j]) * mul +
-                                                  ((int64_t)__float2int_rn(v[j]) * (mul * 256) + (low ? 0 : hi[h + j]));
-                                if (!low) {
-                                    hi[h + j] = t;
-                                } else {
-                                    const uint32_t l = lo[h + j] + (uint32_t)t;
-                                    hi[h + j] += (t >> 32) + (l < (uint32_t)t ? 1 : 0);
-                                    lo[h + j] = l;
-                                }
-                            }
+                            add_weight<16>(sum + h, v, 2 * p);
+                            add_weight<16>(sum + h, u, 2 * p + 1);
                         }
                     }
-                };
-#pragma unroll 1
-                for (int p = 0; p < NP / 2; ++p) drain(p, false, p ? 1 : 65536);
-#pragma unroll 1
-                for (int p = NP / 2; p < NP; ++p) drain(p, true, p == 3 ? 1 : 65536);
+                }
                 if (!G.flush) continue;
                 // one decision of all epilogue warps per flush (also the barrier before s_eB is reused)
                 if (epi_bar_or(failed)) {
@@ -453,33 +438,38 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                 const double alpha = S.alpha;
                 const bool scale = alpha != 1.0;
                 const bool any_bad = epi_bar_or((wa >> 20) >= 2047u || (tid < BN && (s_eB[tid] >> 20) >= 2047u)) != 0;
-                const int slot = lane & 7, rr = warp * 16 + (lane >> 3);         // rows rr, rr + 4, ..
+                const int slot = lane & 7, rr = warp * (4 * SL_NEL) + (lane >> 3);       // rows rr, rr + 4, ..
                 #pragma unroll 1
-                for (int p = 0; p < SL_CW / 4; ++p) {
+                for (int p = 0; p < 8; ++p) {
 #pragma unroll
-                    for (int u = 0; u < SL_CW / 4; ++u) {
+                    for (int u = 0; u < 8; ++u) {
                         if (u != p) continue;
 #pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            s_raw[row][part * 4 + j] = make_longlong2(hi[4 * u + j], (long long)lo[4 * u + j]);
+                        for (int j = 0; j < SL_SUB; ++j)
+                            s_raw[row][part * SL_SUB + j] =
+                                make_uint4(sum[SL_SUB * u + j].w0, sum[SL_SUB * u + j].w1, sum[SL_SUB * u + j].w2, 0u);
                     }
                     epi_bar();
-                    longlong2 raw[4];
+                    Sum96 raw[SL_NEL];
 #pragma unroll
-                    for (int it = 0; it < 4; ++it) raw[it] = s_raw[rr + 4 * it][slot];
+                    for (int it = 0; it < SL_NEL; ++it) {
+                        const uint4 r = s_raw[rr + 4 * it][slot];
+                        raw[it] = Sum96{r.x, r.y, r.z};
+                    }
                     epi_bar();                                   // buffer free
-                    const int jj = (slot >> 2) * SL_CW + 4 * p + (slot & 3);
+                    const int jj = slot / SL_SUB * SL_CW + SL_SUB * p + slot % SL_SUB;
                     if (jj < BN && s_t.n0 + jj < s_t.N) {
                         const uint32_t wb = s_eB[jj];
                         const int eb = exp_of(wb);
-                        double x[4];
+                        double x[SL_NEL];
+                        int te[SL_NEL];
 #pragma unroll
-                        for (int it = 0; it < 4; ++it)
-                            x[it] = sliced_to_double(raw[it].x, (uint32_t)raw[it].y, exp_of(s_eA[rr + 4 * it]) + eb);
+                        for (int it = 0; it < SL_NEL; ++it) te[it] = exp_of(s_eA[rr + 4 * it]) + eb;
+                        sliced_to_doubles<SL_NEL>(raw, te, x);
                         if (any_bad) {
                             // rows or columns with an infinity or a NaN: these K elements in FP64
 #pragma unroll
-                            for (int it = 0; it < 4; ++it) {
+                            for (int it = 0; it < SL_NEL; ++it) {
                                 const int m = s_t.m0 + rr + 4 * it;
                                 if (m >= s_t.M || !((s_eA[rr + 4 * it] >> 20) >= 2047u || (wb >> 20) >= 2047u)) continue;
                                 const double* a = S.A + s_t.batch * S.sA + (int64_t)m * ((S.flags & 1) ? 1 : S.lda);
@@ -494,42 +484,38 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                         }
                         if (scale) {
 #pragma unroll
-                            for (int it = 0; it < 4; ++it) x[it] *= alpha;
+                            for (int it = 0; it < SL_NEL; ++it) x[it] *= alpha;
                         }
-                        double* d[4];
+                        double* d[SL_NEL];
 #pragma unroll
-                        for (int it = 0; it < 4; ++it) d[it] = s_t.C + (int64_t)(s_t.m0 + rr + 4 * it) * s_t.ldc + s_t.n0 + jj;
-                        if (s_t.mode == 2) {
+                        for (int it = 0; it < SL_NEL; ++it) d[it] = s_t.C + s_roff[rr + 4 * it] + s_coff[jj];
+                        if (first && s_t.mode == 2) {
 #pragma unroll
-                            for (int it = 0; it < 4; ++it) {
-                                const int r = rr + 4 * it;
-                                d[it] = s_t.C + (s_rbase[r] + s_rowB[jj]) * s_t.ldc + s_cbase[r] + s_colB[jj];
-                                if (first) {
-                                    if (s_diagB[jj]) x[it] += s_DA[r];
-                                    if (s_diagA[r]) x[it] += s_DB[jj];
-                                }
+                            for (int it = 0; it < SL_NEL; ++it) {
+                                if (s_diagB[jj]) x[it] += s_DA[rr + 4 * it];
+                                if (s_diagA[rr + 4 * it]) x[it] += s_DB[jj];
                             }
                         }
                         if (s_t.mode == 1) {
 #pragma unroll
-                            for (int it = 0; it < 4; ++it)
+                            for (int it = 0; it < SL_NEL; ++it)
                                 if (s_t.m0 + rr + 4 * it < s_t.M) atomicAdd(d[it], x[it]);
                         } else {
                             // later segments add to what the same thread stored for the first one
                             if (!first) {
 #pragma unroll
-                                for (int it = 0; it < 4; ++it)
+                                for (int it = 0; it < SL_NEL; ++it)
                                     if (s_t.m0 + rr + 4 * it < s_t.M) x[it] = *d[it] + x[it];
                             }
 #pragma unroll
-                            for (int it = 0; it < 4; ++it)
+                            for (int it = 0; it < SL_NEL; ++it)
                                 if (s_t.m0 + rr + 4 * it < s_t.M) *d[it] = x[it];
                         }
                     }
                     __syncwarp();
                 }
 #pragma unroll
-                for (int j = 0; j < SL_CW; ++j) hi[j] = lo[j] = 0;
+                for (int j = 0; j < SL_CW; ++j) sum[j] = Sum96{0u, 0u, 0u};
                 first = false;
             }
             if (!failed) epi_bar();                              // metadata reads done before the next tile

@@ -9,13 +9,75 @@ namespace xrh_sliced {
 
 constexpr int NS = XRH_SLICES;
 
-// (hi 2^32 + lo) 2^(x - 68) rounded to FP64 (nearest, ties to even), |hi 2^32 + lo| < 2^94, by about
-// 45 integer operations without a branch (a branch per element serialises the 32 conversions of
-// a thread: 52 000 cycles a tile; the FP64 pipe would need 16 000).  Results outside the normal
-// range are formed by scalbn.
-__device__ __forceinline__ double sliced_to_double(int64_t hi, uint32_t lo, int x) {
-    const uint32_t sg = (uint32_t)(hi >> 63);           // all ones for a negative value
-    uint32_t w0 = lo ^ sg, w1 = (uint32_t)hi ^ sg, w2 = (uint32_t)(hi >> 32) ^ sg;
+// A 96-bit two's complement sum T (w0 lowest).
+struct Sum96 {
+    uint32_t w0, w1, w2;
+};
+
+__device__ __forceinline__ void add96(Sum96& s, uint32_t a0, uint32_t a1, uint32_t a2) {
+    asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+        : "+r"(s.w0), "+r"(s.w1), "+r"(s.w2)
+        : "r"(a0), "r"(a1), "r"(a2));
+}
+
+// s[j] += S_w 256^(7 - w) for the accumulators v[j] of weight w < 8 (integers below 2^24 in magnitude).
+// Conversions (16 lanes/clk/SM) bound it; a 32 x 32 + 64 bit multiply-add also runs at 16 lanes/clk/SM,
+// on another pipe, so the weights that need 64 bits take one and those that need 96 shifts and carries.
+template <int N>
+__device__ __forceinline__ void add_weight(Sum96* s, const float (&v)[N], int w) {
+    const int sh = 8 * (3 - (w & 3));
+    if (w < 4) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const int x = __float2int_rn(v[j]);
+            const uint64_t h = (((uint64_t)s[j].w2 << 32) | s[j].w1) + (uint64_t)((int64_t)x * (1 << sh));
+            s[j].w1 = (uint32_t)h;
+            s[j].w2 = (uint32_t)(h >> 32);
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const int x = __float2int_rn(v[j]);
+            const uint32_t g = (uint32_t)(x >> 31);
+            add96(s[j], (uint32_t)x << sh, __funnelshift_l((uint32_t)x, g, sh), g);
+        }
+    }
+}
+
+// All eight weights of a sum over at most K <= 64 products a pair: T = sum_w v[w] 256^(7 - w).  With
+// |S_w| <= K ((w - 1) 2^14 + 2 * 65 * 128) a sum below 2^22 becomes an integer by an addition on the FP32
+// pipe (1.5 2^23 + S has it in its low bits) instead of a conversion at 16 lanes/clk/SM, and two
+// neighbouring weights fit 32 bits.
+template <int K>
+__device__ __forceinline__ Sum96 collect_weights(const float (&v)[8]) {
+    static_assert(K <= 64, "two weights in 32 bits");
+    int y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (K <= 32 || i < 2) {
+            const uint32_t a = __float_as_uint(v[2 * i] + 12582912.0f), b = __float_as_uint(v[2 * i + 1] + 12582912.0f);
+            y[i] = (int)((a << 8) + b + 0x74c00000u);              // minus 0x4b400000 (256 + 1)
+        } else {
+            y[i] = (int)(((uint32_t)__float2int_rn(v[2 * i]) << 8) + (uint32_t)__float2int_rn(v[2 * i + 1]));
+        }
+    }
+    const int64_t lo = (int64_t)y[2] * 65536 + y[3], hi = (int64_t)y[0] * 65536 + y[1];
+    const uint32_t g = (uint32_t)(lo >> 63);
+    Sum96 s;
+    s.w0 = (uint32_t)lo;
+    const uint64_t h = (uint64_t)hi + (((uint64_t)g << 32) | (uint32_t)(lo >> 32));
+    s.w1 = (uint32_t)h;
+    s.w2 = (uint32_t)(h >> 32);
+    return s;
+}
+
+// T 2^(x - 68) rounded to FP64 (nearest, ties to even), |T| < 2^94, by about 45 integer operations
+// without a branch (a branch per element serialises a thread's conversions; the FP64 pipe, conversions
+// included, runs at 2 lanes/clk/SM).  `rare` is set, and the result is not valid, where it lies outside
+// the normal range (sliced_to_double_rare).
+__device__ __forceinline__ double sliced_to_double_fast(const Sum96& t, int x, bool& rare) {
+    const uint32_t sg = (uint32_t)((int)t.w2 >> 31);    // all ones for a negative value
+    uint32_t w0 = t.w0 ^ sg, w1 = t.w1 ^ sg, w2 = t.w2 ^ sg;
     asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, 0;\n\taddc.u32 %2, %2, 0;"
         : "+r"(w0), "+r"(w1), "+r"(w2)
         : "r"(sg & 1u));
@@ -36,12 +98,28 @@ __device__ __forceinline__ double sliced_to_double(int64_t hi, uint32_t lo, int 
     const int e = 95 - lz + x - 68 + 1023;
     const uint32_t mh = a >> 10, ml = __funnelshift_r(b, a, 10);
     double v = __hiloint2double((int)((mh + ((uint32_t)(e - 1) << 20)) | (sg & 0x80000000u)), (int)ml);
-    if (top == 0u) v = 0.0;
-    else if ((unsigned)(e - 1) >= 2044u) {
-        v = scalbn((double)(((uint64_t)mh << 32) | ml), e - 1075);
-        if (sg) v = -v;
+    rare = rare || (top != 0u && (unsigned)(e - 1) >= 2044u);
+    return top == 0u ? 0.0 : v;
+}
+
+// The same for results that may lie anywhere: two roundings below the normal range, infinite above.
+static __device__ __noinline__ double sliced_to_double_rare(const Sum96& t, int x) {
+    bool rare = false;
+    const int64_t hi = (int64_t)(((uint64_t)t.w2 << 32) | t.w1), mag = hi < 0 ? ~hi : hi;
+    const int bits = 32 + 64 - __clzll(mag | 1);
+    return scalbn(sliced_to_double_fast(t, 68 - bits, rare), x - 68 + bits);
+}
+
+// N sums at once: one branch for all of them, so that their operations interleave.
+template <int N>
+__device__ __forceinline__ void sliced_to_doubles(const Sum96 (&t)[N], const int (&x)[N], double (&v)[N]) {
+    bool rare = false;
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = sliced_to_double_fast(t[i], x[i], rare);
+    if (rare) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] = sliced_to_double_rare(t[i], x[i]);
     }
-    return v;
 }
 
 __device__ __forceinline__ int exp_of(uint32_t hi) {   // |x| < 2^exp_of for the row's largest high word

@@ -315,66 +315,126 @@ def _coupling_units(cp):
     return units, bool((nu > 1).any())
 
 
-class SlicedDensities:
-    """The FP64 coupling-list densities of one builder on the tensor cores
-    (xrh_density_sliced_grouped): digit copies of the state coefficients per charge and side, one unit
-    per operator index with couplings and block of 64 x 64 states, longest first (the CTAs take them
-    in turn, so the long ones do not end up last).
-    blocks: [(couplings, bra side, bra charge, ket side, ket charge, rhoT)]; sides: {side: {charge: zT}}.
-    Operator indices without couplings are never written: rhoT must hold zeros there."""
+class CoeffDigits:
+    """Digit rows of state coefficients for the sliced kernels (xrh_coeff_digits), per side and charge:
+    {(side, charge): (digits, exponent address, zT)}, the common pad width npad and the slices kept."""
 
-    def __init__(self, blocks, sides, device):
-        n_max = max(z.shape[1] for zs in sides.values() for z in zs.values())
+    def __init__(self, sides, device, slices=_lib.SLICES):
+        tabs = [((s, c), z) for s, zs in sides.items() for c, z in zs.items()]
+        n_max = max(z.shape[1] for _, z in tabs)
         self.npad = 16 if n_max <= 16 else 32 if n_max <= 32 else 64
-        tabs = [(s, c, z) for s, zs in sides.items() for c, z in zs.items()]
-        ct = np.zeros(len(tabs), dtype=_lib.COEFF_DIGIT_DTYPE)
-        self.exps = torch.zeros(sum(z.shape[1] for _, _, z in tabs), dtype=torch.int32, device=device)
-        self.digits, at, e0, cta = {}, {}, 0, 0
-        for e, (s, c, z) in zip(ct, tabs):
+        slices = -(-slices * self.npad // 64) * 64 // self.npad            # whole 128-byte row pieces
+        tab = np.zeros(len(tabs), dtype=_lib.COEFF_DIGIT_DTYPE)
+        self.exps = torch.zeros(sum(z.shape[1] for _, z in tabs), dtype=torch.int32, device=device)
+        self.of, e0, cta = {}, 0, 0
+        for e, (key, z) in zip(tab, tabs):
             n_conf, n = z.shape
-            nblk = -(-n // self.npad)
-            d = self.digits[(s, c)] = torch.empty((nblk, max(n_conf, 1), _lib.SLICES, self.npad), dtype=torch.bfloat16,
-                                                  device=device)
-            at[(s, c)] = self.exps.data_ptr() + 4 * e0
-            e["zT"], e["digits"], e["exps"], e["n_conf"] = z.data_ptr(), d.data_ptr(), at[(s, c)], n_conf
-            e["n"], e["npad"], e["cta_begin"] = n, self.npad, cta
+            d = torch.empty((-(-n // self.npad), max(n_conf, 1), slices, self.npad), dtype=torch.bfloat16, device=device)
+            self.of[key] = (d, self.exps.data_ptr() + 4 * e0, z)
+            e["zT"], e["digits"], e["exps"], e["n_conf"] = z.data_ptr(), d.data_ptr(), self.of[key][1], n_conf
+            e["n"], e["npad"], e["slices"], e["cta_begin"] = n, self.npad, slices, cta
             e0 += n
             cta += _lib.lib().xrh_coeff_digit_ctas(n_conf)
-        self.n_coeff, self.coeff_ctas = len(ct), cta
-        tasks = np.zeros(len(blocks), dtype=_lib.DENS_SLICED_TASK_DTYPE)
-        units = []
-        for i, (cp, bs, bc, ks, kc, rhoT) in enumerate(blocks):
-            t, zb, zk = tasks[i], sides[bs][bc], sides[ks][kc]
-            t["P"], t["Q"], t["rhoT"] = cp.P.data_ptr(), cp.Q.data_ptr(), rhoT.data_ptr()
-            t["digb"], t["digk"] = self.digits[(bs, bc)].data_ptr(), self.digits[(ks, kc)].data_ptr()
-            t["eb"], t["ek"], t["zbT"], t["zkT"] = at[(bs, bc)], at[(ks, kc)], zb.data_ptr(), zk.data_ptr()
-            t["conf_b"], t["conf_k"], t["nb"], t["nk"] = zb.shape[0], zk.shape[0], zb.shape[1], zk.shape[1]
-            idx, c0, count, n_pos = cp.ranges()
-            for ib in range(-(-int(t["nb"]) // 64)):
-                for jb in range(-(-int(t["nk"]) // 64)):
-                    un = np.zeros(len(idx), dtype=_lib.DENS_SLICED_UNIT_DTYPE)
-                    un["c0"], un["count"], un["n_pos"] = c0, count, n_pos
-                    un["task"], un["idx"], un["iblk"], un["jblk"] = i, idx, ib, jb
-                    units.append(un)
-        units = np.concatenate(units) if units else np.zeros(0, dtype=_lib.DENS_SLICED_UNIT_DTYPE)
-        units = units[np.argsort(-units["count"], kind="stable")]
-        self.n_tasks, self.n_units = len(tasks), len(units)
-        up = lambda a: torch.from_numpy(np.frombuffer(a.tobytes() or bytes(1), dtype=np.uint8).copy()).to(device)
-        self.coeff_dev, self.tasks_dev, self.units_dev = up(ct), up(tasks), up(units)
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
-        self.keep = (blocks, sides)
+        self.n, self.ctas = len(tab), cta
+        self.dev = torch.from_numpy(tab.view(np.uint8).copy()).to(device)
 
     def run(self, s):
         _lib.zero_(self.exps)
-        call("xrh_coeff_digits", ptr(self.coeff_dev), self.n_coeff, self.coeff_ctas, s)
+        call("xrh_coeff_digits", ptr(self.dev), self.n, self.ctas, s)
+
+    def fill(self, t, bra, ket):
+        """The operand fields of a task between sides bra and ket ((side, charge) keys)."""
+        (db, eb, zb), (dk, ek, zk) = self.of[bra], self.of[ket]
+        t["digb"], t["digk"], t["eb"], t["ek"] = db.data_ptr(), dk.data_ptr(), eb, ek
+        t["zbT"], t["zkT"], t["conf_b"], t["conf_k"] = zb.data_ptr(), zk.data_ptr(), zb.shape[0], zk.shape[0]
+        t["nb"], t["nk"] = zb.shape[1], zk.shape[1]
+
+
+def sliced_units(lists, directions=(0,)):
+    """Work list of the sliced kernels for [(couplings, n_bra, n_ket)] (task i = entry i): a unit per
+    operator index with couplings, block of 64 x 64 states and direction, longest first (the CTAs
+    take them in turn, so the long ones do not end up last); with several directions (gradients, which
+    add up in FP32 on the split paths) task by task instead: sorted over all tasks, the large one-body
+    contributions would come first and every later addition round against them (error of dE/dz of the
+    five-electron states 3.3e-7 instead of 2.1e-7 at 14 orbitals / 60 states).  Direction 1 sets the
+    sign bit of n_pos."""
+    units = [np.zeros(0, dtype=_lib.DENS_SLICED_UNIT_DTYPE)]
+    for i, (cp, nb, nk) in enumerate(lists):
+        idx, c0, count, n_pos = cp.ranges()
+        for ib in range(-(-nb // 64)):
+            for jb in range(-(-nk // 64)):
+                for d in directions:
+                    un = np.zeros(len(idx), dtype=_lib.DENS_SLICED_UNIT_DTYPE)
+                    un["c0"], un["count"] = c0, count
+                    un["n_pos"] = (n_pos.astype(np.uint32) | np.uint32(d << 31)).view(np.int32)
+                    un["task"], un["idx"], un["iblk"], un["jblk"] = i, idx, ib, jb
+                    units.append(un)
+    units = np.concatenate(units)
+    return units[np.lexsort((-units["count"], units["task"] if len(directions) > 1 else 0 * units["task"]))]
+
+
+def _upload(tab, device):
+    return torch.from_numpy(np.frombuffer(tab.tobytes() or bytes(1), dtype=np.uint8).copy()).to(device)
+
+
+class SlicedDensities:
+    """The FP64 coupling-list densities of one builder on the tensor cores (xrh_density_sliced_grouped).
+    blocks: [(couplings, bra key, ket key, rhoT)] with the (side, charge) keys of coeff.  Operator
+    indices without couplings are never written: rhoT must hold zeros there."""
+
+    def __init__(self, blocks, coeff, device):
+        self.coeff, self.keep = coeff, blocks
+        tasks = np.zeros(len(blocks), dtype=_lib.DENS_SLICED_TASK_DTYPE)
+        for t, (cp, bra, ket, rhoT) in zip(tasks, blocks):
+            t["P"], t["Q"], t["rhoT"] = cp.P.data_ptr(), cp.Q.data_ptr(), rhoT.data_ptr()
+            coeff.fill(t, bra, ket)
+        units = sliced_units([(b[0], int(t["nb"]), int(t["nk"])) for b, t in zip(blocks, tasks)])
+        self.n_tasks, self.n_units = len(tasks), len(units)
+        self.tasks_dev, self.units_dev = _upload(tasks, device), _upload(units, device)
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+
+    def run(self, s):
+        self.coeff.run(s)
         call("xrh_density_sliced_grouped", ptr(self.tasks_dev), self.n_tasks, ptr(self.units_dev), self.n_units,
-             self.npad, ptr(self.status), s)
+             self.coeff.npad, ptr(self.status), s)
 
     def check(self):
         """Raise if a bounded device wait gave up (synchronises)."""
         st = int(self.status.item())
         if st != 0:
-            raise _lib.XRHError(f"sliced FP64 densities reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")
+            raise _lib.XRHError(f"sliced densities reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")
+
+
+class SlicedDensityAdjoint:
+    """dE/dz from dE/drho on the tensor cores (xrh_density_adjoint_sliced_grouped) for blocks that share
+    one pad width.  blocks: [(couplings, coeff, bra key, ket key, gT, bra gradient, ket gradient)];
+    refresh: CoeffDigits to run first (those no density build keeps current)."""
+
+    def __init__(self, blocks, precision, refresh, device):
+        self.precision, self.refresh, self.keep = precision, list(refresh), blocks
+        self.npad = blocks[0][1].npad
+        tasks = np.zeros(len(blocks), dtype=_lib.ADJ_SLICED_TASK_DTYPE)
+        for t, (cp, coeff, bra, ket, gT, gzb, gzk) in zip(tasks, blocks):
+            assert coeff.npad == self.npad
+            t["P"], t["Q"], t["gT"] = cp.P.data_ptr(), cp.Q.data_ptr(), gT.data_ptr()
+            t["gzb"], t["gzk"] = gzb.data_ptr(), gzk.data_ptr()
+            coeff.fill(t, bra, ket)
+        units = sliced_units([(b[0], int(t["nb"]), int(t["nk"])) for b, t in zip(blocks, tasks)], (0, 1))
+        self.n_tasks, self.n_units = len(tasks), len(units)
+        self.tasks_dev, self.units_dev = _upload(tasks, device), _upload(units, device)
+        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+
+    def run(self, s):
+        for c in self.refresh:
+            c.run(s)
+        call("xrh_density_adjoint_sliced_grouped", self.precision, ptr(self.tasks_dev), self.n_tasks,
+             ptr(self.units_dev), self.n_units, self.npad, ptr(self.status), s)
+
+    def check(self):
+        """Raise if a bounded device wait gave up (synchronises)."""
+        st = int(self.status.item())
+        if st != 0:
+            raise _lib.XRHError(f"sliced density adjoint reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")
 
 
 class DensityBuilder:
@@ -453,10 +513,10 @@ class DensityBuilder:
         sizes = [(self.n_states_bra[key[1]], self.n_states[key[2]]) for key, _ in direct]
         if not self.f32 and direct and all(min(s) > 0 and sum((x + 3) // 4 * 4 for x in s) <= 400 for s in sizes) and \
                 min(self.n_states.values()) > 0 and min(self.n_states_bra.values()) > 0:
-            kside = "ket" if self.same_bra else "bra"
-            self.sliced = SlicedDensities(
-                [(cp, kside, key[1], "ket", key[2], self._tmp[key]) for key, cp in direct],
-                {"ket": self.zT} if self.same_bra else {"ket": self.zT, "bra": self.zbT}, dev)
+            side = "ket" if self.same_bra else "bra"
+            coeff = CoeffDigits({"ket": self.zT} if self.same_bra else {"ket": self.zT, "bra": self.zbT}, dev)
+            self.sliced = SlicedDensities([(cp, (side, key[1]), ("ket", key[2]), self._tmp[key]) for key, cp in direct],
+                                          coeff, dev)
         self._tr_direct = self._tr_derived = None
         self._mirrors = None
         # FP32 path: coefficients converted once per build, rows padded to 16 bytes

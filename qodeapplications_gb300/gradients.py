@@ -29,6 +29,14 @@ ADJ_UNIT_MAX = 16     # blocks with at most this many states per side use the la
 ORBITAL_FUSED = True  # integral derivatives of the orbital gradient by xrh_orbital_terms
 GAMMA_TC_MIN = 0      # Gamma pair blocks with n * n_K >= this go to the tensor cores (3 x TF32)
 
+def _simt_adjoint_smem(nb, nk):
+    """Shared memory (bytes) of xrh_density_adjoint_f32_grouped: its limit on the state counts."""
+    up = lambda n: (n + 3) // 4 * 4
+    chunk = lambda b, k: max(4, min(128, 4 * (256 // (b // 4 + k // 4))))
+    stage = max(chunk(b, k) * (b + k + 3) for b in range(4, up(nb) + 1, 4) for k in range(4, up(nk) + 1, 4))
+    return 4 * (2 * up(nb) * up(nk) + 2 * stage)
+
+
 class XRDimerAdjoint:
     def __init__(self, plan, density_adjoint="simt", monomer_terms=False, scratch=None):
         """density_adjoint: 'simt' (the grouped CUDA-core kernel) or 'tc' (tensor cores, split-
@@ -414,7 +422,44 @@ class XRDimerAdjoint:
                 self.dens_adj_groups.append((dev_tasks, len(entries), begin,
                                              max(e[5].shape[0] for e in entries), max(e[5].shape[1] for e in entries)))
         else:
-            self._canonicalize()         # the FP64 per-block adjoint
+            self._canonicalize()         # the FP64 adjoint
+        self._setup_sliced()
+
+    def _setup_sliced(self):
+        """The transposed density gradients of self.dens_adj on the tensor cores: every block of the
+        FP64 path (digit rows of the forward builds), and on the FP32 path the blocks of more
+        states than the lane-per-coupling kernel takes (digit rows of 46 bits, made per reverse
+        pass).  State counts the CUDA-core kernels refuse keep their answer."""
+        from .densities import CoeffDigits, SlicedDensityAdjoint
+        plan, dev = self.plan, self.plan.device
+        self.dens_adj_sliced = []
+        entries = [] if self.dens_adj_tc else self.dens_adj
+        if self.prec32:
+            fits = lambda nb, nk: _simt_adjoint_smem(nb, nk) <= 200 * 1024 and max(nb, nk) <= 1024
+        else:
+            fits = lambda nb, nk: 8 * (nb * nk + 64 * (nb + nk)) <= 200 * 1024
+        if not entries or plan.dens_precision == "im" or not all(fits(*e[5].shape[:2]) for e in entries):
+            return
+        coeffs = []
+        for m in (0, 1):
+            b = plan.builders[m]
+            if self.prec32:
+                coeffs.append((CoeffDigits({"ket": b.zT} if b.zbT is b.zT else {"ket": b.zT, "bra": b.zbT}, dev, slices=6)
+                               if any(e[0] == m for e in entries) else None))
+            elif getattr(b, "sliced", None) is None:
+                return
+            else:
+                coeffs.append(b.sliced.coeff)
+        by_pad = {}
+        for (m, op, bc, kc, cp, rt, grho, gT) in entries:
+            c = coeffs[m]
+            bra = ("bra" if ("bra", bc) in c.of else "ket", bc)
+            gz = self.gz32[m] if self.prec32 else {x: self.G[("gzT", m, x)] for x in plan.charges[m]}
+            by_pad.setdefault(c.npad, []).append((cp, c, bra, ("ket", kc), gT, gz[bc], gz[kc]))
+        for blocks in by_pad.values():
+            refresh = list({id(b[1]): b[1] for b in blocks}.values()) if self.prec32 else []
+            self.dens_adj_sliced.append(SlicedDensityAdjoint(blocks, _lib.FP32 if self.prec32 else _lib.FP64, refresh, dev))
+        self.dens_adj_groups = []
 
     def _canonicalize(self, m=None):
         """Entries of self.dens_adj (of fragment m, or all) whose op string has an anticommuting
@@ -472,8 +517,10 @@ class XRDimerAdjoint:
             call("xrh_transpose", ptr(grho), nb * nk, cp.K, ptr(gT), s)
         if self._fold is not None:
             self._fold.run()
+        for sl in self.dens_adj_sliced:
+            sl.run(s)
         for (m, op, bc, kc, cp, rt, grho, gT) in self.dens_adj:
-            if self.prec32:
+            if self.prec32 or self.dens_adj_sliced:
                 break
             nb, nk = rt.shape[0], rt.shape[1]
             bld = plan.builders[m]
@@ -523,7 +570,7 @@ class XRDimerAdjoint:
 
     def check_status(self):
         """Raise if a bounded device wait of the tensor-core launch timed out (syncs)."""
-        for g in (self.L1, self.L2, self.L3, self.Lgamma, self.Lgamma_tc):
+        for g in [self.L1, self.L2, self.L3, self.Lgamma, self.Lgamma_tc] + self.dens_adj_sliced:
             g.check()
         st = int(self.tc_status.item())
         if st != 0:
