@@ -213,6 +213,22 @@ typedef struct {
     int64_t cta_begin;
 } xrh_mirror_task;   /* 48 bytes */
 int xrh_mirror_grouped(const xrh_mirror_task* tasks_dev, int n_tasks, int64_t total_ctas, void* stream);
+/* Three-index density blocks (N <= 64 operators per index) between the [K][R] rows of the coupling-list
+ * kernels (K = N^3 tuples (p, q, r), R = nb nk state pairs) and the [R][K] blocks of the contractions,
+ * with the mirrored block (0: none) of nk x nb states, mirror[(j, i)][(r, q, p)] ~ rho[(i, j)][(p, q, r)].
+ * collect = 0: rho and mirror from rows; anti != 0: the rows with q > r are not read, they are minus
+ * the rows (p, r, q).  collect = 1: rows from rho plus mirror (anti unused).  All tasks have the N of the
+ * call; task t owns CTAs [cta_begin, cta_begin + xrh_density_layout_ctas(collect, N, R)). */
+typedef struct {
+    double* rows;
+    double* rho;
+    double* mirror;
+    int32_t nb, nk, N, anti;
+    int64_t cta_begin;
+} xrh_layout_task;   /* 48 bytes */
+int64_t xrh_density_layout_ctas(int collect, int N, int64_t pairs);
+int xrh_density_layout_grouped(int collect, const xrh_layout_task* tasks_dev, int n_tasks, int64_t total_ctas,
+                               int N, void* stream);
 
 /* Monomer two-electron term without the N^4 density (replaces building rho^ccaa and
  * contracting it, general-XRCC/build_density_tensors.py:122-133 + H_contractions.c:61-78):
@@ -745,6 +761,10 @@ typedef struct {
 } xrh_split_task;   /* 64 bytes */
 int xrh_split_grouped(int precision, const xrh_split_task* tasks_dev, int n_tasks, int64_t total_groups,
                       void* stream);
+/* The same for operands stored transposed, src [K][rows] with row stride ld; group_begin counts tiles of
+ * 32 rows x 64 K (ceil(rows / 32) ceil(Kp / 64) of a task). */
+int xrh_split_trans_grouped(int precision, const xrh_split_task* tasks_dev, int n_tasks, int64_t total_tiles,
+                            void* stream);
 int xrh_tc_encode_map(int precision, const void* base_dev, int64_t rows, int64_t Kp, int box_rows,
                       void* map_out_host);
 int xrh_gemm_tc_grouped(int precision, const xrh_tc_task* tasks_dev, int n_tasks, int64_t total_tiles,

@@ -44,6 +44,9 @@ _SIGS = {
     "xrh_coeff_stage": (_i32, [_vp, _i32, _i64, _vp]),
     "xrh_transpose_grouped": (_i32, [_vp, _i32, _i64, _vp]),
     "xrh_mirror_grouped": (_i32, [_vp, _i32, _i64, _vp]),
+    "xrh_density_layout_ctas": (_i64, [_i32, _i32, _i64]),
+    "xrh_density_layout_grouped": (_i32, [_i32, _vp, _i32, _i64, _i32, _vp]),
+    "xrh_split_trans_grouped": (_i32, [_i32, _vp, _i32, _i64, _vp]),
     "xrh_orbital_terms": (_i32, [_vp, _vp, _vp, _i32, _vp]),
     "xrh_pair_grouped": (_i32, [_i32, _vp, _i32, _i64, _vp]),
     "xrh_gram_grouped": (_i32, [_vp, _i32, _i64, _i32, _vp]),
@@ -143,7 +146,7 @@ class LaunchCounter:
              "xrh_coeff_digits": 2}
     host_only = {"xrh_abi_version", "xrh_status_string", "xrh_last_cuda_error", "xrh_tc_chunk_elems", "xrh_zero",
                  "xrh_tc_encode_map", "xrh_state_ctas", "xrh_abt_ctas", "xrh_lanczos_coop_work",
-                 "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_slice_ctas", "xrh_coeff_digit_ctas"}
+                 "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_density_layout_ctas", "xrh_slice_ctas", "xrh_coeff_digit_ctas"}
     count = 0
 
 
@@ -208,6 +211,9 @@ MIRROR_TASK_DTYPE = np.dtype([("src", np.uint64), ("dst", np.uint64), ("na", np.
                               ("N", np.int32), ("L", np.int32), ("accumulate", np.int32), ("reserved", np.int32),
                               ("cta_begin", np.int64)])
 assert MIRROR_TASK_DTYPE.itemsize == 48
+LAYOUT_TASK_DTYPE = np.dtype([("rows", np.uint64), ("rho", np.uint64), ("mirror", np.uint64), ("nb", np.int32),
+                              ("nk", np.int32), ("N", np.int32), ("anti", np.int32), ("cta_begin", np.int64)])
+assert LAYOUT_TASK_DTYPE.itemsize == 48
 TRANSPOSE_TASK_DTYPE = np.dtype([("in", np.uint64), ("out", np.uint64), ("rows", np.int64), ("cols", np.int64),
                                  ("tile_begin", np.int64)])
 assert TRANSPOSE_TASK_DTYPE.itemsize == 40
@@ -327,6 +333,31 @@ class Mirrors:
     def run(self, stream=None):
         if self.n:
             call("xrh_mirror_grouped", ptr(self.dev), self.n, self.ctas, stream_ptr(stream))
+
+
+class DensityLayout:
+    """A fixed list of three-index density blocks [(rows, rho, mirror or None, nb, nk, anti)] over N
+    operators per index as one xrh_density_layout_grouped launch: rho and mirror from the [K][R] rows, or
+    (collect) the rows from rho plus mirror."""
+
+    def __init__(self, items, N, device, collect=False):
+        import torch
+        tab = np.zeros(len(items), dtype=LAYOUT_TASK_DTYPE)
+        ctas = 0
+        for t, (rows, rho, mirror, nb, nk, anti) in zip(tab, items):
+            for x in (rows, rho, mirror):
+                if x is not None and (x.dtype != torch.float64 or not x.is_contiguous() or x.numel() < nb * nk * N ** 3):
+                    raise ValueError("density layout needs contiguous FP64 blocks of nb nk N^3 elements")
+            t["rows"], t["rho"] = rows.data_ptr(), rho.data_ptr()
+            t["mirror"] = mirror.data_ptr() if mirror is not None else 0
+            t["nb"], t["nk"], t["N"], t["anti"], t["cta_begin"] = nb, nk, N, int(anti), ctas
+            ctas += int(lib().xrh_density_layout_ctas(int(collect), N, nb * nk))
+        self.n, self.ctas, self.N, self.collect, self.keep = len(items), ctas, N, int(collect), items
+        self.dev = torch.from_numpy(tab.view(np.uint8).copy()).to(device) if len(items) else None
+
+    def run(self, stream=None):
+        if self.n:
+            call("xrh_density_layout_grouped", self.collect, ptr(self.dev), self.n, self.ctas, self.N, stream_ptr(stream))
 
 
 class AntisymRows:

@@ -392,6 +392,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 // One thread per group of 4 consecutive K elements of a row (one division per group), one
 // 8- or 16-byte store per group and part.
 template <int KIND>
+__device__ __forceinline__ void split_store(const float (&x)[4], void* __restrict__ hi, void* __restrict__ lo, int64_t o);
+
+template <int KIND>
 __device__ __forceinline__ void split_group(const double* __restrict__ src, int64_t K, int64_t ld, int64_t Kp,
                                             void* __restrict__ hi, void* __restrict__ lo, int64_t t) {
     const int64_t groups = Kp >> 2;
@@ -404,7 +407,11 @@ __device__ __forceinline__ void split_group(const double* __restrict__ src, int6
     float x[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) x[e] = (k0 + e < K) ? xrh_f64_to_f32(__ldg(srow + k0 + e)) : 0.f;
-    const int64_t o = r * Kp + k0;
+    split_store<KIND>(x, hi, lo, r * Kp + k0);
+}
+
+template <int KIND>
+__device__ __forceinline__ void split_store(const float (&x)[4], void* __restrict__ hi, void* __restrict__ lo, int64_t o) {
     if constexpr (KIND == 0) {
         __nv_bfloat16 h[4], l[4];
 #pragma unroll
@@ -460,6 +467,40 @@ __global__ void __launch_bounds__(256) split_grouped_kernel(const xrh_split_task
     }
 }
 
+// Operands stored transposed, src [K][rows]: 32 rows x 64 K per CTA through shared memory, read along
+// the rows, written in 16-byte groups along K (256 bytes a row).  In place of a transposed FP64 copy
+// first: 16 bytes an element through memory instead of 32; bound by memory.
+template <int KIND>
+__global__ void __launch_bounds__(256) split_trans_grouped_kernel(const xrh_split_task* __restrict__ tasks, int n_tasks) {
+    __shared__ __align__(16) double tile[32][66];
+    int lo = 0, hi = n_tasks - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tasks[mid].group_begin <= (int64_t)blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    const xrh_split_task& T = tasks[lo];
+    const int64_t local = (int64_t)blockIdx.x - T.group_begin, tr = (T.rows + 31) / 32;
+    const int64_t r0 = (local % tr) * 32, k0 = (local / tr) * 64;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int64_t k = k0 + warp + 8 * i;
+        v[i] = (k < T.K && r0 + lane < T.rows) ? __ldg(T.src + k * T.ld + r0 + lane) : 0.0;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) tile[lane][warp + 8 * i] = v[i];
+    __syncthreads();
+#pragma unroll
+    for (int item = threadIdx.x; item < 32 * 16; item += 256) {
+        const int r = item >> 4, g = 4 * (item & 15);
+        if (r0 + r >= T.rows || k0 + g >= T.Kp) continue;
+        const double2 a = *reinterpret_cast<const double2*>(&tile[r][g]), b = *reinterpret_cast<const double2*>(&tile[r][g + 2]);
+        const float x[4] = {xrh_f64_to_f32(a.x), xrh_f64_to_f32(a.y), xrh_f64_to_f32(b.x), xrh_f64_to_f32(b.y)};
+        split_store<KIND>(x, T.hi, T.lo, (r0 + r) * T.Kp + k0 + g);
+    }
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     if (!fn) {
@@ -511,6 +552,21 @@ extern "C" int xrh_split_grouped(int precision, const xrh_split_task* tasks_dev,
         split_grouped_kernel<0><<<blocks, 256, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks, total_groups);
     else
         split_grouped_kernel<1><<<blocks, 256, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks, total_groups);
+    XRH_CHECK_LAUNCH();
+    return XRH_OK;
+}
+
+extern "C" int xrh_split_trans_grouped(int precision, const xrh_split_task* tasks_dev, int n_tasks, int64_t total_tiles,
+                                       void* stream) {
+    if (!xrh_tc_chunk_elems(precision)) return XRH_ERR_UNSUPPORTED;
+    if (n_tasks < 0 || total_tiles < 0) return XRH_ERR_ARG;
+    if (n_tasks == 0 || total_tiles == 0) return XRH_OK;
+    if (!tasks_dev) return XRH_ERR_ARG;
+    if (total_tiles > 0x7fffffffLL) return XRH_ERR_CAPACITY;
+    if (precision == XRH_BF16X3)
+        split_trans_grouped_kernel<0><<<(unsigned)total_tiles, 256, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
+    else
+        split_trans_grouped_kernel<1><<<(unsigned)total_tiles, 256, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
     XRH_CHECK_LAUNCH();
     return XRH_OK;
 }

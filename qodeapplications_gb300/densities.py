@@ -484,7 +484,9 @@ class DensityBuilder:
                 arena_off += cp.K * nb * nk
             else:
                 # (the FP64 path writes the operator indices that have couplings only)
-                self._tmp[(op, bc, kc)] = torch.zeros(cp.K * nb * nk, dtype=torch.float64, device=dev)
+                # (a mirrored block comes from its partner and has no rows of its own)
+                if (op, bc, kc) not in self.mirror:
+                    self._tmp[(op, bc, kc)] = torch.zeros(cp.K * nb * nk, dtype=torch.float64, device=dev)
         # canonical lists for the accumulated blocks of op strings with an anticommuting pair (not
         # the warp-per-unit blocks, whose unit tables index the full lists)
         self._canon = {}
@@ -497,7 +499,7 @@ class DensityBuilder:
                 cc = canonical_couplings(space, key)
                 if cc is not None:
                     self._canon[key] = cc
-        self._fill = None
+        self._layout = None
         self.zT = {c: torch.empty((space.n_conf[c], self.n_states[c]), dtype=torch.float64, device=dev)
                    for c in space.charges}
         # the bra side is the ket side unless separate bra states are built (mirror off)
@@ -517,8 +519,6 @@ class DensityBuilder:
             coeff = CoeffDigits({"ket": self.zT} if self.same_bra else {"ket": self.zT, "bra": self.zbT}, dev)
             self.sliced = SlicedDensities([(cp, (side, key[1]), ("ket", key[2]), self._tmp[key]) for key, cp in direct],
                                           coeff, dev)
-        self._tr_direct = self._tr_derived = None
-        self._mirrors = None
         # FP32 path: coefficients converted once per build, rows padded to 16 bytes
         if self.f32:
             pad = lambda n: (n + 3) // 4 * 4
@@ -636,34 +636,31 @@ class DensityBuilder:
                 nb, nk = self.n_states_bra[bc], self.n_states[kc]
                 call("xrh_density_accumulate", self.precision, cp.K, ptr(cp.idx_ptr), ptr(cp.P), ptr(cp.Q),
                      ptr(cp.sign), ptr(self.zbT[bc]), nb, ptr(self.zT[kc]), nk, ptr(self._tmp[(op, bc, kc)]), s)
-        if self._canon:
-            if self._fill is None:
-                self._fill = _lib.AntisymRows(
-                    [(self._tmp[key], self.n_states_bra[key[1]] * self.n_states[key[2]], self.space.N, len(key[0]),
-                      pair_position(key[0])[0], pair_position(key[0])[1]) for key in self._canon], self.space.device)
-            self._fill.run()
-        if self._tr_direct is None:
-            # rho^T [K, nb nk] -> rho [nb nk, K] for the accumulated blocks; the mirrored blocks go
-            # the other way after the mirror kernels (their rho^T feeds the reverse pass)
-            direct, derived = [], []
-            for (op, bc, kc), cp in self.space.couplings.items():
-                nbnk = self.n_states_bra[bc] * self.n_states[kc]
-                tmp, rho = self._tmp[(op, bc, kc)], self.rho[op][(bc, kc)]
-                if (op, bc, kc) in self.mirror:
-                    derived.append((rho, tmp, nbnk, cp.K))
-                else:
-                    direct.append((tmp, rho, cp.K, nbnk))
-            self._tr_direct = _lib.Transposes(direct, self.space.device)
-            self._tr_derived = _lib.Transposes(derived, self.space.device)
-        self._tr_direct.run()
-        if self._mirrors is None:
-            self._mirrors = _lib.Mirrors(
-                [(self.rho[pop][(pbc, pkc)], self.rho[op][(bc, kc)], self.n_states_bra[bc], self.n_states[kc],
-                  self.space.N, len(op), 0) for (op, bc, kc), (pop, pbc, pkc) in self.mirror.items()],
-                self.space.device)
-        self._mirrors.run()
-        self._tr_derived.run()
+        if self._layout is None:
+            self._layout = self._plan_layout()
+        for step in self._layout:
+            step.run()
         return self.rho
+
+    def _plan_layout(self):
+        """rho (and the mirrored blocks) from the accumulated [K, nb nk] rows.  Three-index blocks in
+        one launch; the others, small ones, by row fill, transpose and mirror."""
+        space = self.space
+        partner = {v: k for k, v in self.mirror.items()}
+        wide = {key for key in self._tmp if len(key[0]) == 3 and space.N <= 64 and
+                (key not in self._canon or (key[0] in ANTISYM_PAIR and ANTISYM_PAIR[key[0]] == 1))}
+        size = lambda key: (self.n_states_bra[key[1]], self.n_states[key[2]])
+        rho = lambda key: self.rho[key[0]][key[1:]]
+        fill = [(self._tmp[key], size(key)[0] * size(key)[1], space.N, len(key[0]), *pair_position(key[0])[:2])
+                for key in self._canon if key not in wide]
+        expand = [(self._tmp[key], rho(key), rho(partner[key]) if key in partner else None, *size(key), key in self._canon)
+                  for key in self._tmp if key in wide]
+        flip = [(self._tmp[key], rho(key), space.couplings[key].K, size(key)[0] * size(key)[1])
+                for key in self._tmp if key not in wide]
+        mirrors = [(rho(src), rho(key), *size(key), space.N, len(key[0]), 0)
+                   for key, src in self.mirror.items() if src not in wide]
+        return [_lib.AntisymRows(fill, space.device), _lib.Transposes(flip, space.device),
+                _lib.Mirrors(mirrors, space.device), _lib.DensityLayout(expand, space.N, space.device)]
 
     def check(self):
         """Raise if a bounded device wait of the last builds gave up (synchronises)."""

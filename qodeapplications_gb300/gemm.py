@@ -130,6 +130,16 @@ assert TC_TASK_DTYPE.itemsize == 144 and TC_SEG_DTYPE.itemsize == 32
 TC_BM = 128
 
 
+class Transposed:
+    """An operand stored [K][rows] (base), for SplitRegistry and TCGroupedGemm; its key is not base's."""
+
+    def __init__(self, base):
+        self.base = base
+
+    def data_ptr(self):
+        return -self.base.data_ptr()
+
+
 class SplitRegistry:
     """hi/lo split copies of FP64 operands for the tensor-core path, and their TMA maps.
 
@@ -155,7 +165,11 @@ class SplitRegistry:
             Kp = ((K + self.kch - 1) // self.kch) * self.kch
             hi = torch.zeros((rows, Kp), dtype=self.dtype, device=self.device)
             lo = torch.zeros((rows, Kp), dtype=self.dtype, device=self.device)
-            self.ops[key] = dict(src=t, rows=rows, K=K, ld=ld, Kp=Kp, hi=hi, lo=lo, group=group)
+            src = t.base if isinstance(t, Transposed) else t
+            if src is not t and (src.dtype != torch.float64 or not src.is_contiguous() or
+                                 ld < rows or src.numel() < (K - 1) * ld + rows):
+                raise ValueError("a transposed operand needs contiguous FP64 [K][rows] storage")
+            self.ops[key] = dict(src=src, rows=rows, K=K, ld=ld, Kp=Kp, hi=hi, lo=lo, group=group, trans=src is not t)
         op = self.ops[key]
         assert op["rows"] == rows and op["K"] == K and op["ld"] == ld, "operand registered with another shape"
         return op
@@ -182,19 +196,21 @@ class SplitRegistry:
         after an operand joins the group; not during a graph capture)."""
         s = stream_ptr(stream)
         if group not in self._split_tables:
-            ops = [op for op in self.ops.values() if op["group"] == group]
-            tasks = np.zeros(len(ops), dtype=_lib.SPLIT_TASK_DTYPE)
-            begin = 0
-            for i, op in enumerate(ops):
-                t = tasks[i]
-                t["src"], t["hi"], t["lo"] = op["src"].data_ptr(), op["hi"].data_ptr(), op["lo"].data_ptr()
-                t["rows"], t["K"], t["ld"], t["Kp"], t["group_begin"] = op["rows"], op["K"], op["ld"], op["Kp"], begin
-                begin += op["rows"] * op["Kp"] // 4
-            dev = torch.from_numpy(tasks.view(np.uint8).copy()).to(self.device) if len(ops) else None
-            self._split_tables[group] = (dev, len(ops), begin)
-        dev, n, total = self._split_tables[group]
-        if n:
-            call("xrh_split_grouped", self.prec, ptr(dev), n, total, s)
+            tables = []
+            for trans, fn in ((False, "xrh_split_grouped"), (True, "xrh_split_trans_grouped")):
+                ops = [op for op in self.ops.values() if op["group"] == group and op["trans"] == trans]
+                tasks = np.zeros(len(ops), dtype=_lib.SPLIT_TASK_DTYPE)
+                begin = 0
+                for i, op in enumerate(ops):
+                    t = tasks[i]
+                    t["src"], t["hi"], t["lo"] = op["src"].data_ptr(), op["hi"].data_ptr(), op["lo"].data_ptr()
+                    t["rows"], t["K"], t["ld"], t["Kp"], t["group_begin"] = op["rows"], op["K"], op["ld"], op["Kp"], begin
+                    begin += -(-op["rows"] // 32) * -(-op["Kp"] // 64) if trans else op["rows"] * op["Kp"] // 4
+                if ops:
+                    tables.append((fn, torch.from_numpy(tasks.view(np.uint8).copy()).to(self.device), len(ops), begin))
+            self._split_tables[group] = tables
+        for fn, dev, n, total in self._split_tables[group]:
+            call(fn, self.prec, ptr(dev), n, total, s)
 
 
 _TUNE_CACHE = {}

@@ -21,7 +21,7 @@ import torch
 
 from . import _lib
 from ._lib import call, ptr, stream_ptr
-from .gemm import GroupedGemm, SplitRegistry, TCGroupedGemm
+from .gemm import GroupedGemm, SplitRegistry, TCGroupedGemm, Transposed
 from .hamiltonian import _Arena, _splitk
 
 
@@ -191,41 +191,28 @@ class XRDimerAdjoint:
             for rho_t, wk in segs:
                 writers[rho_t.data_ptr()] = writers.get(rho_t.data_ptr(), 0) + 1
         self.l3_tc = plan.tc
-        self.l3_T = []
-        self._l3_tr = None
-        self._mirror_adj_launch = None
+        self.l3_copies = {}       # contiguous copies of coefficient matrices that are views
+        self._collect = None
         self._gamma_scatter = None
-        self._gam_tr = None
         if plan.tc:
             # tensor cores (split precision, FP32 chunk sums): d rho = dP W on K-major W^T; dW = dP^T rho
-            # on rho^T, which the density build leaves in its pre-transpose buffer
-            rhoT_of = {}
-            for m in (0, 1):
-                b = plan.builders[m]
-                for (op, bc, kc), tmp in b._tmp.items():
-                    rt = b.rho[op][(bc, kc)]
-                    rhoT_of[rt.data_ptr()] = tmp.view(plan.spaces[m].couplings[(op, bc, kc)].K, -1)
+            # on K-major dP^T and rho^T; the transposed operands are split from where they are
             pname = {v: k for k, v in _lib.PRECISIONS.items()}[plan.precision]
             self.reg3 = SplitRegistry(pname, dev)
             L3 = TCGroupedGemm(self.reg3)
-            WT, gPT = {}, {}
             for out, segs in plan.pre_specs:
                 gP = grad_of[out.data_ptr()]
                 M, X = out.shape
-                if gP.data_ptr() not in gPT:
-                    gPT[gP.data_ptr()] = torch.empty((X, M), **f64)
-                    self.l3_T.append((gP, gPT[gP.data_ptr()]))
-                gpt = gPT[gP.data_ptr()]
                 for rho_t, wk in segs:
                     Wt = plan.W[wk]
                     Yk = Wt.shape[1]
-                    if wk not in WT:
-                        WT[wk] = torch.empty((Yk, X), **f64)
-                        self.l3_T.append((Wt, WT[wk]))
+                    if not Wt.is_contiguous():
+                        self.l3_copies.setdefault(wk, (Wt, torch.empty((X, Yk), **f64)))
+                        Wt = self.l3_copies[wk][1]
                     grho = grad_of[rho_t.data_ptr()]
                     mode = 0 if writers[rho_t.data_ptr()] == 1 else 1
-                    L3.add(M, Yk, [(gP, X, WT[wk], X, X, 1.0)], grho, Yk, mode=mode, groups=[("g", "g")])
-                    L3.add(X, Yk, [(gpt, M, rhoT_of[rho_t.data_ptr()], M, M, 1.0)], G[("gW", wk)], Yk, mode=1,
+                    L3.add(M, Yk, [(gP, X, Transposed(Wt), Yk, X, 1.0)], grho, Yk, mode=mode, groups=[("g", "g")])
+                    L3.add(X, Yk, [(Transposed(gP), X, Transposed(rho_t), Yk, M, 1.0)], G[("gW", wk)], Yk, mode=1,
                            groups=[("g", "rhoT")])
             self.reg3.upload()
             self.L3 = L3.finalize().autotune()
@@ -261,7 +248,6 @@ class XRDimerAdjoint:
         Lg = GroupedGemm(dev, gprec)
         self.gam_reg = SplitRegistry("tf32x3", dev)
         Lgt = TCGroupedGemm(self.gam_reg)
-        self.gam_T = []
         self.gam_scatter = []
         for m in (0, 1):
             off = 0
@@ -281,13 +267,10 @@ class XRDimerAdjoint:
                     Gp = self.G[("Gpairs", m)][off:off + npr * npr].view(npr, npr)
                     off += npr * npr
                     if sg.tc and n * nK >= GAMMA_TC_MIN:
-                        # Gamma_c = D^T Dy on the tensor cores (3 x TF32), from K-major transposed
-                        # copies; n states x n_K intermediates is a long K: split-K, FP64 atomics
-                        DT = torch.empty((npr, n * nK), **f64)
-                        DyT = torch.empty((npr, n * nK), **f64)
-                        self.gam_T += [(sg.Dc[k], DT), (Dyc, DyT)]
-                        Lgt.add(npr, npr, [(DT, n * nK, DyT, n * nK, n * nK, 1.0)], Gp, npr, mode=1,
-                                groups=[("gam", "gam")])
+                        # Gamma_c = D^T Dy on the tensor cores (3 x TF32), both split transposed;
+                        # n states x n_K intermediates is a long K: split-K, FP64 atomics
+                        Lgt.add(npr, npr, [(Transposed(sg.Dc[k]), npr, Transposed(Dyc), npr, n * nK, 1.0)], Gp, npr,
+                                mode=1, groups=[("gam", "gam")])
                     else:                 # short K: the SIMT GEMM reads both operands transposed
                         Lg.add(npr, npr, [(sg.Dc[k], npr, Dyc, npr, n * nK, 1.0, 3, 0, 0)], Gp, npr, mode=1,
                                splitk=_splitk(n * nK, 256, 64))
@@ -489,16 +472,28 @@ class XRDimerAdjoint:
     def launch_L3(self):
         """The precontraction adjoint (after launches 1 and 2)."""
         if self.l3_tc:
-            if self._l3_tr is None:
-                flat = [(a, b) for a, b in self.l3_T if a.is_contiguous() and a.dtype == torch.float64]
-                self._l3_tr = _lib.Transposes([(a, b, a.shape[0], a.shape[1]) for a, b in flat], self.plan.device)
-                self._l3_rest = [(a, b) for a, b in self.l3_T if not any(a is x for x, _ in flat)]
-            self._l3_tr.run()
-            for src, dst in self._l3_rest:
-                dst.copy_(src.t())
+            for src, dst in self.l3_copies.values():
+                dst.copy_(src)
             self.reg3.split("g")
             self.reg3.split("rhoT")
         self.L3.run()
+
+    def _plan_collect(self):
+        """The [K, nb nk] rows of the density gradients, mirrored blocks folded in: three-index
+        blocks in one launch per fragment, the others by mirror and transpose."""
+        dev = self.plan.device
+        mirrored = {gdst.data_ptr(): gsrc for (gsrc, gdst, _na, _nb, _N, _L) in self.mirror_adj}
+        wide = [e for e in self.dens_adj if len(e[1]) == 3 and self.plan.N[e[0]] <= 64]
+        taken = {e[6].data_ptr() for e in wide}
+        steps = [_lib.Mirrors([(gsrc, gdst, na, nb, Nm, L, 1) for (gsrc, gdst, na, nb, Nm, L) in self.mirror_adj
+                               if gdst.data_ptr() not in taken], dev),
+                 _lib.Transposes([(e[6], e[7], e[5].shape[0] * e[5].shape[1], e[4].K) for e in self.dens_adj
+                                  if e[6].data_ptr() not in taken], dev)]
+        for m in (0, 1):
+            steps.append(_lib.DensityLayout(
+                [(e[7], e[6], mirrored.get(e[6].data_ptr()), e[5].shape[0], e[5].shape[1], False)
+                 for e in wide if e[0] == m], self.plan.N[m], dev, collect=True))
+        return steps
 
     def launch_density_adjoint(self):
         """dE/dz from the density gradients (after launch 3)."""
@@ -506,15 +501,10 @@ class XRDimerAdjoint:
         s = stream_ptr()
         for (b, grads, gz) in self.im_adj:
             b.adjoint(grads, gz)
-        if self.mirror_adj:
-            if self._mirror_adj_launch is None:
-                self._mirror_adj_launch = _lib.Mirrors(
-                    [(gsrc, gdst, na, nb, Nm, L, 1) for (gsrc, gdst, na, nb, Nm, L) in self.mirror_adj],
-                    self.plan.device)
-            self._mirror_adj_launch.run()
-        for (m, op, bc, kc, cp, rt, grho, gT) in self.dens_adj:
-            nb, nk = rt.shape[0], rt.shape[1]
-            call("xrh_transpose", ptr(grho), nb * nk, cp.K, ptr(gT), s)
+        if self._collect is None:
+            self._collect = self._plan_collect()
+        for step in self._collect:
+            step.run()
         if self._fold is not None:
             self._fold.run()
         for sl in self.dens_adj_sliced:
@@ -549,11 +539,7 @@ class XRDimerAdjoint:
                     [(sg.pl, sg.off_dev, sg.stride_dev, self.G[("YT", m, c)], Dy, sg.n) for (m, c, sg, Dy) in self.gamma_ri],
                     False, self.plan.device)
             self._gamma_scatter.run()
-        if self.gam_T:
-            if self._gam_tr is None:
-                self._gam_tr = _lib.Transposes([(a, b, a.shape[0], a.shape[1]) for a, b in self.gam_T], self.plan.device)
-            self._gam_tr.run()
-            self.gam_reg.split("gam")
+        self.gam_reg.split("gam")
         self.Lgamma.run()
         self.Lgamma_tc.run()
         for (m, idx, vals) in self.gam_scatter:
