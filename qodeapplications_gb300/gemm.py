@@ -80,15 +80,18 @@ class GroupedGemm:
         products = sum(-(-t["M"] // 64) * -(-t["N"] // 64) * 4096 * t["batch"] * K for t, K in long)
         return [t for t, _K in long] if chain >= SLICED_MIN_CHAIN or products >= SLICED_MIN_PRODUCTS else []
 
-    def finalize(self, tile=FP64_TILE):
+    def finalize(self, tile=FP64_TILE, status=None):
         self.sliced = None
         chosen = self._sliced_tasks()
         if chosen:
             self.sliced = SlicedGemm([dict({k: t[k] for k in t if k not in ("seg_begin", "seg_count", "splitk")},
                                            segs=self._segs[t["seg_begin"]:t["seg_begin"] + t["seg_count"]])
-                                      for t in chosen], self.device)
+                                      for t in chosen], self.device, status)
         ids = {id(t) for t in chosen}
         simt = [t for t in self._tasks if id(t) not in ids]
+        self.n_tasks, self.total_tiles = len(simt), 0
+        if not simt and chosen:
+            return self
         tasks = np.zeros(len(simt), dtype=TASK_DTYPE)
         begin = 0
         for i, t in enumerate(simt):
@@ -103,7 +106,6 @@ class GroupedGemm:
         self.tasks_dev = torch.from_numpy(tasks.view(np.uint8).copy()).to(self.device)
         self.segs_dev = torch.from_numpy(segs.view(np.uint8).copy()).to(self.device) if len(segs) else \
             torch.zeros(SEGMENT_DTYPE.itemsize, dtype=torch.uint8, device=self.device)
-        self.n_tasks = len(simt)
         return self
 
     def run(self, stream=None):

@@ -55,83 +55,111 @@ def _spin_block(src, ld_src, frag_sizes, out):
     return out
 
 
-def _pass(X, n, M, out):
-    """out[rest, p] = sum_a X[a, rest] M[a, p] with X of n * rest elements (one GEMM)."""
-    rest = X.numel() // n
-    g = GroupedGemm(X.device)
-    # A = X stored [k = a][m = rest] (flag bit 0), B = M stored [k = a][n = p] (flag bit 1)
-    g.add(rest, n, [(X, rest, M, n, n, 1.0, 3, 0, 0)], out, n, mode=0)
-    g.finalize().run()
-    return out
+def _transform_all(items, status=None):
+    """[(X, batch, mats)] -> transformed arrays: every index of the batch n^k arrays X transformed by
+    its matrix (None for the identity).  The i-th passes of all arrays are one grouped GEMM,
+        Y[rest, p] = sum_a X[a, rest] M[a, p];
+    trailing identities only turn the index order back, one transpose instead of a pass each.  The
+    caller checks `status` (an int32 device word) where it synchronises."""
+    cur, todo = [], []
+    for X, batch, mats in items:
+        n = X.shape[0 if batch is None else 1]
+        if n == 0 or batch == 0:
+            raise RuntimeError("an integral array without elements")
+        last = max((i + 1 for i, M in enumerate(mats) if M is not None), default=0)
+        cur.append(X.contiguous())
+        todo.append((n, batch or 1, len(mats) - last,
+                     [torch.eye(n, dtype=torch.float64, device=X.device) if M is None else M.contiguous() for M in mats[:last]]))
+    for step in range(max((len(t[3]) for t in todo), default=0)):
+        g = GroupedGemm(cur[0].device)
+        for i, (n, batch, _turn, mats) in enumerate(todo):
+            if step >= len(mats):
+                continue
+            X, nxt = cur[i], torch.empty_like(cur[i])
+            size = X.numel() // batch
+            # A = X stored [k = a][m = rest] (flag bit 0), B = M stored [k = a][n = p] (flag bit 1)
+            g.add(size // n, n, [(X, size // n, mats[step], n, n, 1.0, 3, size if batch > 1 else 0, 0)], nxt, n, mode=0,
+                  batch=batch, sC=size if batch > 1 else 0)
+            cur[i] = nxt
+        g.finalize(status=status).run()
+    turns = []
+    for i, (n, batch, turn, _mats) in enumerate(todo):
+        if turn:
+            src, out = cur[i].view(batch, -1), torch.empty_like(cur[i])
+            turns += [(x, y, n ** turn, x.numel() // n ** turn) for x, y in zip(src, out.view(batch, -1))]
+            cur[i] = out
+    if turns:
+        _lib.Transposes(turns, cur[0].device).run()
+    return cur
 
 
 def transform_indices(X, mats):
     """Every index of the n^k array X transformed by its matrix (mats[i] for index i, None
     for the identity): X'[p, q, ...] = sum M0[a, p] M1[b, q] ... X[a, b, ...]."""
-    n = X.shape[0]
-    dev = X.device
-    eye = None
-    cur = X.contiguous()
-    for M in mats:
-        if M is None:
-            if eye is None:
-                eye = torch.eye(n, dtype=torch.float64, device=dev)
-            M = eye
-        nxt = torch.empty_like(cur)
-        _pass(cur, n, M.contiguous(), nxt)
-        cur = nxt.view(cur.shape)
-    return cur
+    return _transform_all([(X, None, mats)])[0]
 
 
-def transform_integrals(M, ints):
+def transform_integrals(M, ints, status=None):
     """The integrals {S, T, U, V} (any subset) in the orbitals transformed by M (n x n):
     every index transformed (the symmetric integrals of orbital_solver.transform_ints)."""
-    out = {}
-    for key, X in ints.items():
-        if X is None:
-            out[key] = None
-        elif key == "U":
-            out[key] = torch.stack([transform_indices(X[k], [M, M]) for k in range(X.shape[0])])
-        else:
-            out[key] = transform_indices(X, [M] * X.dim())
-    return out
+    return _transform_dict({key: (X, [M] * (X.dim() - (key == "U"))) for key, X in ints.items() if X is not None},
+                           ints, status)
+
+
+def _transform_dict(jobs, like, status=None):
+    """{key: (array, mats)} transformed together (U: one matrix per fragment), None for the other keys of like."""
+    done = dict(zip(jobs, _transform_all([(X, X.shape[0] if key == "U" else None, mats)
+                                          for key, (X, mats) in jobs.items()], status)))
+    return {key: done.get(key) for key in like}
 
 
 def inverse_spin_free(S, frag_sizes):
+    """inverse_spin_free_launch, checked (synchronises)."""
+    out, status = inverse_spin_free_launch(S, frag_sizes)
+    _check_inverse(status)
+    return out
+
+
+def _check_inverse(status):
+    if int(status.item()) != 0:
+        raise _lib.XRHError("overlap matrix is singular")
+
+
+def inverse_spin_free_launch(S, frag_sizes):
     """S^-1 of a spin-free spin-orbital overlap (alpha and beta blocks equal, no alpha-beta
     coupling): the inverse of its alpha-alpha block (spatial, <= 64 orbitals), spin-blocked."""
     dev = S.device
     sidx = spin_orbital_spatial_index(frag_sizes)
     spin = _spin_of(frag_sizes)
     n_sp = sum(frag_sizes)
-    alpha = torch.as_tensor(np.array([a for a in range(len(sidx)) if spin[a] == 0], dtype=np.int32), device=dev)
-    # order the alpha spin orbitals by their spatial index
-    order = np.argsort([sidx[a] for a in alpha.cpu().numpy()])
-    alpha = alpha[torch.as_tensor(order, device=dev)].contiguous()
+    # the alpha spin orbitals by their spatial index
+    alpha = sorted((a for a in range(len(sidx)) if spin[a] == 0), key=lambda a: sidx[a])
+    alpha = torch.as_tensor(np.array(alpha, dtype=np.int32), device=dev)
     s_sp = torch.empty((n_sp, n_sp), dtype=torch.float64, device=dev)
     inv_sp = torch.empty_like(s_sp)
     status = torch.zeros(1, dtype=torch.int32, device=dev)
     s = stream_ptr()
     call("xrh_gather_submatrix", n_sp, ptr(alpha), ptr(S), S.shape[1], ptr(s_sp), n_sp, s)
     call("xrh_inverse_small", n_sp, ptr(s_sp), n_sp, ptr(inv_sp), n_sp, ptr(status), s)
-    out = _spin_block(inv_sp, n_sp, frag_sizes, torch.empty_like(S))
-    if int(status.item()) != 0:
-        raise _lib.XRHError("overlap matrix is singular")
-    return out
+    return _spin_block(inv_sp, n_sp, frag_sizes, torch.empty_like(S)), status
 
 
-def biorthogonal_integrals(symm, frag_sizes):
+def biorthogonal_integrals(symm, frag_sizes, status=None):
     """The biorthogonal integrals from the symmetric ones (get_ints.py:62-66,142-143): S^-1
     of symm['S'] contracted into the bra indices of T, U and V.  Returns a dict with S (the
     biorthogonal overlap, the identity up to rounding), T, U, V and Sinv."""
-    Sinv = inverse_spin_free(symm["S"], frag_sizes)
+    Sinv, singular = inverse_spin_free_launch(symm["S"], frag_sizes)
     SinvT = Sinv.t().contiguous()        # pass matrix: M[a, p] = Sinv[p, a]
-    out = {"Sinv": Sinv}
-    out["S"] = transform_indices(symm["S"], [SinvT, None])
-    out["T"] = transform_indices(symm["T"], [SinvT, None])
+    if status is None:
+        status = torch.zeros(1, dtype=torch.int32, device=Sinv.device)
+    jobs = {"S": (symm["S"], [SinvT, None]), "T": (symm["T"], [SinvT, None])}
     if symm.get("U") is not None:
-        out["U"] = torch.stack([transform_indices(symm["U"][k], [SinvT, None]) for k in range(symm["U"].shape[0])])
-    out["V"] = transform_indices(symm["V"], [SinvT, SinvT, None, None])
+        jobs["U"] = (symm["U"], [SinvT, None])
+    jobs["V"] = (symm["V"], [SinvT, SinvT, None, None])
+    out = {"Sinv": Sinv, **_transform_dict(jobs, jobs, status)}
+    _check_inverse(singular)             # one synchronisation, behind everything that was enqueued
+    if int(status.item()) != 0:
+        raise _lib.XRHError("an integral transformation gave up a bounded device wait")
     return out
 
 
@@ -157,6 +185,7 @@ def transform_ints(U_sp, ints, frag_sizes):
     n_so = 2 * sum(frag_sizes)
     Usp = torch.as_tensor(U_sp, dtype=torch.float64, device=dev).contiguous()
     M = _spin_block(Usp, Usp.shape[0], frag_sizes, torch.empty((n_so, n_so), dtype=torch.float64, device=dev))
-    symm = transform_integrals(M, ints)
-    bior = biorthogonal_integrals(symm, frag_sizes)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    symm = transform_integrals(M, ints, status)
+    bior = biorthogonal_integrals(symm, frag_sizes, status)
     return symm, bior

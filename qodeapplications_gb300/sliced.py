@@ -134,16 +134,22 @@ def split_factors(tasks):
     return [max(1, -(-n // per)) if t["mode"] == 1 else 1 for t, n in zip(tasks, stages)]
 
 
+def _table(rows, dtype):
+    """Structured array of rows given as dicts; fields they do not have are zero."""
+    return np.array([tuple(r.get(n, 0) for n in dtype.names) for r in rows], dtype=dtype)
+
+
 class SlicedGemm:
     """tasks: dicts with M, N, mode, C, ldc, batch, sC, mode 2's maps (device addresses) and segs
-    [(A, B, lda, ldb, K, alpha, flags, sA, sB)] (addresses)."""
+    [(A, B, lda, ldb, K, alpha, flags, sA, sB)] (addresses).  status: the int32 device word that a
+    launch sets when a bounded wait gave up (several plans may share one)."""
 
-    def __init__(self, tasks, device):
+    def __init__(self, tasks, device, status=None):
         self.device = device
         waves = plan_waves(tasks)
         self.work = torch.empty(max(w[2] for w in waves) + 1024, dtype=torch.uint8, device=device)
         base = -(-self.work.data_ptr() // 1024) * 1024
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.status = torch.zeros(1, dtype=torch.int32, device=device) if status is None else status
         L = _lib.lib()
         blob, self.waves = bytearray(), []
 
@@ -154,34 +160,27 @@ class SlicedGemm:
             return at
 
         for cur, place, _size, zeroed in waves:
-            st = np.zeros(len(place), dtype=SLICE_TASK_DTYPE)
-            ctas = max_ctas = 0
+            # rows as dicts, then one conversion per table
+            st, ctas, max_ctas = [], 0, 0
             # transposed operands last: their tasks own the CTAs of the row-maximum launch
-            for e, op in zip(st, sorted(place, key=lambda o: o[1])):
+            for op in sorted(place, key=lambda o: o[1]):
                 p, tr, rows, K, ld, batch, sb, block = op
-                e["src"], e["digits"], e["exps"] = p, base + place[op][0], base + place[op][1]
-                e["rows"], e["K"], e["ld"], e["Kp"] = rows, K, ld, _stages(K) * STAGE_K
-                e["batch"], e["sbatch"], e["trans"], e["block"], e["cta_begin"], e["max_begin"] = batch, sb, tr, block, ctas, max_ctas
+                st.append(dict(src=p, digits=base + place[op][0], exps=base + place[op][1], rows=rows, K=K, ld=ld,
+                               Kp=_stages(K) * STAGE_K, batch=batch, sbatch=sb, trans=tr, block=block, cta_begin=ctas,
+                               max_begin=max_ctas))
                 ctas += L.xrh_slice_ctas(rows, K, batch, tr, block, 0)
                 max_ctas += L.xrh_slice_ctas(rows, K, batch, tr, block, 1)
-            gt = np.zeros(len(cur), dtype=TASK_DTYPE)
-            gs = np.zeros(sum(len(t["segs"]) for t in cur), dtype=SLICED_SEG_DTYPE)
-            tiles = k = 0
-            for e, t, sk in zip(gt, cur, split_factors(cur)):
-                for name, v in t.items():
-                    if name != "segs":
-                        e[name] = v
-                e["seg_begin"], e["seg_count"], e["splitk"], e["tile_begin"] = k, len(t["segs"]), sk, tiles
+            gt, gs, tiles = [], [], 0
+            for t, sk in zip(cur, split_factors(cur)):
+                gt.append(dict(t, seg_begin=len(gs), seg_count=len(t["segs"]), splitk=sk, tile_begin=tiles))
                 tiles += _tiles(t) * sk
-                ops = list(_operands(t))
-                for i, (A, B, lda, ldb, K, alpha, flags, sA, sB) in enumerate(t["segs"]):
-                    a, b, s = ops[2 * i], ops[2 * i + 1], gs[k]
-                    s["digA"], s["digB"], s["stages"] = base + place[a][0], base + place[b][0], _stages(K)
-                    s["rA"], s["rB"] = (a[2] if a[5] > 1 else 0), (b[2] if b[5] > 1 else 0)
-                    s["eA"], s["eB"] = base + place[a][1], base + place[b][1]
-                    s["A"], s["B"], s["lda"], s["ldb"], s["K"], s["alpha"] = A, B, lda, ldb, K, alpha
-                    s["flags"], s["sA"], s["sB"] = flags, sA, sB
-                    k += 1
+                ops = _operands(t)
+                for (A, B, lda, ldb, K, alpha, flags, sA, sB), a, b in zip(t["segs"], ops, ops):
+                    gs.append(dict(digA=base + place[a][0], digB=base + place[b][0], stages=_stages(K),
+                                   rA=a[2] if a[5] > 1 else 0, rB=b[2] if b[5] > 1 else 0, eA=base + place[a][1],
+                                   eB=base + place[b][1], A=A, B=B, lda=lda, ldb=ldb, K=K, alpha=alpha, flags=flags,
+                                   sA=sA, sB=sB))
+            st, gt, gs = (_table(rows, dtype) for rows, dtype in ((st, SLICE_TASK_DTYPE), (gt, TASK_DTYPE), (gs, SLICED_SEG_DTYPE)))
             self.waves.append((put(st.tobytes()), len(st), ctas, max_ctas, zeroed, put(gt.tobytes()), len(gt), tiles,
                                put(gs.tobytes())))
         self.tables = torch.frombuffer(blob, dtype=torch.uint8).to(device)

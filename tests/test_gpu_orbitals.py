@@ -113,3 +113,27 @@ def test_transform_ints_biorthogonal():
     np.testing.assert_allclose(bior["V"].cpu().numpy(), Vb, rtol=0, atol=1e-12 * np.abs(Vb).max())
     Ub = np.einsum("pa,kaq->kpq", Sinv, np.einsum("ap,kab,bq->kpq", M, ints["U"], M))
     np.testing.assert_allclose(bior["U"].cpu().numpy(), Ub, rtol=0, atol=1e-12)
+
+
+@pytest.mark.parametrize("n", [1, 7, 24, 33])
+def test_grouped_passes_match_single_ones(n):
+    """Arrays of different index counts, a batch and identities in every place, against einsum in FP64:
+    k chained sums of n products, each within n ulp of sum |x m|."""
+    from qodeapplications_gb300.orbitals import _transform_all, transform_indices
+    g = torch.Generator().manual_seed(n)
+    mk = lambda *s: torch.randn(*s, generator=g, dtype=torch.float64)
+    A, B = mk(n, n), mk(n, n)
+    jobs = [(mk(n, n), None, [A, B]), (mk(3, n, n), 3, [B, None]), (mk(n, n, n), None, [None, A, None]),
+            (mk(n, n, n), None, [None, None, None]), (mk(n, n), None, [None, B])]
+    dev = lambda M: None if M is None else M.cuda()
+    got = _transform_all([(X.cuda(), b, [dev(M) for M in mats]) for X, b, mats in jobs])
+    for (X, batch, mats), out in zip(jobs, got):
+        def apply(Y, f):
+            for M in mats:
+                M = torch.eye(n, dtype=torch.float64) if M is None else f(M)
+                Y = torch.einsum("zar,ap->zrp", Y.reshape(batch or 1, n, -1), M)
+            return Y.reshape(X.shape)
+        ref, size = apply(X, lambda M: M), apply(X.abs(), torch.abs)
+        assert bool(((out.cpu() - ref).abs() <= 4 * n * len(mats) * 2.0 ** -53 * size).all())
+        if batch is None:
+            assert torch.equal(transform_indices(X.cuda(), [dev(M) for M in mats]), out)
