@@ -33,6 +33,7 @@ class GroupedGemm:
         self.tasks_dev = None
         self.segs_dev = None
         self.total_tiles = 0
+        self.sliced = None       # the tasks on the tensor cores (finalize)
         self.flops = 0.0         # algorithmic FLOPs of one launch (2*M*N*K per segment)
 
     def add(self, M, N, segments, C, ldc, mode=0, splitk=1, maps=None, DA=None, DB=None, batch=1, sC=0):

@@ -26,6 +26,9 @@ from .hamiltonian import _Arena, _splitk
 
 
 ADJ_UNIT_MAX = 16     # blocks with at most this many states per side use the lane-per-coupling adjoint
+# Spin orbitals of the system from which V_(1) Gbar_(1)^T runs on the tensor cores in FP64 (whole
+# iterations of 4 states without / with: 48 5.68 / 5.68 ms, 52 8.33 / 8.04, 56 11.35 / 11.07).
+ORBITAL_SLICED_MIN = 50
 ORBITAL_FUSED = True  # integral derivatives of the orbital gradient by xrh_orbital_terms
 GAMMA_TC_MIN = 0      # Gamma pair blocks with n * n_K >= this go to the tensor cores (3 x TF32)
 
@@ -558,6 +561,9 @@ class XRDimerAdjoint:
         """Raise if a bounded device wait of the tensor-core launch timed out (syncs)."""
         for g in [self.L1, self.L2, self.L3, self.Lgamma, self.Lgamma_tc] + self.dens_adj_sliced:
             g.check()
+        orb = getattr(self, "_orb", None)
+        if orb is not None and orb["VG"] is not None:
+            orb["VG"].check()
         st = int(self.tc_status.item())
         if st != 0:
             raise _lib.XRHError(f"tensor-core density adjoint reported status {st}")
@@ -664,6 +670,12 @@ class XRDimerAdjoint:
         # one-electron pieces)
         pairs = [(T, b["dT"], b["Gso"])] + [(U[k], b["dT"], b["Gso"]) for k in range(U.shape[0])]
         b["one_body"] = _one_body_table(pairs, dev)
+        # V_(1) Gbar_(1)^T in FP64: a t x t result over t^3 products, on the tensor cores
+        b["VG"] = None
+        if not self.prec32 and t >= ORBITAL_SLICED_MIN:
+            b["VG"] = GroupedGemm(dev)
+            b["VG"].add(t, t, [(b["A"], t ** 3, b["B"], t ** 3, t ** 3, 0.5)], b["Gso"], t, mode=1)
+            b["VG"].finalize()
         b["inputs"] = self._orbital_inputs()
         self._orb = b
         return b
@@ -726,11 +738,14 @@ class XRDimerAdjoint:
             # real orbitals), so dE/dV may be replaced by its projection on that symmetry; then
             # the four index positions of V' = R^T..R contribute equally: dE/dR = 4 V_(1) Gbar_(1)^T
             # with Gbar = B / 8: a t x t result over t^3 terms, split over CTAs by xrh_abt_small
-            # (FP32 products on the split-precision paths)
+            # (FP32 products on the split-precision paths) or on the tensor cores
             if self.prec32:
                 call("xrh_f64_to_f32", V.numel(), ptr(V), ptr(b["A"]), s)
             K3 = t ** 3
-            call("xrh_abt_small", prec, t, t, K3, ptr(b["A"]), K3, ptr(b["B"]), K3, 0.5, ptr(Gso), s)
+            if b["VG"] is not None:
+                b["VG"].run()
+            else:
+                call("xrh_abt_small", prec, t, t, K3, ptr(b["A"]), K3, ptr(b["B"]), K3, 0.5, ptr(Gso), s)
         if b is None:
             Ga = dV - dV.permute(1, 0, 2, 3) - dV.permute(0, 1, 3, 2) + dV.permute(1, 0, 3, 2)
             Gbar = 0.125 * (Ga + Ga.permute(2, 3, 0, 1))

@@ -305,6 +305,14 @@ def _splitk(K_total, target=384, cap=32):
 
 
 
+# E2 = Zb sigma^T over the determinants: from this many multiply-adds per build on the tensor cores
+# (gemm.py).  Below, xrh_abt_grouped (1.1 TFLOP/s) is as fast: it does not write digits padded to 128 and
+# 64 rows.  Whole FP64 builds without / with: 28 spin orbitals, 20 states (1.0e8) 7.33 / 7.43 ms; 26 and 30
+# (1.5e8) 7.96 / 7.80; 28 and 30 (2.2e8) 10.7 / 10.7; 26 and 45 (3.4e8) 19.0 / 18.4; the terms alone at 28
+# and 60 (8.8e8) 2.00 / 0.50.
+MONO_SLICED_MIN = 1 << 27
+
+
 def _abt_table(entries, device):
     """Task table of xrh_abt_grouped (FP64) for [(m, n, (A, lda, B, ldb, K, alpha), C)], C with
     row stride n; None when empty."""
@@ -511,12 +519,15 @@ class XRDimerPlan:
         # small outputs over long K (E2 = Zb sigma^T, n x n over the determinants): split-K
         # products in one launch instead of 64 x 64 tiles
         abt = [t for t in mono if len(t[2]) == 1 and t[0] <= 64 and t[1] <= 64 and t[4] == t[1]]
+        if sum(t[0] * t[1] * t[2][0][4] for t in abt) >= MONO_SLICED_MIN:
+            abt = []
         mono = [t for t in mono if not any(t is a for a in abt)]
         self.mono_abt = _abt_table([(M_, N_, segs_[0], out_) for (M_, N_, segs_, out_, _l, _s) in abt], dev)
         self.mono_flops += sum(2.0 * M_ * N_ * segs_[0][4] for (M_, N_, segs_, _o, _l, _s) in abt)
         for (M_, N_, segs_, out_, ldc_, sk_) in mono:
             pre.add(M_, N_, segs_, out_, ldc_, mode=1, splitk=sk_)
-        self.pre = pre.finalize()
+        self.tc = self.precision in (_lib.BF16X3, _lib.TF32X3)
+        self.pre = pre if self.tc else pre.finalize()       # (its FLOP count alone with split precision)
 
         # ---- final tasks: one per output charge block ----
         nb = [ns[m] for m in (0, 1)]
@@ -620,10 +631,9 @@ class XRDimerPlan:
                         self.final_tasks.append(dict(key=(ci0, ci1, cj0, cj1), segs=segs, M=M, N=Nn, C=Cbuf, ldc=ldc,
                                                      dims=(ni0, nj0, ni1, nj1),
                                                      maps=(rowA, colA, rowB, colB, diagA, diagB), DA=DA, DB=DB))
-        self.fin = fin.finalize()
+        self.fin = fin if self.tc else fin.finalize()
 
         # ---- split-precision tensor-core variant of both launches ----
-        self.tc = self.precision in (_lib.BF16X3, _lib.TF32X3)
         if self.tc:
             reg = registry if registry is not None else SplitRegistry(precision, dev)
             tag = "%x" % id(self)
