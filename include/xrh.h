@@ -109,6 +109,24 @@ typedef struct {
 int xrh_density_accumulate_f32_grouped(const xrh_dens_task* tasks_dev, int n_tasks, int64_t total_ctas,
                                        int max_nb, int max_nk, void* stream);
 
+/* The same for blocks of more than 128 register tiles of 4 x 4 (ceil(nb / 4) ceil(nk / 4) > 128), with the same
+ * bits; n_pos[idx]: how many couplings of the index, its first ones, have the sign +1.  Task t owns CTAs
+ * [cta_begin, cta_begin + K splits ceil(nb / 64) ceil(nk / 64)). */
+typedef struct {
+    const int64_t* idx_ptr;
+    const int64_t* n_pos;
+    const int32_t* P;
+    const int32_t* Q;
+    const float* zb32;
+    const float* zk32;
+    double* rhoT;
+    int64_t K;
+    int32_t nb, nk;
+    int32_t splits, reserved;
+    int64_t cta_begin;
+} xrh_dens_wide_task;   /* 88 bytes */
+int xrh_density_accumulate_f32_wide(const xrh_dens_wide_task* tasks_dev, int n_tasks, int64_t total_ctas, void* stream);
+
 /* Same product for blocks of at most max_n <= 16 states per side, one warp per unit: unit u
  * covers couplings [idx_ptr[idx] + c_lo, idx_ptr[idx] + c_hi) of operator index idx of task
  * `task` (cta_begin and splits of the tasks are not used).  A unit with c_lo = 0 and c_hi =

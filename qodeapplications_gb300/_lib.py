@@ -25,6 +25,7 @@ _i32, _i64, _vp, _dbl = ctypes.c_int, ctypes.c_longlong, ctypes.c_void_p, ctypes
 _SIGS = {
     "xrh_abi_version": (_i32, []),
     "xrh_density_accumulate_f32_grouped": (_i32, [_vp, _i32, _i64, _i32, _i32, _vp]),
+    "xrh_density_accumulate_f32_wide": (_i32, [_vp, _i32, _i64, _vp]),
     "xrh_density_accumulate_f32_units": (_i32, [_vp, _i32, _vp, _i64, _i32, _vp]),
     "xrh_density_adjoint_f32_grouped": (_i32, [_vp, _i32, _i64, _i32, _i32, _vp]),
     "xrh_density_adjoint_f32_units": (_i32, [_vp, _i32, _vp, _i64, _i32, _i32, _vp]),
@@ -198,6 +199,11 @@ DENS_TASK_DTYPE = np.dtype([("idx_ptr", np.uint64), ("P", np.uint64), ("Q", np.u
                             ("nb", np.int32), ("nk", np.int32), ("splits", np.int32), ("reserved", np.int32),
                             ("cta_begin", np.int64)])
 assert DENS_TASK_DTYPE.itemsize == 88
+DENS_WIDE_TASK_DTYPE = np.dtype([("idx_ptr", np.uint64), ("n_pos", np.uint64), ("P", np.uint64), ("Q", np.uint64),
+                                 ("zb32", np.uint64), ("zk32", np.uint64), ("rhoT", np.uint64), ("K", np.int64),
+                                 ("nb", np.int32), ("nk", np.int32), ("splits", np.int32), ("reserved", np.int32),
+                                 ("cta_begin", np.int64)])
+assert DENS_WIDE_TASK_DTYPE.itemsize == 88
 PAIR_TASK_DTYPE = np.dtype([("X", np.uint64), ("xptr", np.uint64), ("off", np.uint64), ("sign", np.uint64),
                             ("stride", np.uint64), ("src", np.uint64), ("dst", np.uint64), ("count", np.int64),
                             ("n", np.int64)])

@@ -29,6 +29,7 @@ static_assert(sizeof(xrh_gemm_segment) == 72, "xrh_gemm_segment layout is part o
 static_assert(sizeof(xrh_gemm_task) == 152, "xrh_gemm_task layout is part of the ABI");
 static_assert(sizeof(xrh_tc_segment) == 32, "xrh_tc_segment layout is part of the ABI");
 static_assert(sizeof(xrh_dens_task) == 88, "xrh_dens_task layout is part of the ABI");
+static_assert(sizeof(xrh_dens_wide_task) == 88, "xrh_dens_wide_task layout is part of the ABI");
 static_assert(sizeof(xrh_dens_adj_task) == 96, "xrh_dens_adj_task layout is part of the ABI");
 static_assert(sizeof(xrh_dens_adj_tc_task) == 112, "xrh_dens_adj_tc_task layout is part of the ABI");
 static_assert(sizeof(xrh_pair_task) == 72, "xrh_pair_task layout is part of the ABI");
