@@ -15,15 +15,21 @@
 // the segment-independent delta terms are added and the result is scattered like the FP64
 // path.
 //
-// Per CTA (persistent over 128 x BN output tiles, one CTA per SM), 9 warps:
-//   * warp 8, one thread: TMA loads (cp.async.bulk.tensor, 128B swizzle) of the four operand
-//     tiles of a chunk into a 3-stage shared-memory ring, prefetched across tile boundaries,
-//     and the 12 tcgen05.mma of each chunk into one of two TMEM chunk buffers (main +
-//     correction slot, 128 columns each: 512 columns); tcgen05.commit releases the ring stage
-//     (empty) and hands the buffer to the epilogue (ready);
-//   * warps 0-7: per chunk, tcgen05.ld of both slots (warp w reads TMEM lanes 32(w%4).. =
-//     rows, 32-column groups alternate between w<4 and w>=4), add into registers, release the
-//     buffer (drained); at the end of the tile, the FP64 epilogue.
+// Per CTA (persistent over 128 x BN output tiles, one CTA per SM), 18 warps:
+//   * warp 16, one thread: TMA loads (cp.async.bulk.tensor, 128B swizzle) of the four operand
+//     tiles of a chunk into a 3-stage shared-memory ring, prefetched across tile boundaries;
+//   * warp 17, one thread: the 8 tcgen05.mma of each chunk into one of two TMEM chunk buffers (main +
+//     correction slot, 2 BN columns): A_hi x [B_hi; B_lo] goes to both slots at once, then A_lo x B_hi
+//     (12 MMAs of half the width wait longer for their accumulators); tcgen05.commit releases the
+//     ring stage (empty) and hands the buffer to the epilogue (ready);
+//   * warps 0-15: per chunk, tcgen05.ld of both slots (warp w reads TMEM lanes 32(w%4).. = rows, a
+//     quarter of the columns), add into registers, release the buffer (drained); at the end of the
+//     tile, the FP64 epilogue.
+// What bounds it: for short K the store of C, for long K the operand tiles (64 KB a chunk from L2).
+// Measured, TF32 x 3: 3600 x 21952, K = 28 374 -> 227 us (2.6 TB/s of C); 3600 x 3600, K = 784 257 -> 157 us (42
+// bytes/clk/SM of operands; without its drains or a third of its MMAs the same); 1600 x 1120 over 40
+// segments of K = 28 71 -> 45 us; before: one thread for loads and MMAs, 8 epilogue warps that converted on the
+// FP64 pipe and stored 8 bytes a lane behind barriers.
 // Every mbarrier wait is bounded; on timeout the kernel records XRH_ERR_TIMEOUT in *status,
 // every warp leaves its loop (the epilogue warps decide together through bar.red.or once per
 // tile), the producer waits (bounded) for its copies and MMAs in flight, TMEM is freed and the
@@ -40,14 +46,14 @@ using namespace xrh_tc;
 
 constexpr int TC_BM = 128;
 constexpr int TC_STAGES = 3;
-constexpr int TC_EPI_WARPS = 8;
+constexpr int TC_EPI_WARPS = 16;
 constexpr int TC_EPI_THREADS = TC_EPI_WARPS * 32;
-constexpr int TC_THREADS = TC_EPI_THREADS + 32;    // + the producer / MMA warp
+constexpr int TC_THREADS = TC_EPI_THREADS + 64;    // + a warp that loads, a warp that multiplies
+constexpr int TC_TILES = 4;                         // tiles announced to the epilogue
 constexpr uint32_t TC_TMEM_COLS = 512;             // 2 chunk buffers x (main, correction) x 128
 constexpr uint32_t TC_A_BYTES = TC_BM * 128;       // 128 rows x 128 B (one swizzle width of K)
 constexpr uint32_t TC_B_MAX_BYTES = 128 * 128;
 constexpr uint32_t TC_STAGE_BYTES = 2 * TC_A_BYTES + 2 * TC_B_MAX_BYTES;
-constexpr long long TC_IDLE_LIMIT = 1LL << 26;     // producer polls without progress before giving up
 
 // Named barrier 1 over the epilogue warps, returning the OR of a predicate over them.
 __device__ __forceinline__ int epi_bar_or(int pred) {
@@ -60,7 +66,6 @@ __device__ __forceinline__ int epi_bar_or(int pred) {
         : "memory");
     return r;
 }
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(TC_EPI_THREADS) : "memory"); }
 
 __device__ __forceinline__ int find_task(const xrh_tc_task* __restrict__ tasks, int n_tasks, int64_t tile) {
     int lo = 0, hi = n_tasks - 1;
@@ -98,6 +103,7 @@ __device__ __forceinline__ TileInfo tile_info(const xrh_tc_task* __restrict__ ta
         r.n0 = (int)((local % tiles_n) * r.BN);
     }
     int64_t kc_total = 0;
+#pragma unroll 8
     for (int64_t s = 0; s < T.seg_count; ++s) kc_total += segs[T.seg_begin + s].kchunks;
     const int64_t per = (kc_total + T.splitk - 1) / T.splitk;
     r.cb = split * per;
@@ -119,14 +125,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     __shared__ __align__(8) uint64_t done_bar;
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_sh;
-    __shared__ int s_rowB[128], s_colB[128];
-    __shared__ double s_DB[128];
-    // per-row metadata of the tile and the 32-column staging slice of the epilogue
-    __shared__ int64_t s_rbase[128], s_cbase[128];
-    __shared__ double s_DA[128];
-    __shared__ unsigned char s_diagA[128];
-    __shared__ float s_stage[128][33];
-    __shared__ unsigned char s_diagB[128];
+    __shared__ int s_negate[TC_STAGES];                 // of the chunk in a stage
+    // tiles announced by the MMA warp: where, first chunk and number of chunks (0: no more tiles)
+    __shared__ __align__(8) uint64_t tile_bar[TC_TILES];
+    __shared__ TileInfo s_tile[TC_TILES];
+    // element (m, n) of the tile lies at C[s_roff[m] + s_coff[n]]
+    __shared__ int64_t s_roff[128], s_coff[128];
+    __shared__ double s_DA[128], s_DB[128];
+    __shared__ unsigned char s_diagA[128], s_diagB[128];
+    __shared__ __align__(8) float s_stage[TC_EPI_WARPS][16][18];      // 16 x 16 results of a warp, on their way to C
     constexpr int KCH = (KIND == 0) ? 64 : 32;          // elements of K per 128-byte chunk
     constexpr uint32_t FMT = (KIND == 0) ? 1u : 2u;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -140,6 +147,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             mbar_init(smem_u32(&ready_bar[b]), 1);
             mbar_init(smem_u32(&drained_bar[b]), TC_EPI_WARPS);
         }
+        for (int t = 0; t < TC_TILES; ++t) mbar_init(smem_u32(&tile_bar[t]), 1);
         mbar_init(smem_u32(&done_bar), 1);
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -158,139 +166,146 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const uint32_t tmem = tmem_base_sh;
 
     if (warp == TC_EPI_WARPS) {
-        // ------------------------------------------------------------ producer + MMA --
+        // ---------------------------------------------------------------------- loads --
         if (lane == 0) {
-            uint64_t gl = 0, gm = 0;           // chunks loaded / consumed by MMAs (global order)
-            int64_t tl = blockIdx.x, tm = blockIdx.x;
-            int ql = 0, qm = 0;
-            TileInfo L{}, Mi{};
-            bool l_ok = false, m_ok = false;
-            // next tile with at least one chunk, from tile t on
-            auto seek = [&](int64_t& t, TileInfo& I) -> bool {
-                for (; t < total_tiles; t += gridDim.x) {
-                    I = tile_info(tasks, n_tasks, segs, t);
-                    if (I.nk > 0) return true;
-                }
-                return false;
-            };
-            // running (segment, chunk-in-segment) cursors of the loads and the MMAs: a tile's
-            // start is located once (its split-K offset), then each chunk advances the cursor
-            // instead of walking the task's segment list from its first segment again
-            int64_t l_si = 0, l_c = 0, m_si = 0, m_c = 0;
-            l_ok = seek(tl, L);
-            m_ok = seek(tm, Mi);
-            if (l_ok) { l_si = tasks[L.task].seg_begin; l_c = L.cb; }
-            if (m_ok) { m_si = tasks[Mi.task].seg_begin; m_c = Mi.cb; }
+            uint64_t g = 0;                    // chunks loaded
             bool ok = true;
-            // one thread drives both queues without blocking on either: a load is issued as soon
-            // as its ring stage is free, the MMAs of a chunk as soon as its operands have landed
-            // and its TMEM buffer is drained, so that the next chunk's MMAs queue behind the
-            // running ones; a stretch of TC_IDLE_LIMIT polls without progress gives up
-            long long idle = 0;
-            while (m_ok && ok) {
-                bool progress = false;
-                while (l_ok && gl < gm + TC_STAGES) {
-                    const int s = (int)(gl % TC_STAGES);
-                    if (gl >= TC_STAGES && !mbar_test(smem_u32(&empty_bar[s]), (uint32_t)((gl / TC_STAGES) - 1) & 1u))
+            for (int64_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+                const TileInfo I = tile_info(tasks, n_tasks, segs, tile);
+                if (I.nk == 0) continue;
+                const uint32_t b_bytes = (uint32_t)I.BN * 128u;
+                // the tile's first segment is located once (its split-K offset); the next one's fields
+                // are read while this one's chunks are loaded
+                const int64_t seg_end = tasks[I.task].seg_begin + tasks[I.task].seg_count;
+                int64_t si = tasks[I.task].seg_begin, c = I.cb;
+                xrh_tc_segment S = segs[si], nx = si + 1 < seg_end ? segs[si + 1] : S;
+                for (int q = 0; q < I.nk; ++q, ++g) {
+                    while (c >= S.kchunks) {
+                        c -= S.kchunks;
+                        ++si;
+                        S = nx;
+                        if (si + 1 < seg_end) nx = segs[si + 1];
+                    }
+                    const int s = (int)(g % TC_STAGES);
+                    if (g >= TC_STAGES && !mbar_wait(smem_u32(&empty_bar[s]), (uint32_t)(g / TC_STAGES - 1) & 1u, &abort_sh)) {
+                        ok = false;
                         break;
-                    while (l_c >= segs[l_si].kchunks) { l_c -= segs[l_si].kchunks; ++l_si; }
-                    const xrh_tc_segment& S = segs[l_si];
-                    const int kcoord = (int)(l_c * KCH);
-                    ++l_c;
-                    const uint32_t b_bytes = (uint32_t)L.BN * 128u;
+                    }
+                    const int kcoord = (int)(c * KCH);
+                    ++c;
                     uint8_t* st = stages + (size_t)s * TC_STAGE_BYTES;
                     const uint32_t bar = smem_u32(&full_bar[s]);
+                    s_negate[s] = S.negate != 0;
                     mbar_expect_tx(bar, 2u * TC_A_BYTES + 2u * b_bytes);
-                    tma_load_2d(smem_u32(st), maps + S.tmA, bar, kcoord, L.m0);
-                    tma_load_2d(smem_u32(st + TC_A_BYTES), maps + S.tmA + 1, bar, kcoord, L.m0);
-                    tma_load_2d(smem_u32(st + 2 * TC_A_BYTES), maps + S.tmB, bar, kcoord, L.n0);
-                    tma_load_2d(smem_u32(st + 2 * TC_A_BYTES + b_bytes), maps + S.tmB + 1, bar, kcoord, L.n0);
-                    ++gl;
-                    progress = true;
-                    if (++ql == L.nk) {
-                        ql = 0;
-                        tl += gridDim.x;
-                        l_ok = seek(tl, L);
-                        if (l_ok) { l_si = tasks[L.task].seg_begin; l_c = L.cb; }
-                    }
-                }
-                // the MMAs of chunk gm into chunk buffer gm & 1
-                const int s = (int)(gm % TC_STAGES);
-                const uint32_t b = (uint32_t)(gm & 1);
-                if (gm < gl && mbar_test(smem_u32(&full_bar[s]), (uint32_t)(gm / TC_STAGES) & 1u) &&
-                    (gm < 2 || mbar_test(smem_u32(&drained_bar[b]), (uint32_t)((gm >> 1) - 1) & 1u))) {
-                    tc_fence_after();
-                    while (m_c >= segs[m_si].kchunks) { m_c -= segs[m_si].kchunks; ++m_si; }
-                    const uint32_t idesc = make_idesc(FMT, TC_BM, (uint32_t)Mi.BN, segs[m_si].negate != 0);
-                    ++m_c;
-                    const uint32_t b_bytes = (uint32_t)Mi.BN * 128u;
-                    const uint32_t st = smem_u32(stages + (size_t)s * TC_STAGE_BYTES);
-                    const uint64_t da_hi = umma_desc_sw128(st), da_lo = umma_desc_sw128(st + TC_A_BYTES);
-                    const uint64_t db_hi = umma_desc_sw128(st + 2 * TC_A_BYTES);
-                    const uint64_t db_lo = umma_desc_sw128(st + 2 * TC_A_BYTES + b_bytes);
-                    const uint32_t t_main = tmem + b * 256u, t_corr = t_main + 128u;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)              // 4 MMA K-steps of 32 bytes inside the chunk
-                        umma<KIND>(t_main, da_hi + 2 * j, db_hi + 2 * j, idesc, j > 0 ? 1u : 0u);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) umma<KIND>(t_corr, da_hi + 2 * j, db_lo + 2 * j, idesc, j > 0 ? 1u : 0u);
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) umma<KIND>(t_corr, da_lo + 2 * j, db_hi + 2 * j, idesc, 1u);
-                    umma_commit(smem_u32(&empty_bar[s]));
-                    umma_commit(smem_u32(&ready_bar[b]));
-                    ++gm;
-                    progress = true;
-                    if (++qm == Mi.nk) {
-                        qm = 0;
-                        tm += gridDim.x;
-                        m_ok = seek(tm, Mi);
-                        if (m_ok) { m_si = tasks[Mi.task].seg_begin; m_c = Mi.cb; }
-                    }
-                }
-                if (progress) {
-                    idle = 0;
-                } else if (++idle > TC_IDLE_LIMIT || abort_sh) {
-                    ok = false;
+                    tma_load_2d(smem_u32(st), maps + S.tmA, bar, kcoord, I.m0);
+                    tma_load_2d(smem_u32(st + TC_A_BYTES), maps + S.tmA + 1, bar, kcoord, I.m0);
+                    tma_load_2d(smem_u32(st + 2 * TC_A_BYTES), maps + S.tmB, bar, kcoord, I.n0);
+                    tma_load_2d(smem_u32(st + 2 * TC_A_BYTES + b_bytes), maps + S.tmB + 1, bar, kcoord, I.n0);
                 }
             }
             if (!ok) {
                 abort_sh = 1;
                 atomicExch(status, XRH_ERR_TIMEOUT);
             }
-            // before TMEM and shared memory go away: every MMA issued has completed, and every
-            // copy issued has landed (bounded waits)
-            if (gm > 0) {
-                umma_commit(smem_u32(&done_bar));
-                mbar_wait(smem_u32(&done_bar), 0u, nullptr);
+            // every copy issued has landed before shared memory goes away (bounded)
+            for (uint64_t q = g > TC_STAGES ? g - TC_STAGES : 0; q < g; ++q)
+                mbar_wait(smem_u32(&full_bar[q % TC_STAGES]), (uint32_t)(q / TC_STAGES) & 1u, nullptr);
+        }
+    } else if (warp == TC_EPI_WARPS + 1) {
+        // ------------------------------------------------------------------------ MMA --
+        if (lane == 0) {
+            uint64_t g = 0;
+            uint32_t k = 0;                    // tiles announced
+            bool ok = true;
+            // (entry k has been read before its chunk buffers let tile k + 3 begin)
+            auto announce = [&](TileInfo I) {
+                I.cb = (int64_t)g;
+                s_tile[k % TC_TILES] = I;
+                mbar_arrive(smem_u32(&tile_bar[k % TC_TILES]));
+                ++k;
+            };
+            for (int64_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
+                const TileInfo I = tile_info(tasks, n_tasks, segs, tile);
+                if (I.nk == 0) continue;
+                announce(I);
+                const uint32_t bn = (uint32_t)I.BN;
+                for (int q = 0; q < I.nk; ++q, ++g) {
+                    // the MMAs of chunk g into chunk buffer g & 1
+                    const int s = (int)(g % TC_STAGES);
+                    const uint32_t b = (uint32_t)(g & 1);
+                    if (!mbar_wait(smem_u32(&full_bar[s]), (uint32_t)(g / TC_STAGES) & 1u, &abort_sh) ||
+                        (g >= 2 && !mbar_wait(smem_u32(&drained_bar[b]), (uint32_t)((g >> 1) - 1) & 1u, &abort_sh))) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const bool neg = s_negate[s] != 0;
+                    const uint32_t wide = make_idesc(FMT, TC_BM, 2 * bn, neg), narrow = make_idesc(FMT, TC_BM, bn, neg);
+                    const uint32_t st = smem_u32(stages + (size_t)s * TC_STAGE_BYTES);
+                    const uint64_t da_hi = umma_desc_sw128(st), da_lo = umma_desc_sw128(st + TC_A_BYTES);
+                    const uint64_t db = umma_desc_sw128(st + 2 * TC_A_BYTES);
+                    const uint32_t t_main = tmem + b * 256u, t_corr = t_main + bn;
+                    // B_lo lies behind B_hi and the correction slot behind the main one: A_hi times both is
+                    // one MMA a K step (32 bytes), with the same sums in either slot
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) umma<KIND>(t_main, da_hi + 2 * j, db + 2 * j, wide, j > 0 ? 1u : 0u);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) umma<KIND>(t_corr, da_lo + 2 * j, db + 2 * j, narrow, 1u);
+                    umma_commit(smem_u32(&empty_bar[s]));
+                    umma_commit(smem_u32(&ready_bar[b]));
+                }
             }
-            for (uint64_t g = gm; g < gl; ++g)
-                mbar_wait(smem_u32(&full_bar[g % TC_STAGES]), (uint32_t)(g / TC_STAGES) & 1u, nullptr);
+            if (ok) {
+                announce(TileInfo{});
+            } else {
+                abort_sh = 1;
+                atomicExch(status, XRH_ERR_TIMEOUT);
+            }
+            // every MMA issued has completed before TMEM goes away (bounded)
+            umma_commit(smem_u32(&done_bar));
+            mbar_wait(smem_u32(&done_bar), 0u, nullptr);
         }
     } else {
         // ------------------------------------------------------------------ epilogue --
-        const int quarter = warp & 3, half = warp >> 2;      // TMEM lanes 32*quarter.., column half
-        uint64_t ge = 0;
-        bool aborted = false;
-        for (int64_t tile = blockIdx.x; tile < total_tiles && !aborted; tile += gridDim.x) {
-            const TileInfo I = tile_info(tasks, n_tasks, segs, tile);
-            if (I.nk == 0) continue;
+        const int quarter = warp & 3, part = warp >> 2;      // TMEM lanes 32*quarter.., column half
+        for (uint32_t k = 0;; ++k) {
+            const bool here = mbar_wait(smem_u32(&tile_bar[k % TC_TILES]), (k / TC_TILES) & 1u, &abort_sh);
+            const TileInfo I = s_tile[k % TC_TILES];
+            // (also: the metadata of the tile before have been read)
+            if (epi_bar_or(!here)) {
+                abort_sh = 1;
+                if (tid == 0) atomicExch(status, XRH_ERR_TIMEOUT);
+                break;
+            }
+            if (I.nk == 0) break;
+            uint64_t ge = (uint64_t)I.cb;
             const xrh_tc_task& T = tasks[I.task];
             const int BN = I.BN, m0 = I.m0, n0 = I.n0;
-            if (T.mode == 2) {
-                for (int j = tid; j < BN; j += TC_EPI_THREADS) {
-                    const int n = n0 + j;
-                    const bool ok = n < T.N;
-                    s_rowB[j] = ok ? T.rowB[n] : 0;
-                    s_colB[j] = ok ? T.colB[n] : 0;
-                    s_diagB[j] = ok ? T.diagB[n] : 0;
-                    s_DB[j] = (ok && T.DB) ? T.DB[n] : 0.0;
+            // metadata of the tile (the decision barrier below is behind it)
+            {
+                const bool scatter = T.mode == 2;
+                const int64_t ldc = T.ldc;
+                const int M = (int)T.M, N = (int)T.N;
+                for (int x = tid; x < TC_BM + BN; x += TC_EPI_THREADS) {
+                    if (x < TC_BM) {
+                        const int m = m0 + x;
+                        const bool ok = scatter && m < M;
+                        s_roff[x] = ok ? (int64_t)T.rowA[m] * ldc + T.colA[m] : m * ldc;
+                        s_diagA[x] = ok ? T.diagA[m] : 0;
+                        s_DA[x] = (ok && T.DA) ? T.DA[m] : 0.0;
+                    } else {
+                        const int j = x - TC_BM, n = n0 + j;
+                        const bool ok = scatter && n < N;
+                        s_coff[j] = ok ? (int64_t)T.rowB[n] * ldc + T.colB[n] : n;
+                        s_diagB[j] = ok ? T.diagB[n] : 0;
+                        s_DB[j] = (ok && T.DB) ? T.DB[n] : 0.0;
+                    }
                 }
             }
-            float acc[2][32];
+            float acc[32];
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int j = 0; j < 32; ++j) acc[i][j] = 0.f;
+            for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+            const int cw = BN >> 2, cb = part * cw;              // this warp's columns: 8, 16 or 32
             // the warps drain their chunks independently; a wait that gives up raises abort_sh,
             // so the others' waits give up too, and all decide together once per tile below
             bool failed = false;
@@ -303,15 +318,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 }
                 tc_fence_after();
                 const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+                const uint32_t at = tmem + lane_base + b * 256u + (uint32_t)cb;
 #pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const int cc = half * 32 + 64 * i;
-                    if (cc < BN) {
-                        float vm[32], vc[32];
-                        tmem_ld_pair(tmem + lane_base + b * 256u + (uint32_t)cc,
-                                     tmem + lane_base + b * 256u + 128u + (uint32_t)cc, vm, vc);
+                for (int h = 0; h < 32; h += 16) {
+                    if (h < cw) {                                      // uniform
+                        float vm[16], vc[16];
+                        // (8 columns: the 8 behind them are read and not used)
+                        tmem_ld16_pair(at + h, at + h + (uint32_t)BN, vm, vc);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) acc[i][j] += vm[j] + vc[j];
+                        for (int j = 0; j < 16; ++j) acc[h + j] += vm[j] + vc[j];
                     }
                 }
                 tc_fence_before();
@@ -319,65 +334,88 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 if (lane == 0) mbar_arrive(smem_u32(&drained_bar[b]));
             }
             // one collective decision per tile (also the barrier after the column metadata)
-            if (epi_bar_or(failed)) aborted = true;
-            if (aborted) {
+            if (epi_bar_or(failed)) {
                 abort_sh = 1;
                 if (tid == 0) atomicExch(status, XRH_ERR_TIMEOUT);
                 break;
             }
-            // FP64 epilogue, one 32-column slice at a time: the 4 warps that hold the slice put it
-            // into shared memory (a row per lane), then every warp writes 16 rows with its lanes
-            // on consecutive columns, so that stores (and atomics) of a warp touch few cache
-            // lines.  Column metadata came before the decision barrier; row metadata first:
-            for (int rr = tid; rr < TC_BM; rr += TC_EPI_THREADS) {
-                const int m = m0 + rr;
-                int64_t rb = 0, cb2 = 0;
-                unsigned char dgA = 0;
-                double dam = 0.0;
-                if (m < T.M) {
-                    if (T.mode == 2) {
-                        rb = T.rowA[m];
-                        cb2 = T.colA[m];
-                        dgA = T.diagA[m];
-                        dam = T.DA ? T.DA[m] : 0.0;
-                    } else {
-                        rb = (int64_t)m * T.ldc;
-                    }
-                }
-                s_rbase[rr] = rb;
-                s_cbase[rr] = cb2;
-                s_diagA[rr] = dgA;
-                s_DA[rr] = dam;
-            }
+            // FP64 epilogue, 16 rows x 16 columns of a warp at a time, without the other warps: through its
+            // own shared memory to lanes on pairs of columns, four rows an instruction.  16-byte stores
+            // reach 6.7 TB/s here, 8-byte ones 4.4.  FP32 to FP64 by integer operations (the FP64 pipe
+            // converts 2 lanes/clk/SM).
             double* C = T.C;
+            const int mode = (int)T.mode, N = (int)T.N;
+            const int64_t ldc = T.ldc;
+            // a tile inside a plain matrix of 16-byte rows: no bounds, no offsets
+            const bool whole = mode == 0 && m0 + TC_BM <= T.M && n0 + BN <= N && (ldc & 1) == 0 &&
+                               (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+            const int col = 2 * (lane & 7), r_lane = lane >> 3;
+#pragma unroll 1
+            for (int p = 0; p < 4; ++p) {                              // columns 16 (p >> 1).., rows 16 (p & 1)..
+                if (16 * (p >> 1) >= cw) break;                        // uniform
+                if ((lane >> 4) == (p & 1)) {
+                    // (selected value by value: an array indexed at run time would lie in local memory)
 #pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                const int c0 = 32 * p;
-                if (c0 >= BN) break;                                   // uniform
-                if (half == (p & 1)) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) s_stage[quarter * 32 + lane][j] = acc[p >> 1][j];
+                    for (int j = 0; j < 16; ++j) s_stage[warp][lane & 15][j] = p < 2 ? acc[j] : acc[16 + j];
                 }
-                epi_bar();
-                const int jj = c0 + lane;
-                const bool col_ok = n0 + jj < T.N;
-                for (int rr = warp * 16; rr < warp * 16 + 16; ++rr) {
-                    if (m0 + rr >= T.M) break;                         // uniform within the warp
-                    if (!col_ok) continue;
-                    double x = (double)s_stage[rr][lane];
-                    if (T.mode == 2) {
-                        if (s_diagB[jj]) x += s_DA[rr];
-                        if (s_diagA[rr]) x += s_DB[jj];
-                        C[(s_rbase[rr] + s_rowB[jj]) * T.ldc + s_cbase[rr] + s_colB[jj]] = x;
-                    } else if (T.mode == 0) {
-                        C[s_rbase[rr] + n0 + jj] = x;
+                __syncwarp();
+                const int jc = 16 * (p >> 1) + col, jj = cb + jc, row0 = quarter * 32 + 16 * (p & 1) + r_lane;
+                if (jc < cw && n0 + jj < N) {
+                    float f[8];
+                    double x[8];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 v = *reinterpret_cast<const float2*>(&s_stage[warp][r_lane + 4 * i][col]);
+                        f[2 * i] = v.x;
+                        f[2 * i + 1] = v.y;
+                    }
+                    xrh_f32_to_f64s(f, x);
+                    if (mode == 2) {
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const bool diag_col = s_diagB[jj + e];
+                            const double db = s_DB[jj + e];
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                if (diag_col) x[2 * i + e] += s_DA[row0 + 4 * i];
+                                if (s_diagA[row0 + 4 * i]) x[2 * i + e] += db;
+                            }
+                        }
+                    }
+                    if (whole) {
+                        double* d0 = C + (int64_t)(m0 + row0) * ldc + n0 + jj;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            *reinterpret_cast<double2*>(d0 + 4 * i * ldc) = make_double2(x[2 * i], x[2 * i + 1]);
                     } else {
-                        atomicAdd(C + s_rbase[rr] + n0 + jj, x);
+                        const int64_t o0 = s_coff[jj], o1 = s_coff[jj + 1];
+                        const bool two = n0 + jj + 1 < N, pair = two && o1 == o0 + 1;
+                        const int left = (int)T.M - m0 - row0;             // rows from this lane's first one on
+                        double* d[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) d[i] = C + o0 + s_roff[row0 + 4 * i];
+                        if (mode == 1) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                if (4 * i < left) atomicAdd(d[i], x[2 * i]);
+                                if (4 * i < left && two) atomicAdd(d[i] + (o1 - o0), x[2 * i + 1]);
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i) {
+                                if (4 * i >= left) continue;
+                                if (pair && (reinterpret_cast<uintptr_t>(d[i]) & 15) == 0) {
+                                    *reinterpret_cast<double2*>(d[i]) = make_double2(x[2 * i], x[2 * i + 1]);
+                                } else {
+                                    *d[i] = x[2 * i];
+                                    if (two) d[i][o1 - o0] = x[2 * i + 1];
+                                }
+                            }
+                        }
                     }
                 }
-                epi_bar();                                             // slice consumed
+                __syncwarp();
             }
-            epi_bar();          // metadata reads done before the next tile overwrites it
         }
     }
     tc_fence_before();

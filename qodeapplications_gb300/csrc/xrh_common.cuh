@@ -87,6 +87,24 @@ __device__ __forceinline__ double xrh_f32_to_f64(float f) {
     return __longlong_as_double((long long)bits);
 }
 
+// The same for N numbers at once: zeros by selection, one branch for all subnormal, infinite and NaN ones
+// (a branch a number serialises the conversions).
+template <int N>
+__device__ __forceinline__ void xrh_f32_to_f64s(const float (&f)[N], double (&x)[N]) {
+    bool odd = false;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const uint32_t u = __float_as_uint(f[i]), m = u & 0x7fffffffu;
+        const uint32_t hi = (u & 0x80000000u) | (m == 0u ? 0u : (m >> 3) + 0x38000000u);
+        odd = odd || (m != 0u && m - 0x00800000u >= 0x7f000000u);
+        x[i] = __hiloint2double((int)hi, (int)(u << 29));
+    }
+    if (odd) {
+#pragma unroll
+        for (int i = 0; i < N; ++i) x[i] = (double)f[i];
+    }
+}
+
 // FP64 -> FP32 round-to-nearest-even by integer operations (same result as __double2float_rn;
 // zero takes a shortcut, values outside the normal FP32 range the hardware conversion).
 __device__ __forceinline__ float xrh_f64_to_f32(double x) {
