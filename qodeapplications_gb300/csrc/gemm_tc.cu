@@ -26,7 +26,7 @@
 //     quarter of the columns), add into registers, release the buffer (drained); at the end of the
 //     tile, the FP64 epilogue.
 // What bounds it: for short K the store of C, for long K the operand tiles (64 KB a chunk from L2).
-// Measured, TF32 x 3: 3600 x 21952, K = 28 374 -> 227 us (2.6 TB/s of C); 3600 x 3600, K = 784 257 -> 157 us (42
+// Measured, TF32 x 3: 3600 x 21952, K = 28 374 -> 227 us (2.8 TB/s of C); 3600 x 3600, K = 784 257 -> 157 us (42
 // bytes/clk/SM of operands; without its drains or a third of its MMAs the same); 1600 x 1120 over 40
 // segments of K = 28 71 -> 45 us; before: one thread for loads and MMAs, 8 epilogue warps that converted on the
 // FP64 pipe and stored 8 bytes a lane behind barriers.
