@@ -684,6 +684,19 @@ typedef struct {
     int64_t n;
 } xrh_pair_task;   /* 72 bytes */
 int xrh_pair_grouped(int gather, const xrh_pair_task* tasks_dev, int n_tasks, int64_t max_total, void* stream);
+/* The scatter by destination, one task per spin class: dst[s][e] = sign src[X][s] for the class's entries
+ * e = K n_p + pair, inv[e] = sign (X + 1), 0 where no determinant has the pair (dst 0).  Task t owns
+ * CTAs [cta_begin, cta_begin + xrh_pair_rows_ctas(entries, n)). */
+typedef struct {
+    const int32_t* inv;
+    const double* src;
+    double* dst;
+    int64_t entries;
+    int64_t n;
+    int64_t cta_begin;
+} xrh_pair_rows_task;   /* 48 bytes */
+int64_t xrh_pair_rows_ctas(int64_t entries, int64_t n);
+int xrh_pair_rows_grouped(const xrh_pair_rows_task* tasks_dev, int n_tasks, int64_t total_ctas, void* stream);
 
 /* Transition densities through intermediate determinants K (no reference counterpart; they
  * replace the per-coupling outer products of density_tensors.c:142-556 on the split-precision

@@ -49,6 +49,8 @@ _SIGS = {
     "xrh_density_layout_grouped": (_i32, [_i32, _vp, _i32, _i64, _i32, _vp]),
     "xrh_split_trans_grouped": (_i32, [_i32, _vp, _i32, _i64, _vp]),
     "xrh_orbital_terms": (_i32, [_vp, _vp, _vp, _i32, _vp]),
+    "xrh_pair_rows_ctas": (_i64, [_i64, _i64]),
+    "xrh_pair_rows_grouped": (_i32, [_vp, _i32, _i64, _vp]),
     "xrh_pair_grouped": (_i32, [_i32, _vp, _i32, _i64, _vp]),
     "xrh_gram_grouped": (_i32, [_vp, _i32, _i64, _i32, _vp]),
     "xrh_tangent_step": (_i32, [_vp, _i32, _i64, _dbl, _vp, _vp]),
@@ -147,7 +149,7 @@ class LaunchCounter:
              "xrh_coeff_digits": 2}
     host_only = {"xrh_abi_version", "xrh_status_string", "xrh_last_cuda_error", "xrh_tc_chunk_elems", "xrh_zero",
                  "xrh_tc_encode_map", "xrh_state_ctas", "xrh_abt_ctas", "xrh_lanczos_coop_work",
-                 "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_density_layout_ctas", "xrh_slice_ctas", "xrh_coeff_digit_ctas"}
+                 "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_density_layout_ctas", "xrh_pair_rows_ctas", "xrh_slice_ctas", "xrh_coeff_digit_ctas"}
     count = 0
 
 
@@ -392,12 +394,45 @@ class AntisymRows:
             call("xrh_antisym_rows", ptr(self.dev), self.n, self.ctas, stream_ptr(stream))
 
 
+PAIR_ROWS_TASK_DTYPE = np.dtype([("inv", np.uint64), ("src", np.uint64), ("dst", np.uint64), ("entries", np.int64),
+                                 ("n", np.int64), ("cta_begin", np.int64)])
+assert PAIR_ROWS_TASK_DTYPE.itemsize == 48
+
+
+def _pair_inverse(pl, device):
+    """Per class of a pair list, its inverse: sign (X + 1) of every (K, pair), 0 where there is none; kept."""
+    import torch
+    if "inverse" not in pl:
+        at = np.array([cl["base"] for cl in pl["classes"]], dtype=np.int64)[pl["cls"]]
+        at = at + pl["k"] * np.array([cl["n_p"] for cl in pl["classes"]], dtype=np.int64)[pl["cls"]] + pl["p"]
+        inv = np.zeros(max(int(pl["L"]), 1), dtype=np.int32)
+        inv[at] = (pl["X"].astype(np.int64) + 1) * pl["sign"]
+        pl["inverse"] = torch.from_numpy(inv).to(device)
+    return pl["inverse"]
+
+
 class PairLaunch:
     """A fixed list of pair scatters (gather=False: (pl, off, stride, zT, D, n)) or gathers
-    (gather=True: (pl, off, stride, E, sigmaT, n)) run as one xrh_pair_grouped launch."""
+    (gather=True: (pl, off, stride, E, sigmaT, n)) run as one xrh_pair_grouped launch.  Scatters of
+    lists that hold a quarter or more of the (K, pair) positions run by destination
+    (xrh_pair_rows_grouped): below, writing every position moves more than the list's sectors."""
 
     def __init__(self, items, gather, device):
         import torch
+        rows, ctas = [], 0
+        if not gather:
+            by_rows = [it for it in items if 4 * len(it[0]["X"]) >= it[0]["L"] > 0]
+            for pl, _off, _stride, src, dst, n in by_rows:
+                inv = _pair_inverse(pl, device)
+                for cl in pl["classes"]:
+                    size = cl["n_K"] * cl["n_p"]
+                    rows.append((inv.data_ptr() + 4 * cl["base"], src.data_ptr(), dst.data_ptr() + 8 * n * cl["base"],
+                                 size, n, ctas))
+                    ctas += int(lib().xrh_pair_rows_ctas(size, n))
+            self.keep_rows = by_rows
+            items = [it for it in items if not any(it is x for x in by_rows)]
+        self.rows = (torch.from_numpy(np.array(rows, dtype=PAIR_ROWS_TASK_DTYPE).view(np.uint8).copy()).to(device),
+                     len(rows), ctas) if rows else None
         tab = np.zeros(len(items), dtype=PAIR_TASK_DTYPE)
         mx = 0
         for i, (pl, off, stride, src, dst, n) in enumerate(items):
@@ -411,6 +446,8 @@ class PairLaunch:
         self.dev = torch.from_numpy(tab.view(np.uint8).copy()).to(device) if len(items) else None
 
     def run(self, stream=None):
+        if self.rows is not None:
+            call("xrh_pair_rows_grouped", ptr(self.rows[0]), self.rows[1], self.rows[2], stream_ptr(stream))
         if self.n:
             call("xrh_pair_grouped", self.gather, ptr(self.dev), self.n, self.max_total, stream_ptr(stream))
 

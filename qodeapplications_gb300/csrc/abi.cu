@@ -32,6 +32,7 @@ static_assert(sizeof(xrh_dens_task) == 88, "xrh_dens_task layout is part of the 
 static_assert(sizeof(xrh_dens_wide_task) == 88, "xrh_dens_wide_task layout is part of the ABI");
 static_assert(sizeof(xrh_dens_adj_task) == 96, "xrh_dens_adj_task layout is part of the ABI");
 static_assert(sizeof(xrh_dens_adj_tc_task) == 112, "xrh_dens_adj_tc_task layout is part of the ABI");
+static_assert(sizeof(xrh_pair_rows_task) == 48, "xrh_pair_rows_task layout is part of the ABI");
 static_assert(sizeof(xrh_pair_task) == 72, "xrh_pair_task layout is part of the ABI");
 static_assert(sizeof(xrh_orbital_inputs) == 128, "xrh_orbital_inputs layout is part of the ABI");
 static_assert(sizeof(xrh_mirror_task) == 48, "xrh_mirror_task layout is part of the ABI");
