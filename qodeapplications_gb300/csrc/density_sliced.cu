@@ -20,9 +20,9 @@
 //   * warp 12: MMAs;  * warps 0-7: collection and conversion.
 // Bounds: the gathers, 2 x 16 NPAD bytes of L2 per coupling, against 640 / 192 / 64 cycles of the tensor
 // pipe per 16 couplings at NPAD = 64 / 32 / 16, and the collection (8 NPAD columns a group).  Measured,
-// all blocks of a fragment of 28 spin orbitals: 60 states 115 -> 8.3 ms (97 GFLOP of canonical
-// couplings, 12 TFLOP/s FP64 against the pipe's 1.1), 32 states 2.2, 16 states 1.4; 18 spin orbitals, 10
-// states 3.4 -> 0.13 ms.
+// all blocks of a fragment of 28 spin orbitals: 60 states 115 -> 4.9 ms (97 GFLOP of canonical
+// couplings, 20 TFLOP/s FP64 against the pipe's 1.1), 32 states 1.74, 16 states 1.09; 18 spin orbitals, 10
+// states 3.4 -> 0.086 ms.
 // Every wait is bounded; on timeout *status is set and all roles leave after their copies and MMAs
 // have completed.
 #include "sliced_common.cuh"
