@@ -321,13 +321,16 @@ int xrh_gemm_simt_grouped(int precision, const xrh_gemm_task* tasks_dev, int n_t
  * row r of an operand is scaled by the power of two above its largest element and written as
  * XRH_SLICES balanced base-256 digits (integers in [-128, 128], held in BF16): the row in
  * 62-bit fixed point.  Products of digits are summed in FP32 accumulators that stay below 2^24,
- * so exactly, for every digit pair (i, j) with i + j < XRH_SLICES; the sums are collected in 64-bit
- * integers and rounded once per segment to FP64.  Rows with infinities or NaN are recognised and
- * their results formed by FP64 arithmetic from the operands themselves.
+ * so exactly, for every digit pair (i, j) with i + j < XRH_SLICES; the sums are collected in 96-bit
+ * integers and rounded once per segment to FP64: an error of at most K 1.003 2^-59 2^(ea + eb) for row
+ * exponents ea, eb.  Elements for which that could exceed the bound of an FP64 sum, K 2^-53 sum |a||b|
+ * (found by a product of the elements' magnitudes), and rows with infinities or NaN are formed by
+ * FP64 arithmetic from the operands themselves.
  *   xrh_slice_grouped: digits of many operands.  The rows of each batch step are padded to blocks of
  *       `block` rows (128 for an A operand, 64 or 32 for a B operand); digits_dev holds, for every
  *       block and every 32 K, the shared-memory image of one pipeline stage: [XRH_SLICES][block][32]
- *       BF16 in 64-byte swizzle (16-byte aligned); Kp is K rounded up to 32.  exps_dev[batch * rows]
+ *       BF16 in 64-byte swizzle (16-byte aligned), and behind those of a block the magnitudes
+ *       |a| 2^-e, [Kp / 32][block][32] BF16 in the same form; Kp is K rounded up to 32.  exps_dev[batch * rows]
  *       receives the high word of the largest |element| of each row.  Element (b, r, k) of the source
  *       is src[b * sbatch + r * ld + k], or src[b * sbatch + k * ld + r] with trans = 1 (then exps_dev
  *       must be zero on entry).  A task owns xrh_slice_ctas(.., 0) CTAs of the launch from cta_begin

@@ -5,12 +5,22 @@
 // Oishi and Rump, Numer. Algorithms 59, 95 (2012)): a row x of an operand with |x| < 2^e is the
 // integer V = round(x 2^(62 - e)), written in balanced base-256 digits V = sum_t d_t 256^(7 - t),
 // |d_t| <= 128, |d_0| <= 65, each digit exact in BF16.  With S_w = sum_(i+j=w) sum_k d_i(a_k) d_j(b_k),
-//     sum_k a_k b_k = 2^(ea + eb - 68) sum_(w<8) S_w 256^(7 - w)   (+ terms below 2^-63 of the
-//     largest product),
-// 36 digit pairs.  |d_i d_j| <= 2^14 and a weight has at most 8 pairs, so 128 K elements keep every
-// FP32 accumulator at or below 2^24, where integers are exact: the order and the rounding of the
-// tensor core's additions do not matter.  The eight sums of such a group go into two 64-bit integers
-// per output element and are rounded to FP64 once per segment.
+//     sum_k a_k b_k = 2^(ea + eb - 68) sum_(w<8) S_w 256^(7 - w)   (+ what the 36 digit pairs leave out)
+// |d_i d_j| <= 2^14 and a weight has at most 8 pairs, so 128 K elements keep every FP32 accumulator at or
+// below 2^24, where integers are exact: the order and the rounding of the tensor core's additions do
+// not matter.  The eight sums of such a group go into one 96-bit integer per output element, rounded
+// to FP64 once per segment.
+//
+// Error: an element within 2^-9 of its row's largest is represented exactly, a smaller one to 2^-63
+// of 2^e, and the pairs with i + j >= 8 left out are below 2^-59.1 2^(ea + eb) a product: K 1.003 2^-59 2^(ea + eb)
+// in all, K 2^-62 as a rule.  That is relative to the largest elements of the row and the column, an
+// FP64 sum's K 2^-53 sum |a||b| to the products themselves.  So a ninth image holds the magnitudes of
+// the elements as BF16 numbers, one more MMA a K step gives sum |a||b| from below, and the elements where
+// the first bound could exceed the second (low_sum: rows that span many orders of magnitude, whose
+// large elements meet zeros or small ones) are formed by FP64 FMAs from the operands, as those of
+// rows with infinities and NaN are.  Rows of one size have none of them; the magnitudes cost 3 % at
+// 3 600 x 21 952 x 28, the spin blocks and near identities of an integral transformation of 28 spin
+// orbitals 15 % (2.8 -> 3.2 ms; CUDA cores 15.4).
 //
 // What bounds it: 36 pairs of BF16 MMAs are 2 304 cycles of the tensor pipe per 128 x 64 x 32 stage; the
 // integer collection of a group (8 x 8 192 conversions) and the flush of a tile (about 25 000 cycles)
@@ -18,16 +28,13 @@
 // (CUDA cores: 1.0); 3 600 x 784 x 784 0.22 + 0.03 ms digits against 4.65 ms; one tile of 128 K 27 us
 // against 160 us.
 //
-// Error: an element within 2^-9 of its row's largest is represented exactly, smaller ones to 2^-63
-// of the largest; there is no rounding per product or per addition, so a result is closer to the
-// exact sum than an FP64 FMA chain of more than a few terms.
-//
 // Per CTA (persistent over 128 x BN tiles, BN = 64, or 32 for N <= 32), 12 warps:
-//   * warp 8: bulk copies of all eight slices of A and B for 32 K (96 KB: two stages); the digits lie
-//     in global memory as the swizzled shared-memory image of a stage, so a stage is two contiguous
-//     copies;
+//   * warp 8: bulk copies of all eight slices of A and B for 32 K (96 KB: two stages), at the end of a
+//     segment of the magnitudes of 256 K; the digits lie in global memory as the swizzled shared-memory
+//     image of a stage, so a stage is two contiguous copies;
 //   * warp 9: the tcgen05.mma of a stage into eight TMEM accumulators (weight w at column BN w; see
-//     stage_mmas), handed to the epilogue in pairs of weights, the next group starting behind it;
+//     stage_mmas), handed to the epilogue in pairs of weights, the next group starting behind it; the
+//     products of the magnitudes on the first pair's accumulators once they are drained;
 //   * warps 0-7: tcgen05.ld of two weights (32 columns a warp), integer accumulation, release; at the
 //     end of a segment conversion by integer operations (the FP64 pipe is needed only for alpha
 //     and for additions) and the store, scatter or atomic epilogue through shared memory.
@@ -59,7 +66,7 @@ constexpr uint32_t SL_A_SLICE = SL_BM * 64;            // bytes of one slice of 
 constexpr uint32_t SL_A_BYTES = NS * SL_A_SLICE;
 constexpr uint32_t SL_B_BYTES = NS * 64 * 64;
 constexpr uint32_t SL_STAGE_BYTES = SL_A_BYTES + SL_B_BYTES;
-constexpr int SL_RUN_GROUPS = 4096;                    // groups collected in 64 bits before a flush (< 2^93)
+constexpr int SL_RUN_GROUPS = 4096;                    // groups collected in 96 bits before a flush (< 2^93)
 static_assert(NS == 8, "digit weights and shifts below are written for eight slices");
 static_assert((long long)SL_GROUP * SL_KS * NS * (1 << 14) <= (1 << 24), "a group must stay exact in FP32");
 
@@ -117,7 +124,7 @@ __device__ __forceinline__ Tile tile_of(const xrh_gemm_task* __restrict__ tasks,
     return r;
 }
 
-// What the epilogue needs of its tile, in shared memory: its registers hold 32 x 2 64-bit sums.
+// What the epilogue needs of its tile, in shared memory: its registers hold 32 96-bit sums.
 struct EpiTile {
     double* C;
     const xrh_sliced_segment* segs;
@@ -206,6 +213,17 @@ __device__ __forceinline__ bool stage_mmas(uint32_t tmem, uint64_t dA, uint64_t 
     return true;
 }
 
+// The K elements [k0, k1) of row m and column n by FP64 FMAs (at 2 a clock and SM the loads hide behind them).
+__device__ __forceinline__ double fp64_product(const xrh_sliced_segment& S, int64_t batch, int m, int n, int64_t k0, int64_t k1) {
+    const double* a = S.A + batch * S.sA + (int64_t)m * ((S.flags & 1) ? 1 : S.lda);
+    const double* b = S.B + batch * S.sB + (int64_t)n * ((S.flags & 2) ? 1 : S.ldb);
+    const int64_t ka = (S.flags & 1) ? S.lda : 1, kb = (S.flags & 2) ? S.ldb : 1;
+    double y = 0.0;
+#pragma unroll 4
+    for (int64_t k = k0; k < k1; ++k) y = fma(a[k * ka], b[k * kb], y);
+    return y;
+}
+
 __global__ void __launch_bounds__(SL_THREADS, 1)
     gemm_sliced_kernel(const xrh_gemm_task* __restrict__ tasks, int n_tasks, int64_t total_tiles,
                        const xrh_sliced_segment* __restrict__ segs, int32_t* status) {
@@ -213,6 +231,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
     uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __align__(8) uint64_t full_bar[SL_STAGES], empty_bar[SL_STAGES];
     __shared__ __align__(8) uint64_t ready_bar[NP], drained_bar[NP];
+    __shared__ __align__(8) uint64_t mag_ready_bar, mag_drained_bar;
     __shared__ __align__(8) uint64_t done_bar;
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_sh;
@@ -220,7 +239,9 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
     __shared__ int64_t s_roff[SL_BM], s_coff[64];      // element (m, n) lies at C[s_roff[m] + s_coff[n]]
     __shared__ double s_DA[SL_BM], s_DB[64];
     __shared__ uint32_t s_eA[SL_BM], s_eB[64];
+    __shared__ uint32_t s_low[SL_EPI_WARPS / 4][SL_BM];
     __shared__ unsigned char s_diagA[SL_BM], s_diagB[64];
+    __shared__ int s_count;                            // elements to form in FP64
     __shared__ EpiTile s_t;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -233,6 +254,8 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
             mbar_init(smem_u32(&ready_bar[w]), 1);
             mbar_init(smem_u32(&drained_bar[w]), SL_EPI_WARPS);
         }
+        mbar_init(smem_u32(&mag_ready_bar), 1);
+        mbar_init(smem_u32(&mag_drained_bar), SL_EPI_WARPS);
         mbar_init(smem_u32(&done_bar), 1);
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -264,21 +287,27 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                     const xrh_sliced_segment& S = G.segs[G.si];
                     const int64_t blk_a = I.batch * ((S.rA + SL_BM - 1) / SL_BM) + I.m0 / SL_BM;
                     const int64_t blk_b = I.batch * ((S.rB + I.BN - 1) / I.BN) + I.n0 / I.BN;
-                    const uint8_t* pa = reinterpret_cast<const uint8_t*>(S.digA) + (blk_a * S.stages + G.c) * (int64_t)SL_A_BYTES;
-                    const uint8_t* pb = reinterpret_cast<const uint8_t*>(S.digB) + (blk_b * S.stages + G.c) * b_bytes;
-                    for (int q = 0; q < G.take; ++q, ++g) {
+                    const uint32_t b_slice = (uint32_t)I.BN * 64u;
+                    const uint8_t* pa = reinterpret_cast<const uint8_t*>(S.digA) + blk_a * S.stages * (int64_t)(SL_A_BYTES + SL_A_SLICE);
+                    const uint8_t* pb = reinterpret_cast<const uint8_t*>(S.digB) + blk_b * S.stages * (int64_t)(b_bytes + b_slice);
+                    // n slices of either operand into the next slot
+                    auto load = [&](int64_t slice, int n) {
                         const int s = (int)(g % SL_STAGES);
                         if (g >= SL_STAGES &&
-                            !mbar_wait(smem_u32(&empty_bar[s]), (uint32_t)(g / SL_STAGES - 1) & 1u, &abort_sh)) {
-                            ok = false;
-                            break;
-                        }
+                            !mbar_wait(smem_u32(&empty_bar[s]), (uint32_t)(g / SL_STAGES - 1) & 1u, &abort_sh))
+                            return false;
                         uint8_t* st = stages + (size_t)s * SL_STAGE_BYTES;
                         const uint32_t bar = smem_u32(&full_bar[s]);
-                        mbar_expect_tx(bar, SL_A_BYTES + b_bytes);
-                        bulk_load(smem_u32(st), pa + (int64_t)q * SL_A_BYTES, SL_A_BYTES, bar);
-                        bulk_load(smem_u32(st + SL_A_BYTES), pb + (int64_t)q * b_bytes, b_bytes, bar);
-                    }
+                        mbar_expect_tx(bar, (uint32_t)n * (SL_A_SLICE + b_slice));
+                        bulk_load(smem_u32(st), pa + slice * SL_A_SLICE, (uint32_t)n * SL_A_SLICE, bar);
+                        bulk_load(smem_u32(st + SL_A_BYTES), pb + slice * b_slice, (uint32_t)n * b_slice, bar);
+                        ++g;
+                        return true;
+                    };
+                    for (int q = 0; q < G.take && ok; ++q) ok = load((int64_t)(G.c + q) * NS, NS);
+                    if (G.flush)                                 // the magnitudes of the run, NS stages a slot
+                        for (int q = G.g0; q < G.c + G.take && ok; q += NS)
+                            ok = load(S.stages * NS + q, min(NS, G.c + G.take - q));
                 }
             }
             if (!ok) {
@@ -290,7 +319,8 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                 mbar_wait(smem_u32(&full_bar[q % SL_STAGES]), (uint32_t)(q / SL_STAGES) & 1u, nullptr);
         } else if (warp == SL_EPI_WARPS + 1 && lane == 0) {
             // -------------------------------------------------------------------------- MMA --
-            uint64_t g = 0, grp = 0;
+            uint64_t g = 0, grp = 0, runs = 0;
+            bool behind_mag = false;                             // the group before ended its run
             int bn = 0;                                          // N tile of the previous group
             bool ok = true;
             for (int64_t tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -315,6 +345,10 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                             if (!ok) break;
                         }
                         bn = I.BN;
+                        if (q == 0 && behind_mag && !mbar_wait(smem_u32(&mag_drained_bar), (uint32_t)(runs - 1) & 1u, &abort_sh)) {
+                            ok = false;
+                            break;
+                        }
                         ok = I.BN == 64
                                  ? stage_mmas<64>(tmem, dA, dB, q == 0, last, smem_u32(drained_bar), wait_d, par,
                                                   smem_u32(ready_bar), &abort_sh)
@@ -322,6 +356,33 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                                                   smem_u32(ready_bar), &abort_sh);
                         umma_commit(smem_u32(&empty_bar[s]));
                     }
+                    behind_mag = G.flush;
+                    if (!ok || !G.flush) continue;
+                    // the products of the magnitudes, on the accumulators of the first weight pair (a sum
+                    // for either K step, so that two MMAs are in flight)
+                    if (!mbar_wait(smem_u32(&drained_bar[0]), (uint32_t)grp & 1u, &abort_sh)) {
+                        ok = false;
+                        continue;
+                    }
+                    for (int q = G.g0; q < G.c + G.take; q += NS, ++g) {
+                        const int s = (int)(g % SL_STAGES), n = min(NS, G.c + G.take - q);
+                        if (!mbar_wait(smem_u32(&full_bar[s]), (uint32_t)(g / SL_STAGES) & 1u, &abort_sh)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t st = smem_u32(stages + (size_t)s * SL_STAGE_BYTES);
+                        const uint64_t dA = umma_desc_sw64(st), dB = umma_desc_sw64(st + SL_A_BYTES);
+                        for (int j = 0; j < n; ++j)
+#pragma unroll
+                            for (int ks = 0; ks < 2; ++ks)
+                                umma<0>(tmem + (uint32_t)(ks * I.BN), dA + (uint64_t)(j * (SL_A_SLICE >> 4) + 2 * ks),
+                                        dB + (uint64_t)(j * ((I.BN * 64) >> 4) + 2 * ks), make_idesc(1u, SL_BM, (uint32_t)I.BN, false),
+                                        q > G.g0 || j > 0 ? 1u : 0u);
+                        umma_commit(smem_u32(&empty_bar[s]));
+                    }
+                    if (ok) umma_commit(smem_u32(&mag_ready_bar));
+                    ++runs;
                 }
             }
             if (!ok) {
@@ -338,6 +399,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const int row = quarter * 32 + lane;
         uint64_t grp = 0;
+        uint32_t runs = 0;
         bool failed = false;
         for (int64_t tile = blockIdx.x; tile < total_tiles && !failed; tile += gridDim.x) {
             if (tid == 0) {
@@ -418,6 +480,26 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                     }
                 }
                 if (!G.flush) continue;
+                uint32_t low = 0u;                               // bit j: column j needs FP64 arithmetic (s_low)
+                if (!failed && !mbar_wait(smem_u32(&mag_ready_bar), runs & 1u, &abort_sh)) {
+                    failed = true;
+                    abort_sh = 1;
+                }
+                ++runs;
+                if (!failed) {
+                    tc_fence_after();
+#pragma unroll 1
+                    for (int h = 0; h < SL_CW && mine; h += 16) {
+                        float v[16], u[16];
+                        tmem_ld16_pair(tmem + lane_base + (uint32_t)(part * SL_CW + h),
+                                       tmem + lane_base + (uint32_t)(BN + part * SL_CW + h), v, u);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) low |= (low_sum(v[j] + u[j]) ? 1u << j : 0u) << h;
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&mag_drained_bar));
+                }
                 // one decision of all epilogue warps per flush (also the barrier before s_eB is reused)
                 if (epi_bar_or(failed)) {
                     failed = true;
@@ -431,13 +513,19 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                 const uint32_t wa = s_t.m0 + row < s_t.M ? S.eA[s_t.batch * S.rA + s_t.m0 + row] : 0u;
                 const int ea = exp_of(wa);
                 if (part == 0) s_eA[row] = wa;
+                s_low[part][row] = low;
+                if (tid == 0) s_count = 0;
                 epi_bar();
                 // the integer sums of 4 columns of each warp at a time through shared memory; a thread
                 // converts and writes four elements, lanes on consecutive columns.  The register
                 // arrays need constant indices, everything behind them is one rolled body.
                 const double alpha = S.alpha;
                 const bool scale = alpha != 1.0;
-                const bool any_bad = epi_bar_or((wa >> 20) >= 2047u || (tid < BN && (s_eB[tid] >> 20) >= 2047u)) != 0;
+                const bool any_odd = epi_bar_or(low != 0u || (wa >> 20) >= 2047u || (tid < BN && (s_eB[tid] >> 20) >= 2047u)) != 0;
+                // rows or columns with an infinity or a NaN, sums the digits are too coarse for
+                auto odd = [&](int r, int j) {
+                    return (s_eA[r] >> 20) >= 2047u || (s_eB[j] >> 20) >= 2047u || ((s_low[j / SL_CW][r] >> (j % SL_CW)) & 1u);
+                };
                 const int slot = lane & 7, rr = warp * (4 * SL_NEL) + (lane >> 3);       // rows rr, rr + 4, ..
                 #pragma unroll 1
                 for (int p = 0; p < 8; ++p) {
@@ -463,25 +551,13 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                         const int eb = exp_of(wb);
                         double x[SL_NEL];
                         int te[SL_NEL];
+                        bool live[SL_NEL];                       // (the others: below)
+#pragma unroll
+                        for (int it = 0; it < SL_NEL; ++it)
+                            live[it] = s_t.m0 + rr + 4 * it < s_t.M && !(any_odd && odd(rr + 4 * it, jj));
 #pragma unroll
                         for (int it = 0; it < SL_NEL; ++it) te[it] = exp_of(s_eA[rr + 4 * it]) + eb;
                         sliced_to_doubles<SL_NEL>(raw, te, x);
-                        if (any_bad) {
-                            // rows or columns with an infinity or a NaN: these K elements in FP64
-#pragma unroll
-                            for (int it = 0; it < SL_NEL; ++it) {
-                                const int m = s_t.m0 + rr + 4 * it;
-                                if (m >= s_t.M || !((s_eA[rr + 4 * it] >> 20) >= 2047u || (wb >> 20) >= 2047u)) continue;
-                                const double* a = S.A + s_t.batch * S.sA + (int64_t)m * ((S.flags & 1) ? 1 : S.lda);
-                                const double* b = S.B + s_t.batch * S.sB + (int64_t)(s_t.n0 + jj) * ((S.flags & 2) ? 1 : S.ldb);
-                                const int64_t ka = (S.flags & 1) ? S.lda : 1, kb = (S.flags & 2) ? S.ldb : 1;
-                                const int64_t kt = (int64_t)(G.c + G.take) * SL_KS, ke = kt < S.K ? kt : S.K;
-                                double v = 0.0;
-#pragma unroll 1
-                                for (int64_t k = (int64_t)G.g0 * SL_KS; k < ke; ++k) v = fma(a[k * ka], b[k * kb], v);
-                                x[it] = v;
-                            }
-                        }
                         if (scale) {
 #pragma unroll
                             for (int it = 0; it < SL_NEL; ++it) x[it] *= alpha;
@@ -499,23 +575,52 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                         if (s_t.mode == 1) {
 #pragma unroll
                             for (int it = 0; it < SL_NEL; ++it)
-                                if (s_t.m0 + rr + 4 * it < s_t.M) atomicAdd(d[it], x[it]);
+                                if (live[it]) atomicAdd(d[it], x[it]);
                         } else {
                             // later segments add to what the same thread stored for the first one
                             if (!first) {
 #pragma unroll
                                 for (int it = 0; it < SL_NEL; ++it)
-                                    if (s_t.m0 + rr + 4 * it < s_t.M) x[it] = *d[it] + x[it];
+                                    if (live[it]) x[it] = *d[it] + x[it];
                             }
 #pragma unroll
                             for (int it = 0; it < SL_NEL; ++it)
-                                if (s_t.m0 + rr + 4 * it < s_t.M) *d[it] = x[it];
+                                if (live[it]) *d[it] = x[it];
                         }
                     }
                     __syncwarp();
                 }
 #pragma unroll
                 for (int j = 0; j < SL_CW; ++j) sum[j] = Sum96{0u, 0u, 0u};
+                if (any_odd) {
+                    // those elements in FP64, behind the others (the registers of the sums are free here): listed
+                    // first, so that all threads share them
+                    uint16_t* list = reinterpret_cast<uint16_t*>(s_raw);
+                    uint32_t todo = 0u;
+                    if (s_t.m0 + row < s_t.M) {
+#pragma unroll 1
+                        for (int j = 0; j < SL_CW; ++j) {
+                            const int jj = part * SL_CW + j;
+                            if (jj < BN && s_t.n0 + jj < s_t.N && odd(row, jj)) todo |= 1u << j;
+                        }
+                    }
+                    int at = atomicAdd(&s_count, __popc(todo));
+                    for (; todo; todo &= todo - 1u) list[at++] = (uint16_t)(row * 64 + part * SL_CW + __ffs((int)todo) - 1);
+                    epi_bar();
+                    const int64_t kt = (int64_t)(G.c + G.take) * SL_KS, ke = kt < S.K ? kt : S.K;
+#pragma unroll 1
+                    for (int e = tid; e < s_count; e += SL_EPI_THREADS) {
+                        const int r = list[e] >> 6, j = list[e] & 63;
+                        double x = alpha * fp64_product(S, s_t.batch, s_t.m0 + r, s_t.n0 + j, (int64_t)G.g0 * SL_KS, ke);
+                        double* d = s_t.C + s_roff[r] + s_coff[j];
+                        if (first && s_t.mode == 2) {
+                            if (s_diagB[j]) x += s_DA[r];
+                            if (s_diagA[r]) x += s_DB[j];
+                        }
+                        if (s_t.mode == 1) atomicAdd(d, x);
+                        else *d = first ? x : *d + x;
+                    }
+                }
                 first = false;
             }
             if (!failed) epi_bar();                              // metadata reads done before the next tile
@@ -534,15 +639,24 @@ constexpr int DG_WARP_K = 1024;        // rows up to this K: a warp each; longer
 constexpr int DG_TK = 64;              // transposed operands: 32 rows x 64 K per CTA
 constexpr int DG_MAX_K = 512;          // K per CTA of the row-maximum pass
 
-// Digit slices of four consecutive K elements of a row: eight 8-byte stores into the stage image
-// (blocks of `block` rows; per block and 32 K: [slice][row][32 K], 64-byte rows, 64-byte swizzle:
-// 16-byte chunk index xor bits 1..2 of the row).
-__device__ __forceinline__ void put_digits(const uint64_t (&v)[4], const xrh_slice_task& T, int64_t blk, int r, int64_t k) {
-    const int64_t stages = T.Kp / SL_KS;
+// Digit slices and magnitudes of four consecutive K elements of a row: nine 8-byte stores into the stage
+// images (blocks of `block` rows; per block and 32 K: [slice][row][32 K], 64-byte rows, 64-byte swizzle:
+// 16-byte chunk index xor bits 1..2 of the row; behind the digits of a block its magnitudes, [32 K][row]).
+__device__ __forceinline__ void put_digits(const double (&x)[4], int E, const xrh_slice_task& T, int64_t blk, int r, int64_t k) {
+    const int64_t stages = T.Kp / SL_KS, st = k / SL_KS, slice_stride = T.block * 64;
     const int kk = (int)(k & (SL_KS - 1));
-    uint8_t* dst = reinterpret_cast<uint8_t*>(T.digits) + (blk * stages + k / SL_KS) * (T.block * 64 * NS) + r * 64 +
-                   (((kk >> 3) ^ ((r >> 1) & 3)) << 4) + (kk & 7) * 2;
-    const int64_t slice_stride = T.block * 64;
+    uint8_t* base = reinterpret_cast<uint8_t*>(T.digits) + blk * stages * (slice_stride * (NS + 1)) + r * 64 +
+                    (((kk >> 3) ^ ((r >> 1) & 3)) << 4) + (kk & 7) * 2;
+    uint8_t* dst = base + st * NS * slice_stride;
+    const bool bad = E >= 2047;                        // an infinity or a NaN in the row
+    uint64_t v[4];
+    uint32_t m[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        v[e] = bad ? 0x0080808080808080ull : fixed62(x[e], E);
+        m[e] = bad ? 0u : magnitude(x[e], E);
+    }
+    *reinterpret_cast<uint2*>(base + (stages * NS + st) * slice_stride) = make_uint2(m[0] | (m[1] << 16), m[2] | (m[3] << 16));
 #pragma unroll
     for (int t = 0; t < NS; ++t) {
         uint32_t f[4];
@@ -616,11 +730,10 @@ __global__ void __launch_bounds__(DG_THREADS) slice_digits_kernel(const xrh_slic
             if (k >= T.Kp) continue;
             const uint32_t w = r < T.rows ? T.exps[b * T.rows + r] >> 20 : 0u;
             const int E = w < 1u ? 1 : (int)w;
-            uint64_t v[4];
+            double x[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                v[e] = E >= 2047 ? 0x0080808080808080ull : fixed62(tile[4 * (threadIdx.x & 15) + e][rr], E);
-            put_digits(v, T, b * blocks + r / T.block, (int)(r % T.block), k);
+            for (int e = 0; e < 4; ++e) x[e] = tile[4 * (threadIdx.x & 15) + e][rr];
+            put_digits(x, E, T, b * blocks + r / T.block, (int)(r % T.block), k);
         }
         return;
     }
@@ -650,11 +763,10 @@ __global__ void __launch_bounds__(DG_THREADS) slice_digits_kernel(const xrh_slic
     const uint32_t w = m >> 20;
     const int E = w < 1u ? 1 : (int)w;
     for (int64_t k = 4 * me; k < T.Kp; k += 4 * step) {
-        uint64_t v[4];
+        double x[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-            v[e] = E >= 2047 ? 0x0080808080808080ull : fixed62(ok && k + e < T.K ? __ldg(p + k + e) : 0.0, E);
-        put_digits(v, T, b * blocks + r / T.block, (int)(r % T.block), k);
+        for (int e = 0; e < 4; ++e) x[e] = ok && k + e < T.K ? __ldg(p + k + e) : 0.0;
+        put_digits(x, E, T, b * blocks + r / T.block, (int)(r % T.block), k);
     }
 }
 

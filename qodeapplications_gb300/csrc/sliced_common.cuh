@@ -154,4 +154,21 @@ __device__ __forceinline__ uint32_t digit_float(uint64_t v, int t) {
     return __float_as_uint(__uint_as_float(0x4b000000u | byte) - 8388736.0f);
 }
 
+// |x| 2^-e rounded down to BF16 (bits), at least 2^-60 for x != 0, for an x of a row with |x| < 2^e.  A sum
+// of products of magnitudes bounds sum |a||b| 2^-(ea + eb) from below, and is zero only where every
+// product is (2^-60 adds nothing at the threshold below).
+__device__ __forceinline__ uint32_t magnitude(double x, int E) {
+    const uint32_t hi = abs_hi(x);
+    const int m = hi < 0x00100000u ? 0 : (int)(hi >> 13) - ((E - 126) << 7);       // (subnormal: the least one)
+    return hi == 0u && __double2loint(x) == 0 ? 0u : (uint32_t)max(m, 67 << 7);
+}
+
+// Where a sum needs FP64 arithmetic.  What the digits leave out of K products, 2^-63 2^e of an element and
+// the pairs with i + j >= 8 (7 2^14 256^-1 + .. units of 2^-68), is at most K 1.003 2^-59 2^(ea + eb); an FP64
+// sum has the bound K 2^-53 sum |a||b|.  So the digits are as good where sum |a||b| >= 1.003 2^-6
+// 2^(ea + eb): everywhere for rows of elements of like size (there it is about K / 16 and more), not where
+// the large elements of one row meet zeros or small elements of the other.
+constexpr float LOW_SUM = 1.01f / 64.0f;
+__device__ __forceinline__ bool low_sum(float magnitudes) { return magnitudes > 0.0f && magnitudes < LOW_SUM; }
+
 }  // namespace xrh_sliced

@@ -1,7 +1,7 @@
 """Host-side plan of the FP64 grouped GEMM on the tensor cores (csrc/gemm_sliced.cu).
 
 The tasks of one GroupedGemm launch become waves: the operands of a wave are written as digit
-slices into one workspace (xrh_slice_grouped, every distinct operand once), then one
+slices and magnitudes into one workspace (xrh_slice_grouped, every distinct operand once), then one
 xrh_gemm_sliced_grouped launch runs its tasks.  Tasks whose digits exceed the workspace limit are
 divided into panels.  Every table is built once and uploaded in one copy; run() only launches.
 """
@@ -41,7 +41,7 @@ def _operands(t):
 
 def _digit_bytes(op):
     _p, _tr, rows, K, _ld, batch, _st, block = op
-    return 2 * SLICES * -(-rows // block) * block * batch * _stages(K) * STAGE_K
+    return 2 * (SLICES + 1) * -(-rows // block) * block * batch * _stages(K) * STAGE_K
 
 
 def _exp_bytes(op):
