@@ -373,10 +373,13 @@ int xrh_gemm_sliced_grouped(const xrh_gemm_task* tasks_dev, int n_tasks, int64_t
  *   xrh_coeff_digits: state coefficients zT[n_conf][n] as digits [ceil(n / npad)][n_conf][slices]
  *       [npad] BF16 (16-byte aligned; npad = 16, 32 or 64, at least n or 64), each state scaled by the
  *       power of two above its largest coefficient; exps_dev[n] (zero on entry) receives the high word
- *       of that coefficient.  A task owns xrh_coeff_digit_ctas(n_conf) CTAs from cta_begin on.
+ *       of that coefficient.  With slices = 8 there follow the magnitudes |z| 2^-e, [ceil(n / npad)]
+ *       [n_conf][npad] BF16, and masks of the states with a nonzero coefficient, [ceil(n / npad)][n_conf]
+ *       64-bit words.  A task owns xrh_coeff_digit_ctas(n_conf) CTAs from cta_begin on.
  *   xrh_density_sliced_grouped: unit u writes rhoT[idx, iblk 64 .., jblk 64 ..] from its `count` couplings
  *       from c0 on, the first n_pos of sign +1, the rest -1 (count > 0: indices without couplings are
- *       not written).  npad is that of both digit arrays of every task (state counts above 64 in blocks
+ *       not written).  Elements that the digits are too coarse for, relative to the sum of the absolute
+ *       products, and those of states with infinities or NaN are formed by FP64 arithmetic.  npad is that of both digit arrays of every task (state counts above 64 in blocks
  *       of 64: npad = 64).  A device wait that runs out sets *status_dev = XRH_ERR_TIMEOUT. */
 typedef struct {
     const double* zT;

@@ -14,6 +14,16 @@
 // b + g with i = g mod G.  The sums stay below 2^24, so exact, for GROUP stages; they are collected in
 // 96-bit integers, added over the lane groups and rounded once at the end of the index.
 //
+// The digits are relative to a state's largest coefficient: an error of at most count 1.003 2^-59 2^(eI + eJ)
+// (gemm_sliced.cu) where an FP64 sum has count 2^-53 sum |zb||zk|.  Elements that need it are formed by FP64
+// FMAs over their couplings, listed first so that all epilogue threads share them (low_sum in
+// sliced_common.cuh: indices without a large coefficient in their couplings, as in the tails of a
+// wave function).  Which ones is decided from below: one MMA over the magnitudes of 64 couplings spread over
+// the list (all of a shorter one) finds most elements large enough, masks of the determinants' nonzero
+// states find those without any product, and the rest have the magnitudes of all their couplings
+// summed.  Gathering every coupling's magnitudes instead cost 18 % (14 orbitals, 40 states: 4.80 ms without,
+// 4.94 with the sample, 5.70 with all).
+//
 // A CTA (persistent over a work list ordered by length), 16 warps:
 //   * warps 8-11: cp.async gathers of stages of 32 couplings of one sign (positive ones first: the MMA
 //     negates A for the negative ones);
@@ -28,6 +38,7 @@
 #include "sliced_common.cuh"
 #include "tc_common.cuh"
 #include "xrh_common.cuh"
+#include <cuda_bf16.h>
 
 namespace {
 using namespace xrh_tc;
@@ -35,6 +46,7 @@ using namespace xrh_sliced;
 
 constexpr int DS_KS = 32;                              // couplings per stage
 constexpr int DS_EPI = 256, DS_PROD = 128, DS_THREADS = DS_EPI + DS_PROD + 128;
+constexpr int DS_SAMPLE = 64;                          // couplings whose magnitudes are summed
 constexpr uint32_t DS_ATOM = DS_KS * 128;              // bytes between 64-element atoms of a stage side
 
 template <int NPAD>
@@ -78,9 +90,12 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t saddr) {
     return d;
 }
 
+// Coupling i of the sample of an index with n couplings: spread over the list (which is ordered by sign and
+// ket, so that every kind of determinant is met), or all of them.
+__device__ __forceinline__ int sampled(int i, int n) { return n > DS_SAMPLE ? (int)((int64_t)i * n / DS_SAMPLE) : i; }
+
 __device__ __forceinline__ int stages_of(int n) { return (n + DS_KS - 1) / DS_KS; }
 
-// 16 bytes to shared memory, zeros where ok is false
 // The barrier counts this thread's copies as one arrival once they have landed; their reader, not the
 // thread that issued them, orders them before the MMAs (a proxy fence here would wait for the copies
 // in flight: one gather at a time).
@@ -89,6 +104,7 @@ __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
 }
 __device__ __forceinline__ void fence_copies() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// 16 bytes to shared memory, zeros where ok is false
 __device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
@@ -117,6 +133,20 @@ __device__ __forceinline__ void tmem_ld(uint32_t ta, float (&v)[N]) {
     for (int i = 0; i < N; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// The magnitudes of a side's states, [block of 64 states][determinant][NPAD], behind its digits.
+template <int NPAD>
+__device__ __forceinline__ const uint8_t* magnitudes(const xrh_dens_sliced_task& T, int side) {
+    const int64_t rows = (((side ? T.nk : T.nb) + 63) / 64) * (side ? T.conf_k : T.conf_b);
+    return reinterpret_cast<const uint8_t*>(side ? T.digk : T.digb) + rows * (NS * NPAD * 2);
+}
+
+// Which of its block's states a determinant has a coefficient of, [block of 64 states][determinant], behind those.
+template <int NPAD>
+__device__ __forceinline__ const uint64_t* nonzero(const xrh_dens_sliced_task& T, int side) {
+    const int64_t rows = (((side ? T.nk : T.nb) + 63) / 64) * (side ? T.conf_k : T.conf_b);
+    return reinterpret_cast<const uint64_t*>(reinterpret_cast<const uint8_t*>(side ? T.digk : T.digb) + rows * ((NS + 1) * NPAD * 2));
+}
+
 template <int NPAD>
 __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
     density_sliced_kernel(const xrh_dens_sliced_task* __restrict__ tasks, const xrh_dens_sliced_unit* __restrict__ units,
@@ -125,11 +155,13 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
     extern __shared__ unsigned char smem_raw[];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;       // [STAGES][bra, ket][atoms][couplings]
     __shared__ __align__(8) uint64_t full_bar[C::STAGES], empty_bar[C::STAGES];
-    __shared__ __align__(8) uint64_t ready_bar, drained_bar, done_bar;
+    __shared__ __align__(8) uint64_t ready_bar, drained_bar, mag_ready_bar, mag_drained_bar, done_bar;
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_sh;
     __shared__ uint4 s_raw[128][9];
     __shared__ uint32_t s_eb[64], s_ek[64];
+    __shared__ int s_count;                            // elements to form in FP64
+    __shared__ unsigned long long s_nz[64];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < C::STAGES; ++s) {
@@ -138,6 +170,8 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
         }
         mbar_init(smem_u32(&ready_bar), 1);
         mbar_init(smem_u32(&drained_bar), DS_EPI / 32);
+        mbar_init(smem_u32(&mag_ready_bar), 1);
+        mbar_init(smem_u32(&mag_drained_bar), DS_EPI / 32);
         mbar_init(smem_u32(&done_bar), 1);
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -160,33 +194,47 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
         if (warp == 12 && lane == 0) {
             // ------------------------------------------------------------------------ MMA --
             constexpr uint32_t idesc0 = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) | (8u << 24);
-            uint32_t st = 0, grp = 0;
+            uint32_t st = 0, grp = 0, un = 0;
             bool ok = true;
-            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++un) {
                 const int np = units[u].n_pos, nn = units[u].count - np;
                 const int s_pos = stages_of(np), n_st = s_pos + stages_of(nn);
                 for (int q = 0; q < n_st && ok; ++q, ++st) {
                     const int in_group = q % C::GROUP;
                     const uint32_t s = st % C::STAGES;
-                    if (in_group == 0 && grp > 0 && !mbar_wait(smem_u32(&drained_bar), (grp - 1) & 1u, &abort_sh)) ok = false;
+                    if (in_group == 0 && q > 0 && !mbar_wait(smem_u32(&drained_bar), (grp - 1) & 1u, &abort_sh)) ok = false;
                     if (ok && !mbar_wait(smem_u32(&full_bar[s]), (st / C::STAGES) & 1u, &abort_sh)) ok = false;
                     if (!ok) break;
                     fence_copies();
                     tc_fence_after();
                     const uint32_t id = idesc0 | (q >= s_pos ? 1u << 13 : 0u);
                     const uint64_t da = desc_mn_sw128(ring + s * 2 * C::SIDE), db = desc_mn_sw128(ring + s * 2 * C::SIDE + C::SIDE);
+                    // tile t, columns [c0, COLS) of its 128 t ..: slices of B from column c0 on
+                    auto tile = [&](int t, int ks, int c0, int cols, uint32_t acc) {
+                        umma<0>(tmem + 128 * t + c0, da + (uint64_t)((t * 2 * DS_ATOM + ks * 2048) >> 4),
+                                db + (uint64_t)((c0 / 64 * DS_ATOM + ks * 2048) >> 4), id | ((uint32_t)(cols / 8) << 17), acc);
+                    };
+                    // the first 64 columns of a unit's first stage come last: the sums of the magnitudes of the
+                    // unit before are read from there meanwhile
+                    const int skip = q == 0 ? 64 : 0;
 #pragma unroll
                     for (int ks = 0; ks < DS_KS / 16; ++ks) {
 #pragma unroll
                         for (int t = 0; t < C::TILES; ++t) {
+                            const int c0 = t == 0 ? skip : 0, n = C::COLS - 128 * t - c0;
                             const uint32_t acc = (in_group > 0 || ks > 0 || t > 0) ? 1u : 0u;
-                            const uint64_t a = da + (uint64_t)((t * 2 * DS_ATOM + ks * 2048) >> 4);
-                            const int n = C::COLS - 128 * t, n1 = n < 256 ? n : 256;
-                            umma<0>(tmem + 128 * t, a, db + (uint64_t)((ks * 2048) >> 4), id | ((uint32_t)(n1 / 8) << 17), acc);
-                            if (n > 256)
-                                umma<0>(tmem + 128 * t + 256, a, db + (uint64_t)((4 * DS_ATOM + ks * 2048) >> 4),
-                                        id | ((uint32_t)((n - 256) / 8) << 17), acc);
+                            tile(t, ks, c0, n < 256 ? n : 256, acc);
+                            if (n > 256) tile(t, ks, c0 + 256, n - 256, acc);
                         }
+                    }
+                    if (q == 0) {
+                        if (un > 0 && !mbar_wait(smem_u32(&mag_drained_bar), (un - 1) & 1u, &abort_sh)) {
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+#pragma unroll
+                        for (int ks = 0; ks < DS_KS / 16; ++ks) tile(0, ks, 0, 64, ks > 0 ? 1u : 0u);
                     }
                     umma_commit(smem_u32(&empty_bar[s]));
                     if (in_group == C::GROUP - 1 || q == n_st - 1) {
@@ -194,6 +242,23 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                         ++grp;
                     }
                 }
+                // the products of the magnitudes (the rows of A from NPAD on are not written, their sums not read)
+                const uint32_t s = st % C::STAGES;
+                if (ok && (!mbar_wait(smem_u32(&drained_bar), (grp - 1) & 1u, &abort_sh) ||
+                           !mbar_wait(smem_u32(&full_bar[s]), (st / C::STAGES) & 1u, &abort_sh)))
+                    ok = false;
+                if (ok) {
+                    fence_copies();
+                    tc_fence_after();
+                    const uint64_t da = desc_mn_sw128(ring + s * 2 * C::SIDE), db = desc_mn_sw128(ring + s * 2 * C::SIDE + C::SIDE);
+#pragma unroll
+                    for (int k = 0; k < DS_SAMPLE / 16; ++k)
+                        umma<0>(tmem, da + (uint64_t)((k * 2048) >> 4), db + (uint64_t)((k * 2048) >> 4),
+                                idesc0 | ((uint32_t)(NPAD / 8) << 17), k > 0 ? 1u : 0u);
+                    umma_commit(smem_u32(&empty_bar[s]));
+                    ++st;
+                }
+                if (ok) umma_commit(smem_u32(&mag_ready_bar));
             }
             if (!ok) {
                 abort_sh = 1;
@@ -217,6 +282,12 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
             const uint8_t* rows = reinterpret_cast<const uint8_t*>(side ? T.digk : T.digb) +
                                   (int64_t)blk * (side ? T.conf_k : T.conf_b) * (NS * NPAD * 2);
             const int s_pos = stages_of(U.n_pos), n_st = s_pos + stages_of(U.count - U.n_pos);
+            int sample[DS_SAMPLE / 32];
+#pragma unroll
+            for (int i = 0; i < DS_SAMPLE / 32; ++i) {
+                const int c = sampled(i * 32 + lane, U.count);
+                sample[i] = c < U.count ? __ldg(list + c) : -1;
+            }
             for (int q = 0; q < n_st; ++q, ++st) {
                 const uint32_t s = st % C::STAGES;
                 const int c = (q < s_pos ? q * DS_KS : U.n_pos + (q - s_pos) * DS_KS) + lane;
@@ -240,6 +311,34 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                 }
                 cp_async_arrive(smem_u32(&full_bar[s]));
             }
+            // the magnitudes of the sample, 128 bytes a coupling of which NPAD / 8 chunks are written
+            if (ok) {
+                constexpr int CH = NPAD / 8;
+                const uint32_t s = st % C::STAGES;
+                const uint8_t* mags = magnitudes<NPAD>(T, side) + (int64_t)blk * (side ? T.conf_k : T.conf_b) * (NPAD * 2);
+                if (st >= C::STAGES) {
+                    const bool free = mbar_wait(smem_u32(&empty_bar[s]), (st / C::STAGES - 1) & 1u, &abort_sh);
+                    if (!__all_sync(0xffffffffu, free)) {
+                        ok = false;
+                        break;
+                    }
+                }
+                ++st;
+                const uint32_t base = ring + s * 2 * C::SIDE + side * C::SIDE;
+#pragma unroll
+                for (int i = 0; i < DS_SAMPLE * CH / 64; ++i) {
+                    const int item = i * 64 + (pw & 1) * 32 + lane, cc = item / CH, chunk = item % CH;
+                    int row = __shfl_sync(0xffffffffu, sample[0], cc & 31);
+#pragma unroll
+                    for (int k = 1; k < DS_SAMPLE / 32; ++k) {
+                        const int x = __shfl_sync(0xffffffffu, sample[k], cc & 31);
+                        if (cc >> 5 == k) row = x;
+                    }
+                    const uint32_t dst = base + (uint32_t)(cc >> 3) * 1024u + (uint32_t)(cc & 7) * 128u + (uint32_t)((chunk ^ (cc & 7)) << 4);
+                    cp_async16_or_zero(dst, mags + (int64_t)(row < 0 ? 0 : row) * (NPAD * 2) + chunk * 16, row >= 0);
+                }
+                cp_async_arrive(smem_u32(&full_bar[s]));
+            }
         }
         cp_async_commit();
         cp_async_wait<0>();
@@ -254,11 +353,35 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const int row = quarter * 32 + lane;
         const int g = row / NPAD;                      // lane group: weight = column block + g
-        uint32_t grp = 0;
+        uint32_t grp = 0, un = 0;
         bool failed = false;
-        for (int64_t u = blockIdx.x; u < n_units && !failed; u += gridDim.x) {
+        for (int64_t u = blockIdx.x; u < n_units && !failed; u += gridDim.x, ++un) {
             const int np = units[u].n_pos, count = units[u].count;
             const int n_st = stages_of(np) + stages_of(count - np);
+            const bool partial = count > DS_SAMPLE;
+            if (partial) {
+                // s_nz[row]: columns with a product that is not zero.  The determinants' nonzero states come as
+                // masks, few different pairs of them in an index (spin and spatial symmetry)
+                const xrh_dens_sliced_unit U = units[u];
+                const xrh_dens_sliced_task& T = tasks[U.task];
+                const uint64_t *nb_ = nonzero<NPAD>(T, 0) + (int64_t)U.iblk * T.conf_b, *nk_ = nonzero<NPAD>(T, 1) + (int64_t)U.jblk * T.conf_k;
+                if (tid < 64) s_nz[tid] = 0ull;
+                epi_bar();
+                uint64_t done_b = 0ull, done_k = 0ull;
+                for (int c = tid; c - lane < count; c += DS_EPI) {
+                    const uint64_t b = c < count ? __ldg(nb_ + __ldg(T.P + U.c0 + c)) : 0ull, k = c < count ? __ldg(nk_ + __ldg(T.Q + U.c0 + c)) : 0ull;
+                    uint32_t todo = __ballot_sync(0xffffffffu, b != 0ull && k != 0ull && !(b == done_b && k == done_k));
+                    while (todo) {
+                        const int src = __ffs((int)todo) - 1;
+                        done_b = __shfl_sync(0xffffffffu, b, src);
+                        done_k = __shfl_sync(0xffffffffu, k, src);
+#pragma unroll
+                        for (int r = lane; r < 64; r += 32)
+                            if ((done_b >> r) & 1ull) atomicOr(&s_nz[r], (unsigned long long)done_k);
+                        todo &= ~__ballot_sync(0xffffffffu, b == done_b && k == done_k);
+                    }
+                }
+            }
             Sum96 sum[C::CW];
 #pragma unroll
             for (int j = 0; j < C::CW; ++j) sum[j] = Sum96{0u, 0u, 0u};
@@ -285,6 +408,29 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&drained_bar));
             }
+            uint32_t low = 0u;                         // bit j: column j of this row may need FP64 arithmetic
+            if (!failed && !mbar_wait(smem_u32(&mag_ready_bar), un & 1u, &abort_sh)) {
+                failed = true;
+                abort_sh = 1;
+            }
+            if (!failed) {
+                constexpr int CH = 8;                  // (16 spill)
+                tc_fence_after();
+#pragma unroll 1
+                for (int h = 0; h < C::CW && quarter * 32 < NPAD; h += CH) {
+                    float v[CH];
+                    tmem_ld<CH>(tmem + lane_base + (uint32_t)(part * C::CW + h), v);
+#pragma unroll
+                    for (int j = 0; j < CH; ++j) low |= ((partial ? v[j] < LOW_SUM : low_sum(v[j])) ? 1u << j : 0u) << h;
+                }
+                const xrh_dens_sliced_task& T = tasks[units[u].task];
+                const int cols = T.nk - units[u].jblk * 64 - part * C::CW;
+                if (row >= NPAD || units[u].iblk * 64 + row >= T.nb || cols <= 0) low = 0u;
+                else if (cols < 32) low &= (1u << cols) - 1u;
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&mag_drained_bar));
+            }
             if (epi_bar_or(failed)) {                  // (also: s_eb, s_ek of the unit before are read)
                 failed = true;
                 abort_sh = 1;
@@ -296,7 +442,10 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
             const int i0 = U.iblk * 64, j0 = U.jblk * 64;
             if (tid < 64) s_eb[tid] = i0 + tid < T.nb ? T.eb[i0 + tid] : 0u;
             else if (tid < 128) s_ek[tid - 64] = j0 + tid - 64 < T.nk ? T.ek[j0 + tid - 64] : 0u;
+            if (tid == 0) s_count = 0;
+            if (partial && row < NPAD) low &= (uint32_t)(s_nz[row] >> (part * C::CW));
             epi_bar();
+            const bool any_odd = epi_bar_or(low != 0u || (tid < 64 && ((s_eb[tid] >> 20) >= 2047u || (s_ek[tid] >> 20) >= 2047u))) != 0;
             // 4 columns of each part at a time: the lane groups of an element are added, converted, stored
 #pragma unroll 1
             for (int p = 0; p < C::CW / 4; ++p) {
@@ -322,20 +471,51 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                     const int te[1] = {exp_of(s_eb[I]) + exp_of(s_ek[J])};
                     double tv[1];
                     sliced_to_doubles<1>(t, te, tv);
-                    double x = tv[0];
-                    if ((s_eb[I] >> 20) >= 2047u || (s_ek[J] >> 20) >= 2047u) {
-                        // a state with an infinity or a NaN: the couplings in FP64
-                        x = 0.0;
-#pragma unroll 1
-                        for (int c = 0; c < count; ++c) {
-                            const double a = T.zbT[(int64_t)T.P[U.c0 + c] * T.nb + i0 + I];
-                            x = fma(c < np ? a : -a, T.zkT[(int64_t)T.Q[U.c0 + c] * T.nk + j0 + J], x);
-                        }
-                    }
-                    T.rhoT[((int64_t)U.idx * T.nb + i0 + I) * T.nk + j0 + J] = x;
+                    T.rhoT[((int64_t)U.idx * T.nb + i0 + I) * T.nk + j0 + J] = tv[0];
                 }
                 __syncwarp();
                 epi_bar();
+            }
+            if (any_odd) {
+                // sums the digits are too coarse for, states with an infinity or a NaN: the couplings in FP64
+                // (in place of what has been stored), listed first, so that all threads share them
+                uint16_t* odd = reinterpret_cast<uint16_t*>(s_raw);
+                if (row < NPAD && i0 + row < T.nb) {
+                    const bool bad = (s_eb[row] >> 20) >= 2047u;
+#pragma unroll 1
+                    for (int j = 0; j < C::CW; ++j) {
+                        const int J = part * C::CW + j;
+                        if (j0 + J < T.nk && (bad || (s_ek[J] >> 20) >= 2047u)) low |= 1u << j;
+                    }
+                    int at = atomicAdd(&s_count, __popc(low));
+                    for (; low; low &= low - 1u) odd[at++] = (uint16_t)(row * 64 + part * C::CW + __ffs((int)low) - 1);
+                }
+                epi_bar();
+                const int32_t *P = T.P + U.c0, *Q = T.Q + U.c0;
+#pragma unroll 1
+                for (int e = tid; e < s_count; e += DS_EPI) {
+                    const int I = i0 + (odd[e] >> 6), J = j0 + (odd[e] & 63);
+                    if (partial && (s_eb[I - i0] >> 20) < 2047u && (s_ek[J - j0] >> 20) < 2047u) {
+                        // the sample does not show it: the magnitudes of all couplings, as far as needed
+                        const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(magnitudes<NPAD>(T, 0)) + (int64_t)U.iblk * T.conf_b * NPAD + I - i0;
+                        const __nv_bfloat16* mk = reinterpret_cast<const __nv_bfloat16*>(magnitudes<NPAD>(T, 1)) + (int64_t)U.jblk * T.conf_k * NPAD + J - j0;
+                        float m = 0.f;
+                        for (int c = 0; c < count && m < LOW_SUM; c += 8) {
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                                if (c + k < count)
+                                    m = fmaf(__bfloat162float(mb[(int64_t)__ldg(P + c + k) * NPAD]), __bfloat162float(mk[(int64_t)__ldg(Q + c + k) * NPAD]), m);
+                        }
+                        if (!low_sum(m)) continue;
+                    }
+                    double x = 0.0;
+#pragma unroll 4
+                    for (int c = 0; c < count; ++c) {
+                        const double a = __ldg(T.zbT + (int64_t)__ldg(P + c) * T.nb + I);
+                        x = fma(c < np ? a : -a, __ldg(T.zkT + (int64_t)__ldg(Q + c) * T.nk + J), x);
+                    }
+                    T.rhoT[((int64_t)U.idx * T.nb + I) * T.nk + J] = x;
+                }
             }
         }
     }
@@ -383,13 +563,20 @@ __global__ void __launch_bounds__(256) coeff_digits_kernel(const xrh_coeff_digit
         const int r = x / per, o = x - r * per, blk = o / oct, s0 = blk * T.npad + (o - blk * oct) * 8;
         const double* z = T.zT + (r0 + r) * T.n;
         uint64_t v[8];
+        uint32_t m[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int s = s0 + k;
             v[k] = 0x0080808080808080ull;
+            m[k] = 0u;
             if (s < T.n) {
                 const uint32_t w = T.exps[s] >> 20;
-                if (w < 2047u) v[k] = fixed62(__ldg(z + s), w < 1u ? 1 : (int)w);
+                const int E = w < 1u ? 1 : (int)w;
+                if (w < 2047u) {
+                    const double x = __ldg(z + s);
+                    v[k] = fixed62(x, E);
+                    m[k] = magnitude(x, E);
+                }
             }
         }
         uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(T.digits) +
@@ -401,6 +588,20 @@ __global__ void __launch_bounds__(256) coeff_digits_kernel(const xrh_coeff_digit
 #pragma unroll
             for (int k = 0; k < 4; ++k) q[k] = __byte_perm(digit_float(v[2 * k], t), digit_float(v[2 * k + 1], t), 0x7632);
             dst[t * oct] = make_uint4(q[0], q[1], q[2], q[3]);
+        }
+        if (T.slices == NS)                            // behind the digits of all blocks
+            *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(T.digits) +
+                                      ((int64_t)blocks * T.n_conf * NS + (int64_t)blk * T.n_conf + r0 + r) * T.npad + (o - blk * oct) * 8) =
+                make_uint4(m[0] | (m[1] << 16), m[2] | (m[3] << 16), m[4] | (m[5] << 16), m[6] | (m[7] << 16));
+        if (T.slices == NS) {
+            uint8_t bits = 0;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) bits |= m[k] ? 1u << k : 0u;
+            uint8_t* nz = reinterpret_cast<uint8_t*>(reinterpret_cast<uint16_t*>(T.digits) + (int64_t)blocks * T.n_conf * (NS + 1) * T.npad) +
+                          ((int64_t)blk * T.n_conf + r0 + r) * 8;
+            nz[o - blk * oct] = bits;                  // (little-endian: state k is bit k)
+            if (oct < 8 && o == 0)
+                for (int k = oct; k < 8; ++k) nz[k] = 0;
         }
     }
 }

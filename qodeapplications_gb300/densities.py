@@ -326,7 +326,8 @@ def _coupling_units(cp):
 
 class CoeffDigits:
     """Digit rows of state coefficients for the sliced kernels (xrh_coeff_digits), per side and charge:
-    {(side, charge): (digits, exponent address, zT)}, the common pad width npad and the slices kept."""
+    {(side, charge): (digits, exponent address, zT)}, the common pad width npad and the slices kept (all eight:
+    the magnitudes of the coefficients too)."""
 
     def __init__(self, sides, device, slices=_lib.SLICES):
         tabs = [((s, c), z) for s, zs in sides.items() for c, z in zs.items()]
@@ -338,7 +339,9 @@ class CoeffDigits:
         self.of, e0, cta = {}, 0, 0
         for e, (key, z) in zip(tab, tabs):
             n_conf, n = z.shape
-            d = torch.empty((-(-n // self.npad), max(n_conf, 1), slices, self.npad), dtype=torch.bfloat16, device=device)
+            rows = -(-n // self.npad) * max(n_conf, 1)         # (eight slices: magnitudes and a mask behind the digits)
+            d = torch.empty(rows * (slices * self.npad + (self.npad + 4 if slices == _lib.SLICES else 0)), dtype=torch.bfloat16,
+                            device=device)
             self.of[key] = (d, self.exps.data_ptr() + 4 * e0, z)
             e["zT"], e["digits"], e["exps"], e["n_conf"] = z.data_ptr(), d.data_ptr(), self.of[key][1], n_conf
             e["n"], e["npad"], e["slices"], e["cta_begin"] = n, self.npad, slices, cta
