@@ -387,7 +387,7 @@ typedef struct {
     uint32_t* exps;
     int64_t n_conf;
     int32_t n, npad;
-    int64_t slices;            /* digit slices written: 8, or 6 (the leading ones) */
+    int64_t slices;            /* digit slices written: 8, or the leading ones (xrh_coeff_rows: 8 or 3) */
     int64_t cta_begin;
 } xrh_coeff_digit_task;   /* 56 bytes */
 typedef struct {
@@ -409,11 +409,17 @@ typedef struct {
     int32_t task, idx;
     int32_t iblk, jblk;
 } xrh_dens_sliced_unit;   /* 32 bytes */
-/* The adjoint of those densities (xrh_density_adjoint) over the same digit rows: gzk[Q, J] += s sum_I
- * zb[P, I] gT[idx, I, J] (units with n_pos >= 0) and gzb[P, I] += s sum_J zk[Q, J] gT[idx, I, J] (units
- * with the sign bit of n_pos set), one unit per direction, operator index and blocks of 64 states.
- * precision XRH_FP64: digit rows of 8 slices, gz* double; XRH_FP32: rows of 6 slices (8 for npad = 16),
- * gz* float. */
+/* The adjoint of those densities (xrh_density_adjoint): gzk[Q, J] += s sum_I zb[P, I] gT[idx, I, J] (units with
+ * n_pos >= 0) and gzb[P, I] += s sum_J zk[Q, J] gT[idx, I, J] (units with the sign bit of n_pos set), one
+ * unit per direction, operator index and blocks of 64 states.
+ *   xrh_coeff_rows: the coefficients as rows [ceil(n / npad)][n_conf][pieces][npad] BF16 (16-byte aligned,
+ *       pieces rounded up to whole 128 bytes).  slices = 8: nine pieces, magnitudes |z| 2^-e, digits 1 .. 7,
+ *       digit 0, every determinant's states of a block under their own largest coefficient, whose
+ *       high word goes to exps_dev[ceil(n / npad)][n_conf]; slices = 3: z rounded to FP32 as the sum of three
+ *       BF16 numbers (exps_dev is not used).
+ *   xrh_density_adjoint_sliced_grouped: precision XRH_FP64: rows of slices = 8, gz* double, and the
+ *       elements that the digits are too coarse for, relative to the sum of the absolute products, by
+ *       FP64 arithmetic; XRH_FP32: rows of slices = 3, gz* float. */
 typedef struct {
     const int32_t* P;
     const int32_t* Q;

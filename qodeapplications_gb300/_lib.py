@@ -79,6 +79,7 @@ _SIGS = {
     "xrh_gemm_sliced_grouped": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp]),
     "xrh_coeff_digit_ctas": (_i64, [_i64]),
     "xrh_coeff_digits": (_i32, [_vp, _i32, _i64, _vp]),
+    "xrh_coeff_rows": (_i32, [_vp, _i32, _i64, _vp]),
     "xrh_density_adjoint_sliced_grouped": (_i32, [_i32, _vp, _i32, _vp, _i64, _i32, _vp, _vp]),
     "xrh_density_sliced_grouped": (_i32, [_vp, _i32, _vp, _i64, _i32, _vp, _vp]),
     "xrh_gemv_rows": (_i32, [_i64, _i64, _vp, _i64, _vp, _dbl, _dbl, _vp, _vp]),

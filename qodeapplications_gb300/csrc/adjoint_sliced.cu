@@ -1,34 +1,41 @@
-// Adjoint of the transition densities with exact digit products on the tensor cores (sm_103a).
+// Adjoint of the transition densities on the tensor cores (sm_103a).
 //
 // For an operator index with gradient G = dE/drho[idx] (n_b x n_k) and couplings (P_c, Q_c, s_c)
 //     dE/dzk[Q_c, J] += s_c sum_I zb[P_c, I] G[I, J]        (ket direction)
 //     dE/dzb[P_c, I] += s_c sum_J zk[Q_c, J] G[I, J]        (bra direction)
-// Each direction of an index is one unit: A = gathered digit rows of 128 couplings (K = states, the
-// rows the density kernel uses, density_sliced.cu), B = the digits of G for this direction, made in
-// shared memory once per unit.  A's digits are scaled per state, by 2^e_I; that factor goes into G
-// before its columns are scaled by their own largest element.  Slice i of A times all slices j of B
-// with i + j < NS is one MMA of N = (NS - i) NPAD columns that lands on the accumulators of the weights
-// i + j; a tile sums at most 8 pairs of 64 states, 2^23, exactly.
-//   FP64 (NS = 8): the eight weights of a sum become one 96-bit integer, rounded once;
-//   FP32 (NS = 6, 46 bits: states and gradients down to 2^-22 of their column's largest keep the 24 bits
-//   of FP32): the weights are combined by FP32 fused multiply-adds.
+// Each direction of an index is one unit: A = gathered rows of 128 couplings (K = states) in pieces of BF16
+// numbers, B = the pieces of G for this direction, made in shared memory once per unit.  Piece i of A
+// times all pieces j of B with i + j < NSL is one MMA of N = (NSL - i) NPAD columns that lands on the
+// accumulators of the weights i + j.
+//   FP64 (NSL = 8): digits (sliced_common.cuh) of determinants (rows of A) and columns of G under their own
+//       largest elements; a tile sums at most 8 pairs of 64 states, 2^23, exactly, and the eight weights
+//       of a sum become one 96-bit integer, rounded once.  An error of at most K 1.003 2^-59 2^(eP + eJ) where
+//       an FP64 sum has K 2^-53 sum |z||G|: one more piece holds magnitudes, their products show from
+//       below where the first bound could exceed the second, and those elements are formed by FP64
+//       FMAs.  The magnitudes go first, to the accumulators of weight 0, and digit 0 of A, the only one that
+//       adds there, last: they are read meanwhile.
+//   FP32 (NSL = 3): an FP32 number is the sum of three BF16 numbers of falling size, whatever its size; six
+//       products with FP32 accumulators leave out less than 2^-23 |z||G| each.  Results that are not finite
+//       are formed again by FP32 FMAs (infinities meet the zeros of the smaller parts).
 // The results of a tile are staged in shared memory and added to the gradient rows with the lanes along
 // the outputs of a row: additions by a lane per row (one 32-byte sector each) held up the gathers on
-// the way to L2, 13.5 against 11.9 ms at the FP32 size below; one bulk reduction per row was slower
-// than either (12.9 ms, and 9.9 against 7.6 at the FP64 size, whose rows are not 16-byte units).
+// the way to L2, 13.5 against 11.9 ms with six pieces at the FP32 size below; one bulk reduction per row was
+// slower than either (12.9 ms, and 9.9 against 7.6 at the FP64 size, whose rows are not 16-byte units).
 //
 // A CTA (persistent), 16 or 20 warps: 8-11 gather (ring of 16 KB slots: 128 couplings x 64 elements,
-// K-major, 128-byte swizzle), 12 issues the MMAs, 13 and up make the digits of the next unit's G, 0-7
+// K-major, 128-byte swizzle), 12 issues the MMAs, 13 and up make the pieces of the next unit's G, 0-7
 // collect and add.
 //
 // What bounds it: FP64, the collection, about 75 integer operations a result, and the FP64 additions in
-// L2; FP32, the gathers, 96 KB a tile for 60 states, and the MMAs (3 500 cycles a tile, of about 5 500).
-// Measured, all indices of a fragment: FP64 24 spin orbitals, 21 states 48.6 (FP64 FMAs) -> 4.4 ms; FP64
-// 18 spin orbitals, 10 states 3.5 -> 0.53 ms; FP32 28 spin orbitals, 60 states 16.4 (TF32 x 3) -> 11.7 ms.
+// L2; FP32, the gathers, 48 KB a tile for 60 states, and the additions in L2.
+// Measured, all indices of a fragment: FP64 24 spin orbitals, 21 states 48.6 (FP64 FMAs) -> 5.2 ms (4.4 without
+// the magnitudes, 4.9 with no element to form in FP64); FP64 18 spin orbitals, 10 states 3.5 -> 0.6 ms; FP32
+// 28 spin orbitals, 60 states 16.4 (TF32 x 3) -> 7.6 ms (46-bit digits, six pieces: 11.7).
 // Every wait is bounded; on timeout *status is set and all roles leave after their copies and MMAs
 // have completed.
 #include "sliced_common.cuh"
 #include "tc_common.cuh"
+#include <cuda_bf16.h>
 #include <type_traits>
 
 namespace {
@@ -41,30 +48,31 @@ constexpr uint32_t AS_SLOT = AS_M * 128;
 
 template <int NPAD, int NSL>
 struct Cfg {
-    static constexpr int PER = 64 / NPAD;                              // slices per 128-byte row chunk
-    static constexpr int CHUNKS = (NSL + PER - 1) / PER;               // chunks of a tile
-    static constexpr int ROW = CHUNKS * 128;                           // bytes of a determinant's digit row
-    static constexpr int GROW = NPAD == 32 ? 64 : 128;                 // bytes of a row of B: (slice, output)
-    static constexpr uint32_t GBYTES = (uint32_t)NSL * NPAD * GROW;    // one buffer of it
+    static constexpr int MAG = NSL == 8 ? 1 : 0;                       // a piece of magnitudes
+    static constexpr int PER = 64 / NPAD;                              // pieces per 128-byte row chunk
+    static constexpr int CHUNKS = (NSL + MAG + PER - 1) / PER;         // chunks of a tile
+    static constexpr int ROW = CHUNKS * 128;                           // bytes of a determinant's row
+    static constexpr int GROW = NPAD == 32 ? 64 : 128;                 // bytes of a row of B: (piece, output)
+    static constexpr uint32_t GBYTES = (uint32_t)(NSL + MAG) * NPAD * GROW;        // one buffer of it
     static constexpr int NBUF = NPAD == 64 && NSL == 8 ? 1 : 2;        // buffers of B
     static constexpr int ESIZE = NSL == 8 ? 8 : 4;                     // bytes of a result
     static constexpr int SROW = NPAD * ESIZE + (NSL == 8 ? 8 : 16);                   // bytes of a staged row of results
-    static constexpr int SLOTS = NPAD == 64 ? 5 : (NPAD == 32 && NSL == 8 ? 2 : 3);
+    static constexpr int SLOTS = NPAD == 64 ? (NSL == 8 ? 5 : 8) : (NPAD == 32 && NSL == 8 ? 2 : 3);
     static constexpr uint32_t SMEM = NBUF * GBYTES + SLOTS * AS_SLOT + AS_M * SROW + 1024;
     static constexpr int CTAS = NPAD == 64 ? 1 : 2;
-    static constexpr int DIG = NPAD == 64 ? 7 : 3;                     // warps that make digits of G
+    static constexpr int DIG = NPAD == 64 ? 7 : 3;                     // warps that make the pieces of G
     static constexpr int THREADS = AS_EPI + AS_PROD + 32 + DIG * 32;
-    static constexpr uint32_t COLS = NPAD == 64 ? 512 : 8 * NPAD;      // TMEM columns (a power of two)
-    static constexpr int CW = NPAD / 2;
+    static constexpr uint32_t COLS = (NSL == 8 ? 8 : 4) * NPAD;        // TMEM columns (a power of two)
+    static constexpr int CW = NPAD / 2;                                // output columns per epilogue thread
     // registers: 640 threads x 96 (one CTA an SM) or 512 x 64 (two) at launch
     static constexpr int EPI_REGS = CTAS == 2 ? 80 : (NSL == 8 ? 168 : 152);
-    static constexpr int IO_REGS = CTAS == 1 && NSL == 6 ? 56 : 48;
+    static constexpr int IO_REGS = CTAS == 1 && NSL == 3 ? 56 : 48;
     static_assert(AS_EPI * EPI_REGS + (THREADS - AS_EPI) * IO_REGS <= THREADS * (CTAS == 1 ? 96 : 64),
                   "register split exceeds the launch");
 };
 
 template <int N>
-__device__ __forceinline__ bool all_digit(bool x) {        // barrier of the warps that make digits of G
+__device__ __forceinline__ bool all_digit(bool x) {        // barrier of the warps that make the pieces of G
     int r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 3, %2, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
@@ -122,13 +130,18 @@ __device__ __forceinline__ void tmem_wait(float (&v)[32]) {
                  : "memory");
 }
 
-__device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }      // -126 <= e <= 127
-
 __device__ __forceinline__ void tmem_ld4(uint32_t ta, float* v) {         // v is there after a wait
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
                  : "r"(ta)
                  : "memory");
+}
+
+// The bits of x rounded to BF16, which is taken off x (exactly).
+__device__ __forceinline__ uint32_t bf16_part(float& x) {
+    const __nv_bfloat16 h = __float2bfloat16_rn(x);
+    x = __fsub_rn(x, __bfloat162float(h));
+    return __bfloat16_as_ushort(h);
 }
 
 template <typename T>
@@ -150,14 +163,15 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
     const uint32_t gsm = (smem_u32(smem_raw) + 1023u) & ~1023u, ring = gsm + C::NBUF * C::GBYTES;
     const uint32_t stage = ring + C::SLOTS * AS_SLOT;  // [row][output] results of a tile, on their way to memory
     __shared__ __align__(8) uint64_t full_bar[C::SLOTS], empty_bar[C::SLOTS];
-    __shared__ __align__(8) uint64_t ready_bar, drained_bar, gfull_bar[2], gfree_bar[2], done_bar;
+    __shared__ __align__(8) uint64_t ready_bar, drained_bar, mag_ready_bar, mag_drained_bar, gfull_bar[2], gfree_bar[2], done_bar;
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_sh;
     __shared__ int s_src[2][AS_M];                     // gathered rows of a tile (producers)
     __shared__ int s_dst[AS_M];                        // output rows of a tile (epilogue)
-    __shared__ int s_max[2][64];                       // exponents of the columns of G
-    __shared__ float2 s_scale[2][F64 ? 1 : 64];        // factor of a column's sums, as a product of two floats
-    __shared__ int s_bad[2];                           // an infinity or a NaN in G or its states
+    __shared__ int s_max[2][F64 ? 64 : 1];             // exponents of the columns of G (biased)
+    __shared__ int s_bad[2];                           // an infinity or a NaN in G (FP64)
+    __shared__ uint32_t s_low[2][F64 ? AS_M : 1];      // elements of a tile to form in FP64
+    __shared__ uint16_t s_odd[AS_EPI / 32][F64 ? 64 : 1];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (tid == 0) {
         for (int s = 0; s < C::SLOTS; ++s) {
@@ -166,6 +180,8 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
         }
         mbar_init(smem_u32(&ready_bar), 1);
         mbar_init(smem_u32(&drained_bar), AS_EPI / 32);
+        mbar_init(smem_u32(&mag_ready_bar), 1);
+        mbar_init(smem_u32(&mag_drained_bar), AS_EPI / 32);
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&gfull_bar[b]), C::DIG);
             mbar_init(smem_u32(&gfree_bar[b]), 2);     // the MMAs and the epilogue of the unit
@@ -213,19 +229,38 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                         fence_copies();
                         tc_fence_after();
                         const uint64_t da = umma_desc_sw128(ring + s * AS_SLOT);
-#pragma unroll
-                        for (int p = 0; p < C::PER; ++p) {
-                            const int i = k * C::PER + p;
-                            if (i >= NSL) break;
-                            const int n = (NSL - i) * NPAD, n1 = n < 256 ? n : 256;
+                        // columns [c0, c0 + n) from B's row c0 - NPAD i on, piece p of this chunk
+                        auto mma = [&](int p, int c0, int from, int n, uint32_t later) {
 #pragma unroll
                             for (int ks = 0; ks < NPAD / 16; ++ks) {
-                                const uint64_t a = da + (uint64_t)((p * NPAD * 2 + ks * 32) >> 4), b = db + 2 * ks;
-                                const uint32_t acc = (i > 0 || ks > 0) ? 1u : 0u;
-                                umma<0>(tmem + i * NPAD, a, b, idesc0 | ((uint32_t)(n1 / 8) << 17), acc);
+                                const uint64_t a = da + (uint64_t)((p * NPAD * 2 + ks * 32) >> 4), b = db + (uint64_t)((from * C::GROW) >> 4) + 2 * ks;
+                                const uint32_t acc = ks > 0 ? 1u : later;
+                                const int n1 = n < 256 ? n : 256;
+                                umma<0>(tmem + c0, a, b, idesc0 | ((uint32_t)(n1 / 8) << 17), acc);
                                 if (n > 256)
-                                    umma<0>(tmem + i * NPAD + 256, a, b + (uint64_t)((256 * C::GROW) >> 4),
+                                    umma<0>(tmem + c0 + 256, a, b + (uint64_t)((256 * C::GROW) >> 4),
                                             idesc0 | ((uint32_t)((n - 256) / 8) << 17), acc);
+                            }
+                        };
+#pragma unroll
+                        for (int p = 0; p < C::PER; ++p) {
+                            const int at = k * C::PER + p;               // FP64: magnitudes, digits 1 .. 7, digit 0
+                            if (at >= NSL + C::MAG) break;
+                            if (!F64) {
+                                mma(p, at * NPAD, 0, (NSL - at) * NPAD, at > 0 ? 1u : 0u);
+                            } else if (at == 0) {
+                                mma(p, 0, NSL * NPAD, NPAD, 0u);
+                                umma_commit(smem_u32(&mag_ready_bar));
+                            } else if (at < NSL) {
+                                mma(p, at * NPAD, 0, (NSL - at) * NPAD, at > 1 ? 1u : 0u);
+                            } else {
+                                if (!mbar_wait(smem_u32(&mag_drained_bar), tile & 1u, &abort_sh)) {
+                                    ok = false;
+                                    break;
+                                }
+                                tc_fence_after();
+                                mma(p, 0, 0, NPAD, 0u);
+                                mma(p, NPAD, NPAD, (NSL - 1) * NPAD, 1u);
                             }
                         }
                         umma_commit(smem_u32(&empty_bar[s]));
@@ -241,7 +276,7 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
             umma_commit(smem_u32(&done_bar));
             mbar_wait(smem_u32(&done_bar), 0u, nullptr);
         } else if (warp > 12) {
-            // ------------------------------------------------------------ digits of G --
+            // ------------------------------------------------------------ pieces of G --
             // an item: OL outputs along the lanes, KC consecutive contracted states per lane
             constexpr int OL = NPAD < 32 ? NPAD : 32, KC = 4, KL = 32 / OL;
             constexpr int ITEMS = (NPAD / OL) * (NPAD / (KC * KL));
@@ -255,10 +290,11 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                     if (!__all_sync(0xffffffffu, free)) ok = false;
                 }
                 if (dw == 0) {
-                    for (int o = lane; o < 64; o += 32) s_max[b][o] = -100000;
+                    if constexpr (F64)
+                        for (int o = lane; o < 64; o += 32) s_max[b][o] = 1;
                     if (lane == 0) s_bad[b] = 0;
                 }
-                ok = all_digit<C::DIG * 32>(ok);                        // (the three warps go on or stop together)
+                ok = all_digit<C::DIG * 32>(ok);                        // (these warps go on or stop together)
                 if (!ok) break;
                 const xrh_dens_sliced_unit U = units[u];
                 const xrh_adj_sliced_task& T = tasks[U.task];
@@ -266,64 +302,63 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                 const int i0 = U.iblk * 64, j0 = U.jblk * 64;
                 const int nk_ = bra ? T.nk - j0 : T.nb - i0, no_ = bra ? T.nb - i0 : T.nk - j0;
                 const int n_con = nk_ < NPAD ? nk_ : NPAD, n_out = no_ < NPAD ? no_ : NPAD;
-                const uint32_t* ecoef = bra ? T.ek + j0 : T.eb + i0;
                 const double* g = T.gT + ((int64_t)U.idx * T.nb + i0) * T.nk + j0;
                 const int64_t so = bra ? T.nk : 1, sk = bra ? 1 : T.nk;
-                // x and the exponent (biased as FP64's) of x 2^e_k
-                auto load = [&](int item, double (&x)[KC], int (&ex)[KC], int& o, int& k0) {
+                auto load = [&](int item, double (&x)[KC], int& o, int& k0) {
                     o = (item % (NPAD / OL)) * OL + lane % OL;
                     k0 = (item / (NPAD / OL) * KL + lane / OL) * KC;
-                    bool odd = false;
 #pragma unroll
-                    for (int k = 0; k < KC; ++k) {
-                        const bool in = o < n_out && k0 + k < n_con;
-                        x[k] = in ? g[o * so + (k0 + k) * sk] : 0.0;
-                        const uint32_t we = in ? ecoef[k0 + k] >> 20 : 0u, wx = abs_hi(x[k]) >> 20;
-                        odd = odd || we >= 2047u || wx >= 2047u;
-                        ex[k] = (int)(wx < 1u ? 1u : wx) + (int)(we < 1u ? 1u : we) - 1022;
-                    }
-                    return odd;
+                    for (int k = 0; k < KC; ++k) x[k] = o < n_out && k0 + k < n_con ? g[o * so + (k0 + k) * sk] : 0.0;
                 };
+                if constexpr (F64) {
 #pragma unroll 1
-                for (int item = dw; item < ITEMS; item += C::DIG) {
-                    double x[KC];
-                    int ex[KC], o, k0, top = -100000;
-                    if (load(item, x, ex, o, k0)) s_bad[b] = 1;
+                    for (int item = dw; item < ITEMS; item += C::DIG) {
+                        double x[KC];
+                        int o, k0, top = 0;
+                        load(item, x, o, k0);
 #pragma unroll
-                    for (int k = 0; k < KC; ++k)
-                        if (x[k] != 0.0 && ex[k] > top) top = ex[k];
-                    if (top > -100000) atomicMax(&s_max[b][o], top);
-                }
-                asm volatile("bar.sync 3, %0;" ::"n"(C::DIG * 32) : "memory");
-                const bool bad = s_bad[b] != 0;
-                if (!F64 && dw == 0) {
-                    for (int o = lane; o < NPAD; o += 32) {
-                        int e = s_max[b][o] - 1022 - 12;
-                        e = e < -250 ? -250 : (e > 250 ? 250 : e);
-                        s_scale[b][o] = make_float2(pow2f(e / 2), pow2f(e - e / 2));
+                        for (int k = 0; k < KC; ++k) top = max(top, (int)(abs_hi(x[k]) >> 20));
+                        if (top >= 2047) s_bad[b] = 1;
+                        if (top > 0) atomicMax(&s_max[b][o], top);
                     }
+                    asm volatile("bar.sync 3, %0;" ::"n"(C::DIG * 32) : "memory");
                 }
+                const bool bad = F64 && s_bad[b] != 0;
 #pragma unroll 1
                 for (int item = dw; item < ITEMS; item += C::DIG) {
                     double x[KC];
-                    int ex[KC], o, k0;
-                    load(item, x, ex, o, k0);
-                    const int E = s_max[b][o];
-                    uint64_t v[KC];
-#pragma unroll
-                    for (int k = 0; k < KC; ++k)
-                        v[k] = bad || x[k] == 0.0 ? 0x0080808080808080ull
-                                                  : fixed62(x[k], E - (ex[k] - (int)max(1u, abs_hi(x[k]) >> 20)));
-#pragma unroll
-                    for (int t = 0; t < NSL; ++t) {
+                    int o, k0;
+                    load(item, x, o, k0);
+                    // four BF16 numbers of piece t
+                    auto put = [&](int t, uint32_t q0, uint32_t q1) {
                         const uint32_t r = (uint32_t)(t * NPAD + o), kk = (uint32_t)k0;
                         const uint32_t sw = NPAD == 32 ? (r >> 1) & 3u : r & 7u;
                         const uint32_t dst = gsm + b * C::GBYTES + r * C::GROW + (((kk >> 3) ^ sw) << 4) + (kk & 7u) * 2u;
-                        uint32_t q[KC / 2];
+                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"(q0), "r"(q1) : "memory");
+                    };
+                    if constexpr (F64) {
+                        const int E = s_max[b][o];
+                        uint64_t v[KC];
+                        uint32_t m[KC];
 #pragma unroll
-                        for (int k = 0; k < KC / 2; ++k)
-                            q[k] = __byte_perm(digit_float(v[2 * k], t), digit_float(v[2 * k + 1], t), 0x7632);
-                        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(dst), "r"(q[0]), "r"(q[1]) : "memory");
+                        for (int k = 0; k < KC; ++k) {
+                            v[k] = bad ? 0x0080808080808080ull : fixed62(x[k], E);
+                            m[k] = bad ? 0u : magnitude(x[k], E);
+                        }
+#pragma unroll
+                        for (int t = 0; t < NSL; ++t)
+                            put(t, __byte_perm(digit_float(v[0], t), digit_float(v[1], t), 0x7632),
+                                __byte_perm(digit_float(v[2], t), digit_float(v[3], t), 0x7632));
+                        put(NSL, m[0] | (m[1] << 16), m[2] | (m[3] << 16));
+                    } else {
+                        float f[KC];
+#pragma unroll
+                        for (int k = 0; k < KC; ++k) f[k] = xrh_f64_to_f32(x[k]);
+#pragma unroll
+                        for (int t = 0; t < NSL; ++t) {
+                            const uint32_t q0 = bf16_part(f[0]) | (bf16_part(f[1]) << 16), q1 = bf16_part(f[2]) | (bf16_part(f[3]) << 16);
+                            put(t, q0, q1);
+                        }
                     }
                 }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -362,12 +397,13 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                         if (!__all_sync(0xffffffffu, free)) ok = false;
                     }
                     if (ok) {
-                        // 8 lanes per 128-byte row piece, 16 rows at a time
+                        // 8 lanes per 128-byte row chunk, 16 rows at a time (the last chunk may be filled in part)
+                        const int used = (NSL + C::MAG - k * C::PER) * (NPAD / 8);
 #pragma unroll
                         for (int i = 0; i < 8; ++i) {
                             const int r = i * 16 + pw * 4 + (lane >> 3), c16 = lane & 7;
                             const int row = src[r];
-                            cp_async16_or_zero(ring + s * AS_SLOT + (uint32_t)r * 128u + (uint32_t)((c16 ^ (r & 7)) << 4),
+                            if (c16 < used) cp_async16_or_zero(ring + s * AS_SLOT + (uint32_t)r * 128u + (uint32_t)((c16 ^ (r & 7)) << 4),
                                                rows + (int64_t)(row < 0 ? 0 : row) * C::ROW + k * 128 + c16 * 16, row >= 0);
                         }
                     }
@@ -403,7 +439,9 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
             const double* g = T.gT + ((int64_t)U.idx * T.nb + i0) * T.nk + j0;             // G[i][j], row stride nk
             const int64_t so = bra ? T.nk : 1, sk = bra ? 1 : T.nk;
             // ---- tiles ----
-            const int32_t* out_list = (bra ? T.P : T.Q) + U.c0;
+            const int32_t *out_list = (bra ? T.P : T.Q) + U.c0, *in_list = (bra ? T.Q : T.P) + U.c0;
+            const uint32_t* row_exps = (bra ? T.ek + U.jblk * T.conf_k : T.eb + U.iblk * T.conf_b);      // (FP64)
+            int next_src = F64 && row < U.count ? __ldg(in_list + row) : -1;
             const int64_t n_row = bra ? T.nb : T.nk;
             const int o0 = bra ? i0 : j0;
             const int n_tiles = (U.count + AS_M - 1) / AS_M;
@@ -413,6 +451,37 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                 // this tile's output rows (loaded during the tile before)
                 if (tid < AS_M) s_dst[tid] = next_dst;
                 if (tid < AS_M) next_dst = (q + 1) * AS_M + tid < U.count ? __ldg(out_list + (q + 1) * AS_M + tid) : -1;
+                uint32_t low = 0u, er = 0u;            // bit 4 p + j: column 8 p + 4 part + j; the row's largest element
+                if constexpr (F64) {
+                    if (next_src >= 0) er = __ldg(row_exps + next_src);
+                    next_src = (q + 1) * AS_M + row < U.count ? __ldg(in_list + (q + 1) * AS_M + row) : -1;
+                    if (!failed && !mbar_wait(smem_u32(&mag_ready_bar), tile & 1u, &abort_sh)) {
+                        failed = true;
+                        abort_sh = 1;
+                    }
+                    if (!failed) {
+                        tc_fence_after();
+#pragma unroll 1
+                        for (int p = 0; p < NPAD / 8; p += 2) {
+                            float v[2][4];
+#pragma unroll
+                            for (int h = 0; h < 2; ++h) tmem_ld4(tmem + lane_base + (uint32_t)(8 * (p + h) + 4 * part), v[h]);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                                for (int j = 0; j < 4; ++j) {
+                                    asm volatile("" : "+f"(v[h][j]));          // (not before the wait)
+                                    low |= (low_sum(v[h][j]) ? 1u << (4 * h + j) : 0u) << (4 * p);
+                                }
+                        }
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(smem_u32(&mag_drained_bar));
+                    }
+                    if (bad || (er >> 20) >= 2047u) low = 0xffffffffu;
+                    s_low[part][row] = low;
+                }
                 if (!failed && !mbar_wait(smem_u32(&ready_bar), tile & 1u, &abort_sh)) {
                     failed = true;
                     abort_sh = 1;
@@ -449,20 +518,9 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                                 x[w] = v[w][j];
                             }
                             if constexpr (NSL == 8) t[j] = collect_weights<NPAD>(x);
-                            te[j] = s_max[b][J + j] - 1022;
+                            te[j] = s_max[b][J + j] - 1022 + exp_of(er);
                         }
                         sliced_to_doubles<4>(t, te, y);
-                        if (bad && d >= 0) {
-                            // an infinity or a NaN in G or the states: the products in FP64
-                            const double* z = bra ? T.zkT + (int64_t)T.Q[U.c0 + q * AS_M + row] * T.nk + j0
-                                                  : T.zbT + (int64_t)T.P[U.c0 + q * AS_M + row] * T.nb + i0;
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                y[j] = 0.0;
-#pragma unroll 1
-                                for (int k = 0; k < n_con && J + j < n_out; ++k) y[j] = fma(z[k], g[(J + j) * so + k * sk], y[j]);
-                            }
-                        }
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             if (neg) y[j] = -y[j];
@@ -476,33 +534,32 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                     // the sums of this thread's columns into registers, the accumulators back to the MMA
                     // warp, then scaling and additions while the next tile is multiplied
                     float acc[C::CW];
-#pragma unroll
-                    for (int j = 0; j < C::CW; ++j) acc[j] = 0.f;
-                    if constexpr (NPAD == 64) {        // two weights in flight
+                    if constexpr (NPAD == 64) {
                         float va[32], vb[32];
                         const uint32_t t0 = tmem + lane_base + (uint32_t)(part * 32);
-                        tmem_ld32(t0 + (NSL - 1) * 64, va);
+                        tmem_ld32(t0 + 2 * 64, va);
+                        tmem_wait(va);
+                        tmem_ld32(t0 + 64, vb);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) acc[j] = va[j];
+                        tmem_wait(vb);
+                        tmem_ld32(t0, va);
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) acc[j] += vb[j];
                         tmem_wait(va);
 #pragma unroll
-                        for (int w = NSL - 1; w > 0; w -= 2) {
-                            tmem_ld32(t0 + (w - 1) * 64, vb);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) acc[j] = fmaf(acc[j], 0.00390625f, va[j]);
-                            tmem_wait(vb);
-                            if (w > 1) tmem_ld32(t0 + (w - 2) * 64, va);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) acc[j] = fmaf(acc[j], 0.00390625f, vb[j]);
-                            if (w > 1) tmem_wait(va);
-                        }
+                        for (int j = 0; j < 32; ++j) acc[j] += va[j];
                     } else {
-#pragma unroll 1
+#pragma unroll
+                        for (int j = 0; j < C::CW; ++j) acc[j] = 0.f;
+#pragma unroll
                         for (int w = NSL - 1; w >= 0; --w) {
 #pragma unroll
                             for (int h = 0; h < C::CW; h += 8) {
                                 float v[8];
                                 tmem_ld8(tmem + lane_base + (uint32_t)(w * NPAD + part * C::CW + h), v);
 #pragma unroll
-                                for (int j = 0; j < 8; ++j) acc[h + j] = fmaf(acc[h + j], 0.00390625f, v[j]);
+                                for (int j = 0; j < 8; ++j) acc[h + j] += v[j];
                             }
                         }
                     }
@@ -516,9 +573,12 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                         if (J < n_out) {
                             float v[4];
 #pragma unroll
-                            for (int j = 0; j < 4; ++j) v[j] = (acc[h + j] * s_scale[b][J + j].x) * (sg * s_scale[b][J + j].y);
-                            if (bad && d >= 0) {
-                                // an infinity or a NaN in G or the states: FP32 products of the operands
+                            for (int j = 0; j < 4; ++j) v[j] = sg * acc[h + j];
+                            bool odd = false;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) odd = odd || (__float_as_uint(v[j]) & 0x7f800000u) == 0x7f800000u;
+                            if (odd && d >= 0) {
+                                // FP32 products of the operands
                                 const double* z = bra ? T.zkT + (int64_t)T.Q[U.c0 + q * AS_M + row] * T.nk + j0
                                                       : T.zbT + (int64_t)T.P[U.c0 + q * AS_M + row] * T.nb + i0;
 #pragma unroll
@@ -535,10 +595,44 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
                         }
                     }
                 }
-                epi_bar();                             // the tile is staged
+                const bool any_odd = epi_bar_or(low != 0u) != 0;       // also: the tile is staged
                 // a warp adds 16 rows, lanes along the outputs of a row: whole sectors in every addition
                 const int to_lane = s_dst[warp * 16 + (lane & 15)];
                 const uint32_t rows = stage + (uint32_t)(warp * 16) * C::SROW;
+                if constexpr (F64) {
+                    if (any_odd) {
+                        // elements of these rows the digits are too coarse for, or with an infinity or a NaN: in
+                        // FP64 in place of what is staged, 32 at a time
+                        auto redo = [&](int e) {
+                            const int r = warp * 16 + e / NPAD, J = e % NPAD;
+                            const int c = in_list[q * AS_M + r];
+                            const double* z = bra ? T.zkT + (int64_t)c * T.nk + j0 : T.zbT + (int64_t)c * T.nb + i0;
+                            double y = 0.0;
+#pragma unroll 4
+                            for (int k = 0; k < n_con; ++k) y = fma(z[k], g[J * so + k * sk], y);
+                            if (q * AS_M + r >= n_pos) y = -y;
+                            asm volatile("st.shared.f64 [%0], %1;" ::"r"(rows + (uint32_t)((e / NPAD) * C::SROW + J * 8)), "d"(y) : "memory");
+                        };
+                        int n = 0;
+#pragma unroll 1
+                        for (int i = 0; i < NPAD / 2; ++i) {
+                            const int e = i * 32 + lane, r = warp * 16 + e / NPAD, J = e % NPAD;
+                            const bool odd = s_dst[r] >= 0 && J < n_out && ((s_low[(J >> 2) & 1][r] >> (4 * (J >> 3) + (J & 3))) & 1u);
+                            const uint32_t m = __ballot_sync(0xffffffffu, odd);
+                            if (odd) s_odd[warp][n + __popc(m & ((1u << lane) - 1u))] = (uint16_t)e;
+                            n += __popc(m);
+                            __syncwarp();
+                            if (n >= 32 || (i == NPAD / 2 - 1 && n > 0)) {
+                                const int take = n < 32 ? n : 32;
+                                if (lane < take) redo(s_odd[warp][n - take + lane]);
+                                n -= take;
+                                __syncwarp();
+                                if (i == NPAD / 2 - 1 && lane < n) redo(s_odd[warp][lane]);
+                            }
+                        }
+                        __syncwarp();
+                    }
+                }
                 unsigned char* out = reinterpret_cast<unsigned char*>(bra ? T.gzb : T.gzk) + o0 * C::ESIZE;
                 if (!F64 && vec) {
 #pragma unroll
@@ -582,6 +676,71 @@ __global__ void __launch_bounds__(Cfg<NPAD, NSL>::THREADS, Cfg<NPAD, NSL>::CTAS)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::COLS) : "memory");
 }
 
+// ---- rows of the state coefficients ---------------------------------------------------------
+constexpr int CR_ROWS = 64;                            // determinants per CTA
+
+// [block of 64 states][determinant][piece][npad]: a thread per (determinant, 8 states)
+__global__ void __launch_bounds__(256) coeff_rows_kernel(const xrh_coeff_digit_task* __restrict__ tasks, int n_tasks) {
+    int lo = 0, hi = n_tasks - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tasks[mid].cta_begin <= (int64_t)blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    const xrh_coeff_digit_task& T = tasks[lo];
+    const int64_t r0 = ((int64_t)blockIdx.x - T.cta_begin) * CR_ROWS;
+    const int rows = T.n_conf - r0 < CR_ROWS ? (int)(T.n_conf - r0) : CR_ROWS;
+    const bool f64 = T.slices == NS;
+    const int blocks = (T.n + T.npad - 1) / T.npad, oct = T.npad / 8, per = blocks * oct, chunk = 64 / T.npad;
+    const int pieces = (f64 ? NS + chunk : 2 + chunk) / chunk * chunk;           // 9 or 3, to whole 128 bytes
+    const uint32_t group = (oct == 8 ? 0xffu : (1u << oct) - 1u) << ((threadIdx.x & 31) & ~(oct - 1));
+    for (int x = threadIdx.x; x < rows * per; x += 256) {
+        const int r = x / per, o = x - r * per, blk = o / oct, oo = o - blk * oct, s0 = blk * T.npad + oo * 8;
+        const double* z = T.zT + (r0 + r) * T.n;
+        double v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = s0 + k < T.n ? __ldg(z + s0 + k) : 0.0;
+        uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(T.digits) + ((int64_t)blk * T.n_conf + r0 + r) * (pieces * T.npad)) + oo;
+        if (f64) {
+            uint32_t top = 0u;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) top = max(top, abs_hi(v[k]));
+            for (int w = oct / 2; w > 0; w >>= 1) top = max(top, __shfl_xor_sync(group, top, w));
+            if (oo == 0) T.exps[(int64_t)blk * T.n_conf + r0 + r] = top;
+            const bool bad = (top >> 20) >= 2047u;
+            const int E = (top >> 20) < 1u ? 1 : (int)(top >> 20);
+            uint64_t f[8];
+            uint32_t m[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                f[k] = bad ? 0x0080808080808080ull : fixed62(v[k], E);
+                m[k] = bad ? 0u : magnitude(v[k], E);
+            }
+            dst[0] = make_uint4(m[0] | (m[1] << 16), m[2] | (m[3] << 16), m[4] | (m[5] << 16), m[6] | (m[7] << 16));
+#pragma unroll
+            for (int t = 0; t < NS; ++t) {
+                uint32_t q[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) q[k] = __byte_perm(digit_float(f[2 * k], t), digit_float(f[2 * k + 1], t), 0x7632);
+                dst[(t == 0 ? NS : t) * oct] = make_uint4(q[0], q[1], q[2], q[3]);
+            }
+        } else {
+            float f[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) f[k] = xrh_f64_to_f32(v[k]);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                uint32_t q[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t a = bf16_part(f[2 * k]);
+                    q[k] = a | (bf16_part(f[2 * k + 1]) << 16);
+                }
+                dst[t * oct] = make_uint4(q[0], q[1], q[2], q[3]);
+            }
+        }
+    }
+}
+
 template <int NPAD, int NSL>
 int launch(const xrh_adj_sliced_task* tasks, const xrh_dens_sliced_unit* units, int64_t n_units, int32_t* status,
            cudaStream_t s) {
@@ -598,6 +757,16 @@ int launch(const xrh_adj_sliced_task* tasks, const xrh_dens_sliced_unit* units, 
 
 }  // namespace
 
+extern "C" int xrh_coeff_rows(const xrh_coeff_digit_task* tasks_dev, int n_tasks, int64_t total_ctas, void* stream) {
+    if (n_tasks < 0 || total_ctas < 0) return XRH_ERR_ARG;
+    if (n_tasks == 0 || total_ctas == 0) return XRH_OK;
+    if (!tasks_dev) return XRH_ERR_ARG;
+    if (total_ctas > 0x7fffffffLL) return XRH_ERR_CAPACITY;
+    coeff_rows_kernel<<<(unsigned)total_ctas, 256, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
+    XRH_CHECK_LAUNCH();
+    return XRH_OK;
+}
+
 extern "C" int xrh_density_adjoint_sliced_grouped(int precision, const xrh_adj_sliced_task* tasks_dev, int n_tasks,
                                                   const xrh_dens_sliced_unit* units_dev, int64_t n_units, int npad,
                                                   int32_t* status_dev, void* stream) {
@@ -611,7 +780,7 @@ extern "C" int xrh_density_adjoint_sliced_grouped(int precision, const xrh_adj_s
         if (npad == 32) return launch<32, 8>(tasks_dev, units_dev, n_units, status_dev, s);
         return launch<64, 8>(tasks_dev, units_dev, n_units, status_dev, s);
     }
-    if (npad == 16) return launch<16, 6>(tasks_dev, units_dev, n_units, status_dev, s);
-    if (npad == 32) return launch<32, 6>(tasks_dev, units_dev, n_units, status_dev, s);
-    return launch<64, 6>(tasks_dev, units_dev, n_units, status_dev, s);
+    if (npad == 16) return launch<16, 3>(tasks_dev, units_dev, n_units, status_dev, s);
+    if (npad == 32) return launch<32, 3>(tasks_dev, units_dev, n_units, status_dev, s);
+    return launch<64, 3>(tasks_dev, units_dev, n_units, status_dev, s);
 }

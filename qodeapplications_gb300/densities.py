@@ -324,35 +324,13 @@ def _coupling_units(cp):
     return units, bool((nu > 1).any())
 
 
-class CoeffDigits:
-    """Digit rows of state coefficients for the sliced kernels (xrh_coeff_digits), per side and charge:
-    {(side, charge): (digits, exponent address, zT)}, the common pad width npad and the slices kept (all eight:
-    the magnitudes of the coefficients too)."""
+class StateTables:
+    """The coefficients of the sliced kernels: zT per side and charge, and the common pad width npad."""
 
-    def __init__(self, sides, device, slices=_lib.SLICES):
-        tabs = [((s, c), z) for s, zs in sides.items() for c, z in zs.items()]
-        n_max = max(z.shape[1] for _, z in tabs)
+    def __init__(self, sides):
+        self.tabs = [((s, c), z) for s, zs in sides.items() for c, z in zs.items()]
+        n_max = max(z.shape[1] for _, z in self.tabs)
         self.npad = 16 if n_max <= 16 else 32 if n_max <= 32 else 64
-        slices = -(-slices * self.npad // 64) * 64 // self.npad            # whole 128-byte row pieces
-        tab = np.zeros(len(tabs), dtype=_lib.COEFF_DIGIT_DTYPE)
-        self.exps = torch.zeros(sum(z.shape[1] for _, z in tabs), dtype=torch.int32, device=device)
-        self.of, e0, cta = {}, 0, 0
-        for e, (key, z) in zip(tab, tabs):
-            n_conf, n = z.shape
-            rows = -(-n // self.npad) * max(n_conf, 1)         # (eight slices: magnitudes and a mask behind the digits)
-            d = torch.empty(rows * (slices * self.npad + (self.npad + 4 if slices == _lib.SLICES else 0)), dtype=torch.bfloat16,
-                            device=device)
-            self.of[key] = (d, self.exps.data_ptr() + 4 * e0, z)
-            e["zT"], e["digits"], e["exps"], e["n_conf"] = z.data_ptr(), d.data_ptr(), self.of[key][1], n_conf
-            e["n"], e["npad"], e["slices"], e["cta_begin"] = n, self.npad, slices, cta
-            e0 += n
-            cta += _lib.lib().xrh_coeff_digit_ctas(n_conf)
-        self.n, self.ctas = len(tab), cta
-        self.dev = torch.from_numpy(tab.view(np.uint8).copy()).to(device)
-
-    def run(self, s):
-        _lib.zero_(self.exps)
-        call("xrh_coeff_digits", ptr(self.dev), self.n, self.ctas, s)
 
     def fill(self, t, bra, ket):
         """The operand fields of a task between sides bra and ket ((side, charge) keys)."""
@@ -360,6 +338,53 @@ class CoeffDigits:
         t["digb"], t["digk"], t["eb"], t["ek"] = db.data_ptr(), dk.data_ptr(), eb, ek
         t["zbT"], t["zkT"], t["conf_b"], t["conf_k"] = zb.data_ptr(), zk.data_ptr(), zb.shape[0], zk.shape[0]
         t["nb"], t["nk"] = zb.shape[1], zk.shape[1]
+
+    def _table(self, exps, slices, elements, device):
+        """Task table: `elements` BF16 numbers a determinant and block of states, exps(n_conf, blocks, n) exponents."""
+        tab = np.zeros(len(self.tabs), dtype=_lib.COEFF_DIGIT_DTYPE)
+        size = [(z.shape[0], -(-z.shape[1] // self.npad), z.shape[1]) for _, z in self.tabs]
+        self.exps = torch.zeros(max(sum(exps(*x) for x in size), 1), dtype=torch.int32, device=device)
+        self.of, e0, cta = {}, 0, 0
+        for e, (key, z), x in zip(tab, self.tabs, size):
+            d = torch.empty(max(x[0], 1) * x[1] * elements, dtype=torch.bfloat16, device=device)
+            self.of[key] = (d, self.exps.data_ptr() + 4 * e0, z)
+            e["zT"], e["digits"], e["exps"], e["n_conf"] = z.data_ptr(), d.data_ptr(), self.of[key][1], x[0]
+            e["n"], e["npad"], e["slices"], e["cta_begin"] = x[2], self.npad, slices, cta
+            e0 += exps(*x)
+            cta += _lib.lib().xrh_coeff_digit_ctas(x[0])
+        self.n, self.ctas = len(tab), cta
+        self.dev = torch.from_numpy(tab.view(np.uint8).copy()).to(device)
+
+
+class CoeffDigits(StateTables):
+    """Digit rows of state coefficients for the sliced kernels (xrh_coeff_digits), per side and charge:
+    {(side, charge): (digits, exponent address, zT)}, the common pad width npad and the slices kept (all eight:
+    the magnitudes of the coefficients too)."""
+
+    def __init__(self, sides, device, slices=_lib.SLICES):
+        super().__init__(sides)
+        slices = -(-slices * self.npad // 64) * 64 // self.npad            # whole 128-byte row pieces
+        # (eight slices: magnitudes and a mask behind the digits)
+        extra = self.npad + 4 if slices == _lib.SLICES else 0
+        self._table(lambda n_conf, blocks, n: n, slices, slices * self.npad + extra, device)
+
+    def run(self, s):
+        _lib.zero_(self.exps)
+        call("xrh_coeff_digits", ptr(self.dev), self.n, self.ctas, s)
+
+
+class CoeffRows(StateTables):
+    """The coefficients as rows of the density adjoint (xrh_coeff_rows): FP64 digits and magnitudes of every
+    determinant under its own largest coefficient, or FP32 numbers as three BF16 numbers."""
+
+    def __init__(self, states, precision, device):
+        self.tabs, self.npad = states.tabs, states.npad
+        slices, pieces = (_lib.SLICES, _lib.SLICES + 1) if precision == _lib.FP64 else (3, 3)
+        row = -(-pieces * self.npad // 64) * 64                            # whole 128-byte chunks
+        self._table(lambda n_conf, blocks, n: n_conf * blocks, slices, row, device)
+
+    def run(self, s):
+        call("xrh_coeff_rows", ptr(self.dev), self.n, self.ctas, s)
 
 
 def sliced_units(lists, directions=(0,)):
@@ -419,25 +444,27 @@ class SlicedDensities:
 
 class SlicedDensityAdjoint:
     """dE/dz from dE/drho on the tensor cores (xrh_density_adjoint_sliced_grouped) for blocks that share
-    one pad width.  blocks: [(couplings, coeff, bra key, ket key, gT, bra gradient, ket gradient)];
-    refresh: CoeffDigits to run first (those no density build keeps current)."""
+    one pad width.  blocks: [(couplings, states, bra key, ket key, gT, bra gradient, ket gradient)] (states:
+    StateTables); refresh: CoeffDigits to run first."""
 
     def __init__(self, blocks, precision, refresh, device):
         self.precision, self.refresh, self.keep = precision, list(refresh), blocks
         self.npad = blocks[0][1].npad
+        rows = {id(b[1]): b[1] for b in blocks}
+        self.rows = {k: CoeffRows(st, precision, device) for k, st in rows.items()}
         tasks = np.zeros(len(blocks), dtype=_lib.ADJ_SLICED_TASK_DTYPE)
         for t, (cp, coeff, bra, ket, gT, gzb, gzk) in zip(tasks, blocks):
             assert coeff.npad == self.npad
             t["P"], t["Q"], t["gT"] = cp.P.data_ptr(), cp.Q.data_ptr(), gT.data_ptr()
             t["gzb"], t["gzk"] = gzb.data_ptr(), gzk.data_ptr()
-            coeff.fill(t, bra, ket)
+            self.rows[id(coeff)].fill(t, bra, ket)
         units = sliced_units([(b[0], int(t["nb"]), int(t["nk"])) for b, t in zip(blocks, tasks)], (0, 1))
         self.n_tasks, self.n_units = len(tasks), len(units)
         self.tasks_dev, self.units_dev = _upload(tasks, device), _upload(units, device)
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
 
     def run(self, s):
-        for c in self.refresh:
+        for c in [*self.refresh, *self.rows.values()]:
             c.run(s)
         call("xrh_density_adjoint_sliced_grouped", self.precision, ptr(self.tasks_dev), self.n_tasks,
              ptr(self.units_dev), self.n_units, self.npad, ptr(self.status), s)

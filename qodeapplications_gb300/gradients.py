@@ -413,10 +413,9 @@ class XRDimerAdjoint:
 
     def _setup_sliced(self):
         """The transposed density gradients of self.dens_adj on the tensor cores: every block of the
-        FP64 path (digit rows of the forward builds), and on the FP32 path the blocks of more
-        states than the lane-per-coupling kernel takes (digit rows of 46 bits, made per reverse
-        pass).  State counts the CUDA-core kernels refuse keep their answer."""
-        from .densities import CoeffDigits, SlicedDensityAdjoint
+        FP64 path, and on the FP32 path the blocks of more states than the lane-per-coupling kernel
+        takes.  State counts the CUDA-core kernels refuse keep their answer."""
+        from .densities import SlicedDensityAdjoint, StateTables
         plan, dev = self.plan, self.plan.device
         self.dens_adj_sliced = []
         entries = [] if self.dens_adj_tc else self.dens_adj
@@ -430,7 +429,7 @@ class XRDimerAdjoint:
         for m in (0, 1):
             b = plan.builders[m]
             if self.prec32:
-                coeffs.append((CoeffDigits({"ket": b.zT} if b.zbT is b.zT else {"ket": b.zT, "bra": b.zbT}, dev, slices=6)
+                coeffs.append((StateTables({"ket": b.zT} if b.zbT is b.zT else {"ket": b.zT, "bra": b.zbT})
                                if any(e[0] == m for e in entries) else None))
             elif getattr(b, "sliced", None) is None:
                 return
@@ -439,12 +438,11 @@ class XRDimerAdjoint:
         by_pad = {}
         for (m, op, bc, kc, cp, rt, grho, gT) in entries:
             c = coeffs[m]
-            bra = ("bra" if ("bra", bc) in c.of else "ket", bc)
+            bra = ("bra" if ("bra", bc) in dict(c.tabs) else "ket", bc)
             gz = self.gz32[m] if self.prec32 else {x: self.G[("gzT", m, x)] for x in plan.charges[m]}
             by_pad.setdefault(c.npad, []).append((cp, c, bra, ("ket", kc), gT, gz[bc], gz[kc]))
         for blocks in by_pad.values():
-            refresh = list({id(b[1]): b[1] for b in blocks}.values()) if self.prec32 else []
-            self.dens_adj_sliced.append(SlicedDensityAdjoint(blocks, _lib.FP32 if self.prec32 else _lib.FP64, refresh, dev))
+            self.dens_adj_sliced.append(SlicedDensityAdjoint(blocks, _lib.FP32 if self.prec32 else _lib.FP64, [], dev))
         self.dens_adj_groups = []
 
     def _canonicalize(self, m=None):
