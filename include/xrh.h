@@ -364,9 +364,16 @@ typedef struct {
 } xrh_sliced_segment;   /* 128 bytes */
 int64_t xrh_slice_ctas(int64_t rows, int64_t K, int64_t batch, int trans, int block, int max_pass);
 int xrh_slice_grouped(const xrh_slice_task* tasks_dev, int n_tasks, int64_t total_ctas, int64_t max_ctas,
-                      void* stream);
+                      uint32_t* odd_list_dev, void* stream);
+/* Marks of the elements formed by FP64 arithmetic, one range per task: begin and runs per tile in units of 256
+ * words of odd_bits_dev (a run: the stages of a tile in one segment, at most 16 384).  odd_list_dev:
+ * 1 + total_tiles words, cleared by the xrh_slice_grouped in front of the GEMM. */
+typedef struct {
+    int64_t begin, runs;
+} xrh_odd_range;   /* 16 bytes */
 int xrh_gemm_sliced_grouped(const xrh_gemm_task* tasks_dev, int n_tasks, int64_t total_tiles,
-                            const xrh_sliced_segment* segs_dev, int32_t* status_dev, void* stream);
+                            const xrh_sliced_segment* segs_dev, const xrh_odd_range* odd_ranges_dev,
+                            uint32_t* odd_bits_dev, uint32_t* odd_list_dev, int32_t* status_dev, void* stream);
 
 /* The FP64 densities of xrh_density_accumulate over digit slices (exact products on the tensor cores;
  * no reference counterpart).

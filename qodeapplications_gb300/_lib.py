@@ -75,8 +75,8 @@ _SIGS = {
     "xrh_gemm_fp64_grouped": (_i32, [_vp, _i32, _i64, _vp, _vp]),
     "xrh_gemm_simt_grouped": (_i32, [_i32, _vp, _i32, _i64, _vp, _vp]),
     "xrh_slice_ctas": (_i64, [_i64, _i64, _i64, _i32, _i32, _i32]),
-    "xrh_slice_grouped": (_i32, [_vp, _i32, _i64, _i64, _vp]),
-    "xrh_gemm_sliced_grouped": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp]),
+    "xrh_slice_grouped": (_i32, [_vp, _i32, _i64, _i64, _vp, _vp]),
+    "xrh_gemm_sliced_grouped": (_i32, [_vp, _i32, _i64, _vp, _vp, _vp, _vp, _vp, _vp]),
     "xrh_coeff_digit_ctas": (_i64, [_i64]),
     "xrh_coeff_digits": (_i32, [_vp, _i32, _i64, _vp]),
     "xrh_coeff_rows": (_i32, [_vp, _i32, _i64, _vp]),
@@ -147,7 +147,7 @@ class LaunchCounter:
     except the host-only ones below launches one kernel of this library (those in `multi` the
     number given)."""
     multi = {"xrh_orbital_terms": 2, "xrh_gemv_rows_split": 2, "xrh_lanczos_normalize_split": 2,
-             "xrh_coeff_digits": 2}
+             "xrh_coeff_digits": 2, "xrh_gemm_sliced_grouped": 2}
     host_only = {"xrh_abi_version", "xrh_status_string", "xrh_last_cuda_error", "xrh_tc_chunk_elems", "xrh_zero",
                  "xrh_tc_encode_map", "xrh_state_ctas", "xrh_abt_ctas", "xrh_lanczos_coop_work",
                  "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_density_layout_ctas", "xrh_pair_rows_ctas", "xrh_slice_ctas", "xrh_coeff_digit_ctas"}

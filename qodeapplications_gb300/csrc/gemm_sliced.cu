@@ -18,9 +18,9 @@
 // the elements as BF16 numbers, one more MMA a K step gives sum |a||b| from below, and the elements where
 // the first bound could exceed the second (low_sum: rows that span many orders of magnitude, whose
 // large elements meet zeros or small ones) are formed by FP64 FMAs from the operands, as those of
-// rows with infinities and NaN are.  Rows of one size have none of them; the magnitudes cost 3 % at
-// 3 600 x 21 952 x 28, the spin blocks and near identities of an integral transformation of 28 spin
-// orbitals 15 % (2.8 -> 3.2 ms; CUDA cores 15.4).
+// rows with infinities and NaN are (odd_products_kernel).  Rows of one size have none of them; the
+// magnitudes cost 3 % at 3 600 x 21 952 x 28, the spin blocks and near identities of an integral
+// transformation of 28 spin orbitals 15 % (2.8 -> 3.2 ms; CUDA cores 15.4).
 //
 // What bounds it: 36 pairs of BF16 MMAs are 2 304 cycles of the tensor pipe per 128 x 64 x 32 stage; the
 // integer collection of a group (8 x 8 192 conversions) and the flush of a tile (about 25 000 cycles)
@@ -128,6 +128,7 @@ __device__ __forceinline__ Tile tile_of(const xrh_gemm_task* __restrict__ tasks,
 struct EpiTile {
     double* C;
     const xrh_sliced_segment* segs;
+    uint32_t* odd;                // marks of the tile's runs
     int64_t ldc, batch;
     int M, N, m0, n0, mode, BN, sb, left, task;
 };
@@ -213,20 +214,10 @@ __device__ __forceinline__ bool stage_mmas(uint32_t tmem, uint64_t dA, uint64_t 
     return true;
 }
 
-// The K elements [k0, k1) of row m and column n by FP64 FMAs (at 2 a clock and SM the loads hide behind them).
-__device__ __forceinline__ double fp64_product(const xrh_sliced_segment& S, int64_t batch, int m, int n, int64_t k0, int64_t k1) {
-    const double* a = S.A + batch * S.sA + (int64_t)m * ((S.flags & 1) ? 1 : S.lda);
-    const double* b = S.B + batch * S.sB + (int64_t)n * ((S.flags & 2) ? 1 : S.ldb);
-    const int64_t ka = (S.flags & 1) ? S.lda : 1, kb = (S.flags & 2) ? S.ldb : 1;
-    double y = 0.0;
-#pragma unroll 4
-    for (int64_t k = k0; k < k1; ++k) y = fma(a[k * ka], b[k * kb], y);
-    return y;
-}
-
 __global__ void __launch_bounds__(SL_THREADS, 1)
     gemm_sliced_kernel(const xrh_gemm_task* __restrict__ tasks, int n_tasks, int64_t total_tiles,
-                       const xrh_sliced_segment* __restrict__ segs, int32_t* status) {
+                       const xrh_sliced_segment* __restrict__ segs, const xrh_odd_range* __restrict__ odd_ranges,
+                       uint32_t* __restrict__ odd_bits, uint32_t* __restrict__ odd_list, int32_t* status) {
     extern __shared__ unsigned char smem_raw[];
     uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     __shared__ __align__(8) uint64_t full_bar[SL_STAGES], empty_bar[SL_STAGES];
@@ -241,7 +232,6 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
     __shared__ uint32_t s_eA[SL_BM], s_eB[64];
     __shared__ uint32_t s_low[SL_EPI_WARPS / 4][SL_BM];
     __shared__ unsigned char s_diagA[SL_BM], s_diagB[64];
-    __shared__ int s_count;                            // elements to form in FP64
     __shared__ EpiTile s_t;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -418,6 +408,7 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                 s_t.sb = I.sb;
                 s_t.left = I.left;
                 s_t.task = I.task;
+                s_t.odd = odd_bits + (odd_ranges[I.task].begin + (tile - T.tile_begin) * odd_ranges[I.task].runs) * (2 * SL_BM);
             }
             epi_bar();
             if (s_t.left == 0) {                                 // (uniform)
@@ -445,6 +436,8 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                 }
             }
             bool first = true;                                   // first flush of the tile
+            bool tile_odd = false;                               // it has elements for odd_products_kernel
+            int run = 0;
             Sum96 sum[SL_CW];
 #pragma unroll
             for (int j = 0; j < SL_CW; ++j) sum[j] = Sum96{0u, 0u, 0u};
@@ -508,24 +501,32 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                     break;
                 }
                 const xrh_sliced_segment& S = G.segs[G.si];
-                for (int j = tid; j < BN; j += SL_EPI_THREADS)
-                    s_eB[j] = s_t.n0 + j < s_t.N ? S.eB[s_t.batch * S.rB + s_t.n0 + j] : 0u;
+                bool bad = false;                                // an infinity or a NaN
+                if (tid < BN) {
+                    const uint32_t wb = s_t.n0 + tid < s_t.N ? S.eB[s_t.batch * S.rB + s_t.n0 + tid] : 0u;
+                    s_eB[tid] = wb;
+                    bad = (wb >> 20) >= 2047u;
+                }
                 const uint32_t wa = s_t.m0 + row < s_t.M ? S.eA[s_t.batch * S.rA + s_t.m0 + row] : 0u;
-                const int ea = exp_of(wa);
                 if (part == 0) s_eA[row] = wa;
+                if (epi_bar_or(bad || (wa >> 20) >= 2047u) && s_t.m0 + row < s_t.M) {
+#pragma unroll 1
+                    for (int j = 0; j < SL_CW; ++j) {
+                        const int jj = part * SL_CW + j;
+                        if (jj < BN && s_t.n0 + jj < s_t.N && ((wa >> 20) >= 2047u || (s_eB[jj] >> 20) >= 2047u)) low |= 1u << j;
+                    }
+                }
                 s_low[part][row] = low;
-                if (tid == 0) s_count = 0;
-                epi_bar();
+                s_t.odd[run * (2 * SL_BM) + 2 * row + part] = low;
+                ++run;
                 // the integer sums of 4 columns of each warp at a time through shared memory; a thread
                 // converts and writes four elements, lanes on consecutive columns.  The register
                 // arrays need constant indices, everything behind them is one rolled body.
                 const double alpha = S.alpha;
                 const bool scale = alpha != 1.0;
-                const bool any_odd = epi_bar_or(low != 0u || (wa >> 20) >= 2047u || (tid < BN && (s_eB[tid] >> 20) >= 2047u)) != 0;
-                // rows or columns with an infinity or a NaN, sums the digits are too coarse for
-                auto odd = [&](int r, int j) {
-                    return (s_eA[r] >> 20) >= 2047u || (s_eB[j] >> 20) >= 2047u || ((s_low[j / SL_CW][r] >> (j % SL_CW)) & 1u);
-                };
+                // the elements of s_low: nothing here, odd_products_kernel adds what they are
+                const bool any_odd = epi_bar_or(low != 0u) != 0;
+                tile_odd = tile_odd || any_odd;
                 const int slot = lane & 7, rr = warp * (4 * SL_NEL) + (lane >> 3);       // rows rr, rr + 4, ..
                 #pragma unroll 1
                 for (int p = 0; p < 8; ++p) {
@@ -551,13 +552,14 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                         const int eb = exp_of(wb);
                         double x[SL_NEL];
                         int te[SL_NEL];
-                        bool live[SL_NEL];                       // (the others: below)
-#pragma unroll
-                        for (int it = 0; it < SL_NEL; ++it)
-                            live[it] = s_t.m0 + rr + 4 * it < s_t.M && !(any_odd && odd(rr + 4 * it, jj));
 #pragma unroll
                         for (int it = 0; it < SL_NEL; ++it) te[it] = exp_of(s_eA[rr + 4 * it]) + eb;
                         sliced_to_doubles<SL_NEL>(raw, te, x);
+                        if (any_odd) {
+#pragma unroll
+                            for (int it = 0; it < SL_NEL; ++it)
+                                if ((s_low[jj / SL_CW][rr + 4 * it] >> (jj % SL_CW)) & 1u) x[it] = 0.0;
+                        }
                         if (scale) {
 #pragma unroll
                             for (int it = 0; it < SL_NEL; ++it) x[it] *= alpha;
@@ -575,54 +577,26 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
                         if (s_t.mode == 1) {
 #pragma unroll
                             for (int it = 0; it < SL_NEL; ++it)
-                                if (live[it]) atomicAdd(d[it], x[it]);
+                                if (s_t.m0 + rr + 4 * it < s_t.M) atomicAdd(d[it], x[it]);
                         } else {
                             // later segments add to what the same thread stored for the first one
                             if (!first) {
 #pragma unroll
                                 for (int it = 0; it < SL_NEL; ++it)
-                                    if (live[it]) x[it] = *d[it] + x[it];
+                                    if (s_t.m0 + rr + 4 * it < s_t.M) x[it] = *d[it] + x[it];
                             }
 #pragma unroll
                             for (int it = 0; it < SL_NEL; ++it)
-                                if (live[it]) *d[it] = x[it];
+                                if (s_t.m0 + rr + 4 * it < s_t.M) *d[it] = x[it];
                         }
                     }
                     __syncwarp();
                 }
 #pragma unroll
                 for (int j = 0; j < SL_CW; ++j) sum[j] = Sum96{0u, 0u, 0u};
-                if (any_odd) {
-                    // those elements in FP64, behind the others (the registers of the sums are free here): listed
-                    // first, so that all threads share them
-                    uint16_t* list = reinterpret_cast<uint16_t*>(s_raw);
-                    uint32_t todo = 0u;
-                    if (s_t.m0 + row < s_t.M) {
-#pragma unroll 1
-                        for (int j = 0; j < SL_CW; ++j) {
-                            const int jj = part * SL_CW + j;
-                            if (jj < BN && s_t.n0 + jj < s_t.N && odd(row, jj)) todo |= 1u << j;
-                        }
-                    }
-                    int at = atomicAdd(&s_count, __popc(todo));
-                    for (; todo; todo &= todo - 1u) list[at++] = (uint16_t)(row * 64 + part * SL_CW + __ffs((int)todo) - 1);
-                    epi_bar();
-                    const int64_t kt = (int64_t)(G.c + G.take) * SL_KS, ke = kt < S.K ? kt : S.K;
-#pragma unroll 1
-                    for (int e = tid; e < s_count; e += SL_EPI_THREADS) {
-                        const int r = list[e] >> 6, j = list[e] & 63;
-                        double x = alpha * fp64_product(S, s_t.batch, s_t.m0 + r, s_t.n0 + j, (int64_t)G.g0 * SL_KS, ke);
-                        double* d = s_t.C + s_roff[r] + s_coff[j];
-                        if (first && s_t.mode == 2) {
-                            if (s_diagB[j]) x += s_DA[r];
-                            if (s_diagA[r]) x += s_DB[j];
-                        }
-                        if (s_t.mode == 1) atomicAdd(d, x);
-                        else *d = first ? x : *d + x;
-                    }
-                }
                 first = false;
             }
+            if (tile_odd && !failed && tid == 0) odd_list[1 + atomicAdd(odd_list, 1u)] = (uint32_t)tile;
             if (!failed) epi_bar();                              // metadata reads done before the next tile
         }
     }
@@ -631,6 +605,83 @@ __global__ void __launch_bounds__(SL_THREADS, 1)
     tc_fence_after();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
+// ---- the elements in FP64 -------------------------------------------------------------------
+// A tile's marked elements: sums of the marked runs of stages by FP64 FMAs, added to C, where the tile left
+// nothing (delta terms apart).  Eight rows of a tile per CTA and step, or 32 where there are many tiles, the
+// elements listed so that all threads share them: a few tiles that are marked throughout spread over the chip
+// (in the GEMM's own epilogue they took 1.9 ms of an FP64 iteration of 18 spin orbitals, here 0.85).
+constexpr int OD_ROWS = 8, OD_MORE_ROWS = 32, OD_THREADS = 256;
+
+__global__ void __launch_bounds__(OD_THREADS, 4) odd_products_kernel(const xrh_gemm_task* __restrict__ tasks, int n_tasks,
+                                                                  const xrh_sliced_segment* __restrict__ segs,
+                                                                  const xrh_odd_range* __restrict__ odd_ranges,
+                                                                  const uint32_t* __restrict__ odd_bits, const uint32_t* __restrict__ odd_list) {
+    __shared__ uint16_t list[OD_MORE_ROWS * 64];
+    __shared__ int s_count;
+    __shared__ Tile s_tile;
+    const int64_t n_odd = odd_list[0];
+    const int rows = n_odd * (SL_BM / OD_ROWS) <= 2 * (int64_t)gridDim.x ? OD_ROWS : OD_MORE_ROWS, steps = SL_BM / rows;
+    for (int64_t w = blockIdx.x; w < n_odd * steps; w += gridDim.x) {
+        const int64_t tile = odd_list[1 + w / steps];
+        const int r0 = (int)(w % steps) * rows;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_tile = tile_of(tasks, n_tasks, segs, tile);
+            s_count = 0;
+        }
+        __syncthreads();
+        const Tile I = s_tile;
+        const xrh_gemm_task& T = tasks[I.task];
+        const xrh_sliced_segment* S0 = segs + T.seg_begin;
+        const int runs = (int)odd_ranges[I.task].runs;
+        const uint32_t* bits = odd_bits + (odd_ranges[I.task].begin + (tile - T.tile_begin) * runs) * (2 * SL_BM);
+        // the runs of the tile (Groups): f(run, segment, first K, behind the last K)
+        auto each_run = [&](auto&& f) {
+            int si = 0, c = I.sb, run = 0;
+            for (int left = I.left; left > 0; ++run) {
+                while (c >= S0[si].stages) {
+                    c -= (int)S0[si].stages;
+                    ++si;
+                }
+                int k = (int)S0[si].stages - c;
+                if (k > left) k = left;
+                if (k > SL_RUN_GROUPS * SL_GROUP) k = SL_RUN_GROUPS * SL_GROUP;
+                const int64_t end = (int64_t)(c + k) * SL_KS;
+                f(run, S0[si], (int64_t)c * SL_KS, end < S0[si].K ? end : S0[si].K);
+                c += k;
+                left -= k;
+            }
+        };
+        if (threadIdx.x < rows * 2) {
+            const int r = r0 + (threadIdx.x >> 1), part = threadIdx.x & 1;
+            uint32_t any = 0u;
+            each_run([&](int run, const xrh_sliced_segment&, int64_t, int64_t) { any |= bits[run * (2 * SL_BM) + 2 * r + part]; });
+            int at = atomicAdd(&s_count, __popc(any));
+            for (; any; any &= any - 1u) list[at++] = (uint16_t)(r * 64 + part * SL_CW + __ffs((int)any) - 1);
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < s_count; e += OD_THREADS) {
+            const int r = list[e] >> 6, j = list[e] & 63;
+            const int64_t m = I.m0 + r, col = I.n0 + j;
+            double x = 0.0;
+            each_run([&](int run, const xrh_sliced_segment& S, int64_t k0, int64_t k1) {
+                if (!((bits[run * (2 * SL_BM) + 2 * r + j / SL_CW] >> (j % SL_CW)) & 1u)) return;
+                const double* a = S.A + I.batch * S.sA + m * ((S.flags & 1) ? 1 : S.lda);
+                const double* b = S.B + I.batch * S.sB + col * ((S.flags & 2) ? 1 : S.ldb);
+                const int64_t ka = (S.flags & 1) ? S.lda : 1, kb = (S.flags & 2) ? S.ldb : 1;
+                double y = 0.0;
+#pragma unroll 8
+                for (int64_t k = k0; k < k1; ++k) y = fma(a[k * ka], b[k * kb], y);
+                x += S.alpha * y;
+            });
+            double* d = T.C + I.batch * T.sC +
+                        (T.mode == 2 ? (int64_t)(T.rowA[m] + T.rowB[col]) * T.ldc + T.colA[m] + T.colB[col] : m * T.ldc + col);
+            if (T.mode == 1) atomicAdd(d, x);
+            else *d += x;
+        }
+    }
 }
 
 // ---- digits -------------------------------------------------------------------------------
@@ -704,11 +755,13 @@ __global__ void __launch_bounds__(DG_THREADS) slice_max_kernel(const xrh_slice_t
     }
 }
 
-__global__ void __launch_bounds__(DG_THREADS) slice_digits_kernel(const xrh_slice_task* __restrict__ tasks, int n_tasks) {
+__global__ void __launch_bounds__(DG_THREADS) slice_digits_kernel(const xrh_slice_task* __restrict__ tasks, int n_tasks,
+                                                                  uint32_t* odd_list) {
     __shared__ uint32_t part[8];
     __shared__ double tile[DG_TK][33];
     const xrh_slice_task& T = tasks[find_slice_task(tasks, n_tasks, blockIdx.x, false)];
     int64_t local = (int64_t)blockIdx.x - T.cta_begin;
+    if (blockIdx.x == 0 && threadIdx.x == 0) odd_list[0] = 0u;         // of the GEMM that follows
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // rows are padded with zero digits to whole blocks (block: 32, 64 or 128)
     const int64_t blocks = (T.rows + T.block - 1) / T.block, rows_p = blocks * T.block;
@@ -784,25 +837,27 @@ extern "C" int64_t xrh_slice_ctas(int64_t rows, int64_t K, int64_t batch, int tr
 }
 
 extern "C" int xrh_slice_grouped(const xrh_slice_task* tasks_dev, int n_tasks, int64_t total_ctas, int64_t max_ctas,
-                                 void* stream) {
+                                 uint32_t* odd_list_dev, void* stream) {
     if (n_tasks < 0 || total_ctas < 0 || max_ctas < 0) return XRH_ERR_ARG;
     if (n_tasks == 0 || total_ctas == 0) return XRH_OK;
-    if (!tasks_dev) return XRH_ERR_ARG;
+    if (!tasks_dev || !odd_list_dev) return XRH_ERR_ARG;
     if (total_ctas > 0x7fffffffLL || max_ctas > 0x7fffffffLL) return XRH_ERR_CAPACITY;
     if (max_ctas > 0) {
         slice_max_kernel<<<(unsigned)max_ctas, DG_THREADS, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
         XRH_CHECK_LAUNCH();
     }
-    slice_digits_kernel<<<(unsigned)total_ctas, DG_THREADS, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks);
+    slice_digits_kernel<<<(unsigned)total_ctas, DG_THREADS, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks, odd_list_dev);
     XRH_CHECK_LAUNCH();
     return XRH_OK;
 }
 
 extern "C" int xrh_gemm_sliced_grouped(const xrh_gemm_task* tasks_dev, int n_tasks, int64_t total_tiles,
-                                       const xrh_sliced_segment* segs_dev, int32_t* status_dev, void* stream) {
+                                       const xrh_sliced_segment* segs_dev, const xrh_odd_range* odd_ranges_dev,
+                                       uint32_t* odd_bits_dev, uint32_t* odd_list_dev, int32_t* status_dev, void* stream) {
     if (n_tasks < 0 || total_tiles < 0) return XRH_ERR_ARG;
     if (n_tasks == 0 || total_tiles == 0) return XRH_OK;
-    if (!tasks_dev || !segs_dev || !status_dev) return XRH_ERR_ARG;
+    if (!tasks_dev || !segs_dev || !odd_ranges_dev || !odd_bits_dev || !odd_list_dev || !status_dev) return XRH_ERR_ARG;
+    if (total_tiles > 0x7fffffffLL) return XRH_ERR_CAPACITY;
     int dev = 0, n_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev);
@@ -810,7 +865,11 @@ extern "C" int xrh_gemm_sliced_grouped(const xrh_gemm_task* tasks_dev, int n_tas
     cudaFuncSetAttribute(gemm_sliced_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     const int64_t grid = total_tiles < n_sm ? total_tiles : n_sm;
     gemm_sliced_kernel<<<(unsigned)grid, SL_THREADS, smem, (cudaStream_t)stream>>>(
-        tasks_dev, n_tasks, total_tiles, segs_dev, status_dev);
+        tasks_dev, n_tasks, total_tiles, segs_dev, odd_ranges_dev, odd_bits_dev, odd_list_dev, status_dev);
+    XRH_CHECK_LAUNCH();
+    const int64_t odd_grid = total_tiles * (SL_BM / OD_ROWS) < 4 * n_sm ? total_tiles * (SL_BM / OD_ROWS) : 4 * n_sm;
+    odd_products_kernel<<<(unsigned)odd_grid, OD_THREADS, 0, (cudaStream_t)stream>>>(tasks_dev, n_tasks, segs_dev, odd_ranges_dev,
+                                                                                     odd_bits_dev, odd_list_dev);
     XRH_CHECK_LAUNCH();
     return XRH_OK;
 }

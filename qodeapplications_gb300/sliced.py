@@ -14,6 +14,8 @@ from ._lib import SLICE_TASK_DTYPE, SLICED_SEG_DTYPE, SLICES, TASK_DTYPE, call, 
 STAGE_K = 32
 BM = 128
 SMS = 152
+RUN_STAGES = 16384               # stages of a segment collected before a rounding (csrc/gemm_sliced.cu)
+ODD_BYTES = 1024                 # marks of a tile and run
 WORKSPACE_LIMIT = 1 << 30        # bytes of digits per wave
 MIN_STAGES_PER_SPLIT = 8         # 256 K: an accumulating tile is not divided below this
 
@@ -147,7 +149,13 @@ class SlicedGemm:
     def __init__(self, tasks, device, status=None):
         self.device = device
         waves = plan_waves(tasks)
-        self.work = torch.empty(max(w[2] for w in waves) + 1024, dtype=torch.uint8, device=device)
+        splits = [split_factors(w[0]) for w in waves]
+        # behind the digits of a wave the marks of its tiles (a range per task) and the list of marked tiles
+        runs = lambda t: sum(-(-_stages(s[4]) // RUN_STAGES) for s in t["segs"])
+        marks = [[_tiles(t) * k * runs(t) for t, k in zip(w[0], sk)] for w, sk in zip(waves, splits)]
+        tiles_of = [sum(_tiles(t) * k for t, k in zip(w[0], sk)) for w, sk in zip(waves, splits)]
+        size_of = lambda w, m, n: -(-w[2] // 1024) * 1024 + sum(m) * ODD_BYTES + 4 * (1 + n)
+        self.work = torch.empty(max(map(size_of, waves, marks, tiles_of)) + 1024, dtype=torch.uint8, device=device)
         base = -(-self.work.data_ptr() // 1024) * 1024
         self.status = torch.zeros(1, dtype=torch.int32, device=device) if status is None else status
         L = _lib.lib()
@@ -159,7 +167,7 @@ class SlicedGemm:
             blob.extend(bytes(-len(blob) % 128))
             return at
 
-        for cur, place, _size, zeroed in waves:
+        for (cur, place, size, zeroed), splitk, mark in zip(waves, splits, marks):
             # rows as dicts, then one conversion per table
             st, ctas, max_ctas = [], 0, 0
             # transposed operands last: their tasks own the CTAs of the row-maximum launch
@@ -171,7 +179,7 @@ class SlicedGemm:
                 ctas += L.xrh_slice_ctas(rows, K, batch, tr, block, 0)
                 max_ctas += L.xrh_slice_ctas(rows, K, batch, tr, block, 1)
             gt, gs, tiles = [], [], 0
-            for t, sk in zip(cur, split_factors(cur)):
+            for t, sk in zip(cur, splitk):
                 gt.append(dict(t, seg_begin=len(gs), seg_count=len(t["segs"]), splitk=sk, tile_begin=tiles))
                 tiles += _tiles(t) * sk
                 ops = _operands(t)
@@ -181,19 +189,21 @@ class SlicedGemm:
                                    eB=base + place[b][1], A=A, B=B, lda=lda, ldb=ldb, K=K, alpha=alpha, flags=flags,
                                    sA=sA, sB=sB))
             st, gt, gs = (_table(rows, dtype) for rows, dtype in ((st, SLICE_TASK_DTYPE), (gt, TASK_DTYPE), (gs, SLICED_SEG_DTYPE)))
+            odd = np.stack([np.cumsum([0] + mark[:-1]), [runs(t) for t in cur]], axis=1).astype(np.int64)
             self.waves.append((put(st.tobytes()), len(st), ctas, max_ctas, zeroed, put(gt.tobytes()), len(gt), tiles,
-                               put(gs.tobytes())))
+                               put(gs.tobytes()), put(odd.tobytes()), base + -(-size // 1024) * 1024,
+                               base + -(-size // 1024) * 1024 + sum(mark) * ODD_BYTES))
         self.tables = torch.frombuffer(blob, dtype=torch.uint8).to(device)
         self.base = base
 
     def run(self, stream=None):
         s = stream_ptr(stream)
         t = self.tables.data_ptr()
-        for st, n_s, ctas, max_ctas, zeroed, gt, n_t, tiles, gs in self.waves:
+        for st, n_s, ctas, max_ctas, zeroed, gt, n_t, tiles, gs, odd, bits, marked in self.waves:
             if zeroed:
                 call("xrh_zero", self.base, zeroed, s)
-            call("xrh_slice_grouped", t + st, n_s, ctas, max_ctas, s)
-            call("xrh_gemm_sliced_grouped", t + gt, n_t, tiles, t + gs, ptr(self.status), s)
+            call("xrh_slice_grouped", t + st, n_s, ctas, max_ctas, marked, s)
+            call("xrh_gemm_sliced_grouped", t + gt, n_t, tiles, t + gs, t + odd, bits, marked, ptr(self.status), s)
 
     def check(self):
         """Raise if a bounded device wait gave up (synchronises)."""
