@@ -164,6 +164,21 @@ def call(name, *args):
         raise XRHError(f"{name} failed: {msg} (status {st}, cuda error {lib().xrh_last_cuda_error()})")
 
 
+def status_word(device):
+    """An int32 device word that a launch sets when a bounded device wait gave up.  Launches whose results are
+    read together share one; whoever hands the results out checks it (check_status) where it waits for the
+    device anyway."""
+    import torch
+    return torch.zeros(1, dtype=torch.int32, device=device)
+
+
+def check_status(word, what):
+    """Raise if a bounded device wait of `what` gave up (synchronises)."""
+    st = int(word.item())
+    if st != XRH_OK:
+        raise XRHError(f"{what} reported status {st} ({lib().xrh_status_string(st).decode()})")
+
+
 def ptr(t):
     """Device (or host) address of a torch tensor, or None."""
     return None if t is None else ctypes.c_void_p(t.data_ptr())

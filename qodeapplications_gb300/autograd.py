@@ -97,6 +97,7 @@ class XRDimerEnergy:
                     break
             if best is None or w[0] < best[0]:
                 best = (float(w[0]), t, float(res))
+        self.plan.check_status()
         E, t, res = best
         self.sector, self.residual = t, res
         d = self.lz[t].v0
@@ -109,6 +110,7 @@ class XRDimerEnergy:
         g = self.adj.state_gradient()
         gz = [g[m][c].clone() for m in (0, 1) for c in self.charges[m]]
         dT, _dU, dV = self.adj.integral_gradients()
+        self.adj.check_status()
         return dT, dV, gz
 
     def __call__(self, h, V, coeffs):

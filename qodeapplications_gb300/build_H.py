@@ -96,6 +96,7 @@ class build_matrix_elements(object):
                                builders=[ExternalBuilder(self.rho[m1]), ExternalBuilder(self.rho[m2])],
                                monomer_2e="none", autotune=False)
             plan.launch(build_densities=False)
+            plan.check_status()
             offs = []
             for k in (0, 1):
                 off, acc = {}, 0
@@ -131,6 +132,7 @@ class build_matrix_elements(object):
             plan = XRTrimerPlan([self.rho[m] for m in frags], self.ints, [self.n_elec[m] for m in frags], charges,
                                 ns, frags=frags, device=self.device)
             plan.launch()
+            plan.check_status()
             self._trimer[frags] = {k: plan.block(*k).cpu().numpy() for k in plan.keys()}
             del plan
         return self._trimer[frags]

@@ -419,7 +419,7 @@ class SlicedDensities:
     blocks: [(couplings, bra key, ket key, rhoT)] with the (side, charge) keys of coeff.  Operator
     indices without couplings are never written: rhoT must hold zeros there."""
 
-    def __init__(self, blocks, coeff, device):
+    def __init__(self, blocks, coeff, device, status=None):
         self.coeff, self.keep = coeff, blocks
         tasks = np.zeros(len(blocks), dtype=_lib.DENS_SLICED_TASK_DTYPE)
         for t, (cp, bra, ket, rhoT) in zip(tasks, blocks):
@@ -428,7 +428,7 @@ class SlicedDensities:
         units = sliced_units([(b[0], int(t["nb"]), int(t["nk"])) for b, t in zip(blocks, tasks)])
         self.n_tasks, self.n_units = len(tasks), len(units)
         self.tasks_dev, self.units_dev = _upload(tasks, device), _upload(units, device)
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.status = _lib.status_word(device) if status is None else status
 
     def run(self, s):
         self.coeff.run(s)
@@ -437,9 +437,7 @@ class SlicedDensities:
 
     def check(self):
         """Raise if a bounded device wait gave up (synchronises)."""
-        st = int(self.status.item())
-        if st != 0:
-            raise _lib.XRHError(f"sliced densities reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")
+        _lib.check_status(self.status, "sliced densities")
 
 
 class SlicedDensityAdjoint:
@@ -447,7 +445,7 @@ class SlicedDensityAdjoint:
     one pad width.  blocks: [(couplings, states, bra key, ket key, gT, bra gradient, ket gradient)] (states:
     StateTables); refresh: CoeffDigits to run first."""
 
-    def __init__(self, blocks, precision, refresh, device):
+    def __init__(self, blocks, precision, refresh, device, status=None):
         self.precision, self.refresh, self.keep = precision, list(refresh), blocks
         self.npad = blocks[0][1].npad
         rows = {id(b[1]): b[1] for b in blocks}
@@ -461,7 +459,7 @@ class SlicedDensityAdjoint:
         units = sliced_units([(b[0], int(t["nb"]), int(t["nk"])) for b, t in zip(blocks, tasks)], (0, 1))
         self.n_tasks, self.n_units = len(tasks), len(units)
         self.tasks_dev, self.units_dev = _upload(tasks, device), _upload(units, device)
-        self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self.status = _lib.status_word(device) if status is None else status
 
     def run(self, s):
         for c in [*self.refresh, *self.rows.values()]:
@@ -471,9 +469,7 @@ class SlicedDensityAdjoint:
 
     def check(self):
         """Raise if a bounded device wait gave up (synchronises)."""
-        st = int(self.status.item())
-        if st != 0:
-            raise _lib.XRHError(f"sliced density adjoint reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")
+        _lib.check_status(self.status, "sliced density adjoint")
 
 
 class DensityBuilder:
@@ -485,8 +481,10 @@ class DensityBuilder:
     With the same states on both sides (mirror=True, no bra_coeffs) the c, cc and cca
     blocks are mirrored from their a, aa and caa partners instead of accumulated."""
 
-    def __init__(self, space, n_states, precision="fp64", n_states_bra=None, mirror=True, antisym=True):
+    def __init__(self, space, n_states, precision="fp64", n_states_bra=None, mirror=True, antisym=True,
+                 status=None):
         self.space = space
+        self.status = status                     # word for the launches (None: one of their own)
         self.precision = _lib.PRECISIONS[precision]
         if self.precision not in (_lib.FP64, _lib.FP32):
             self.precision = _lib.FP32       # tensor-core variants build densities with FP32 products
@@ -557,7 +555,7 @@ class DensityBuilder:
             side = "ket" if self.same_bra else "bra"
             coeff = CoeffDigits({"ket": self.zT} if self.same_bra else {"ket": self.zT, "bra": self.zbT}, dev)
             self.sliced = SlicedDensities([(cp, (side, key[1]), ("ket", key[2]), self._tmp[key]) for key, cp in direct],
-                                          coeff, dev)
+                                          coeff, dev, self.status)
         # FP32 path: coefficients converted once per build, rows padded to 16 bytes
         if self.f32:
             pad = lambda n: (n + 3) // 4 * 4
@@ -754,6 +752,7 @@ def build_density_tensors(z_lists, n_orbs, Vints, n_core, n_threads=1):
     space = FragmentSpace(sectors, n_orbs, n_core, n_elec_ref=0)
     builder = DensityBuilder(space, {c: coeffs[c].shape[0] for c in sectors})
     rho = builder.build({c: torch.as_tensor(coeffs[c], device=space.device) for c in sectors})
+    builder.check()
     out = {op: {} for op in ("aa", "a", "caa", "ca", "ccaa", "c", "cca", "cc")}
     total = 0
     for op, blocks in rho.items():

@@ -22,7 +22,9 @@ bra_det / ket_det.
 """
 import torch
 
+from . import _lib
 from ._external import device_densities
+from ._lib import check_status
 
 
 class _charges(object):
@@ -48,7 +50,10 @@ class _charges(object):
                 reorder = list(perm) + [order + p for p in perm]
                 r = r.permute(*reorder) if order > 1 else r
                 total = r if total is None else total + r
-            self._results[label] = None if total is None else total.contiguous().cpu().numpy()
+            if total is not None:
+                total = total.contiguous().cpu().numpy()
+                check_status(self._info["status"], f"diagram '{label}'")
+            self._results[label] = total
         return self._results[label]
 
 
@@ -87,7 +92,7 @@ class blocks(object):
                         blk = src[(m, m)] if kind == "T" else (src[(m, m, m, m)] if kind == "V" else src[(m, m, m)])
                         break
             N.append(int(blk.shape[0]))
-        self._info = {"rho": rho, "integrals": integrals, "N": N, "device": dev}
+        self._info = {"rho": rho, "integrals": integrals, "N": N, "device": dev, "status": _lib.status_word(dev)}
         self._diagrams = diagrams
         self._items = {}
         self.densities = densities

@@ -22,12 +22,15 @@ import torch
 from .gemm import GroupedGemm
 
 
-def _gemm(A, W, M, x, K, alpha=1.0):
-    """C[M, x] = alpha * A[M, K] W[x, K]^T on the device (one FP64 grouped-GEMM task)."""
+def _gemm(A, W, M, x, K, alpha=1.0, status=None):
+    """C[M, x] = alpha * A[M, K] W[x, K]^T on the device (one FP64 grouped-GEMM task).  status: the word that
+    whoever reads the result checks (diagrammatic_expansion.blocks); without one it is checked here."""
     C = torch.zeros((M, x), dtype=torch.float64, device=A.device)
     g = GroupedGemm(A.device)
     g.add(M, x, [(A.contiguous(), K, W.contiguous(), K, K, float(alpha))], C, x, mode=0)
-    g.finalize().run()
+    g.finalize(status=status).run()
+    if status is None:
+        g.check()
     return C
 
 
@@ -52,6 +55,7 @@ class Resolved:
         self.rho, self.ints = info["rho"], info["integrals"]
         self.frags, self.charges, self.n_j0 = frags, charges, n_j0
         self.N = [info["N"][f] for f in frags]
+        self.status = info.get("status")
 
     def dens(self, k, op):
         return self.rho[self.frags[k]][op].get(tuple(self.charges[k]))
@@ -85,7 +89,7 @@ def _monomer(op, kind, idx, weight_perm=None):
         if weight_perm is not None:
             w = w.permute(*weight_perm)
         k = N ** len(op)
-        return _gemm(r.reshape(ni * nj, k), w.reshape(1, k), ni * nj, 1, k).view(ni, nj)
+        return _gemm(r.reshape(ni * nj, k), w.reshape(1, k), ni * nj, 1, k, status=X.status).view(ni, nj)
     return body
 
 
@@ -101,8 +105,8 @@ def _dimer(op0, op1, kind, idx, weight_perm, ext0, ext1, prefactor):
         ni1, nj1 = X.n(1)
         k0, k1 = X.N[0] ** ext0, X.N[1] ** ext1
         W = _int_block(X, kind, *idx).permute(*weight_perm).reshape(k1, k0)
-        P = _gemm(r0.reshape(ni0 * nj0, k0), W, ni0 * nj0, k1, k0)
-        out = _gemm(P, r1.reshape(ni1 * nj1, k1), ni0 * nj0, ni1 * nj1, k1, prefactor(X.n_j0))
+        P = _gemm(r0.reshape(ni0 * nj0, k0), W, ni0 * nj0, k1, k0, status=X.status)
+        out = _gemm(P, r1.reshape(ni1 * nj1, k1), ni0 * nj0, ni1 * nj1, k1, prefactor(X.n_j0), X.status)
         return out.view(ni0, nj0, ni1, nj1).permute(0, 2, 1, 3)
     return body
 
@@ -116,7 +120,7 @@ def _u100(X):
     ni1, nj1 = X.n(1)
     N = X.N[0]
     w = _int_block(X, "U", 1, 0, 0).reshape(1, N * N)
-    P = _gemm(r0.reshape(ni0 * nj0, N * N), w, ni0 * nj0, 1, N * N).view(ni0, nj0)
+    P = _gemm(r0.reshape(ni0 * nj0, N * N), w, ni0 * nj0, 1, N * N, status=X.status).view(ni0, nj0)
     out = torch.zeros((ni0, ni1, nj0, nj1), dtype=torch.float64, device=P.device)
     for i in range(min(ni1, nj1)):
         out[:, i, :, i] = P

@@ -62,7 +62,8 @@ class FragmentHamiltonian:
         self.zT = torch.zeros((self.n_conf, self.n_vec), dtype=torch.float64, device=dev)
 
     def apply(self, Psi, out=None):
-        """H Psi for Psi (n_vec, n_conf) (rows = CI vectors); returns (n_vec, n_conf)."""
+        """H Psi for Psi (n_vec, n_conf) (rows = CI vectors); returns (n_vec, n_conf).  Does not wait for the
+        device (check_status does)."""
         s = stream_ptr()
         Psi = Psi.contiguous()             # kept alive until the launch is enqueued
         call("xrh_transpose", ptr(Psi), self.n_vec, self.n_conf, ptr(self.zT), s)
@@ -71,6 +72,10 @@ class FragmentHamiltonian:
             return self.sigma.sigmaT
         out.copy_(self.sigma.sigmaT)
         return out
+
+    def check_status(self):
+        """Raise if a bounded device wait of the launches gave up (synchronises)."""
+        self.sigma.check()
 
     def matrix(self):
         """The dense FCI matrix (generic_fci): H applied to the unit vectors, n_vec at a time."""
@@ -83,6 +88,7 @@ class FragmentHamiltonian:
             E[torch.arange(k), torch.arange(c0, c0 + k)] = 1.0
             HE = self.apply(E)
             H[c0:c0 + k].copy_(HE[:k])
+        self.check_status()
         return H
 
     def lowest(self, k=1, m=None, tol=1e-10, max_restarts=50):
@@ -112,6 +118,7 @@ class FragmentHamiltonian:
                 break
             v0 = vecs[:len(w)].sum(0)
             lz.v0.copy_(v0 / v0.norm())
+        self.check_status()
         return w, vecs[:len(w)]
 
 

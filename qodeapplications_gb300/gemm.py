@@ -236,7 +236,7 @@ class TCGroupedGemm:
         self._logical = []
         self.flops = 0.0
         self.policy = (128, 16)
-        self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
+        self.status = _lib.status_word(self.device)
         self.tuning = None
 
     def add(self, M, N, segments, C, ldc, mode=0, splitk=None, maps=None, DA=None, DB=None, groups=None):
@@ -346,6 +346,4 @@ class TCGroupedGemm:
              ptr(self.segs_dev), ptr(self.reg.maps_dev), ptr(self.status), stream_ptr(stream))
 
     def check(self):
-        st = int(self.status.item())
-        if st != 0:
-            raise _lib.XRHError(f"tensor-core GEMM reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")
+        _lib.check_status(self.status, "tensor-core GEMM")

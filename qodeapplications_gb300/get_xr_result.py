@@ -74,8 +74,7 @@ def get_xr_H(ints, dens, xr_order, monomer_charges, bra_det=False, ket_det=False
     plan.launch(build_densities=False)
     H1 = plan.H1()
     H2 = plan.H
-    if plan.tc or not device:        # the host copies below wait for the device anyway
-        plan.check_status()
+    plan.check_status()
     if device:
         return H1, H2
     return [h.cpu().numpy() for h in H1], H2.cpu().numpy()

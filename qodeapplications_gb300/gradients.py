@@ -149,7 +149,7 @@ class XRDimerAdjoint:
                 # Z[i1, (j0,x)] = a sum_i0 D[i0,i1] A[(i0,j0),x]
                 L1.add(ni1, nj0 * K, [(Di, tot1, A, nj0 * K, ni0, a, 3, 0, 0)], Z, nj0 * K)
                 self.final_adj.append((A, B, K, Y, Z, Dj, (ni0, nj0, ni1, nj1)))
-        self.L1 = L1.finalize()
+        self.L1 = L1.finalize(status=plan.status)
 
         # ---- launch 2: dA, dB (batched), monomer pieces ----
         L2 = GroupedGemm(dev, gprec)
@@ -178,7 +178,7 @@ class XRDimerAdjoint:
                 L2.add(nconf, n, [(sg.sigmaT, nconf, gb, n, n, 2.0, 1, 0, 0)], G[("gzT", m, c)], n, mode=1)
                 # Y^T = z^T g^T for the two-particle density of the weighted ensemble
                 L2.add(nconf, n, [(plan.builders[m].zT[c], n, gb, n, n, 1.0)], G[("YT", m, c)], n)
-        self.L2 = L2.finalize()
+        self.L2 = L2.finalize(status=plan.status)
 
         # ---- launch 3: precontraction adjoint ----
         # every gradient buffer's writers: outputs written by this launch alone take plain stores
@@ -218,6 +218,7 @@ class XRDimerAdjoint:
                     L3.add(X, Yk, [(Transposed(gP), X, Transposed(rho_t), Yk, M, 1.0)], G[("gW", wk)], Yk, mode=1,
                            groups=[("g", "rhoT")])
             self.reg3.upload()
+            L3.status = plan.status
             self.L3 = L3.finalize().autotune()
         else:
             L3 = GroupedGemm(dev, gprec)
@@ -234,7 +235,7 @@ class XRDimerAdjoint:
                     # dW[x, y] += sum_m dP[m, x] rho[m, y]
                     L3.add(X, Yk, [(gP, X, rho_t, Yk, M, 1.0, 3, 0, 0)], G[("gW", wk)], Yk, mode=1,
                            splitk=_splitk(M, 256, 32))
-            self.L3 = L3.finalize()
+            self.L3 = L3.finalize(status=plan.status)
 
         # ---- launch 4 inputs: transposed density gradients for the coupling-list adjoint ----
         # (FP32 accumulation buffers on the split-precision paths)
@@ -283,8 +284,9 @@ class XRDimerAdjoint:
             if flat_all:
                 idx = torch.as_tensor(np.concatenate(flat_all), dtype=torch.int64, device=dev)
                 self.gam_scatter.append((m, idx, self.G[("Gpairs", m)][:off]))
-        self.Lgamma = Lg.finalize()
+        self.Lgamma = Lg.finalize(status=plan.status)
         self.gam_reg.upload()
+        Lgt.status = plan.status
         self.Lgamma_tc = Lgt.finalize().autotune()
 
         pool = [t.reshape(-1) for t in (scratch or ())]
@@ -332,7 +334,6 @@ class XRDimerAdjoint:
         # every block has at most 64 states per side (else the CUDA-core kernel)
         self.dens_adj_groups = []
         self.dens_adj_tc = []
-        self.tc_status = torch.zeros(1, dtype=torch.int32, device=dev)
         use_tc = (density_adjoint == "tc" and self.prec32 and plan.tc and
                   all(e[5].shape[0] <= 64 and e[5].shape[1] <= 64 for e in self.dens_adj))
         if density_adjoint == "tc" and not use_tc:
@@ -442,7 +443,8 @@ class XRDimerAdjoint:
             gz = self.gz32[m] if self.prec32 else {x: self.G[("gzT", m, x)] for x in plan.charges[m]}
             by_pad.setdefault(c.npad, []).append((cp, c, bra, ("ket", kc), gT, gz[bc], gz[kc]))
         for blocks in by_pad.values():
-            self.dens_adj_sliced.append(SlicedDensityAdjoint(blocks, _lib.FP32 if self.prec32 else _lib.FP64, [], dev))
+            self.dens_adj_sliced.append(SlicedDensityAdjoint(blocks, _lib.FP32 if self.prec32 else _lib.FP64, [], dev,
+                                                             plan.status))
         self.dens_adj_groups = []
 
     def _canonicalize(self, m=None):
@@ -528,7 +530,7 @@ class XRDimerAdjoint:
                     n = bld.zT[c].shape[1]
                     call("xrh_split_operand", _lib.TF32X3, ptr(bld.zT[c]), zh.shape[0], n, n, 64, ptr(zh), ptr(zl), s)
             for (tasks, n_t, ctas) in self.dens_adj_tc:
-                call("xrh_density_adjoint_tc_grouped", ptr(tasks), n_t, ctas, ptr(self.tc_status), s)
+                call("xrh_density_adjoint_tc_grouped", ptr(tasks), n_t, ctas, ptr(self.plan.status), s)
 
     def launch_gamma(self):
         """Two-particle densities of the monomer two-electron terms (after launch 2)."""
@@ -557,14 +559,7 @@ class XRDimerAdjoint:
 
     def check_status(self):
         """Raise if a bounded device wait of the tensor-core launch timed out (syncs)."""
-        for g in [self.L1, self.L2, self.L3, self.Lgamma, self.Lgamma_tc] + self.dens_adj_sliced:
-            g.check()
-        orb = getattr(self, "_orb", None)
-        if orb is not None and orb["VG"] is not None:
-            orb["VG"].check()
-        st = int(self.tc_status.item())
-        if st != 0:
-            raise _lib.XRHError(f"tensor-core density adjoint reported status {st}")
+        _lib.check_status(self.plan.status, "reverse pass")
 
     def launch(self, d):
         """Enqueue the reverse pass for ground-state vector d (device, product order)."""
@@ -673,7 +668,7 @@ class XRDimerAdjoint:
         if not self.prec32 and t >= ORBITAL_SLICED_MIN:
             b["VG"] = GroupedGemm(dev)
             b["VG"].add(t, t, [(b["A"], t ** 3, b["B"], t ** 3, t ** 3, 0.5)], b["Gso"], t, mode=1)
-            b["VG"].finalize()
+            b["VG"].finalize(status=self.plan.status)
         b["inputs"] = self._orbital_inputs()
         self._orb = b
         return b

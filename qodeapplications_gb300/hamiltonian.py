@@ -156,6 +156,11 @@ class SigmaTwoElectron:
             elif g is not None:
                 self.gemm = g.finalize()
 
+    def check(self):
+        """Raise if a bounded device wait of the own GEMM gave up (synchronises)."""
+        if self.pl is not None and self.gemm is not None:
+            self.gemm.check()
+
     def add_gemm_tasks(self, g, k):
         """E[c][(s, K)][pq] = sum_rs D[c][(s, K)][rs] W_c[pq, rs] for spin class k into grouped
         GEMM g (tensor cores, 3 x TF32, when self.tc)."""
@@ -213,7 +218,7 @@ class SigmaBatch:
     split (tensor-core plans), one grouped GEMM over all spin classes, fragments and charges,
     one grouped pair gather.  items: [(SigmaTwoElectron built with own_gemm=False, its zT)]."""
 
-    def __init__(self, items, device):
+    def __init__(self, items, device, status=None):
         self.items = items
         self.tc = bool(items) and items[0][0].tc
         if not items:
@@ -231,9 +236,10 @@ class SigmaBatch:
         if self.tc:
             self.reg.upload()
             self.reg.split("sigW")
+            g.status = g.status if status is None else status
             self.gemm = g.finalize().autotune()
         else:
-            self.gemm = g.finalize()
+            self.gemm = g.finalize(status=status)
 
     def run(self):
         if not self.items:
@@ -255,7 +261,7 @@ class SigmaBatch:
 
 
 def monomer_two_electron(space, coeffs, V_block, c):
-    """sum_pqrs V_pqrs rho^ccaa_IJ[p,q,s,r] for all state pairs of charge c (FP64)."""
+    """sum_pqrs V_pqrs rho^ccaa_IJ[p,q,s,r] for all state pairs of charge c (FP64).  Waits for the device."""
     z = coeffs[c].contiguous()
     n = z.shape[0]
     zT = z.t().contiguous()
@@ -267,6 +273,8 @@ def monomer_two_electron(space, coeffs, V_block, c):
     splitk = max(1, min(64, nconf // 512))
     g.add(n, n, [(z, nconf, s2.sigmaT, nconf, nconf, 1.0)], out, n, mode=1, splitk=splitk)
     g.finalize().run()
+    s2.check()
+    g.check()
     return out
 
 
@@ -379,6 +387,7 @@ class XRDimerPlan:
         self.device = spaces[0].device
         dev = self.device
         f64 = dict(dtype=torch.float64, device=dev)
+        self.status = _lib.status_word(dev)      # of every launch of this plan and of its reverse pass
         self.coeffs = [{c: torch.zeros((self.n_states[m][c], spaces[m].n_conf[c]), **f64) for c in self.charges[m]}
                        for m in (0, 1)]
         # densities and sigma vectors: FP64 on the fp64 path; FP32 products with FP64 sums on the
@@ -402,7 +411,7 @@ class XRDimerPlan:
             # owner builds them once per iteration and calls launch(build_densities=False)
             self.builders = list(builders)
         else:
-            self.builders = [DensityBuilder(spaces[m], self.n_states[m], precision=self.dens_precision)
+            self.builders = [DensityBuilder(spaces[m], self.n_states[m], precision=self.dens_precision, status=self.status)
                              for m in (0, 1)]
         N = [spaces[0].N, spaces[1].N]
         self.N = N
@@ -500,7 +509,7 @@ class XRDimerPlan:
                     mono.append((n * n, 1, [(ca, N[m] ** 2, W[("u100", m)], N[m] ** 2, N[m] ** 2, 1.0)], tgt, 1,
                                  _splitk(N[m] ** 2)))
         self.sigma_batch = SigmaBatch([(sg, self.builders[m].zT[c]) for m in (0, 1)
-                                       for c, sg in self.sigma[m].items() if sg.pl is not None], dev)
+                                       for c, sg in self.sigma[m].items() if sg.pl is not None], dev, self.status)
         # one-column terms (rho^ca . h) are row GEMVs: a 64 x 64 FP64 tile would spend 64x the
         # FMAs of the result on them, and an FP64 tile is slow on this part
         self.mono_gemv = [(sg_[0][0], sg_[0][2], out_, M_, sg_[0][4]) for (M_, N_, sg_, out_, _l, _s) in mono if N_ == 1]
@@ -527,7 +536,7 @@ class XRDimerPlan:
         for (M_, N_, segs_, out_, ldc_, sk_) in mono:
             pre.add(M_, N_, segs_, out_, ldc_, mode=1, splitk=sk_)
         self.tc = self.precision in (_lib.BF16X3, _lib.TF32X3)
-        self.pre = pre if self.tc else pre.finalize()       # (its FLOP count alone with split precision)
+        self.pre = pre if self.tc else pre.finalize(status=self.status)       # (its FLOP count alone with split precision)
 
         # ---- final tasks: one per output charge block ----
         nb = [ns[m] for m in (0, 1)]
@@ -631,7 +640,7 @@ class XRDimerPlan:
                         self.final_tasks.append(dict(key=(ci0, ci1, cj0, cj1), segs=segs, M=M, N=Nn, C=Cbuf, ldc=ldc,
                                                      dims=(ni0, nj0, ni1, nj1),
                                                      maps=(rowA, colA, rowB, colB, diagA, diagB), DA=DA, DB=DB))
-        self.fin = fin if self.tc else fin.finalize()
+        self.fin = fin if self.tc else fin.finalize(status=self.status)
 
         # ---- split-precision tensor-core variant of both launches ----
         if self.tc:
@@ -676,7 +685,9 @@ class XRDimerPlan:
             reg.upload()
             reg.split(self._grp_W)
             self._grp_in = sorted(self._grp_in)
-            self.reg, self.pre_tc, self.pre64, self.fin_tc = reg, pre_tc.finalize(), pre64.finalize(), fin_tc.finalize()
+            pre_tc.status = fin_tc.status = self.status
+            self.reg, self.pre_tc, self.fin_tc = reg, pre_tc.finalize(), fin_tc.finalize()
+            self.pre64 = pre64.finalize(status=self.status)
             if autotune:
                 self.pre_tc.autotune()
                 self.fin_tc.autotune()
@@ -813,12 +824,10 @@ class XRDimerPlan:
 
     def check_status(self):
         """Raise if a bounded device wait of the tensor-core kernels timed out (syncs)."""
-        for g in (self.pre_tc, self.pre64, self.fin_tc) if self.tc else (self.pre, self.fin):
-            g.check()
+        _lib.check_status(self.status, "excitonic Hamiltonian")
         for b in self.builders:
-            if hasattr(b, "check"):
+            if hasattr(b, "check") and getattr(b, "status", None) is not self.status:
                 b.check()
-        self.sigma_batch.check()
 
 
 def lowest_eigenpairs(H, k=5, tol=1e-10):

@@ -243,8 +243,14 @@ class XRStateOptimizer:
                 self._graphs[1].replay()
             else:
                 self._backward(t, warm=True)
+        # (of this forward and of the reverse passes before: the states they left are in this energy)
+        self.check_status()
         self.energy, self.residual = float(E), float(resid)
         return self.energy
+
+    def check_status(self):
+        """Raise if a bounded device wait of the iterations so far gave up (synchronises)."""
+        self.plan.check_status()                 # (the reverse pass shares the plan's word)
 
     def _ritz_padded(self, t):
         lz = self.lz_warm[t]
@@ -301,4 +307,5 @@ class XRStateOptimizer:
 
     @property
     def gradient_norm(self):
+        self.check_status()
         return float(self._gsq.sqrt())

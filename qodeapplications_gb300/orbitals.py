@@ -60,8 +60,11 @@ def _transform_all(items, status=None):
     its matrix (None for the identity).  The i-th passes of all arrays are one grouped GEMM,
         Y[rest, p] = sum_a X[a, rest] M[a, p];
     trailing identities only turn the index order back, one transpose instead of a pass each.  The
-    caller checks `status` (an int32 device word) where it synchronises."""
+    caller checks `status` (_lib.status_word) where it waits for the device; without one it is checked here."""
+    own = status is None
     cur, todo = [], []
+    if own and items:
+        status = _lib.status_word(items[0][0].device)
     for X, batch, mats in items:
         n = X.shape[0 if batch is None else 1]
         if n == 0 or batch == 0:
@@ -90,6 +93,8 @@ def _transform_all(items, status=None):
             cur[i] = out
     if turns:
         _lib.Transposes(turns, cur[0].device).run()
+    if own and cur:
+        _lib.check_status(status, "integral transformation")
     return cur
 
 
@@ -151,15 +156,14 @@ def biorthogonal_integrals(symm, frag_sizes, status=None):
     Sinv, singular = inverse_spin_free_launch(symm["S"], frag_sizes)
     SinvT = Sinv.t().contiguous()        # pass matrix: M[a, p] = Sinv[p, a]
     if status is None:
-        status = torch.zeros(1, dtype=torch.int32, device=Sinv.device)
+        status = _lib.status_word(Sinv.device)
     jobs = {"S": (symm["S"], [SinvT, None]), "T": (symm["T"], [SinvT, None])}
     if symm.get("U") is not None:
         jobs["U"] = (symm["U"], [SinvT, None])
     jobs["V"] = (symm["V"], [SinvT, SinvT, None, None])
     out = {"Sinv": Sinv, **_transform_dict(jobs, jobs, status)}
     _check_inverse(singular)             # one synchronisation, behind everything that was enqueued
-    if int(status.item()) != 0:
-        raise _lib.XRHError("an integral transformation gave up a bounded device wait")
+    _lib.check_status(status, "integral transformation")
     return out
 
 
@@ -185,7 +189,7 @@ def transform_ints(U_sp, ints, frag_sizes):
     n_so = 2 * sum(frag_sizes)
     Usp = torch.as_tensor(U_sp, dtype=torch.float64, device=dev).contiguous()
     M = _spin_block(Usp, Usp.shape[0], frag_sizes, torch.empty((n_so, n_so), dtype=torch.float64, device=dev))
-    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    status = _lib.status_word(dev)
     symm = transform_integrals(M, ints, status)
     bior = biorthogonal_integrals(symm, frag_sizes, status)
     return symm, bior

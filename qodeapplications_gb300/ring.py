@@ -315,6 +315,7 @@ class XRRing:
             self.run_triple(T)
         ev[2].record()
         torch.cuda.current_stream().synchronize()
+        self.check_status()
         self.phase_ms = {"pairs": ev[0].elapsed_time(ev[1]), "triples": ev[1].elapsed_time(ev[2])}
         E2, E3 = mbe_energies(self.E_mono, self.E_pair, self.E_triple, self.n_frag)
         self.E2, self.E3 = E2, (E3 if self.triples and with_triples else None)

@@ -157,7 +157,7 @@ class SlicedGemm:
         size_of = lambda w, m, n: -(-w[2] // 1024) * 1024 + sum(m) * ODD_BYTES + 4 * (1 + n)
         self.work = torch.empty(max(map(size_of, waves, marks, tiles_of)) + 1024, dtype=torch.uint8, device=device)
         base = -(-self.work.data_ptr() // 1024) * 1024
-        self.status = torch.zeros(1, dtype=torch.int32, device=device) if status is None else status
+        self.status = _lib.status_word(device) if status is None else status
         L = _lib.lib()
         blob, self.waves = bytearray(), []
 
@@ -207,6 +207,4 @@ class SlicedGemm:
 
     def check(self):
         """Raise if a bounded device wait gave up (synchronises)."""
-        st = int(self.status.item())
-        if st != 0:
-            raise _lib.XRHError(f"sliced FP64 GEMM reported status {st} ({_lib.lib().xrh_status_string(st).decode()})")
+        _lib.check_status(self.status, "sliced FP64 GEMM")

@@ -138,13 +138,18 @@ class XRTrimerPlan:
                 perm = [2 * order.index(f) for f in range(3)] + [2 * order.index(f) + 1 for f in range(3)]
                 self.blocks_out[(chg_i, chg_j)] = (B, shape, perm)
                 self._keep += [P, Q, R1, R2, R3]
-        self.stages = [st1.finalize(), st2.finalize(), st3.finalize()]
+        self.status = _lib.status_word(dev)
+        self.stages = [st.finalize(status=self.status) for st in (st1, st2, st3)]
         self.flops = sum(s.flops for s in self.stages)
 
     def launch(self, stream=None):
         """Enqueue the three grouped stages (no host synchronisation)."""
         for st in self.stages:
             st.run(stream)
+
+    def check_status(self):
+        """Raise if a bounded device wait of the launches gave up (synchronises)."""
+        _lib.check_status(self.status, "trimer blocks")
 
     def block(self, chg_i, chg_j):
         """(n_I1, n_I2, n_I3, n_J1, n_J2, n_J3) view of one charge block, or None."""

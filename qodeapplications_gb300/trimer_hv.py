@@ -709,4 +709,5 @@ class XRTrimerHamiltonian:
             if tol is None or resid <= tol * max(1.0, abs(float(w[0]))):
                 break
             lz.v0.copy_(lz.ground_vector())
+        self.check_status()
         return w, resid
