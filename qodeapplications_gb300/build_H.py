@@ -94,7 +94,7 @@ class build_matrix_elements(object):
             plan = XRDimerPlan(spaces, ns, charges, _PairIntegrals(self.ints, (m1, m2)), output="split",
                                precision="fp64", convention="general", layout="product",
                                builders=[ExternalBuilder(self.rho[m1]), ExternalBuilder(self.rho[m2])],
-                               monomer_2e="none", autotune=False)
+                               monomer_2e="none", autotune=False, once=True)
             plan.launch(build_densities=False)
             plan.check_status()
             offs = []
@@ -130,7 +130,7 @@ class build_matrix_elements(object):
             charges = [self.info[m][0] for m in frags]
             ns = [self.info[m][1] for m in frags]
             plan = XRTrimerPlan([self.rho[m] for m in frags], self.ints, [self.n_elec[m] for m in frags], charges,
-                                ns, frags=frags, device=self.device)
+                                ns, frags=frags, device=self.device, once=True)
             plan.launch()
             plan.check_status()
             self._trimer[frags] = {k: plan.block(*k).cpu().numpy() for k in plan.keys()}

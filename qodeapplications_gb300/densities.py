@@ -41,15 +41,8 @@ class Couplings:
         """(operator indices with couplings, first coupling, number, number of sign +1) on the host;
         kept with the list."""
         if self._ranges is None:
-            dev = self.idx_ptr.device
-            pos = torch.zeros(self.count + 1, dtype=torch.int64, device=dev)
-            pos[1:] = torch.cumsum((self.sign > 0).to(torch.int64), 0)
-            p = torch.stack([self.idx_ptr, pos[self.idx_ptr]]).cpu().numpy()
-            n = np.diff(p, axis=1)
-            idx = np.nonzero(n[0])[0]
-            self._ranges = (idx, p[0, idx], n[0, idx], n[1, idx])
+            _fetch_ranges([self])
         return self._ranges
-
 
     def positives(self):
         """Number of couplings of sign +1 (the first ones) of every operator index, on the device; kept."""
@@ -58,6 +51,24 @@ class Couplings:
             pos[1:] = torch.cumsum((self.sign > 0).to(torch.int64), 0)
             self._positives = torch.diff(pos[self.idx_ptr]).contiguous()
         return self._positives
+
+
+def _fetch_ranges(lists):
+    """Couplings.ranges of the lists that have none yet, with one copy to the host for all of them."""
+    lists = [cp for cp in {id(cp): cp for cp in lists}.values() if cp._ranges is None]
+    if not lists:
+        return
+    pos = torch.zeros(sum(cp.count for cp in lists) + 1, dtype=torch.int64, device=lists[0].idx_ptr.device)
+    torch.cumsum(torch.cat([cp.sign for cp in lists]) > 0, 0, out=pos[1:])
+    first = np.cumsum([0] + [cp.count for cp in lists])
+    p = torch.stack([torch.cat([cp.idx_ptr for cp in lists]), pos[torch.cat([cp.idx_ptr + int(f) for cp, f in zip(lists, first)])]])
+    p, at = p.cpu().numpy(), 0
+    for cp in lists:
+        q = p[:, at:at + cp.idx_ptr.numel()]
+        at += cp.idx_ptr.numel()
+        n = np.diff(q, axis=1)
+        idx = np.nonzero(n[0])[0]
+        cp._ranges = (idx, q[0, idx], n[0, idx], n[1, idx])
 
 
 # op strings with two adjacent operators of one kind: position u of the anticommuting pair
@@ -395,23 +406,31 @@ def sliced_units(lists, directions=(0,)):
     contributions would come first and every later addition round against them (error of dE/dz of the
     five-electron states 3.3e-7 instead of 2.1e-7 at 14 orbitals / 60 states).  Direction 1 sets the
     sign bit of n_pos."""
-    units = [np.zeros(0, dtype=_lib.DENS_SLICED_UNIT_DTYPE)]
+    _fetch_ranges([cp for cp, _nb, _nk in lists])
+    parts = []                       # (couplings' ranges, task, block of bra and ket states, direction)
     for i, (cp, nb, nk) in enumerate(lists):
-        idx, c0, count, n_pos = cp.ranges()
-        for ib in range(-(-nb // 64)):
-            for jb in range(-(-nk // 64)):
-                for d in directions:
-                    un = np.zeros(len(idx), dtype=_lib.DENS_SLICED_UNIT_DTYPE)
-                    un["c0"], un["count"] = c0, count
-                    un["n_pos"] = (n_pos.astype(np.uint32) | np.uint32(d << 31)).view(np.int32)
-                    un["task"], un["idx"], un["iblk"], un["jblk"] = i, idx, ib, jb
-                    units.append(un)
-    units = np.concatenate(units)
+        parts += [(cp.ranges(), i, ib, jb, d) for ib in range(-(-nb // 64)) for jb in range(-(-nk // 64)) for d in directions]
+    units = np.zeros(sum(len(p[0][0]) for p in parts), dtype=_lib.DENS_SLICED_UNIT_DTYPE)
+    size = [len(p[0][0]) for p in parts]
+    if parts:
+        for name, k in (("idx", 0), ("c0", 1), ("count", 2)):
+            units[name] = np.concatenate([p[0][k] for p in parts])
+        n_pos = np.concatenate([p[0][3] for p in parts]).astype(np.uint32)
+        units["n_pos"] = (n_pos | np.repeat(np.array([p[4] << 31 for p in parts], dtype=np.uint32), size)).view(np.int32)
+        for name, k in (("task", 1), ("iblk", 2), ("jblk", 3)):
+            units[name] = np.repeat([p[k] for p in parts], size)
     return units[np.lexsort((-units["count"], units["task"] if len(directions) > 1 else 0 * units["task"]))]
 
 
-def _upload(tab, device):
-    return torch.from_numpy(np.frombuffer(tab.tobytes() or bytes(1), dtype=np.uint8).copy()).to(device)
+def _upload(tabs, device):
+    """Structured arrays on the device, one copy: a byte tensor each (128-byte aligned)."""
+    raw = [t.tobytes() or bytes(1) for t in tabs]
+    at = np.cumsum([0] + [-(-len(r) // 128) * 128 for r in raw])
+    host = np.zeros(int(at[-1]), dtype=np.uint8)
+    for a, r in zip(at, raw):
+        host[a:a + len(r)] = np.frombuffer(r, dtype=np.uint8)
+    dev = torch.from_numpy(host).to(device)
+    return [dev[int(a):int(a) + len(r)] for a, r in zip(at, raw)]
 
 
 class SlicedDensities:
@@ -427,7 +446,7 @@ class SlicedDensities:
             coeff.fill(t, bra, ket)
         units = sliced_units([(b[0], int(t["nb"]), int(t["nk"])) for b, t in zip(blocks, tasks)])
         self.n_tasks, self.n_units = len(tasks), len(units)
-        self.tasks_dev, self.units_dev = _upload(tasks, device), _upload(units, device)
+        self.tasks_dev, self.units_dev = _upload((tasks, units), device)
         self.status = _lib.status_word(device) if status is None else status
 
     def run(self, s):
@@ -458,7 +477,7 @@ class SlicedDensityAdjoint:
             self.rows[id(coeff)].fill(t, bra, ket)
         units = sliced_units([(b[0], int(t["nb"]), int(t["nk"])) for b, t in zip(blocks, tasks)], (0, 1))
         self.n_tasks, self.n_units = len(tasks), len(units)
-        self.tasks_dev, self.units_dev = _upload(tasks, device), _upload(units, device)
+        self.tasks_dev, self.units_dev = _upload((tasks, units), device)
         self.status = _lib.status_word(device) if status is None else status
 
     def run(self, s):
@@ -512,6 +531,7 @@ class DensityBuilder:
         arena_n = sum(space.couplings[k].K * self.n_states_bra[k[1]] * self.n_states[k[2]] for k in split_keys)
         self._unit_zero = torch.zeros(arena_n, dtype=torch.float64, device=dev) if arena_n else None
         arena_off = 0
+        rows = []                                # blocks with rows of their own
         for (op, bc, kc), cp in space.couplings.items():
             nb, nk = self.n_states_bra[bc], self.n_states[kc]
             shape = (nb, nk) + (space.N,) * len(op)
@@ -520,10 +540,13 @@ class DensityBuilder:
                 self._tmp[(op, bc, kc)] = self._unit_zero[arena_off:arena_off + cp.K * nb * nk]
                 arena_off += cp.K * nb * nk
             else:
-                # (the FP64 path writes the operator indices that have couplings only)
                 # (a mirrored block comes from its partner and has no rows of its own)
                 if (op, bc, kc) not in self.mirror:
-                    self._tmp[(op, bc, kc)] = torch.zeros(cp.K * nb * nk, dtype=torch.float64, device=dev)
+                    rows.append(((op, bc, kc), cp.K * nb * nk))
+        # (the FP64 path writes the operator indices that have couplings only)
+        off = np.cumsum([0] + [-(-n // 16) * 16 for _, n in rows])
+        arena = (torch.empty if self.f32 else torch.zeros)(int(off[-1]), dtype=torch.float64, device=dev)
+        self._tmp.update({key: arena[int(o):int(o) + n] for (key, n), o in zip(rows, off)})
         # canonical lists for the accumulated blocks of op strings with an anticommuting pair (not
         # the warp-per-unit blocks, whose unit tables index the full lists)
         self._canon = {}

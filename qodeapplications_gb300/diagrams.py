@@ -28,7 +28,7 @@ def _gemm(A, W, M, x, K, alpha=1.0, status=None):
     C = torch.zeros((M, x), dtype=torch.float64, device=A.device)
     g = GroupedGemm(A.device)
     g.add(M, x, [(A.contiguous(), K, W.contiguous(), K, K, float(alpha))], C, x, mode=0)
-    g.finalize(status=status).run()
+    g.finalize(status=status, once=True).run()
     if status is None:
         g.check()
     return C

@@ -21,6 +21,9 @@ FP64_TILE = 64
 SLICED_MIN_CHAIN = 24            # longest K chain of a launch from which it is worth the fixed time
 SLICED_MIN_PRODUCTS = 1 << 24    # or all products of a launch (64 x 64 tiles): 28 us of the FP64 pipe
 SLICED_MIN_K = 8                 # shorter tasks cost the epilogues and stores either way
+# A launch that runs once (finalize(once=True)) also pays its plan: about 60 us and 9 us of host work a task,
+# against the CUDA cores' 1.3 us per K of the longest chain and 0.55e6 multiply-adds a us.
+ONCE_US, ONCE_TASK_US, SIMT_K_US, SIMT_PRODUCTS_US = 60.0, 9.0, 1.3, 0.55e6
 
 
 class GroupedGemm:
@@ -70,7 +73,7 @@ class GroupedGemm:
             self._keep += [x for x in (DA, DB) if x is not None]
         self._tasks.append(t)
 
-    def _sliced_tasks(self):
+    def _sliced_tasks(self, once=False):
         """The FP64 tasks that run on the tensor cores (all long enough ones of the launch, or none)."""
         if self.precision != _lib.FP64:
             return []
@@ -79,11 +82,16 @@ class GroupedGemm:
                 sum(K_of(t)) >= SLICED_MIN_K]
         chain = max((K // t["splitk"] for t, K in long), default=0)
         products = sum(-(-t["M"] // 64) * -(-t["N"] // 64) * 4096 * t["batch"] * K for t, K in long)
-        return [t for t, _K in long] if chain >= SLICED_MIN_CHAIN or products >= SLICED_MIN_PRODUCTS else []
+        if chain < SLICED_MIN_CHAIN and products < SLICED_MIN_PRODUCTS:
+            return []
+        if once and max(SIMT_K_US * chain, products / SIMT_PRODUCTS_US) < ONCE_US + ONCE_TASK_US * len(long):
+            return []
+        return [t for t, _K in long]
 
-    def finalize(self, tile=FP64_TILE, status=None):
+    def finalize(self, tile=FP64_TILE, status=None, once=False):
+        """Task tables for run().  status: a word shared with other launches; once: the launch runs one time."""
         self.sliced = None
-        chosen = self._sliced_tasks()
+        chosen = self._sliced_tasks(once)
         if chosen:
             self.sliced = SlicedGemm([dict({k: t[k] for k in t if k not in ("seg_begin", "seg_count", "splitk")},
                                            segs=self._segs[t["seg_begin"]:t["seg_begin"] + t["seg_count"]])

@@ -37,9 +37,10 @@ from .hamiltonian import DeviceIntegrals, XRDimerPlan
 
 
 def dimer_plan_from_densities(dens, integrals, monomer_charges, precision="fp64", output="split",
-                              convention="hermitian", monomer_2e="ccaa", device="cuda"):
+                              convention="hermitian", monomer_2e="ccaa", device="cuda",
+                              once=False):
     """An XRDimerPlan over densities given as reference dictionaries (the two fragments of
-    dens), built once: launch() then forms H without rebuilding densities."""
+    dens), built once: launch() then forms H without rebuilding densities (once: it is called one time)."""
     charges = [list(c) for c in monomer_charges]
     dev = torch.device(device)
     ints = DeviceIntegrals(source=integrals, device=dev)
@@ -59,7 +60,7 @@ def dimer_plan_from_densities(dens, integrals, monomer_charges, precision="fp64"
         ns.append(ns_m)
     return XRDimerPlan(spaces, ns, charges, ints, output=output, precision=precision, convention=convention,
                        layout="product", builders=[ExternalBuilder(r) for r in rho], monomer_2e=monomer_2e,
-                       autotune=False)
+                       autotune=False, once=once)
 
 
 def get_xr_H(ints, dens, xr_order, monomer_charges, bra_det=False, ket_det=False, precision="fp64",
@@ -70,7 +71,7 @@ def get_xr_H(ints, dens, xr_order, monomer_charges, bra_det=False, ket_det=False
         raise NotImplementedError("bra_det / ket_det builds are not provided: the state gradient comes from the "
                                   "adjoint (qodeapplications_gb300.gradients) instead")
     symm_ints, bior_ints, nuc_rep = ints
-    plan = dimer_plan_from_densities(dens, bior_ints, monomer_charges, precision=precision)
+    plan = dimer_plan_from_densities(dens, bior_ints, monomer_charges, precision=precision, once=True)
     plan.launch(build_densities=False)
     H1 = plan.H1()
     H2 = plan.H

@@ -104,7 +104,7 @@ class SigmaTwoElectron:
     density then holds the same-class blocks only: the entries between pairs of different
     spin classes multiply integrals that vanish by spin symmetry."""
 
-    def __init__(self, space, charge, n_states, V_block, precision=_lib.FP64, own_gemm=True):
+    def __init__(self, space, charge, n_states, V_block, precision=_lib.FP64, own_gemm=True, once=False):
         self.space, self.c, self.n = space, charge, n_states
         self.V = V_block.contiguous()
         self.precision = precision if precision in (_lib.FP64, _lib.FP32) else _lib.FP32
@@ -154,7 +154,7 @@ class SigmaTwoElectron:
                 self.reg.split("sigW")
                 self.gemm = g.finalize().autotune()
             elif g is not None:
-                self.gemm = g.finalize()
+                self.gemm = g.finalize(once=once)
 
     def check(self):
         """Raise if a bounded device wait of the own GEMM gave up (synchronises)."""
@@ -265,14 +265,14 @@ def monomer_two_electron(space, coeffs, V_block, c):
     z = coeffs[c].contiguous()
     n = z.shape[0]
     zT = z.t().contiguous()
-    s2 = SigmaTwoElectron(space, c, n, V_block)
+    s2 = SigmaTwoElectron(space, c, n, V_block, once=True)
     s2.run_sigma(zT)
     out = torch.zeros((n, n), dtype=torch.float64, device=space.device)
     g = GroupedGemm(space.device)
     nconf = space.n_conf[c]
     splitk = max(1, min(64, nconf // 512))
     g.add(n, n, [(z, nconf, s2.sigmaT, nconf, nconf, 1.0)], out, n, mode=1, splitk=splitk)
-    g.finalize().run()
+    g.finalize(once=True).run()
     s2.check()
     g.check()
     return out
@@ -364,6 +364,7 @@ class XRDimerPlan:
               precision): each builder's densities are split copies held once, in the split
               group named by the builder (builder.split_group); precontraction outputs and
               integral matrices stay in groups of this plan.
+    once:     the plan is launched one time (its FP64 products are planned accordingly)
 
     The inputs are the persistent coefficient buffers self.coeffs[m][charge]
     (n_states x n_conf); launch() enqueues the whole build on the current stream without
@@ -372,7 +373,7 @@ class XRDimerPlan:
 
     def __init__(self, spaces, n_states, charges, ints, output="full", precision="fp64",
                  convention="hermitian", layout="product", dens_precision=None, sigma_precision=None,
-                 autotune=True, builders=None, monomer_2e="sigma", total_charges=None, registry=None):
+                 autotune=True, builders=None, monomer_2e="sigma", total_charges=None, registry=None, once=False):
         if monomer_2e not in ("sigma", "ccaa", "none"):
             raise ValueError("monomer_2e must be 'sigma', 'ccaa' or 'none'")
         if total_charges is not None and layout == "product":
@@ -536,7 +537,7 @@ class XRDimerPlan:
         for (M_, N_, segs_, out_, ldc_, sk_) in mono:
             pre.add(M_, N_, segs_, out_, ldc_, mode=1, splitk=sk_)
         self.tc = self.precision in (_lib.BF16X3, _lib.TF32X3)
-        self.pre = pre if self.tc else pre.finalize(status=self.status)       # (its FLOP count alone with split precision)
+        self.pre = pre if self.tc else pre.finalize(status=self.status, once=once)       # (its FLOP count alone with split precision)
 
         # ---- final tasks: one per output charge block ----
         nb = [ns[m] for m in (0, 1)]
@@ -640,7 +641,7 @@ class XRDimerPlan:
                         self.final_tasks.append(dict(key=(ci0, ci1, cj0, cj1), segs=segs, M=M, N=Nn, C=Cbuf, ldc=ldc,
                                                      dims=(ni0, nj0, ni1, nj1),
                                                      maps=(rowA, colA, rowB, colB, diagA, diagB), DA=DA, DB=DB))
-        self.fin = fin if self.tc else fin.finalize(status=self.status)
+        self.fin = fin if self.tc else fin.finalize(status=self.status, once=once)
 
         # ---- split-precision tensor-core variant of both launches ----
         if self.tc:
@@ -687,7 +688,7 @@ class XRDimerPlan:
             self._grp_in = sorted(self._grp_in)
             pre_tc.status = fin_tc.status = self.status
             self.reg, self.pre_tc, self.fin_tc = reg, pre_tc.finalize(), fin_tc.finalize()
-            self.pre64 = pre64.finalize(status=self.status)
+            self.pre64 = pre64.finalize(status=self.status, once=once)
             if autotune:
                 self.pre_tc.autotune()
                 self.fin_tc.autotune()

@@ -34,16 +34,26 @@ def _stages(K):
 
 def _operands(t):
     """(pointer, transposed, rows, K, ld, batch, batch stride, block) of A and B of every segment."""
+    M, N, batch, bn, ops = t["M"], t["N"], t["batch"], _bn(t["N"]), []
     for (A, B, lda, ldb, K, _alpha, flags, sA, sB) in t["segs"]:
-        for p, tr, rows, ld, st, block in ((A, flags & 1, t["M"], lda, sA, BM),
-                                           (B, flags >> 1 & 1, t["N"], ldb, sB, _bn(t["N"]))):
-            batch = t["batch"] if st else 1
-            yield (p, tr, rows, K, ld, batch, st if batch > 1 else 0, block)
+        ops.append((A, flags & 1, M, K, lda, batch, sA, BM) if sA and batch > 1 else (A, flags & 1, M, K, lda, 1, 0, BM))
+        ops.append((B, flags >> 1 & 1, N, K, ldb, batch, sB, bn) if sB and batch > 1 else
+                   (B, flags >> 1 & 1, N, K, ldb, 1, 0, bn))
+    return ops
 
 
 def _digit_bytes(op):
     _p, _tr, rows, K, _ld, batch, _st, block = op
     return 2 * (SLICES + 1) * -(-rows // block) * block * batch * _stages(K) * STAGE_K
+
+
+def slice_ctas(rows, K, batch, trans, block):
+    """xrh_slice_ctas of an operand with rows, K and batch > 0 (tables have hundreds of them): CTAs of the digit
+    launch and of the row-maximum launch."""
+    rows_p = -(-rows // block) * block
+    if trans:
+        return batch * (rows_p // 32) * -(-_stages(K) * STAGE_K // 64), batch * -(-rows // 32) * -(-K // 512)
+    return (rows_p * batch if K > 1024 else rows_p * batch // 8), 0
 
 
 def _exp_bytes(op):
@@ -79,7 +89,7 @@ def _part(t, axis, lo, hi):
 
 def _panels(t, limit):
     """The task as parts whose digits fit the limit."""
-    if sum(_digit_bytes(op) for op in set(_operands(t))) <= limit:
+    if sum(map(_digit_bytes, set(_operands(t)))) <= limit:
         return [t]
     if t["batch"] > 1:
         axis, n, unit = "batch", t["batch"], 1
@@ -97,17 +107,16 @@ def plan_waves(tasks, limit=None):
     """[(tasks, {operand: (digit offset, exponent offset)}, bytes, zeroed bytes)]: row exponents of
     transposed operands first (they are zeroed before each run), then the rest."""
     limit = WORKSPACE_LIMIT if limit is None else limit
-    waves, cur, ops, size = [], [], {}, 0
+    waves, cur, ops, size = [], [], {}, 0            # ops: {operand: (digit bytes, exponent bytes)}
     for t in (p for t in tasks for p in _panels(t, limit)):
-        new = [op for op in dict.fromkeys(_operands(t)) if op not in ops]
-        extra = sum(_digit_bytes(op) + _exp_bytes(op) for op in new)
+        mine = {op: ops.get(op) or (_digit_bytes(op), _exp_bytes(op)) for op in _operands(t)}
+        extra = sum(sum(b) for op, b in mine.items() if op not in ops)
         if cur and size + extra > limit:
             waves.append((cur, ops))
             cur, ops, size = [], {}, 0
-            new = list(dict.fromkeys(_operands(t)))
-            extra = sum(_digit_bytes(op) + _exp_bytes(op) for op in new)
+            extra = sum(map(sum, mine.values()))
         cur.append(t)
-        ops.update(dict.fromkeys(new))
+        ops.update(mine)
         size += extra
     if cur:
         waves.append((cur, ops))
@@ -116,13 +125,13 @@ def plan_waves(tasks, limit=None):
         off, at = 0, {}
         for op in sorted(ops, key=lambda o: not o[1]):
             at[op] = off
-            off += _exp_bytes(op)
-        zeroed = sum(_exp_bytes(op) for op in ops if op[1])
+            off += ops[op][1]
+        zeroed = sum(b for op, (_d, b) in ops.items() if op[1])
         off = -(-off // 1024) * 1024
         place = {}
-        for op in ops:
+        for op, (b, _e) in ops.items():
             place[op] = (off, at[op])
-            off += _digit_bytes(op)
+            off += b
         out.append((cur, place, off, zeroed))
     return out
 
@@ -136,9 +145,14 @@ def split_factors(tasks):
     return [max(1, -(-n // per)) if t["mode"] == 1 else 1 for t, n in zip(tasks, stages)]
 
 
-def _table(rows, dtype):
-    """Structured array of rows given as dicts; fields they do not have are zero."""
-    return np.array([tuple(r.get(n, 0) for n in dtype.names) for r in rows], dtype=dtype)
+# the fields of a task that only the scatter epilogue has
+_MAPS = ("rowA", "colA", "rowB", "colB", "DA", "DB", "diagA", "diagB")
+_NO_MAPS = (0,) * len(_MAPS)
+assert TASK_DTYPE.names == ("M", "N", "seg_begin", "seg_count", "mode", "splitk", "tile_begin", "C", "ldc") + _MAPS + ("batch", "sC")
+assert SLICE_TASK_DTYPE.names == ("src", "digits", "exps", "rows", "K", "ld", "Kp", "batch", "sbatch", "trans", "block", "cta_begin",
+                                  "max_begin")
+assert SLICED_SEG_DTYPE.names == ("digA", "digB", "stages", "rA", "rB", "eA", "eB", "A", "B", "lda", "ldb", "K", "flags", "sA", "sB",
+                                  "alpha")
 
 
 class SlicedGemm:
@@ -151,14 +165,13 @@ class SlicedGemm:
         waves = plan_waves(tasks)
         splits = [split_factors(w[0]) for w in waves]
         # behind the digits of a wave the marks of its tiles (a range per task) and the list of marked tiles
-        runs = lambda t: sum(-(-_stages(s[4]) // RUN_STAGES) for s in t["segs"])
-        marks = [[_tiles(t) * k * runs(t) for t, k in zip(w[0], sk)] for w, sk in zip(waves, splits)]
-        tiles_of = [sum(_tiles(t) * k for t, k in zip(w[0], sk)) for w, sk in zip(waves, splits)]
-        size_of = lambda w, m, n: -(-w[2] // 1024) * 1024 + sum(m) * ODD_BYTES + 4 * (1 + n)
+        tiles_of = [[_tiles(t) * k for t, k in zip(w[0], sk)] for w, sk in zip(waves, splits)]
+        runs_of = [[sum(-(-_stages(s[4]) // RUN_STAGES) for s in t["segs"]) for t in w[0]] for w in waves]
+        marks = [[n * r for n, r in zip(*x)] for x in zip(tiles_of, runs_of)]
+        size_of = lambda w, m, n: -(-w[2] // 1024) * 1024 + sum(m) * ODD_BYTES + 4 * (1 + sum(n))
         self.work = torch.empty(max(map(size_of, waves, marks, tiles_of)) + 1024, dtype=torch.uint8, device=device)
         base = -(-self.work.data_ptr() // 1024) * 1024
         self.status = _lib.status_word(device) if status is None else status
-        L = _lib.lib()
         blob, self.waves = bytearray(), []
 
         def put(raw):
@@ -167,29 +180,29 @@ class SlicedGemm:
             blob.extend(bytes(-len(blob) % 128))
             return at
 
-        for (cur, place, size, zeroed), splitk, mark in zip(waves, splits, marks):
-            # rows as dicts, then one conversion per table
+        for (cur, place, size, zeroed), splitk, count, runs, mark in zip(waves, splits, tiles_of, runs_of, marks):
+            # rows as tuples, then one conversion per table
             st, ctas, max_ctas = [], 0, 0
             # transposed operands last: their tasks own the CTAs of the row-maximum launch
             for op in sorted(place, key=lambda o: o[1]):
                 p, tr, rows, K, ld, batch, sb, block = op
-                st.append(dict(src=p, digits=base + place[op][0], exps=base + place[op][1], rows=rows, K=K, ld=ld,
-                               Kp=_stages(K) * STAGE_K, batch=batch, sbatch=sb, trans=tr, block=block, cta_begin=ctas,
-                               max_begin=max_ctas))
-                ctas += L.xrh_slice_ctas(rows, K, batch, tr, block, 0)
-                max_ctas += L.xrh_slice_ctas(rows, K, batch, tr, block, 1)
+                st.append((p, base + place[op][0], base + place[op][1], rows, K, ld, _stages(K) * STAGE_K, batch, sb, tr,
+                           block, ctas, max_ctas))
+                c, m = slice_ctas(rows, K, batch, tr, block)
+                ctas, max_ctas = ctas + c, max_ctas + m
             gt, gs, tiles = [], [], 0
-            for t, sk in zip(cur, splitk):
-                gt.append(dict(t, seg_begin=len(gs), seg_count=len(t["segs"]), splitk=sk, tile_begin=tiles))
-                tiles += _tiles(t) * sk
+            for t, sk, n in zip(cur, splitk, count):
+                gt.append((t["M"], t["N"], len(gs), len(t["segs"]), t["mode"], sk, tiles, t["C"], t["ldc"],
+                           *([t[n] for n in _MAPS] if t["mode"] == 2 else _NO_MAPS), t["batch"], t["sC"]))
+                tiles += n
                 ops = _operands(t)
-                for (A, B, lda, ldb, K, alpha, flags, sA, sB), a, b in zip(t["segs"], ops, ops):
-                    gs.append(dict(digA=base + place[a][0], digB=base + place[b][0], stages=_stages(K),
-                                   rA=a[2] if a[5] > 1 else 0, rB=b[2] if b[5] > 1 else 0, eA=base + place[a][1],
-                                   eB=base + place[b][1], A=A, B=B, lda=lda, ldb=ldb, K=K, alpha=alpha, flags=flags,
-                                   sA=sA, sB=sB))
-            st, gt, gs = (_table(rows, dtype) for rows, dtype in ((st, SLICE_TASK_DTYPE), (gt, TASK_DTYPE), (gs, SLICED_SEG_DTYPE)))
-            odd = np.stack([np.cumsum([0] + mark[:-1]), [runs(t) for t in cur]], axis=1).astype(np.int64)
+                for (A, B, lda, ldb, K, alpha, flags, sA, sB), a, b in zip(t["segs"], ops[::2], ops[1::2]):
+                    (dA, eA), (dB, eB) = place[a], place[b]
+                    gs.append((base + dA, base + dB, _stages(K), a[2] if a[5] > 1 else 0, b[2] if b[5] > 1 else 0, base + eA,
+                               base + eB, A, B, lda, ldb, K, flags, sA, sB, alpha))
+            st, gt, gs = (np.array(rows, dtype=dtype)
+                          for rows, dtype in ((st, SLICE_TASK_DTYPE), (gt, TASK_DTYPE), (gs, SLICED_SEG_DTYPE)))
+            odd = np.stack([np.cumsum([0] + mark[:-1]), runs], axis=1).astype(np.int64)
             self.waves.append((put(st.tobytes()), len(st), ctas, max_ctas, zeroed, put(gt.tobytes()), len(gt), tiles,
                                put(gs.tobytes()), put(odd.tobytes()), base + -(-size // 1024) * 1024,
                                base + -(-size // 1024) * 1024 + sum(mark) * ODD_BYTES))

@@ -63,9 +63,10 @@ class XRTrimerPlan:
     ints:     DeviceIntegrals over the three fragments (T, U, V block accessors)
     n_elec:   reference electron counts of the three fragments
     charges:  three charge lists;  n_states: three {charge: n}
+    once:     the plan is launched one time
     The density tensors are read in place: rebuild them, then launch() again."""
 
-    def __init__(self, rho, ints, n_elec, charges, n_states, frags=(0, 1, 2), device="cuda"):
+    def __init__(self, rho, ints, n_elec, charges, n_states, frags=(0, 1, 2), device="cuda", once=False):
         dev = torch.device(device)
         self.device = dev
         f64 = dict(dtype=torch.float64, device=dev)
@@ -139,7 +140,7 @@ class XRTrimerPlan:
                 self.blocks_out[(chg_i, chg_j)] = (B, shape, perm)
                 self._keep += [P, Q, R1, R2, R3]
         self.status = _lib.status_word(dev)
-        self.stages = [st.finalize(status=self.status) for st in (st1, st2, st3)]
+        self.stages = [st.finalize(status=self.status, once=once) for st in (st1, st2, st3)]
         self.flops = sum(s.flops for s in self.stages)
 
     def launch(self, stream=None):
