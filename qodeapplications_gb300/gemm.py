@@ -88,14 +88,15 @@ class GroupedGemm:
             return []
         return [t for t, _K in long]
 
-    def finalize(self, tile=FP64_TILE, status=None, once=False):
-        """Task tables for run().  status: a word shared with other launches; once: the launch runs one time."""
+    def finalize(self, tile=FP64_TILE, status=None, once=False, work=None):
+        """Task tables for run().  status: a word shared with other launches; once: the launch runs one time;
+        work: a digit Workspace shared with other launches (its owner allocates it before the first run)."""
         self.sliced = None
         chosen = self._sliced_tasks(once)
         if chosen:
             self.sliced = SlicedGemm([dict({k: t[k] for k in t if k not in ("seg_begin", "seg_count", "splitk")},
                                            segs=self._segs[t["seg_begin"]:t["seg_begin"] + t["seg_count"]])
-                                      for t in chosen], self.device, status)
+                                      for t in chosen], self.device, status, work)
         ids = {id(t) for t in chosen}
         simt = [t for t in self._tasks if id(t) not in ids]
         self.n_tasks, self.total_tiles = len(simt), 0

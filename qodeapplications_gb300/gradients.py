@@ -149,7 +149,7 @@ class XRDimerAdjoint:
                 # Z[i1, (j0,x)] = a sum_i0 D[i0,i1] A[(i0,j0),x]
                 L1.add(ni1, nj0 * K, [(Di, tot1, A, nj0 * K, ni0, a, 3, 0, 0)], Z, nj0 * K)
                 self.final_adj.append((A, B, K, Y, Z, Dj, (ni0, nj0, ni1, nj1)))
-        self.L1 = L1.finalize(status=plan.status)
+        self.L1 = L1.finalize(status=plan.status, work=plan.workspace)
 
         # ---- launch 2: dA, dB (batched), monomer pieces ----
         L2 = GroupedGemm(dev, gprec)
@@ -178,7 +178,7 @@ class XRDimerAdjoint:
                 L2.add(nconf, n, [(sg.sigmaT, nconf, gb, n, n, 2.0, 1, 0, 0)], G[("gzT", m, c)], n, mode=1)
                 # Y^T = z^T g^T for the two-particle density of the weighted ensemble
                 L2.add(nconf, n, [(plan.builders[m].zT[c], n, gb, n, n, 1.0)], G[("YT", m, c)], n)
-        self.L2 = L2.finalize(status=plan.status)
+        self.L2 = L2.finalize(status=plan.status, work=plan.workspace)
 
         # ---- launch 3: precontraction adjoint ----
         # every gradient buffer's writers: outputs written by this launch alone take plain stores
@@ -235,7 +235,7 @@ class XRDimerAdjoint:
                     # dW[x, y] += sum_m dP[m, x] rho[m, y]
                     L3.add(X, Yk, [(gP, X, rho_t, Yk, M, 1.0, 3, 0, 0)], G[("gW", wk)], Yk, mode=1,
                            splitk=_splitk(M, 256, 32))
-            self.L3 = L3.finalize(status=plan.status)
+            self.L3 = L3.finalize(status=plan.status, work=plan.workspace)
 
         # ---- launch 4 inputs: transposed density gradients for the coupling-list adjoint ----
         # (FP32 accumulation buffers on the split-precision paths)
@@ -284,7 +284,8 @@ class XRDimerAdjoint:
             if flat_all:
                 idx = torch.as_tensor(np.concatenate(flat_all), dtype=torch.int64, device=dev)
                 self.gam_scatter.append((m, idx, self.G[("Gpairs", m)][:off]))
-        self.Lgamma = Lg.finalize(status=plan.status)
+        self.Lgamma = Lg.finalize(status=plan.status, work=plan.workspace)
+        plan.workspace.allocate()
         self.gam_reg.upload()
         Lgt.status = plan.status
         self.Lgamma_tc = Lgt.finalize().autotune()
@@ -668,7 +669,8 @@ class XRDimerAdjoint:
         if not self.prec32 and t >= ORBITAL_SLICED_MIN:
             b["VG"] = GroupedGemm(dev)
             b["VG"].add(t, t, [(b["A"], t ** 3, b["B"], t ** 3, t ** 3, 0.5)], b["Gso"], t, mode=1)
-            b["VG"].finalize(status=self.plan.status)
+            b["VG"].finalize(status=self.plan.status, work=self.plan.workspace)
+            self.plan.workspace.allocate()
         b["inputs"] = self._orbital_inputs()
         self._orb = b
         return b

@@ -25,6 +25,7 @@ from . import _lib
 from ._lib import call, ptr, stream_ptr
 from .densities import DensityBuilder, FragmentSpace
 from .gemm import GroupedGemm, SplitRegistry, TCGroupedGemm
+from .sliced import Workspace
 
 
 class DeviceIntegrals:
@@ -218,7 +219,7 @@ class SigmaBatch:
     split (tensor-core plans), one grouped GEMM over all spin classes, fragments and charges,
     one grouped pair gather.  items: [(SigmaTwoElectron built with own_gemm=False, its zT)]."""
 
-    def __init__(self, items, device, status=None):
+    def __init__(self, items, device, status=None, work=None):
         self.items = items
         self.tc = bool(items) and items[0][0].tc
         if not items:
@@ -239,7 +240,7 @@ class SigmaBatch:
             g.status = g.status if status is None else status
             self.gemm = g.finalize().autotune()
         else:
-            self.gemm = g.finalize(status=status)
+            self.gemm = g.finalize(status=status, work=work)
 
     def run(self):
         if not self.items:
@@ -365,6 +366,8 @@ class XRDimerPlan:
               group named by the builder (builder.split_group); precontraction outputs and
               integral matrices stay in groups of this plan.
     once:     the plan is launched one time (its FP64 products are planned accordingly)
+    workspace: a digit Workspace shared with other plans of one stream, allocated by its owner before the
+              first launch (None: the plan's own, which its reverse pass shares)
 
     The inputs are the persistent coefficient buffers self.coeffs[m][charge]
     (n_states x n_conf); launch() enqueues the whole build on the current stream without
@@ -373,7 +376,7 @@ class XRDimerPlan:
 
     def __init__(self, spaces, n_states, charges, ints, output="full", precision="fp64",
                  convention="hermitian", layout="product", dens_precision=None, sigma_precision=None,
-                 autotune=True, builders=None, monomer_2e="sigma", total_charges=None, registry=None, once=False):
+                 autotune=True, builders=None, monomer_2e="sigma", total_charges=None, registry=None, once=False, workspace=None):
         if monomer_2e not in ("sigma", "ccaa", "none"):
             raise ValueError("monomer_2e must be 'sigma', 'ccaa' or 'none'")
         if total_charges is not None and layout == "product":
@@ -388,6 +391,7 @@ class XRDimerPlan:
         self.device = spaces[0].device
         dev = self.device
         f64 = dict(dtype=torch.float64, device=dev)
+        self.workspace = Workspace(dev) if workspace is None else workspace
         self.status = _lib.status_word(dev)      # of every launch of this plan and of its reverse pass
         self.coeffs = [{c: torch.zeros((self.n_states[m][c], spaces[m].n_conf[c]), **f64) for c in self.charges[m]}
                        for m in (0, 1)]
@@ -510,7 +514,7 @@ class XRDimerPlan:
                     mono.append((n * n, 1, [(ca, N[m] ** 2, W[("u100", m)], N[m] ** 2, N[m] ** 2, 1.0)], tgt, 1,
                                  _splitk(N[m] ** 2)))
         self.sigma_batch = SigmaBatch([(sg, self.builders[m].zT[c]) for m in (0, 1)
-                                       for c, sg in self.sigma[m].items() if sg.pl is not None], dev, self.status)
+                                       for c, sg in self.sigma[m].items() if sg.pl is not None], dev, self.status, self.workspace)
         # one-column terms (rho^ca . h) are row GEMVs: a 64 x 64 FP64 tile would spend 64x the
         # FMAs of the result on them, and an FP64 tile is slow on this part
         self.mono_gemv = [(sg_[0][0], sg_[0][2], out_, M_, sg_[0][4]) for (M_, N_, sg_, out_, _l, _s) in mono if N_ == 1]
@@ -537,7 +541,7 @@ class XRDimerPlan:
         for (M_, N_, segs_, out_, ldc_, sk_) in mono:
             pre.add(M_, N_, segs_, out_, ldc_, mode=1, splitk=sk_)
         self.tc = self.precision in (_lib.BF16X3, _lib.TF32X3)
-        self.pre = pre if self.tc else pre.finalize(status=self.status, once=once)       # (its FLOP count alone with split precision)
+        self.pre = pre if self.tc else pre.finalize(status=self.status, once=once, work=self.workspace)       # (its FLOP count alone with split precision)
 
         # ---- final tasks: one per output charge block ----
         nb = [ns[m] for m in (0, 1)]
@@ -641,7 +645,7 @@ class XRDimerPlan:
                         self.final_tasks.append(dict(key=(ci0, ci1, cj0, cj1), segs=segs, M=M, N=Nn, C=Cbuf, ldc=ldc,
                                                      dims=(ni0, nj0, ni1, nj1),
                                                      maps=(rowA, colA, rowB, colB, diagA, diagB), DA=DA, DB=DB))
-        self.fin = fin if self.tc else fin.finalize(status=self.status, once=once)
+        self.fin = fin if self.tc else fin.finalize(status=self.status, once=once, work=self.workspace)
 
         # ---- split-precision tensor-core variant of both launches ----
         if self.tc:
@@ -688,10 +692,12 @@ class XRDimerPlan:
             self._grp_in = sorted(self._grp_in)
             pre_tc.status = fin_tc.status = self.status
             self.reg, self.pre_tc, self.fin_tc = reg, pre_tc.finalize(), fin_tc.finalize()
-            self.pre64 = pre64.finalize(status=self.status, once=once)
+            self.pre64 = pre64.finalize(status=self.status, once=once, work=self.workspace)
             if autotune:
                 self.pre_tc.autotune()
                 self.fin_tc.autotune()
+        if workspace is None:
+            self.workspace.allocate()
 
     # ------------------------------------------------------------------------------------
     def _integral_matrices(self, ints):

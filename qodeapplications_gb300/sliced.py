@@ -155,13 +155,35 @@ assert SLICED_SEG_DTYPE.names == ("digA", "digB", "stages", "rA", "rB", "eA", "e
                                   "alpha")
 
 
+class Workspace:
+    """Device memory for the digits of launches that run one after the other (those of a plan and its
+    reverse pass, in the order of one stream).  They join when they are planned; allocate(), before the
+    first run, gives those that have joined since the last call one buffer as large as the largest needs,
+    an earlier one where it is large enough."""
+
+    def __init__(self, device):
+        self.device, self.buf, self.waiting = device, None, []
+
+    def join(self, g):
+        self.waiting.append(g)
+
+    def allocate(self):
+        need = max((g.size for g in self.waiting), default=0)
+        if need and (self.buf is None or self.buf.numel() < need):
+            self.buf = torch.empty(need, dtype=torch.uint8, device=self.device)
+        for g in self.waiting:
+            g.bind(self.buf)
+        self.waiting = []
+
+
 class SlicedGemm:
     """tasks: dicts with M, N, mode, C, ldc, batch, sC, mode 2's maps (device addresses) and segs
     [(A, B, lda, ldb, K, alpha, flags, sA, sB)] (addresses).  status: the int32 device word that a
-    launch sets when a bounded wait gave up (several plans may share one)."""
+    launch sets when a bounded wait gave up (several plans may share one).  work: a Workspace, whose owner
+    allocates it; without one the launch has its own."""
 
-    def __init__(self, tasks, device, status=None):
-        self.device = device
+    def __init__(self, tasks, device, status=None, work=None):
+        self.device, self.tables = device, None
         waves = plan_waves(tasks)
         splits = [split_factors(w[0]) for w in waves]
         # behind the digits of a wave the marks of its tiles (a range per task) and the list of marked tiles
@@ -169,9 +191,20 @@ class SlicedGemm:
         runs_of = [[sum(-(-_stages(s[4]) // RUN_STAGES) for s in t["segs"]) for t in w[0]] for w in waves]
         marks = [[n * r for n, r in zip(*x)] for x in zip(tiles_of, runs_of)]
         size_of = lambda w, m, n: -(-w[2] // 1024) * 1024 + sum(m) * ODD_BYTES + 4 * (1 + sum(n))
-        self.work = torch.empty(max(map(size_of, waves, marks, tiles_of)) + 1024, dtype=torch.uint8, device=device)
-        base = -(-self.work.data_ptr() // 1024) * 1024
+        self.size = max(map(size_of, waves, marks, tiles_of)) + 1024
+        self._plan = list(zip(waves, splits, tiles_of, runs_of, marks))
         self.status = _lib.status_word(device) if status is None else status
+        if work is None:
+            work = Workspace(device)
+            work.join(self)
+            work.allocate()
+        else:
+            work.join(self)
+
+    def bind(self, work):
+        """Task tables over the workspace `work` (a byte tensor), uploaded in one copy."""
+        self.work = work
+        self.base = base = -(-work.data_ptr() // 1024) * 1024
         blob, self.waves = bytearray(), []
 
         def put(raw):
@@ -180,7 +213,7 @@ class SlicedGemm:
             blob.extend(bytes(-len(blob) % 128))
             return at
 
-        for (cur, place, size, zeroed), splitk, count, runs, mark in zip(waves, splits, tiles_of, runs_of, marks):
+        for (cur, place, size, zeroed), splitk, count, runs, mark in self._plan:
             # rows as tuples, then one conversion per table
             st, ctas, max_ctas = [], 0, 0
             # transposed operands last: their tasks own the CTAs of the row-maximum launch
@@ -206,10 +239,12 @@ class SlicedGemm:
             self.waves.append((put(st.tobytes()), len(st), ctas, max_ctas, zeroed, put(gt.tobytes()), len(gt), tiles,
                                put(gs.tobytes()), put(odd.tobytes()), base + -(-size // 1024) * 1024,
                                base + -(-size // 1024) * 1024 + sum(mark) * ODD_BYTES))
-        self.tables = torch.frombuffer(blob, dtype=torch.uint8).to(device)
-        self.base = base
+        self.tables = torch.frombuffer(blob, dtype=torch.uint8).to(self.device)
+        self._plan = None
 
     def run(self, stream=None):
+        if self.tables is None:
+            raise RuntimeError("the workspace of this launch has not been allocated")
         s = stream_ptr(stream)
         t = self.tables.data_ptr()
         for st, n_s, ctas, max_ctas, zeroed, gt, n_t, tiles, gs, odd, bits, marked in self.waves:

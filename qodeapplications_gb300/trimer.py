@@ -28,6 +28,7 @@ import torch
 
 from . import _lib
 from .gemm import GroupedGemm
+from .sliced import Workspace
 
 
 def _case(ci, cj):
@@ -140,7 +141,9 @@ class XRTrimerPlan:
                 self.blocks_out[(chg_i, chg_j)] = (B, shape, perm)
                 self._keep += [P, Q, R1, R2, R3]
         self.status = _lib.status_word(dev)
-        self.stages = [st.finalize(status=self.status, once=once) for st in (st1, st2, st3)]
+        work = Workspace(dev)
+        self.stages = [st.finalize(status=self.status, once=once, work=work) for st in (st1, st2, st3)]
+        work.allocate()
         self.flops = sum(s.flops for s in self.stages)
 
     def launch(self, stream=None):

@@ -42,6 +42,7 @@ import torch
 from . import _lib
 from ._lib import call, ptr, stream_ptr
 from .gemm import GroupedGemm
+from .sliced import Workspace
 from .trimer import _case, _phase
 
 IDENTITY = (0, 1, 2)
@@ -426,12 +427,13 @@ class XRTrimerHamiltonian:
                 pair_sectors[p] = sorted({total_charge - c for c in self.charges[s_]})
         # the three pair plans share one split registry: each fragment's densities are split once
         from .gemm import SplitRegistry
+        self.workspace = Workspace(dev)          # digits of all FP64 launches, one after the other
         self.pair_registry = SplitRegistry(precision, dev) if precision in ("bf16x3", "tf32x3") else None
         self.plans = [XRDimerPlan([spaces[a], spaces[b]], [self.n_states[a], self.n_states[b]],
                                   [self.charges[a], self.charges[b]], _PairIntegrals(ints, (a, b)), output=pair_output,
                                   precision=precision, convention="general", layout="sector", autotune=autotune,
                                   builders=[self.builders[a], self.builders[b]], total_charges=pair_sectors[p],
-                                  registry=self.pair_registry)
+                                  registry=self.pair_registry, workspace=self.workspace)
                       for p, (a, b) in enumerate(PAIRS)]
         # each fragment's coefficient buffers and monomer blocks from one pair plan that holds it
         holder = {0: (0, 0), 1: (0, 1), 2: (1, 1)}
@@ -489,6 +491,7 @@ class XRTrimerHamiltonian:
         tc_roles = (("pair",) if pair_terms_tc else ()) + ("A", "B", "C") if self.tc else ()
         self.stage1 = self._grouped(plan.build_tasks, simt)
         self.simt = [self._grouped([t for t in L if t.get("role") not in tc_roles], simt) for L in plan.launches]
+        self.workspace.allocate()
         self.tcs = [[] for _ in plan.launches]
         self.stage_b = self.simt[1]
         if self.tc:
@@ -566,7 +569,7 @@ class XRTrimerHamiltonian:
                              s["flags"], s["sA"], s["sB"]))
             g.add(t["M"], t["N"], segs, self._resolve(t["C"]), t["ldc"], mode=t["mode"], batch=t["batch"], sC=t["sC"],
                   maps=self._maps(t))
-        return g.finalize()
+        return g.finalize(work=self.workspace)
 
     # ---------------------------------------------------------------------------------
     def trimer_integral_set(self, ints):
