@@ -145,9 +145,10 @@ def register(name, restype, argtypes):
 class LaunchCounter:
     """Counts library calls that launch a kernel (the gpu_launches figure): every entry point
     except the host-only ones below launches one kernel of this library (those in `multi` the
-    number given)."""
+    number given, which may depend on the arguments)."""
     multi = {"xrh_orbital_terms": 2, "xrh_gemv_rows_split": 2, "xrh_lanczos_normalize_split": 2,
-             "xrh_coeff_digits": 2, "xrh_gemm_sliced_grouped": 2}
+             "xrh_coeff_digits": 2, "xrh_gemm_sliced_grouped": 2,
+             "xrh_slice_grouped": lambda _tasks, _n, _ctas, max_ctas, *_: 2 if max_ctas else 1}
     host_only = {"xrh_abi_version", "xrh_status_string", "xrh_last_cuda_error", "xrh_tc_chunk_elems", "xrh_zero",
                  "xrh_tc_encode_map", "xrh_state_ctas", "xrh_abt_ctas", "xrh_lanczos_coop_work",
                  "xrh_lanczos_cluster_fits", "xrh_gemv_split_work", "xrh_mirror_ctas", "xrh_density_layout_ctas", "xrh_pair_rows_ctas", "xrh_slice_ctas", "xrh_coeff_digit_ctas"}
@@ -157,7 +158,8 @@ class LaunchCounter:
 def call(name, *args):
     """Call one ABI function; raise XRHError on a non-zero status."""
     if name not in LaunchCounter.host_only:
-        LaunchCounter.count += LaunchCounter.multi.get(name, 1)
+        n = LaunchCounter.multi.get(name, 1)
+        LaunchCounter.count += n(*args) if callable(n) else n
     st = getattr(lib(), name)(*args)
     if st != XRH_OK:
         msg = lib().xrh_status_string(st).decode()
