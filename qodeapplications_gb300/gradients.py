@@ -331,8 +331,9 @@ class XRDimerAdjoint:
                 self.dens_adj.append((m, op, bc, kc, cp, rt, grad_of[rt.data_ptr()], gT))
         self.dens_adj_all = list(self.dens_adj)
         self._fold = None
-        # FP32 path: every block of a fragment in one grouped launch, on the tensor cores when
-        # every block has at most 64 states per side (else the CUDA-core kernel)
+        # density adjoint: FP64, and FP32 blocks of more than ADJ_UNIT_MAX states, on the tensor cores
+        # (_setup_sliced); smaller FP32 blocks a lane per coupling; or all FP32 blocks of at most 64 states
+        # by the split-precision kernel (density_adjoint='tc')
         self.dens_adj_groups = []
         self.dens_adj_tc = []
         use_tc = (density_adjoint == "tc" and self.prec32 and plan.tc and
@@ -392,26 +393,33 @@ class XRDimerAdjoint:
                                                 max(max(e[5].shape[0], e[5].shape[1]) for e in small)))
                     self.dens_adj = [e for e in self.dens_adj if not any(e is x for x in small)]
                 self._canonicalize(m)
-                entries = [e for e in self.dens_adj if e[0] == m]
-                if not entries:
-                    continue
-                tasks = np.zeros(len(entries), dtype=_lib.DENS_ADJ_TASK_DTYPE)
-                begin = 0
-                for i, (_m, op, bc, kc, cp, rt, grho, gT) in enumerate(entries):
-                    t = tasks[i]
-                    t["idx_ptr"], t["P"], t["Q"], t["sign"] = (cp.idx_ptr.data_ptr(), cp.P.data_ptr(),
-                                                               cp.Q.data_ptr(), cp.sign.data_ptr())
-                    t["zb32"], t["zk32"] = bld.zbT32[bc].data_ptr(), bld.zT32[kc].data_ptr()
-                    t["gT"] = gT.data_ptr()
-                    t["gzb"], t["gzk"] = self.gz32[m][bc].data_ptr(), self.gz32[m][kc].data_ptr()
-                    t["K"], t["nb"], t["nk"], t["cta_begin"] = cp.K, rt.shape[0], rt.shape[1], begin
-                    begin += cp.K
-                dev_tasks = torch.from_numpy(tasks.view(np.uint8).copy()).to(dev)
-                self.dens_adj_groups.append((dev_tasks, len(entries), begin,
-                                             max(e[5].shape[0] for e in entries), max(e[5].shape[1] for e in entries)))
         else:
             self._canonicalize()         # the FP64 adjoint
         self._setup_sliced()
+        if self.prec32 and not self.dens_adj_tc and not self.dens_adj_sliced:
+            self._setup_groups()
+
+    def _setup_groups(self):
+        """Launch tables of xrh_density_adjoint_f32_grouped, one per fragment: for state counts the tensor-core
+        kernel leaves to it (it refuses them), and as its reference."""
+        plan, dev = self.plan, self.plan.device
+        for m in (0, 1):
+            entries = [e for e in self.dens_adj if e[0] == m]
+            if not entries:
+                continue
+            bld = plan.builders[m]
+            tasks = np.zeros(len(entries), dtype=_lib.DENS_ADJ_TASK_DTYPE)
+            begin = 0
+            for t, (_m, op, bc, kc, cp, rt, grho, gT) in zip(tasks, entries):
+                t["idx_ptr"], t["P"], t["Q"], t["sign"] = (cp.idx_ptr.data_ptr(), cp.P.data_ptr(), cp.Q.data_ptr(),
+                                                           cp.sign.data_ptr())
+                t["zb32"], t["zk32"] = bld.zbT32[bc].data_ptr(), bld.zT32[kc].data_ptr()
+                t["gT"] = gT.data_ptr()
+                t["gzb"], t["gzk"] = self.gz32[m][bc].data_ptr(), self.gz32[m][kc].data_ptr()
+                t["K"], t["nb"], t["nk"], t["cta_begin"] = cp.K, rt.shape[0], rt.shape[1], begin
+                begin += cp.K
+            self.dens_adj_groups.append((torch.from_numpy(tasks.view(np.uint8).copy()).to(dev), len(entries), begin,
+                                         max(e[5].shape[0] for e in entries), max(e[5].shape[1] for e in entries)))
 
     def _setup_sliced(self):
         """The transposed density gradients of self.dens_adj on the tensor cores: every block of the
@@ -446,7 +454,6 @@ class XRDimerAdjoint:
         for blocks in by_pad.values():
             self.dens_adj_sliced.append(SlicedDensityAdjoint(blocks, _lib.FP32 if self.prec32 else _lib.FP64, [], dev,
                                                              plan.status))
-        self.dens_adj_groups = []
 
     def _canonicalize(self, m=None):
         """Entries of self.dens_adj (of fragment m, or all) whose op string has an anticommuting
