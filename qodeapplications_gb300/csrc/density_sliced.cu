@@ -492,29 +492,34 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                 }
                 epi_bar();
                 const int32_t *P = T.P + U.c0, *Q = T.Q + U.c0;
+                const int n_odd = s_count, lanes = lanes_per_sum(n_odd, DS_EPI, count), sub = tid % lanes;
 #pragma unroll 1
-                for (int e = tid; e < s_count; e += DS_EPI) {
-                    const int I = i0 + (odd[e] >> 6), J = j0 + (odd[e] & 63);
-                    if (partial && (s_eb[I - i0] >> 20) < 2047u && (s_ek[J - j0] >> 20) < 2047u) {
-                        // the sample does not show it: the magnitudes of all couplings, as far as needed
+                for (int e0 = 0; e0 < n_odd; e0 += DS_EPI / lanes) {
+                    const int e = e0 + tid / lanes, at = odd[e < n_odd ? e : 0];
+                    const int I = i0 + (at >> 6), J = j0 + (at & 63);
+                    bool wanted = e < n_odd;
+                    if (partial) {
+                        // the sample does not show it: the magnitudes of all couplings
                         const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(magnitudes<NPAD>(T, 0)) + (int64_t)U.iblk * T.conf_b * NPAD + I - i0;
                         const __nv_bfloat16* mk = reinterpret_cast<const __nv_bfloat16*>(magnitudes<NPAD>(T, 1)) + (int64_t)U.jblk * T.conf_k * NPAD + J - j0;
+                        const bool finite = (s_eb[I - i0] >> 20) < 2047u && (s_ek[J - j0] >> 20) < 2047u;
                         float m = 0.f;
-                        for (int c = 0; c < count && m < LOW_SUM; c += 8) {
-#pragma unroll
-                            for (int k = 0; k < 8; ++k)
-                                if (c + k < count)
-                                    m = fmaf(__bfloat162float(mb[(int64_t)__ldg(P + c + k) * NPAD]), __bfloat162float(mk[(int64_t)__ldg(Q + c + k) * NPAD]), m);
-                        }
-                        if (!low_sum(m)) continue;
+#pragma unroll 4
+                        for (int c = sub; c < count; c += lanes)
+                            m = fmaf(__bfloat162float(mb[(int64_t)__ldg(P + c) * NPAD]), __bfloat162float(mk[(int64_t)__ldg(Q + c) * NPAD]), m);
+                        for (int o = lanes / 2; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
+                        wanted = wanted && (!finite || low_sum(m));
                     }
                     double x = 0.0;
+                    if (wanted) {
 #pragma unroll 4
-                    for (int c = 0; c < count; ++c) {
-                        const double a = __ldg(T.zbT + (int64_t)__ldg(P + c) * T.nb + I);
-                        x = fma(c < np ? a : -a, __ldg(T.zkT + (int64_t)__ldg(Q + c) * T.nk + J), x);
+                        for (int c = sub; c < count; c += lanes) {
+                            const double a = __ldg(T.zbT + (int64_t)__ldg(P + c) * T.nb + I);
+                            x = fma(c < np ? a : -a, __ldg(T.zkT + (int64_t)__ldg(Q + c) * T.nk + J), x);
+                        }
                     }
-                    T.rhoT[((int64_t)U.idx * T.nb + I) * T.nk + J] = x;
+                    x = sum_lanes(x, lanes);
+                    if (wanted && sub == 0) T.rhoT[((int64_t)U.idx * T.nb + I) * T.nk + J] = x;
                 }
             }
         }

@@ -619,10 +619,11 @@ __global__ void __launch_bounds__(OD_THREADS, 4) odd_products_kernel(const xrh_g
                                                                   const xrh_odd_range* __restrict__ odd_ranges,
                                                                   const uint32_t* __restrict__ odd_bits, const uint32_t* __restrict__ odd_list) {
     __shared__ uint16_t list[OD_MORE_ROWS * 64];
+    __shared__ double s_part[OD_THREADS];
     __shared__ int s_count;
     __shared__ Tile s_tile;
     const int64_t n_odd = odd_list[0];
-    const int rows = n_odd * (SL_BM / OD_ROWS) <= 2 * (int64_t)gridDim.x ? OD_ROWS : OD_MORE_ROWS, steps = SL_BM / rows;
+    const int rows = n_odd * (SL_BM / OD_ROWS) <= 8 * (int64_t)gridDim.x ? OD_ROWS : OD_MORE_ROWS, steps = SL_BM / rows;
     for (int64_t w = blockIdx.x; w < n_odd * steps; w += gridDim.x) {
         const int64_t tile = odd_list[1 + w / steps];
         const int r0 = (int)(w % steps) * rows;
@@ -662,20 +663,36 @@ __global__ void __launch_bounds__(OD_THREADS, 4) odd_products_kernel(const xrh_g
             for (; any; any &= any - 1u) list[at++] = (uint16_t)(r * 64 + part * SL_CW + __ffs((int)any) - 1);
         }
         __syncthreads();
-        for (int e = threadIdx.x; e < s_count; e += OD_THREADS) {
-            const int r = list[e] >> 6, j = list[e] & 63;
+        // a group of threads per element: neighbours, which read neighbouring K of stored rows, or (both operands
+        // stored [k][row]) one of every `step` threads, so that neighbours read neighbouring elements
+        const int count = s_count, lanes = lanes_per_sum(count, OD_THREADS, S0->K), step = OD_THREADS / lanes;
+        const bool across = lanes > 1 && (S0->flags & 3) == 3;
+        const int sub = across ? threadIdx.x / step : threadIdx.x % lanes;
+        for (int e0 = 0; e0 < count; e0 += step) {
+            const int e = e0 + (across ? threadIdx.x % step : threadIdx.x / lanes), at = list[e < count ? e : 0];
+            const int r = at >> 6, j = at & 63;
             const int64_t m = I.m0 + r, col = I.n0 + j;
             double x = 0.0;
             each_run([&](int run, const xrh_sliced_segment& S, int64_t k0, int64_t k1) {
-                if (!((bits[run * (2 * SL_BM) + 2 * r + j / SL_CW] >> (j % SL_CW)) & 1u)) return;
+                if (e >= count || !((bits[run * (2 * SL_BM) + 2 * r + j / SL_CW] >> (j % SL_CW)) & 1u)) return;
                 const double* a = S.A + I.batch * S.sA + m * ((S.flags & 1) ? 1 : S.lda);
                 const double* b = S.B + I.batch * S.sB + col * ((S.flags & 2) ? 1 : S.ldb);
                 const int64_t ka = (S.flags & 1) ? S.lda : 1, kb = (S.flags & 2) ? S.ldb : 1;
                 double y = 0.0;
 #pragma unroll 8
-                for (int64_t k = k0; k < k1; ++k) y = fma(a[k * ka], b[k * kb], y);
+                for (int64_t k = k0 + sub; k < k1; k += lanes) y = fma(a[k * ka], b[k * kb], y);
                 x += S.alpha * y;
             });
+            if (across) {
+                s_part[threadIdx.x] = x;
+                __syncthreads();
+                if (sub == 0)
+                    for (int i = 1; i < lanes; ++i) x += s_part[threadIdx.x + i * step];
+                __syncthreads();
+            } else {
+                x = sum_lanes(x, lanes);
+            }
+            if (e >= count || sub != 0) continue;
             double* d = T.C + I.batch * T.sC +
                         (T.mode == 2 ? (int64_t)(T.rowA[m] + T.rowB[col]) * T.ldc + T.colA[m] + T.colB[col] : m * T.ldc + col);
             if (T.mode == 1) atomicAdd(d, x);

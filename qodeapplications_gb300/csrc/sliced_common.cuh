@@ -168,6 +168,19 @@ __device__ __forceinline__ uint32_t magnitude(double x, int E) {
 // sum has the bound K 2^-53 sum |a||b|.  So the digits are as good where sum |a||b| >= 1.003 2^-6
 // 2^(ea + eb): everywhere for rows of elements of like size (there it is about K / 16 and more), not where
 // the large elements of one row meet zeros or small elements of the other.
+// Lanes that share one of `elements` sums of `terms` terms, for `threads` threads: a power of two, so that few
+// elements keep the threads busy (and neighbouring lanes read neighbouring terms).
+__device__ __forceinline__ int lanes_per_sum(int elements, int threads, int64_t terms) {
+    int n = 1;
+    while (n < 32 && 2 * n * elements <= threads && 2 * n <= terms) n *= 2;
+    return n;
+}
+// The sum over a group of n lanes (a power of two, whole warps call), in every lane.
+__device__ __forceinline__ double sum_lanes(double x, int n) {
+    for (int o = n / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
 constexpr float LOW_SUM = 1.01f / 64.0f;
 __device__ __forceinline__ bool low_sum(float magnitudes) { return magnitudes > 0.0f && magnitudes < LOW_SUM; }
 
