@@ -20,8 +20,7 @@
 // sliced_common.cuh: indices without a large coefficient in their couplings, as in the tails of a
 // wave function).  Which ones is decided from below: one MMA over the magnitudes of 64 couplings spread over
 // the list (all of a shorter one) finds most elements large enough, masks of the determinants' nonzero
-// states find those without any product, and the rest have the magnitudes of all their couplings
-// summed.  Gathering every coupling's magnitudes instead cost 18 % (14 orbitals, 40 states: 4.80 ms without,
+// states find those without any product, and the rest are formed in FP64.  Gathering every coupling's magnitudes instead cost 18 % (14 orbitals, 40 states: 4.80 ms without,
 // 4.94 with the sample, 5.70 with all).
 //
 // A CTA (persistent over a work list ordered by length), 16 warps:
@@ -38,7 +37,6 @@
 #include "sliced_common.cuh"
 #include "tc_common.cuh"
 #include "xrh_common.cuh"
-#include <cuda_bf16.h>
 
 namespace {
 using namespace xrh_tc;
@@ -493,33 +491,82 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                 epi_bar();
                 const int32_t *P = T.P + U.c0, *Q = T.Q + U.c0;
                 const int n_odd = s_count, lanes = lanes_per_sum(n_odd, DS_EPI, count), sub = tid % lanes;
-#pragma unroll 1
-                for (int e0 = 0; e0 < n_odd; e0 += DS_EPI / lanes) {
-                    const int e = e0 + tid / lanes, at = odd[e < n_odd ? e : 0];
-                    const int I = i0 + (at >> 6), J = j0 + (at & 63);
-                    bool wanted = e < n_odd;
-                    if (partial) {
-                        // the sample does not show it: the magnitudes of all couplings
-                        const __nv_bfloat16* mb = reinterpret_cast<const __nv_bfloat16*>(magnitudes<NPAD>(T, 0)) + (int64_t)U.iblk * T.conf_b * NPAD + I - i0;
-                        const __nv_bfloat16* mk = reinterpret_cast<const __nv_bfloat16*>(magnitudes<NPAD>(T, 1)) + (int64_t)U.jblk * T.conf_k * NPAD + J - j0;
-                        const bool finite = (s_eb[I - i0] >> 20) < 2047u && (s_ek[J - j0] >> 20) < 2047u;
-                        float m = 0.f;
-#pragma unroll 4
-                        for (int c = sub; c < count; c += lanes)
-                            m = fmaf(__bfloat162float(mb[(int64_t)__ldg(P + c) * NPAD]), __bfloat162float(mk[(int64_t)__ldg(Q + c) * NPAD]), m);
-                        for (int o = lanes / 2; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
-                        wanted = wanted && (!finite || low_sum(m));
+                // the couplings' determinants staged behind the list, so that only the coefficients are waited for
+                constexpr int CH = 1024;
+                int *s_p = reinterpret_cast<int*>(odd + 4096), *s_q = s_p + CH;
+                static_assert(sizeof(s_raw) >= 4096 * 2 + 2 * CH * 4, "list and couplings share the buffer of the sums");
+                auto stage = [&](int c0, int n) {
+                    epi_bar();
+                    for (int i = tid; i < n; i += DS_EPI) {
+                        s_p[i] = __ldg(P + c0 + i);
+                        s_q[i] = __ldg(Q + c0 + i);
                     }
-                    double x = 0.0;
-                    if (wanted) {
+                    epi_bar();
+                };
+                const int rows = T.nb - i0 < NPAD ? T.nb - i0 : NPAD, cols = T.nk - j0 < NPAD ? T.nk - j0 : NPAD;
+                if (NPAD == 64 && 3 * n_odd >= rows * cols) {
+                    // most of a large block: all of it, 4 x 2 elements a thread (6 loads for 8 FMAs; a thread an
+                    // element: 119 ms instead of 79 for all indices of 28 spin orbitals, 40 states, CUDA-core
+                    // kernel 61; 60 x 60 states of 20 spin orbitals 21.8 and 19)
+                    const int tk = (cols + 1) / 2, tiles = (rows + 3) / 4 * tk;
+#pragma unroll 1
+                    for (int t0 = 0; t0 < tiles; t0 += DS_EPI) {
+                        const int t = t0 + tid, I = t / tk * 4, J = t % tk * 2;
+                        const double* zb[4];
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) zb[r] = T.zbT + i0 + (I + r < rows ? I + r : 0);
+                        const double *zk0 = T.zkT + j0 + J, *zk1 = J + 1 < cols ? zk0 + 1 : zk0;
+                        double x[4][2];
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) x[r][0] = x[r][1] = 0.0;
+#pragma unroll 1
+                        for (int c0 = 0; c0 < count; c0 += CH) {
+                            const int n = count - c0 < CH ? count - c0 : CH;
+                            if (t0 == 0 || count > CH) stage(c0, n);
+                            if (t >= tiles) continue;
 #pragma unroll 4
-                        for (int c = sub; c < count; c += lanes) {
-                            const double a = __ldg(T.zbT + (int64_t)__ldg(P + c) * T.nb + I);
-                            x = fma(c < np ? a : -a, __ldg(T.zkT + (int64_t)__ldg(Q + c) * T.nk + J), x);
+                            for (int c = 0; c < n; ++c) {
+                                const int64_t p = (int64_t)s_p[c] * T.nb, q = (int64_t)s_q[c] * T.nk;
+                                const double k0 = __ldg(zk0 + q), k1 = __ldg(zk1 + q);
+                                const bool neg = c0 + c >= np;
+#pragma unroll
+                                for (int r = 0; r < 4; ++r) {
+                                    const double a = neg ? -__ldg(zb[r] + p) : __ldg(zb[r] + p);
+                                    x[r][0] = fma(a, k0, x[r][0]);
+                                    x[r][1] = fma(a, k1, x[r][1]);
+                                }
+                            }
+                        }
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) {
+                            if (t >= tiles || I + r >= rows) break;
+                            double* out = T.rhoT + ((int64_t)U.idx * T.nb + i0 + I + r) * T.nk + j0 + J;
+                            out[0] = x[r][0];
+                            if (J + 1 < cols) out[1] = x[r][1];
                         }
                     }
-                    x = sum_lanes(x, lanes);
-                    if (wanted && sub == 0) T.rhoT[((int64_t)U.idx * T.nb + I) * T.nk + J] = x;
+                } else {
+#pragma unroll 1
+                    for (int e0 = 0; e0 < n_odd; e0 += DS_EPI / lanes) {
+                        const int e = e0 + tid / lanes, at = odd[e < n_odd ? e : 0];
+                        const int I = i0 + (at >> 6), J = j0 + (at & 63);
+                        const double *zb = T.zbT + I, *zk = T.zkT + J;
+                        double x = 0.0;
+#pragma unroll 1
+                        for (int c0 = 0; c0 < count; c0 += CH) {
+                            const int n = count - c0 < CH ? count - c0 : CH;
+                            if (e0 == 0 || count > CH) stage(c0, n);
+                            if (e < n_odd) {
+#pragma unroll 8
+                                for (int c = sub; c < n; c += lanes) {
+                                    const double a = __ldg(zb + (int64_t)s_p[c] * T.nb);
+                                    x = fma(c0 + c < np ? a : -a, __ldg(zk + (int64_t)s_q[c] * T.nk), x);
+                                }
+                            }
+                        }
+                        x = sum_lanes(x, lanes);
+                        if (e < n_odd && sub == 0) T.rhoT[((int64_t)U.idx * T.nb + I) * T.nk + J] = x;
+                    }
                 }
             }
         }
