@@ -325,7 +325,7 @@ def time_variant(sysd, precision, steps, warmup, l2_flush):
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from ncu captures of the bench
 # command (the summaries are in profiles/); None where no capture of the current kernel exists
-DENSITY_ADJ_TRAFFIC = {(3, "density_adjoint_f32_grouped_kernel"): 0.675e9}
+DENSITY_ADJ_TRAFFIC = {}
 
 
 def measure_peaks():
@@ -359,6 +359,27 @@ def measure_peaks():
     torch.set_float32_matmul_precision(prev)
     torch.cuda.empty_cache()
     out["how"] = "torch.matmul (cuBLAS), best of 3, CUDA events: fp64 4096^3, fp32 IEEE 8192^3, tf32 8192^3"
+    # L2 reads: sums over 64 MB, half of L2, in one graph (no launch gaps)
+    x = torch.zeros(1 << 24, device="cuda")
+    y = torch.empty(1, device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.sum(x, 0, keepdim=True, out=y)
+    torch.cuda.current_stream().wait_stream(side)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        for _ in range(20):
+            torch.sum(x, 0, keepdim=True, out=y)
+    best = 1e9
+    for _ in range(4):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        g.replay()
+        e1.record()
+        torch.cuda.synchronize()
+        best = min(best, e0.elapsed_time(e1))
+    out["l2_read_gbs"] = 20 * x.numel() * 4 / (best * 1e-3) / 1e9
     return out
 
 
@@ -386,8 +407,9 @@ def density_adjoint_work(adj, m):
 def dominant_kernel_roofline(it, config, reps=20):
     """Live CUDA-event timing, on the launching stream, of the dominant kernel of the step in
     the ncu launch list: the FP32 density adjoint (dE/dz from dE/drho): lane per coupling on unit
-    tables for blocks of at most 16 states, one launch per fragment; above, digit slices on the
-    tensor cores, both fragments in one launch.  Timed with the buffers the last iteration left (the launches add
+    tables for blocks of at most 16 states, one launch per fragment; above, BF16 pieces on the
+    tensor cores, both fragments in one launch.  l2: bytes that kernel gathers from L2 (384 of a
+    row of 64 states, both directions of a coupling) and adds to it (4 a result).  Timed with the buffers the last iteration left (the launches add
     into the gradient buffers, which the next iteration zeroes)."""
     import torch
     from qodeapplications_gb300 import _lib
@@ -423,7 +445,13 @@ def dominant_kernel_roofline(it, config, reps=20):
     by = sum(w[0] for w in work) / len(work)
     fl = sum(w[1] for w in work) / len(work)
     kname = "density_adjoint_units_kernel" if name.endswith("units") else "adjoint_sliced_kernel"
-    return dict(name=f"{kname} (FP32 density adjoint)", ms=ms, bytes=by, flops=fl,
+    l2 = 0.0
+    if kname == "adjoint_sliced_kernel":
+        for sl in adj.dens_adj_sliced:
+            for cp, _st, _b, _k, _g, gzb, gzk in sl.keep:
+                blocks = -(-gzb.shape[1] // 64) * -(-gzk.shape[1] // 64)
+                l2 += cp.count * blocks * (2 * 6 * sl.npad) + 4.0 * cp.count * (gzb.shape[1] + gzk.shape[1])
+    return dict(name=f"{kname} (FP32 density adjoint)", ms=ms, bytes=by, flops=fl, l2=l2,
                 kernel=kname, traffic=DENSITY_ADJ_TRAFFIC.get((config, kname)))
 
 
@@ -514,21 +542,31 @@ def run_ours(args):
         hbm = float(peaks.get("hbm_gbs", 6800.0))
         gbs = dk["bytes"] / (dk["ms"] * 1e-3) / 1e9
         tflops = dk["flops"] / (dk["ms"] * 1e-3) / 1e12
-        roofline = {"bound": "fp32 (CUDA-core FMA)", "kernel": dk["name"], "achieved": tflops,
-                    "peak": live["fp32_simt_tflops"], "unit": "TFLOP/s", "frac": tflops / live["fp32_simt_tflops"],
+        tensor = dk["kernel"] == "adjoint_sliced_kernel"
+        l2_gbs = dk["l2"] / (dk["ms"] * 1e-3) / 1e9
+        bf16 = 6.0 * tflops                      # an FP32 product is six of BF16 parts
+        bf16_peak = float(peaks.get("bf16_tflops", 1900.0))
+        roofline = {"bound": "l2" if tensor else "fp32 (CUDA-core FMA)", "kernel": dk["name"],
+                    "achieved": l2_gbs if tensor else tflops, "peak": live["l2_read_gbs"] if tensor else live["fp32_simt_tflops"],
+                    "unit": "GB/s" if tensor else "TFLOP/s",
+                    "frac": l2_gbs / live["l2_read_gbs"] if tensor else tflops / live["fp32_simt_tflops"],
                     "traffic": dk["traffic"], "launch_ms": dk["ms"],
                     "algorithmic_bytes_per_launch": dk["bytes"], "flops_per_launch": dk["flops"],
-                    "peak_source": "fp32 IEEE cuBLAS GEMM measured in this run (of measured)",
+                    "peak_source": ("sum over 64 MB that stay in L2, measured in this run" if tensor else
+                                    "fp32 IEEE cuBLAS GEMM measured in this run") + " (of measured)",
+                    "tensor": {"achieved_tflops": bf16, "peak_tflops": bf16_peak, "frac": bf16 / bf16_peak,
+                               "peak_source": "MEASURED_PEAKS.json bf16_tflops (of measured)" if "bf16_tflops" in peaks
+                               else "fallback 1.9 PFLOP/s (of fallback)"} if tensor else None,
                     "hbm": {"achieved_gbs": gbs, "peak_gbs": hbm, "frac": gbs / hbm,
                             "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if "hbm_gbs" in peaks
                             else "fallback 6.8 TB/s (of fallback)"},
                     "traffic_source": ("ncu dram__bytes_read.sum + dram__bytes_write.sum of this kernel in a "
                                        "capture of the bench command (profiles/)") if dk["traffic"] else
                                       "null: no ncu capture of the current kernel build at this workload",
-                    "note": "products over coupling lists (4 n_b n_k FLOPs and 9 bytes per coupling; coefficient rows "
-                            "gathered from L2), FLOPs as on the CUDA cores; above 16 states the kernel forms them from "
-                            "21 BF16 digit-slice products on the tensor cores, so the FP32 rate is a yardstick there, "
-                            "not its bound; the HBM fraction is given beside it"}
+                    "note": ("rows of BF16 pieces gathered from L2 and results added to it; six BF16 products an FP32 "
+                             "one on the tensor cores, whose fraction is given beside it") if tensor else
+                            ("products over coupling lists (4 n_b n_k FLOPs and 9 bytes per coupling; coefficient "
+                             "rows gathered from L2); the HBM fraction is given beside it")}
     else:
         roofline = None
 
