@@ -81,29 +81,8 @@ __device__ __forceinline__ bool all_digit(bool x) {        // barrier of the war
         : "memory");
     return r != 0;
 }
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(AS_EPI) : "memory"); }
-__device__ __forceinline__ int epi_bar_or(int pred) {
-    int r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(r)
-        : "r"(pred), "n"(AS_EPI)
-        : "memory");
-    return r;
-}
-
-// The barrier counts this thread's copies as one arrival once they have landed; their reader, not the
-// thread that issued them, orders them before the MMAs (a proxy fence here would wait for the copies
-// in flight: one gather at a time).
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void fence_copies() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool ok) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
+__device__ __forceinline__ void epi_bar() { named_bar<1, AS_EPI>(); }
+__device__ __forceinline__ int epi_bar_or(int pred) { return named_bar_or<1, AS_EPI>(pred); }
 
 __device__ __forceinline__ void tmem_ld8(uint32_t ta, float (&v)[8]) {
     uint32_t r[8];
@@ -780,6 +759,7 @@ extern "C" int xrh_density_adjoint_sliced_grouped(int precision, const xrh_adj_s
         if (npad == 32) return launch<32, 8>(tasks_dev, units_dev, n_units, status_dev, s);
         return launch<64, 8>(tasks_dev, units_dev, n_units, status_dev, s);
     }
+    // (npad 16: for callers of this entry point; a reverse pass gives such blocks to xrh_density_adjoint_f32_units)
     if (npad == 16) return launch<16, 3>(tasks_dev, units_dev, n_units, status_dev, s);
     if (npad == 32) return launch<32, 3>(tasks_dev, units_dev, n_units, status_dev, s);
     return launch<64, 3>(tasks_dev, units_dev, n_units, status_dev, s);

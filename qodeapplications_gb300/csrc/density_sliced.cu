@@ -65,17 +65,8 @@ struct Cfg {
                   "register split exceeds the launch");
 };
 
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(DS_EPI) : "memory"); }
-__device__ __forceinline__ int epi_bar_or(int pred) {
-    int r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(r)
-        : "r"(pred), "n"(DS_EPI)
-        : "memory");
-    return r;
-}
+__device__ __forceinline__ void epi_bar() { named_bar<1, DS_EPI>(); }
+__device__ __forceinline__ int epi_bar_or(int pred) { return named_bar_or<1, DS_EPI>(pred); }
 
 // MN-major operand: 64-element atoms DS_ATOM apart, 8-coupling groups 1024 B apart.
 __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t saddr) {
@@ -93,19 +84,6 @@ __device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t saddr) {
 __device__ __forceinline__ int sampled(int i, int n) { return n > DS_SAMPLE ? (int)((int64_t)i * n / DS_SAMPLE) : i; }
 
 __device__ __forceinline__ int stages_of(int n) { return (n + DS_KS - 1) / DS_KS; }
-
-// The barrier counts this thread's copies as one arrival once they have landed; their reader, not the
-// thread that issued them, orders them before the MMAs (a proxy fence here would wait for the copies
-// in flight: one gather at a time).
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void fence_copies() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// 16 bytes to shared memory, zeros where ok is false
-__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool ok) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
-}
 
 // columns [c, c + n) of an accumulator, n = 8, 16, 32
 template <int N>

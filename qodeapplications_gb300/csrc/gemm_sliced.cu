@@ -70,17 +70,8 @@ constexpr int SL_RUN_GROUPS = 4096;                    // groups collected in 96
 static_assert(NS == 8, "digit weights and shifts below are written for eight slices");
 static_assert((long long)SL_GROUP * SL_KS * NS * (1 << 14) <= (1 << 24), "a group must stay exact in FP32");
 
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(SL_EPI_THREADS) : "memory"); }
-__device__ __forceinline__ int epi_bar_or(int pred) {
-    int r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(r)
-        : "r"(pred), "n"(SL_EPI_THREADS)
-        : "memory");
-    return r;
-}
+__device__ __forceinline__ void epi_bar() { named_bar<1, SL_EPI_THREADS>(); }
+__device__ __forceinline__ int epi_bar_or(int pred) { return named_bar_or<1, SL_EPI_THREADS>(pred); }
 
 // A persistent CTA's tile: task, batch, output corner, N tile, range of K stages.
 struct Tile {

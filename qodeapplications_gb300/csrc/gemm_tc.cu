@@ -56,16 +56,7 @@ constexpr uint32_t TC_B_MAX_BYTES = 128 * 128;
 constexpr uint32_t TC_STAGE_BYTES = 2 * TC_A_BYTES + 2 * TC_B_MAX_BYTES;
 
 // Named barrier 1 over the epilogue warps, returning the OR of a predicate over them.
-__device__ __forceinline__ int epi_bar_or(int pred) {
-    int r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
-        : "=r"(r)
-        : "r"(pred), "n"(TC_EPI_THREADS)
-        : "memory");
-    return r;
-}
+__device__ __forceinline__ int epi_bar_or(int pred) { return named_bar_or<1, TC_EPI_THREADS>(pred); }
 
 __device__ __forceinline__ int find_task(const xrh_tc_task* __restrict__ tasks, int n_tasks, int64_t tile) {
     int lo = 0, hi = n_tasks - 1;
@@ -267,7 +258,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
     } else {
         // ------------------------------------------------------------------ epilogue --
-        const int quarter = warp & 3, part = warp >> 2;      // TMEM lanes 32*quarter.., column half
+        const int quarter = warp & 3, part = warp >> 2;      // TMEM lanes 32*quarter.., a quarter of the columns
         for (uint32_t k = 0;; ++k) {
             const bool here = mbar_wait(smem_u32(&tile_bar[k % TC_TILES]), (k / TC_TILES) & 1u, &abort_sh);
             const TileInfo I = s_tile[k % TC_TILES];

@@ -56,6 +56,35 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
         : "memory");
 }
 
+// Barrier ID of N threads, alone or with the OR of a predicate.
+template <int ID, int N>
+__device__ __forceinline__ void named_bar() {
+    asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+template <int ID, int N>
+__device__ __forceinline__ int named_bar_or(int pred) {
+    int r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, %2, %3, p;\n\tselp.b32 %0, 1, 0, q;\n\t}\n"
+        : "=r"(r)
+        : "r"(pred), "n"(ID), "n"(N)
+        : "memory");
+    return r;
+}
+
+// The barrier counts this thread's cp.async copies as one arrival once they have landed; their reader, not
+// the thread that issued them, orders them before its MMAs by fence_copies (a proxy fence behind the copies
+// would wait for those in flight: one gather at a time).
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void fence_copies() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// 16 bytes to shared memory, zeros where ok is false
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+
 // Untiled bulk copy of `bytes` contiguous bytes (a multiple of 16; both addresses 16-byte aligned).
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
