@@ -654,10 +654,13 @@ __global__ void __launch_bounds__(OD_THREADS, 4) odd_products_kernel(const xrh_g
             for (; any; any &= any - 1u) list[at++] = (uint16_t)(r * 64 + part * SL_CW + __ffs((int)any) - 1);
         }
         __syncthreads();
-        // a group of threads per element: neighbours, which read neighbouring K of stored rows, or (both operands
-        // stored [k][row]) one of every `step` threads, so that neighbours read neighbouring elements
-        const int count = s_count, lanes = lanes_per_sum(count, OD_THREADS, S0->K), step = OD_THREADS / lanes;
-        const bool across = lanes > 1 && (S0->flags & 3) == 3;
+        // a group of threads per element: neighbours, which read neighbouring K of stored rows (a lane a row would
+        // touch 32 lines an instruction, twice the time of its FMAs), or, both operands stored [k][row], one of
+        // every `step` threads, so that neighbours read neighbouring elements
+        const bool trans = (S0->flags & 3) == 3;
+        const int count = s_count, lanes = lanes_per_sum(count, OD_THREADS, S0->K, trans ? 1 : S0->K >= 64 ? 8 : 2);
+        const int step = OD_THREADS / lanes;
+        const bool across = lanes > 1 && trans;
         const int sub = across ? threadIdx.x / step : threadIdx.x % lanes;
         for (int e0 = 0; e0 < count; e0 += step) {
             const int e = e0 + (across ? threadIdx.x % step : threadIdx.x / lanes), at = list[e < count ? e : 0];

@@ -170,8 +170,8 @@ __device__ __forceinline__ uint32_t magnitude(double x, int E) {
 // the large elements of one row meet zeros or small elements of the other.
 // Lanes that share one of `elements` sums of `terms` terms, for `threads` threads: a power of two, so that few
 // elements keep the threads busy (and neighbouring lanes read neighbouring terms).
-__device__ __forceinline__ int lanes_per_sum(int elements, int threads, int64_t terms) {
-    int n = 1;
+__device__ __forceinline__ int lanes_per_sum(int elements, int threads, int64_t terms, int least = 1) {
+    int n = least;
     while (n < 32 && 2 * n * elements <= threads && 2 * n <= terms) n *= 2;
     return n;
 }
