@@ -20,8 +20,9 @@
 // sliced_common.cuh: indices without a large coefficient in their couplings, as in the tails of a
 // wave function).  Which ones is decided from below: one MMA over the magnitudes of 64 couplings spread over
 // the list (all of a shorter one) finds most elements large enough, masks of the determinants' nonzero
-// states find those without any product, and the rest are formed in FP64.  Gathering every coupling's magnitudes instead cost 18 % (14 orbitals, 40 states: 4.80 ms without,
-// 4.94 with the sample, 5.70 with all).
+// states find those without any product, and the rest are formed in FP64.  Gathering every coupling's
+// magnitudes instead cost 18 % (14 orbitals, 40 states: 4.80 ms without, 4.94 with the sample, 5.70 with all;
+// 5.06 with the sample and the masks).
 //
 // A CTA (persistent over a work list ordered by length), 16 warps:
 //   * warps 8-11: cp.async gathers of stages of 32 couplings of one sign (positive ones first: the MMA
@@ -29,9 +30,8 @@
 //   * warp 12: MMAs;  * warps 0-7: collection and conversion.
 // Bounds: the gathers, 2 x 16 NPAD bytes of L2 per coupling, against 640 / 192 / 64 cycles of the tensor
 // pipe per 16 couplings at NPAD = 64 / 32 / 16, and the collection (8 NPAD columns a group).  Measured,
-// all blocks of a fragment of 28 spin orbitals: 60 states 115 -> 4.9 ms (97 GFLOP of canonical
-// couplings, 20 TFLOP/s FP64 against the pipe's 1.1), 32 states 1.74, 16 states 1.09; 18 spin orbitals, 10
-// states 3.4 -> 0.086 ms.
+// all blocks of a fragment, no element in FP64: 28 spin orbitals, 60 states 115 -> 5.1 ms (97 GFLOP of
+// canonical couplings, 19 TFLOP/s FP64 against the pipe's 1.1); 22, 27 states 0.47; 18, 10 states 3.4 -> 0.11.
 // Every wait is bounded; on timeout *status is set and all roles leave after their copies and MMAs
 // have completed.
 #include "sliced_common.cuh"
@@ -456,23 +456,35 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                 // sums the digits are too coarse for, states with an infinity or a NaN: the couplings in FP64
                 // (in place of what has been stored), listed first, so that all threads share them
                 uint16_t* odd = reinterpret_cast<uint16_t*>(s_raw);
-                if (row < NPAD && i0 + row < T.nb) {
+                // the couplings' determinants staged behind the list, so that only the coefficients are waited for;
+                // behind those the marked columns of a row and the tiles that begin at it
+                constexpr int CH = 1024;
+                int *s_p = reinterpret_cast<int*>(odd + 4096), *s_q = s_p + CH;
+                uint32_t* s_m = reinterpret_cast<uint32_t*>(s_q + CH);
+                int* s_n = reinterpret_cast<int*>(s_m + 2 * NPAD);
+                static_assert(sizeof(s_raw) >= 4096 * 2 + 2 * CH * 4 + 3 * NPAD * 4, "list, couplings and masks share the buffer of the sums");
+                if (row < NPAD) {
                     const bool bad = (s_eb[row] >> 20) >= 2047u;
 #pragma unroll 1
                     for (int j = 0; j < C::CW; ++j) {
                         const int J = part * C::CW + j;
-                        if (j0 + J < T.nk && (bad || (s_ek[J] >> 20) >= 2047u)) low |= 1u << j;
+                        if (i0 + row < T.nb && j0 + J < T.nk && (bad || (s_ek[J] >> 20) >= 2047u)) low |= 1u << j;
                     }
+                    s_m[2 * row + part] = low;
                     int at = atomicAdd(&s_count, __popc(low));
                     for (; low; low &= low - 1u) odd[at++] = (uint16_t)(row * 64 + part * C::CW + __ffs((int)low) - 1);
                 }
                 epi_bar();
+                auto marked = [&](int r) { return (uint64_t)s_m[2 * r] | ((uint64_t)s_m[2 * r + 1] << C::CW); };
+                if (tid < NPAD) {
+                    const uint64_t m = marked(tid);
+                    int rank = 0;
+                    for (int r = 0; r < tid; ++r) rank += marked(r) == m;
+                    s_n[tid] = rank % 4 == 0 ? (__popcll(m) + 1) / 2 : 0;
+                }
+                epi_bar();
                 const int32_t *P = T.P + U.c0, *Q = T.Q + U.c0;
-                const int n_odd = s_count, lanes = lanes_per_sum(n_odd, DS_EPI, count), sub = tid % lanes;
-                // the couplings' determinants staged behind the list, so that only the coefficients are waited for
-                constexpr int CH = 1024;
-                int *s_p = reinterpret_cast<int*>(odd + 4096), *s_q = s_p + CH;
-                static_assert(sizeof(s_raw) >= 4096 * 2 + 2 * CH * 4, "list and couplings share the buffer of the sums");
+                const int n_odd = s_count;
                 auto stage = [&](int c0, int n) {
                     epi_bar();
                     for (int i = tid; i < n; i += DS_EPI) {
@@ -482,18 +494,56 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                     epi_bar();
                 };
                 const int rows = T.nb - i0 < NPAD ? T.nb - i0 : NPAD, cols = T.nk - j0 < NPAD ? T.nk - j0 : NPAD;
-                if (NPAD == 64 && 3 * n_odd >= rows * cols) {
-                    // most of a large block: all of it, 4 x 2 elements a thread (6 loads for 8 FMAs; a thread an
-                    // element: 119 ms instead of 79 for all indices of 28 spin orbitals, 40 states, CUDA-core
-                    // kernel 61; 60 x 60 states of 20 spin orbitals 21.8 and 19)
-                    const int tk = (cols + 1) / 2, tiles = (rows + 3) / 4 * tk;
+                int grouped = 0;
+                for (int r = 0; r < NPAD; ++r) grouped += s_n[r];
+                const int tk = (cols + 1) / 2, all = (rows + 3) / 4 * tk;
+                const bool whole = grouped > all;
+                const int tiles = whole ? all : grouped;
+                if (2 * 8 * tiles <= 3 * n_odd) {
+                    // tiles of 4 x 2 elements, a group of lanes each: 6 loads for 8 FMAs.  Four rows with the same marked
+                    // columns (a symmetry marks whole classes of states) and two of these columns, or, where the rows
+                    // differ too much, all of the block.  Where they are mostly filled: an element by itself
+                    // costs 1.5 times one of a tile.  Evolved states of two Sz classes, all indices of two
+                    // fragments, ms, by elements / whole blocks / tiles of this kind: 28 spin orbitals, 60 states - / 290 /
+                    // 167, 40 - / 141 / 79, 30 52.2 / - / 40.3; 24, 21 states (tiles filled to 0.8) 11.3 / - /
+                    // 10.6, 16 6.2 / - / 4.8; 18, 10 states (tiles filled to 0.5) 0.61 / - / 0.75
+                    const int lanes = lanes_per_sum(tiles, DS_EPI, count), sub = tid % lanes;
 #pragma unroll 1
-                    for (int t0 = 0; t0 < tiles; t0 += DS_EPI) {
-                        const int t = t0 + tid, I = t / tk * 4, J = t % tk * 2;
-                        const double* zb[4];
+                    for (int t0 = 0; t0 < tiles; t0 += DS_EPI / lanes) {
+                        const int t = t0 + tid / lanes;
+                        int I[4], J[2], n_r = 0, n_c = 0;
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) zb[r] = T.zbT + i0 + (I + r < rows ? I + r : 0);
-                        const double *zk0 = T.zkT + j0 + J, *zk1 = J + 1 < cols ? zk0 + 1 : zk0;
+                        for (int r = 0; r < 4; ++r) I[r] = 0;
+                        J[0] = J[1] = 0;
+                        if (t < tiles && whole) {
+                            const int a = t / tk * 4, b = t % tk * 2;
+                            n_r = rows - a < 4 ? rows - a : 4;
+                            n_c = cols - b < 2 ? cols - b : 2;
+#pragma unroll
+                            for (int r = 0; r < 4; ++r) I[r] = r < n_r ? a + r : a;
+                            J[0] = b;
+                            J[1] = n_c > 1 ? b + 1 : b;
+                        } else if (t < tiles) {
+                            int r0 = 0, c = t;
+                            for (; c >= s_n[r0]; ++r0) c -= s_n[r0];
+                            const uint64_t m = marked(r0);
+                            uint64_t left = m;
+                            for (int k = 0; k < 2 * c; ++k) left &= left - 1ull;
+                            J[0] = J[1] = __ffsll((long long)left) - 1;
+                            left &= left - 1ull;
+                            n_c = left ? 2 : 1;
+                            if (left) J[1] = __ffsll((long long)left) - 1;
+                            I[0] = I[1] = I[2] = I[3] = r0;
+                            n_r = 1;
+                            for (int r = r0 + 1; r < NPAD && n_r < 4; ++r) {
+                                if (marked(r) != m) continue;
+#pragma unroll
+                                for (int k = 1; k < 4; ++k)
+                                    if (k == n_r) I[k] = r;
+                                ++n_r;
+                            }
+                        }
+                        const double *zb = T.zbT + i0, *zk = T.zkT + j0;
                         double x[4][2];
 #pragma unroll
                         for (int r = 0; r < 4; ++r) x[r][0] = x[r][1] = 0.0;
@@ -503,27 +553,29 @@ __global__ void __launch_bounds__(DS_THREADS, Cfg<NPAD>::CTAS)
                             if (t0 == 0 || count > CH) stage(c0, n);
                             if (t >= tiles) continue;
 #pragma unroll 4
-                            for (int c = 0; c < n; ++c) {
-                                const int64_t p = (int64_t)s_p[c] * T.nb, q = (int64_t)s_q[c] * T.nk;
-                                const double k0 = __ldg(zk0 + q), k1 = __ldg(zk1 + q);
+                            for (int c = sub; c < n; c += lanes) {
+                                const double *p = zb + (int64_t)s_p[c] * T.nb, *q = zk + (int64_t)s_q[c] * T.nk;
+                                const double k0 = __ldg(q + J[0]), k1 = __ldg(q + J[1]);
                                 const bool neg = c0 + c >= np;
 #pragma unroll
                                 for (int r = 0; r < 4; ++r) {
-                                    const double a = neg ? -__ldg(zb[r] + p) : __ldg(zb[r] + p);
+                                    const double a = neg ? -__ldg(p + I[r]) : __ldg(p + I[r]);
                                     x[r][0] = fma(a, k0, x[r][0]);
                                     x[r][1] = fma(a, k1, x[r][1]);
                                 }
                             }
                         }
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            if (t >= tiles || I + r >= rows) break;
-                            double* out = T.rhoT + ((int64_t)U.idx * T.nb + i0 + I + r) * T.nk + j0 + J;
-                            out[0] = x[r][0];
-                            if (J + 1 < cols) out[1] = x[r][1];
-                        }
+                        for (int r = 0; r < 4; ++r)
+#pragma unroll
+                            for (int k = 0; k < 2; ++k) {
+                                const double y = sum_lanes(x[r][k], lanes);
+                                if (sub == 0 && r < n_r && k < n_c)
+                                    T.rhoT[((int64_t)U.idx * T.nb + i0 + I[r]) * T.nk + j0 + J[k]] = y;
+                            }
                     }
                 } else {
+                    const int lanes = lanes_per_sum(n_odd, DS_EPI, count), sub = tid % lanes;
 #pragma unroll 1
                     for (int e0 = 0; e0 < n_odd; e0 += DS_EPI / lanes) {
                         const int e = e0 + tid / lanes, at = odd[e < n_odd ? e : 0];
