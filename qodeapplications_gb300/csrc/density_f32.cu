@@ -23,7 +23,7 @@ namespace {
 constexpr int FW_SUB = 32, FW_RING = 3, FW_ROW = 128;  // floats of a staged coupling: bra 64 | ket 64
 constexpr int FW_TN = 4;                               // a lane: 8 rows x 4 columns
 constexpr int FW_THREADS = 64 * 8 / FW_TN, FW_WARPS = FW_THREADS / 32, FW_PER = FW_SUB / FW_WARPS;
-constexpr int FW_CTAS = 3;                             // 168 registers; four (128) spill and are slower
+constexpr int FW_CTAS = 3;                             // 168 registers (4 bytes spilled); four (128) spill more and are slower
 constexpr int FW_STAGE_FLOATS = 8192;
 
 __device__ __forceinline__ void copy16(uint32_t dst, const float* src) {

@@ -24,9 +24,9 @@
 //
 // What bounds it: 36 pairs of BF16 MMAs are 2 304 cycles of the tensor pipe per 128 x 64 x 32 stage; the
 // integer collection of a group (8 x 8 192 conversions) and the flush of a tile (about 25 000 cycles)
-// overlap with it in part.  Measured at M = N = 3 600, K = 784: 0.77 ms, 26 TFLOP/s of FP64 products
-// (CUDA cores: 1.0); 3 600 x 784 x 784 0.22 + 0.03 ms digits against 4.65 ms; one tile of 128 K 27 us
-// against 160 us.
+// overlap with it in part.  Measured, whole launches with their digits: M = N = 3 600, K = 784 0.82 ms, 25 TFLOP/s
+// of FP64 products (CUDA cores: 20.8 ms, 1.0); 3 600 x 784 x 784 0.26 ms against 4.64; one tile of 128 K 39 us
+// against 158 us.
 //
 // Per CTA (persistent over 128 x BN tiles, BN = 64, or 32 for N <= 32), 12 warps:
 //   * warp 8: bulk copies of all eight slices of A and B for 32 K (96 KB: two stages), at the end of a

@@ -163,11 +163,6 @@ __device__ __forceinline__ uint32_t magnitude(double x, int E) {
     return hi == 0u && __double2loint(x) == 0 ? 0u : (uint32_t)max(m, 67 << 7);
 }
 
-// Where a sum needs FP64 arithmetic.  What the digits leave out of K products, 2^-63 2^e of an element and
-// the pairs with i + j >= 8 (7 2^14 256^-1 + .. units of 2^-68), is at most K 1.003 2^-59 2^(ea + eb); an FP64
-// sum has the bound K 2^-53 sum |a||b|.  So the digits are as good where sum |a||b| >= 1.003 2^-6
-// 2^(ea + eb): everywhere for rows of elements of like size (there it is about K / 16 and more), not where
-// the large elements of one row meet zeros or small elements of the other.
 // Lanes that share one of `elements` sums of `terms` terms, for `threads` threads: a power of two, so that few
 // elements keep the threads busy (and neighbouring lanes read neighbouring terms).
 __device__ __forceinline__ int lanes_per_sum(int elements, int threads, int64_t terms, int least = 1) {
@@ -181,6 +176,11 @@ __device__ __forceinline__ double sum_lanes(double x, int n) {
     return x;
 }
 
+// Where a sum needs FP64 arithmetic.  What the digits leave out of K products, 2^-63 2^e of an element and
+// the pairs with i + j >= 8 (7 2^14 256^-1 + .. units of 2^-68), is at most K 1.003 2^-59 2^(ea + eb); an FP64
+// sum has the bound K 2^-53 sum |a||b|.  So the digits are as good where sum |a||b| >= 1.003 2^-6
+// 2^(ea + eb): everywhere for rows of elements of like size (there it is about K / 16 and more), not where
+// the large elements of one row meet zeros or small elements of the other.
 constexpr float LOW_SUM = 1.01f / 64.0f;
 __device__ __forceinline__ bool low_sum(float magnitudes) { return magnitudes > 0.0f && magnitudes < LOW_SUM; }
 

@@ -16,8 +16,8 @@ from .sliced import SlicedGemm
 FP64_TILE = 64
 # FP64 launches on the tensor cores (sliced.py).  The CUDA-core kernel takes about 1.3 us per K
 # element of a tile's chain and 2 DFMA/clk/SM in all; a sliced launch takes about 32 us (digits and one
-# tile of up to 128 K), then 27 TFLOP/s: measured alone at M = 128, N = 64: K = 32 33 against 47 us,
-# K = 128 38 against 160 us; at 3600 x 784 x 784 249 against 4 650 us.
+# tile of up to 128 K), then 25 TFLOP/s: measured alone at M = 128, N = 64: K = 24 33 against 43 us,
+# K = 128 39 against 158 us; at 3600 x 784 x 784 258 against 4 635 us.
 SLICED_MIN_CHAIN = 24            # longest K chain of a launch from which it is worth the fixed time
 SLICED_MIN_PRODUCTS = 1 << 24    # or all products of a launch (64 x 64 tiles): 28 us of the FP64 pipe
 SLICED_MIN_K = 8                 # shorter tasks cost the epilogues and stores either way

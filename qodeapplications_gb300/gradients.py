@@ -25,7 +25,11 @@ from .gemm import GroupedGemm, SplitRegistry, TCGroupedGemm, Transposed
 from .hamiltonian import _Arena, _splitk
 
 
-ADJ_UNIT_MAX = 16     # blocks with at most this many states per side use the lane-per-coupling adjoint
+# FP32 blocks with at most this many states per side use the lane-per-coupling adjoint, not the pieces on the
+# tensor cores (reverse passes with either, us: 9 orbitals, 4 states 570 / 675, 10 states 756 / 797, 16 states
+# 1013 / 928; 14 orbitals, 8 states 2460 / 3007, 10 states 4226 / 4194, 16 states 5567 / 3843: a line at 10 would be as
+# good up to there and better above).
+ADJ_UNIT_MAX = 16
 # Spin orbitals of the system from which V_(1) Gbar_(1)^T runs on the tensor cores in FP64 (whole
 # iterations of 4 states without / with: 48 5.68 / 5.68 ms, 52 8.33 / 8.04, 56 11.35 / 11.07).
 ORBITAL_SLICED_MIN = 50
